@@ -67,6 +67,7 @@
 #include "jc_check.cuh"
 #include "jc_common.h"
 #include "jc_engine.h"
+#include "jc_exact.cuh"
 #include "jc_params.h"
 #include "jc_sort.cuh"
 #include "jc_pool.h"
@@ -1247,35 +1248,110 @@ k_speed_graphs(Forest F, float jitter_tolerance, const DevState* st) {
 }
 
 // ------------------------------------------------------- brute force --
-__global__ void __launch_bounds__(256)
+// All pairs, each body's terms added in ascending j as the shader does
+// (force_atlas2.wgsl:69-165). A body's sum is a serial chain of n additions,
+// but the terms do not depend on it: eight warps compute the terms of I bodies
+// against BRUTE_J others into shared memory while further warps, one lane per
+// (body, axis), add the chunk before in order. The self term and the entries
+// past n are -0.0f, which leaves any sum as it is (x + -0 = x, signs of zero
+// included), so the sums are the roundings of the one-thread loop. Bound by
+// instruction issue from about n = 5,000 on (52-66 % of issue slots, FP32 pipe
+// 43 %), below that by the chain of additions. A lane per body doing both ran
+// n IEEE divisions one after another on n / 256 blocks. B200, us a pass, before
+// and after: n = 400: 84 -> 7.6; 2,500: 497 -> 23; 10,000: 2,029 -> 186;
+// 50,000: 10,790 -> 3,490; 200,000: 70,800 -> 53,100.
+constexpr int BRUTE_J = 256;
+constexpr int BRUTE_ROW = BRUTE_J + 4;  // rows 4 banks apart: 16-byte reads of 8 rows touch every bank once
+constexpr int brute_threads(int I) { return BRUTE_J + (3 * I + 31) / 32 * 32; }
+constexpr int brute_smem(int I) { return 2 * 3 * I * BRUTE_ROW * (int)sizeof(float); }
+
+// The terms of one body j against the block's I bodies. With IN_RANGE the
+// quotients come from div_in_range: independent of each other with no call
+// between them, so the I chains overlap (with __fdiv_rn the pass took 39.6 us
+// at n = 2,500); `ok` comes back false when a squared distance was too large
+// for it, and the caller repeats the chunk with the general division.
+template <int I, bool IN_RANGE, bool SELECT>
+__device__ __forceinline__ bool brute_terms(const float4* body, const float4 cur, float mcur, uint32_t i0, uint32_t j,
+                                            uint32_t n, bool ok, float* out) {
+#pragma unroll
+  for (int b = 0; b < I; ++b) {
+    const float4 p = body[b];
+    const float dx = __fsub_rn(p.x, cur.x), dy = __fsub_rn(p.y, cur.y), dz = __fsub_rn(p.z, cur.z);
+    const float r2 = fmaxf(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)), 1.0e-4f);
+    const float num = __fmul_rn(p.w, mcur);
+    if (IN_RANGE) ok = ok && r2 <= dev::DIV_HI;
+    const float k = IN_RANGE ? dev::div_in_range(num, r2) : __fdiv_rn(num, r2);
+    const bool use = !SELECT || (j < n && j != i0 + (uint32_t)b);
+    out[b * BRUTE_ROW] = use ? __fmul_rn(dx, k) : -0.0f;
+    out[(I + b) * BRUTE_ROW] = use ? __fmul_rn(dy, k) : -0.0f;
+    out[(2 * I + b) * BRUTE_ROW] = use ? __fmul_rn(dz, k) : -0.0f;
+  }
+  return ok;
+}
+
+template <int I>
+__global__ void __launch_bounds__(brute_threads(I))
 k_brute(const float4* __restrict__ pos, const float* __restrict__ degf, uint32_t n, KParams P,
         float4* __restrict__ frep) {
-  __shared__ float4 tile[256];
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  float4 p = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float srd = i < n ? __fmul_rn(P.scaling_ratio, degf[i]) : 0.0f;
-  float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-  for (uint32_t base = 0; base < n; base += 256) {
-    uint32_t j = base + threadIdx.x;
-    if (j < n) {
-      float4 q = pos[j];
-      tile[threadIdx.x] = make_float4(q.x, q.y, q.z, degf[j]);
-    }
-    __syncthreads();
-    uint32_t lim = min(256u, n - base);
-    for (uint32_t t = 0; t < lim; ++t) {
-      if (base + t == i) continue;
-      float4 q = tile[t];
-      float dx = __fsub_rn(p.x, q.x), dy = __fsub_rn(p.y, q.y), dz = __fsub_rn(p.z, q.z);
-      float r2 = fmaxf(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)), 1.0e-4f);
-      float k = __fdiv_rn(__fmul_rn(srd, q.w), r2);
-      fx = __fadd_rn(fx, __fmul_rn(dx, k));
-      fy = __fadd_rn(fy, __fmul_rn(dy, k));
-      fz = __fadd_rn(fz, __fmul_rn(dz, k));
+  extern __shared__ float4 brute_sm[];  // float4: 16-byte aligned rows
+  float* term = reinterpret_cast<float*>(brute_sm);  // [2][3][I][BRUTE_ROW]
+  __shared__ float4 body[I];
+  __shared__ float sums[3][I];
+  const uint32_t i0 = blockIdx.x * I;
+  const uint32_t t = threadIdx.x;
+  if (t < I) {
+    const uint32_t i = i0 + t;
+    const float4 p = i < n ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    body[t] = make_float4(p.x, p.y, p.z, i < n ? __fmul_rn(P.scaling_ratio, degf[i]) : 1.0f);
+  }
+  __syncthreads();
+  // numerators srd * m of [1e-18, 1e18] suit div_in_range
+  bool srd_ok = true;
+#pragma unroll
+  for (int b = 0; b < I; ++b) srd_ok = srd_ok && body[b].w >= 1e-9f && body[b].w <= 1e9f;
+  const bool computes = t < BRUTE_J;
+  const uint32_t s = t - BRUTE_J;           // summing lane: body s % I, axis s / I
+  const bool adds = !computes && s < 3 * I;
+  float sum = 0.0f;
+  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+  float mq = 0.0f;
+  if (computes && t < n) {
+    q = pos[t];
+    mq = degf[t];
+  }
+  const uint32_t chunks = (n + BRUTE_J - 1) / BRUTE_J;
+  for (uint32_t c = 0; c <= chunks; ++c) {
+    if (computes) {
+      if (c < chunks) {
+        const uint32_t j = c * BRUTE_J + t;
+        const float4 cur = q;
+        const float mcur = mq;
+        if (j + BRUTE_J < n) {
+          q = pos[j + BRUTE_J];
+          mq = degf[j + BRUTE_J];
+        }
+        float* out = term + (size_t)(c & 1u) * 3 * I * BRUTE_ROW + t;
+        // chunks without a self term or an entry past n need no selects
+        const bool plain = (c + 1) * BRUTE_J <= n && (i0 + I <= c * BRUTE_J || i0 >= (c + 1) * BRUTE_J);
+        bool ok = srd_ok && mcur >= 1e-9f && mcur <= 1e9f;
+        if (plain) ok = brute_terms<I, true, false>(body, cur, mcur, i0, j, n, ok, out);
+        else ok = brute_terms<I, true, true>(body, cur, mcur, i0, j, n, ok, out);
+        if (!ok) brute_terms<I, false, true>(body, cur, mcur, i0, j, n, true, out);
+      }
+    } else if (adds && c > 0) {
+      const float4* in =
+          reinterpret_cast<const float4*>(term + (size_t)((c - 1) & 1u) * 3 * I * BRUTE_ROW + s * BRUTE_ROW);
+#pragma unroll 8
+      for (int k = 0; k < BRUTE_J / 4; ++k) {
+        const float4 v = in[k];
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
+      }
     }
     __syncthreads();
   }
-  if (i < n) frep[i] = make_float4(fx, fy, fz, 0.0f);
+  if (adds) (&sums[0][0])[s] = sum;
+  __syncthreads();
+  if (t < I && i0 + t < n) frep[i0 + t] = make_float4(sums[0][t], sums[1][t], sums[2][t], 0.0f);
 }
 
 // ----------------------------------------------- attraction + speed --
@@ -2548,7 +2624,7 @@ class Fa2Engine : public Engine {
       L += 1;
     } else {
       record_phase(1);
-      k_brute<<<cdiv(n, 256), 256, 0, stream_>>>(pos_.p, degf_.p, n, P, frep_.p);
+      launch_brute(P);
       L += 1;
     }
     record_phase(2);
@@ -2567,6 +2643,22 @@ class Fa2Engine : public Engine {
     L += 2;
     JC_CUDA_CHECK(cudaGetLastError());
     return L;
+  }
+
+  template <int I>
+  void launch_brute_as(const KParams& P) {
+    if (brute_smem(I) > 48 * 1024)
+      JC_CUDA_CHECK(cudaFuncSetAttribute(k_brute<I>, cudaFuncAttributeMaxDynamicSharedMemorySize, brute_smem(I)));
+    k_brute<I><<<cdiv(n_, I), brute_threads(I), brute_smem(I), stream_>>>(pos_.p, degf_.p, n_, P, frep_.p);
+  }
+
+  // Bodies per block: the most (fewest loads of the others' positions) that
+  // still give every SM a block; with 16 throughout, a graph of 400 nodes
+  // would run on 25 of the 148 SMs.
+  void launch_brute(const KParams& P) {
+    if (n_ > 8u * 148u) launch_brute_as<16>(P);
+    else if (n_ > 4u * 148u) launch_brute_as<8>(P);
+    else launch_brute_as<4>(P);
   }
 
   // The staged-top walk: a single graph, walk group 1.
