@@ -40,6 +40,7 @@
 
 #include "jc_common.h"
 #include "jc_engine.h"
+#include "jc_exact.cuh"
 #include "jc_params.h"
 
 namespace jc {
@@ -58,70 +59,149 @@ __device__ __forceinline__ uint64_t smix(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-template <typename D>
-__device__ __forceinline__ float dist_value(D du) {
-  // sgd_stress_gpu.rs:203-207: unreachable or self -> 0.0 (skipped)
-  const D sent = (D)~(D)0;
-  return (du == sent || du == 0) ? 0.0f : (float)du;
+// Node i's term with the pivot at q, hop distance d and mu = min(1, eta / d^2):
+// the general operations (any f32 input).
+__device__ __forceinline__ void jacobi_term(float& px, float& py, float& pz, const float4 q, float d, float mu) {
+  const float ex = __fsub_rn(px, q.x), ey = __fsub_rn(py, q.y), ez = __fsub_rn(pz, q.z);
+  const float mag = fmaxf(len3(ex, ey, ez), 1e-6f);
+  const float r = __fdiv_rn(__fmul_rn(mu, __fsub_rn(mag, d)), mag);
+  px = __fsub_rn(px, __fmul_rn(r, ex));
+  py = __fsub_rn(py, __fmul_rn(r, ey));
+  pz = __fsub_rn(pz, __fmul_rn(r, ez));
 }
 
-// One Jacobi sweep (sgd_stress.wgsl:34-62). eta_idx points at the step's
-// sweep counter; eta comes from the host-computed schedule table.
+// The same term where root and quotient may come from jc_exact.cuh. Below
+// 1e-12 the squared distance's root is not exact, but it is under the 1e-6
+// clamp (or NaN, which fmaxf drops) as the exact one is.
+__device__ __forceinline__ void jacobi_term_in_range(float& px, float& py, float& pz, const float4 q, float d,
+                                                     float mu, bool use) {
+  const float ex = __fsub_rn(px, q.x), ey = __fsub_rn(py, q.y), ez = __fsub_rn(pz, q.z);
+  const float s = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
+  const float mag = fmaxf(dev::sqrt_in_range(s), 1e-6f);
+  const float r = dev::div_in_range(__fmul_rn(mu, __fsub_rn(mag, d)), mag);
+  if (use) {  // (the three subtractions alone are predicated: no branch in the chain)
+    px = __fsub_rn(px, __fmul_rn(r, ex));
+    py = __fsub_rn(py, __fmul_rn(r, ey));
+    pz = __fsub_rn(pz, __fmul_rn(r, ez));
+  }
+}
+
+// Where that holds: mu >= 2^-44 (eta >= JACOBI_ETA_LO, d < JACOBI_MU_MAX), since
+// |mag - d| is 0 or at least 2^-25 of max(mag, 1), so that neither the quotient
+// nor its remainders underflow; and every coordinate of the pivots and of the
+// node within JACOBI_POS_HI at the sweep's start. A term moves the node along
+// its line with the pivot to a distance between mag and d, so its coordinates
+// stay within JACOBI_POS_HI + d + rounding and squared distances under 2^60.
+constexpr float JACOBI_ETA_LO = 9.5367431640625e-7f;  // 2^-20
+constexpr uint32_t JACOBI_MU_MAX = 4096u;
+constexpr float JACOBI_POS_HI = 1.34217728e8f;        // 2^27
+__device__ __forceinline__ bool jacobi_pos_ok(const float4 p) {
+  return fabsf(p.x) <= JACOBI_POS_HI && fabsf(p.y) <= JACOBI_POS_HI && fabsf(p.z) <= JACOBI_POS_HI;
+}
+constexpr uint32_t JACOBI_PF = 8;
+
+// (unreachable, all ones, and the node itself, 0, are skipped)
+template <typename D>
+__device__ __forceinline__ bool jacobi_skipped(D dv) {
+  return (D)(dv - (D)1) >= (D)~(D)1;
+}
+
+// Pivot positions and the (mu, d) table into shared memory; whether the
+// in-range terms hold as far as these decide it.
+__device__ __forceinline__ bool jacobi_stage(float4* piv, float2* mu_tab, const float4* __restrict__ pin,
+                                             const uint32_t* __restrict__ pivots, uint32_t k, uint32_t mu_len,
+                                             float eta) {
+  bool ok = mu_len != 0u && eta >= JACOBI_ETA_LO;
+  for (uint32_t t = threadIdx.x; t < k; t += blockDim.x) {
+    const float4 q = pin[pivots[t]];
+    ok = ok && jacobi_pos_ok(q);
+    piv[t] = q;
+  }
+  for (uint32_t du = threadIdx.x; du < mu_len; du += blockDim.x) {
+    const float d = (float)du;
+    mu_tab[du] = make_float2(fminf(1.0f, __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(d, d)), eta)), d);
+  }
+  return __syncthreads_and(ok);
+}
+
+// One Jacobi sweep (sgd_stress.wgsl:34-62); eta comes from the host-computed
+// schedule table at the device's sweep counter. The position update is a
+// serial chain over the pivots, k links long; a sweep is bound by the
+// instructions of the chain where nodes fill the GPU and by its latency where
+// they do not, not by the n k 2 B of distances. So:
+// - mu = min(1, eta / d^2) depends only on the hop distance d and the sweep's
+//   eta and is tabulated beside d for d < mu_len (the same operations, once
+//   per block), which takes a division and a conversion out of a link;
+// - the root and the quotient come without range tests and calls, correctly
+//   rounded both (jc_exact.cuh): bit-identical to the general operations;
+// - the next JACOBI_PF distances are in flight during a group's links, and a
+//   skipped pivot only predicates the three subtractions, so a link holds no
+//   branch.
+// About 47 instructions a link, 71 % of issue slots used at 250,000 nodes.
+// B200, us a step with 200 pivots, before and after: 500 x 500 grid 135 -> 98;
+// random geometric graphs of 200,000 nodes 119 -> 84, of 70,000 55 -> 35; of
+// 30,011 with 100 pivots 29 -> 14. Two nodes per thread in packed f32
+// operations gave 95 (grid) but for the moves it needs, and was not kept.
 template <typename D>
 __global__ void __launch_bounds__(256)
 k_jacobi(const float4* __restrict__ pin, float4* __restrict__ pout, const uint32_t* __restrict__ pivots,
          const D* __restrict__ dist, uint32_t n, uint32_t k, const float* __restrict__ eta_table, uint32_t n_eta,
          const uint32_t* __restrict__ sweep_ctr, uint32_t mu_len) {
   extern __shared__ float4 piv[];
-  // mu = min(1, eta / d^2) depends only on the hop distance d and this sweep's
-  // eta: with mu_len > 0 it is tabulated for d < mu_len (the same operations
-  // as below, once per block), which takes one IEEE division per term out of
-  // the serial chain
-  float* mu_tab = reinterpret_cast<float*>(piv + k);
+  float2* mu_tab = reinterpret_cast<float2*>(piv + k);  // (mu, d)
   const uint32_t sw = *sweep_ctr;
   const float eta = eta_table[sw < n_eta ? sw : n_eta - 1];
-  for (uint32_t t = threadIdx.x; t < k; t += blockDim.x) {
-    float4 q = pin[pivots[t]];
-    piv[t] = make_float4(q.x, q.y, q.z, __uint_as_float(pivots[t]));
-  }
-  for (uint32_t du = threadIdx.x; du < mu_len; du += blockDim.x) {
-    const float d = (float)du;
-    mu_tab[du] = fminf(1.0f, __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(d, d)), eta));
-  }
-  __syncthreads();
+  const bool block_ok = jacobi_stage(piv, mu_tab, pin, pivots, k, mu_len, eta);
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float4 p4 = pin[i];
+  const float4 p4 = pin[i];
   float px = p4.x, py = p4.y, pz = p4.z;
-  // The position update is a serial chain over the pivots; the distances do
-  // not depend on it, so JACOBI_PF of them are loaded ahead (in flight
-  // together) instead of one exposed load per pivot. Same operations, same
-  // order.
-  constexpr uint32_t JACOBI_PF = 8;
-  for (uint32_t t0 = 0; t0 < k; t0 += JACOBI_PF) {
-    D dv[JACOBI_PF];
+  if (!block_ok || !jacobi_pos_ok(p4)) {
+    for (uint32_t t0 = 0; t0 < k; t0 += JACOBI_PF) {
+      D dv[JACOBI_PF];
 #pragma unroll
-    for (uint32_t u = 0; u < JACOBI_PF; ++u) dv[u] = t0 + u < k ? dist[(size_t)(t0 + u) * n + i] : (D)0;
+      for (uint32_t u = 0; u < JACOBI_PF; ++u) dv[u] = t0 + u < k ? dist[(size_t)(t0 + u) * n + i] : (D)0;
+#pragma unroll
+      for (uint32_t u = 0; u < JACOBI_PF; ++u) {
+        if (jacobi_skipped(dv[u])) continue;
+        const float d = (float)dv[u];
+        jacobi_term(px, py, pz, piv[t0 + u], d, fminf(1.0f, __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(d, d)), eta)));
+      }
+    }
+    pout[i] = make_float4(px, py, pz, 0.0f);
+    return;
+  }
+  const uint32_t top = mu_len - 1u;
+  const D* row = dist;  // the next group's first row
+  uint32_t t = 0;
+  D nx[JACOBI_PF];
+#pragma unroll
+  for (uint32_t u = 0; u < JACOBI_PF; ++u) nx[u] = u < k ? (row + (size_t)u * n)[i] : (D)0;
+  for (; t + JACOBI_PF <= k; t += JACOBI_PF) {
+    D dv[JACOBI_PF];
+    row += (size_t)JACOBI_PF * n;
 #pragma unroll
     for (uint32_t u = 0; u < JACOBI_PF; ++u) {
-      const uint32_t t = t0 + u;
-      if (t >= k) break;
-      const float4 q = piv[t];
-      if (__float_as_uint(q.w) == i) continue;
-      const float d = dist_value<D>(dv[u]);
-      if (d <= 0.0f) continue;
-      const float ex = __fsub_rn(px, q.x), ey = __fsub_rn(py, q.y), ez = __fsub_rn(pz, q.z);
-      const float mag = fmaxf(len3(ex, ey, ez), 1e-6f);
-      const float mu = (uint32_t)dv[u] < mu_len ? mu_tab[(uint32_t)dv[u]]
-                                                 : fminf(1.0f, __fmul_rn(__fdiv_rn(1.0f, __fmul_rn(d, d)), eta));
-      const float r = __fdiv_rn(__fmul_rn(mu, __fsub_rn(mag, d)), mag);
-      px = __fsub_rn(px, __fmul_rn(r, ex));
-      py = __fsub_rn(py, __fmul_rn(r, ey));
-      pz = __fsub_rn(pz, __fmul_rn(r, ez));
+      dv[u] = nx[u];
+      nx[u] = t + JACOBI_PF + u < k ? (row + (size_t)u * n)[i] : (D)0;
     }
+#pragma unroll
+    for (uint32_t u = 0; u < JACOBI_PF; ++u) {
+      const float2 md = mu_tab[min((uint32_t)dv[u], top)];
+      jacobi_term_in_range(px, py, pz, piv[t + u], md.y, md.x, !jacobi_skipped(dv[u]));
+    }
+  }
+#pragma unroll
+  for (uint32_t u = 0; u < JACOBI_PF; ++u) {
+    if (t + u >= k) break;
+    const float2 md = mu_tab[min((uint32_t)nx[u], top)];
+    jacobi_term_in_range(px, py, pz, piv[t + u], md.y, md.x, !jacobi_skipped(nx[u]));
   }
   pout[i] = make_float4(px, py, pz, 0.0f);
 }
+
+// Up to here 64-thread blocks, so that the nodes spread over every SM.
+constexpr uint32_t JACOBI_SMALL_N = 148u * 512u;
 
 // One batch of the per-pair scatter. Sample q = sweep * n + q0 + t.
 template <typename D>
@@ -183,6 +263,20 @@ k_pairs_apply(float4* __restrict__ pos, long long* __restrict__ acc, uint32_t* _
 }
 
 __global__ void k_add_counter(uint32_t* ctr, uint32_t by) { *ctr += by; }
+
+// The end of a step's Jacobi sweeps: the last sweep's output to the engine's
+// positions and the read-back array, and the sweep counter (one launch).
+__global__ void __launch_bounds__(256)
+k_jacobi_end(const float4* v, uint32_t n, float4* pos, float* __restrict__ xyz, uint32_t* ctr, uint32_t sweeps) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *ctr += sweeps;
+  if (i >= n) return;
+  const float4 p = v[i];
+  if (v != pos) pos[i] = p;
+  xyz[3 * (size_t)i] = p.x;
+  xyz[3 * (size_t)i + 1] = p.y;
+  xyz[3 * (size_t)i + 2] = p.z;
+}
 
 __global__ void k_pack(const float4* __restrict__ v, uint32_t n, float* __restrict__ xyz) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -716,26 +810,27 @@ class SgdEngine : public Engine {
     int L = 0;
     if (jacobi_) {
       // sgd_stress_gpu.rs:377-428: one eta per step, `sweeps` ping-pong sweeps.
-      // the mu table covers distances up to the largest one when it fits in 16 KB
-      const uint32_t mu_len = max_dist_ + 1 <= 4096u ? max_dist_ + 1 : 0u;
-      const size_t smem = sizeof(float4) * k + sizeof(float) * mu_len;
-      if (smem > 200 * 1024) fail(JC_ERR_ARG, "too many pivots for the shared-memory pivot stage");
+      // the mu table covers distances up to the largest one when it fits in 32 KB
+      const uint32_t mu_len = max_dist_ + 1 <= JACOBI_MU_MAX ? max_dist_ + 1 : 0u;
+      // (rounded to whole 16 bytes; the 200 KB below leave room for the table)
+      const size_t smem = sizeof(float4) * k + sizeof(float2) * mu_len;
+      if (sizeof(float4) * k + sizeof(float) * mu_len > 200 * 1024)
+        fail(JC_ERR_ARG, "too many pivots for the shared-memory pivot stage");
       if (smem > 48 * 1024)
         JC_CUDA_CHECK(cudaFuncSetAttribute(k_jacobi<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       float4* in = pos_a_.p;
       float4* out = pos_b_.p;
+      const uint32_t threads = n <= JACOBI_SMALL_N ? 64u : 256u;
       for (uint32_t s = 0; s < sweeps; ++s) {
-        k_jacobi<D><<<cdiv(n, 256), 256, smem, stream_>>>(in, out, piv_.p, dist, n, k, eta_.p, n_eta_, ctr_.p,
-                                                           mu_len);
+        k_jacobi<D><<<cdiv(n, threads), threads, smem, stream_>>>(in, out, piv_.p, dist, n, k, eta_.p, n_eta_, ctr_.p,
+                                                                  mu_len);
         std::swap(in, out);
         ++L;
       }
-      if (in != pos_a_.p) {
-        JC_CUDA_CHECK(cudaMemcpyAsync(pos_a_.p, in, sizeof(float4) * n, cudaMemcpyDeviceToDevice, stream_));
-        ++L;
-      }
-      k_add_counter<<<1, 1, 0, stream_>>>(ctr_.p, sweeps);
+      k_jacobi_end<<<cdiv(n, 256), 256, 0, stream_>>>(in, n, pos_a_.p, xyz_.p, ctr_.p, sweeps);
       ++L;
+      JC_CUDA_CHECK(cudaGetLastError());
+      return L;
     } else {
       // sgd_stress.rs:287-315: per sweep, eta(sweep), n samples, sweep += 1.
       // Default: batches of max(256, n/64) samples (at most 64 per sweep).
