@@ -62,6 +62,7 @@
 #include "jc_common.h"
 #include "jc_engine.h"
 #include "jc_params.h"
+#include "jc_exact.cuh"
 #include "jc_tc_gemm.cuh"
 
 namespace jc {
@@ -78,7 +79,14 @@ constexpr int NPROJ = 8;
 constexpr uint32_t RECENTER = 8;  // smoothing steps between re-centrings
 constexpr uint32_t HUB_DEG = 1024;  // longer rows are summed in HUB_SEGS segments by a block
 constexpr int HUB_SEGS = 8;
-constexpr uint32_t ITEM_NODES = 4096;  // nodes per reduction item
+// Rows longer than this (up to HUB_DEG) are listed and taken by whole warps in
+// the first blocks of a pass: one thread or warp alone on a row of hundreds of
+// entries outlasted the rest of the pass.
+constexpr uint32_t LONG_DEG = 32;
+// Nodes per reduction item (one warp). At 4,096 a set of 64 graphs had about
+// 100 warps to sum with: k_proj_center_sums 80 us over 227,000 nodes, now 10 (and 11 for
+// the pair in one launch).
+constexpr uint32_t ITEM_NODES = 256;
 constexpr int HEAD_W = HID * 4 + 4;    // head weight (128 x 4) + bias (4) gradient row
 constexpr uint32_t NO_PIVOT = 0xFFFFFFFFu;
 constexpr uint16_t NO_DIST = 0xFFFFu;
@@ -182,12 +190,22 @@ struct GView {
   const uint32_t* go;   // graph -> first node (G + 1 entries)
   uint32_t n0, nb;      // nodes [n0, n0 + nb)
   uint32_t g0;          // first graph
+  const uint32_t* longs;  // its rows of LONG_DEG < deg <= HUB_DEG (global node ids)
+  uint32_t n_long;
 };
 
 // ========================================================== features ==
 // One warp per node. Lane w walks WALK_LEN steps from i; a ballot counts the
 // walks that are back at i after each step. Isolated nodes stay put.
-__global__ void __launch_bounds__(256) k_features(GView v, uint64_t seed, bf16* __restrict__ X,
+// The walks gather at random nodes and are bound by L1 requests: a node's row
+// start and length come in one 8-byte load (rows) instead of two.
+__global__ void k_pack_rows(const uint32_t* __restrict__ off, const uint32_t* __restrict__ deg, uint32_t n,
+                            uint2* __restrict__ rows) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) rows[i] = make_uint2(off[i], deg[i]);
+}
+
+__global__ void __launch_bounds__(256) k_features(GView v, const uint2* __restrict__ rows, uint64_t seed, bf16* __restrict__ X,
                                                   float* __restrict__ P) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= v.nb) return;
@@ -195,8 +213,8 @@ __global__ void __launch_bounds__(256) k_features(GView v, uint64_t seed, bf16* 
   bf16* x = X + (size_t)i * FEAT;
   uint32_t cur = i;
   for (int t = 1; t <= WALK_LEN; ++t) {
-    const uint32_t d = v.deg[cur];
-    if (d) cur = v.nbr[v.off[cur] + pick(hash4(seed ^ SALT_WALK, i, lane, (uint64_t)t), d)];
+    const uint2 r = rows[cur];
+    if (r.y) cur = v.nbr[r.x + pick(hash4(seed ^ SALT_WALK, i, lane, (uint64_t)t), r.y)];
     const uint32_t back = __popc(__ballot_sync(0xffffffffu, cur == i));
     if (lane == 0) x[t] = __float2bfloat16_rn((float)back * (1.0f / WALKS));
   }
@@ -234,13 +252,67 @@ __device__ __forceinline__ float filter_out(float px, float x, float xp, float c
 // latency-bound, so more resident warps keep more rows in flight (128 filter
 // steps over 13.4 M nodes 131.8 -> 127.8 ms, with the node's own row read
 // after the sum).
+//
+// The first blocks take the long rows, a warp each: lane (q, c) holds column c
+// of neighbours q, q + 4, ... of a chunk of 16, the next chunk's rows and the
+// ids after it in flight, and every lane of a column adds the chunk in CSR
+// order from shuffles (the same sums as one thread's; lanes past the row add
+// +0 to a sum that is never -0). One thread alone on a row of hundreds of
+// entries outlasted the rest of the step: 227,000 nodes 78 -> 18 us, 3.3 M
+// nodes 248 -> 142.
+template <int MODE>
+__device__ __forceinline__ void smooth_long(const GView& v, uint32_t i, const float* __restrict__ pin,
+                                            float* __restrict__ pout, const float* __restrict__ pprev, float c1) {
+  constexpr int K = 4;  // chunk: 4 K neighbours
+  const uint32_t lane = threadIdx.x & 31, q = lane >> 3, c = lane & 7, d = v.deg[i];
+  const uint32_t* row = v.nbr + v.off[i];
+  uint32_t id[K];
+  float val[K];
+  auto ids = [&](uint32_t base) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) id[k] = base + 4 * k + q < d ? __ldg(row + base + 4 * k + q) : i;
+  };
+  auto vals = [&](uint32_t base) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) val[k] = base + 4 * k + q < d ? __ldg(pin + 8 * (size_t)id[k] + c) : 0.0f;
+  };
+  ids(0);
+  vals(0);
+  ids(4 * K);
+  float a = 0.0f;
+  for (uint32_t base = 0; base < d; base += 4 * K) {
+    float cur[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) cur[k] = val[k];
+    vals(base + 4 * K);
+    ids(base + 8 * K);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a = __fadd_rn(a, __shfl_sync(0xffffffffu, cur[k], (int)c + 8 * u));
+  }
+  if (q == 0) {
+    const float x = pin[8 * (size_t)i + c];
+    const float xp = MODE == 2 ? pprev[8 * (size_t)i + c] : 0.0f;
+    pout[8 * (size_t)i + c] =
+        filter_out<MODE>(__fmul_rn(__fadd_rn(x, __fdiv_rn(a, (float)d)), 0.5f), x, xp, c1);
+  }
+}
+
+inline uint32_t long_blocks(uint32_t n_long) { return cdiv(n_long, 8); }  // a warp per long row
+
 template <int MODE>
 __global__ void __launch_bounds__(256, 6) k_smooth(GView v, const float* __restrict__ pin, float* __restrict__ pout,
-                                                const float* __restrict__ pprev, float c1) {
-  const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+                                                const float* __restrict__ pprev, float c1, uint32_t lb) {
+  if (blockIdx.x < lb) {
+    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k < v.n_long) smooth_long<MODE>(v, v.longs[k], pin, pout, pprev, c1);
+    return;
+  }
+  const uint32_t w = (blockIdx.x - lb) * blockDim.x + threadIdx.x;
   if (w >= v.nb) return;
   const uint32_t i = v.n0 + w, d = v.deg[i];
-  if (d > HUB_DEG) return;
+  if (d > LONG_DEG) return;
   const float4* src = reinterpret_cast<const float4*>(pin);
   float4* dst = reinterpret_cast<float4*>(pout);
   // the node's own row and the previous iterate are read after the neighbour
@@ -358,15 +430,20 @@ __global__ void __launch_bounds__(256) k_smooth_hub(GView v, const uint32_t* __r
 // leaks into it while every other mode decays), and each column is rescaled
 // to unit mean square at the same time so the decaying modes never underflow.
 constexpr int CEN = 2 * NPROJ + 1;
-__global__ void __launch_bounds__(256) k_proj_center_sums(const float* __restrict__ P, const uint32_t* __restrict__ deg,
+// blockIdx.y picks the array (x, or the Chebyshev pair's x_prev).
+__global__ void __launch_bounds__(256) k_proj_center_sums(const float* __restrict__ P0, const float* __restrict__ P1,
+                                                          const uint32_t* __restrict__ deg,
                                                           const int4* __restrict__ items, uint32_t n_items,
-                                                          double* __restrict__ part) {
+                                                          double* __restrict__ part0, double* __restrict__ part1) {
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= n_items) return;
+  const float* __restrict__ P = blockIdx.y ? P1 : P0;
+  double* __restrict__ part = blockIdx.y ? part1 : part0;
   const int4 it = items[w];
   double acc[CEN];
 #pragma unroll
   for (int k = 0; k < CEN; ++k) acc[k] = 0.0;
+#pragma unroll 4
   for (uint32_t i = (uint32_t)it.y + lane; i < (uint32_t)it.z; i += 32) {
     const double d = (double)deg[i];
 #pragma unroll
@@ -385,38 +462,66 @@ __global__ void __launch_bounds__(256) k_proj_center_sums(const float* __restric
   }
 }
 
-// x <- (x - m) * sc with m the degree-weighted mean (graphs with edges) and
-// sc = 1 / sqrt(mean of x^2) (columns that are not all zero).
-__global__ void k_proj_center(GView v, const double* __restrict__ gsum, float* __restrict__ P) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t w = t >> 3, c = t & 7;
-  if (w >= v.nb) return;
-  const uint32_t i = v.n0 + w, g = v.gid[i];
-  const double* s = gsum + (size_t)(g - v.g0) * CEN;
-  const double ms = s[NPROJ + 1 + c] / (double)(v.go[g + 1] - v.go[g]);
-  const float m = s[NPROJ] > 0.0 ? (float)(s[c] / s[NPROJ]) : 0.0f;
-  const float sc = ms > 0.0 ? (float)(1.0 / sqrt(ms)) : 1.0f;
-  P[(size_t)i * NPROJ + c] = __fmul_rn(__fsub_rn(P[(size_t)i * NPROJ + c], m), sc);
+// Per graph and column: m, the degree-weighted mean (graphs with edges), sc =
+// 1 / sqrt(mean of x^2) (columns that are not all zero) and the pair's mean
+// m_prev, from the items' sums: one block per graph, warp w adds items w,
+// w + 8, ..., then the warps' sums in order (one shape on every run). Every
+// node recomputing them from the sums spent its pass on f64 divisions
+// (227,000 nodes: 15 us a pass and 21 for the pair, now 6 with 6 here).
+__global__ void __launch_bounds__(256) k_center_coef(const double* __restrict__ part, const double* __restrict__ part_prev,
+                                                     const uint32_t* __restrict__ item_off,
+                                                     const uint32_t* __restrict__ go,
+                                                     float4* __restrict__ coef) {
+  __shared__ double sm[8][2][32];
+  const uint32_t g = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t a = item_off[g], b = item_off[g + 1];
+  double s = 0.0, sp = 0.0;
+  if (lane < CEN)
+#pragma unroll 4
+    for (uint32_t it = a + w; it < b; it += 8) {
+      s += part[(size_t)it * CEN + lane];
+      if (part_prev) sp += part_prev[(size_t)it * CEN + lane];
+    }
+  sm[w][0][lane] = s;
+  sm[w][1][lane] = sp;
+  __syncthreads();
+  if (w != 0) return;
+#pragma unroll
+  for (int q = 1; q < 8; ++q) {
+    s += sm[q][0][lane];
+    sp += sm[q][1][lane];
+  }
+  const double sd = __shfl_sync(0xffffffffu, s, NPROJ), sdp = __shfl_sync(0xffffffffu, sp, NPROJ);
+  const double sq = __shfl_sync(0xffffffffu, s, (int)(NPROJ + 1 + lane) & 31);
+  if (lane >= NPROJ) return;
+  const double ms = sq / (double)(go[g + 1] - go[g]);
+  coef[(size_t)g * NPROJ + lane] = make_float4(sd > 0.0 ? (float)(s / sd) : 0.0f,
+                                               ms > 0.0 ? (float)(1.0 / sqrt(ms)) : 1.0f,
+                                               sdp > 0.0 ? (float)(sp / sdp) : 0.0f, 0.0f);
 }
 
-// The Chebyshev pair (x, x_prev): each loses its own degree-weighted mean and
-// both are scaled by x's factor, which keeps the three-term recurrence intact
-// (the constant vector is an eigenvector of the walk and the projection that
-// removes it commutes with the walk).
-__global__ void k_proj_center_pair(GView v, const double* __restrict__ gsum, const double* __restrict__ gsum_prev,
-                                   float* __restrict__ P, float* __restrict__ Pprev) {
+// x <- (x - m) * sc, and with Pprev the Chebyshev pair (x, x_prev): each loses
+// its own degree-weighted mean and both are scaled by x's factor, which keeps
+// the three-term recurrence intact (the constant vector is an eigenvector of
+// the walk and the projection that removes it commutes with the walk). Four
+// columns per thread.
+__global__ void __launch_bounds__(256) k_proj_center(GView v, const float4* __restrict__ coef,
+                                                     float* __restrict__ P, float* __restrict__ Pprev) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t w = t >> 3, c = t & 7;
+  const uint32_t w = t >> 1, h = t & 1;
   if (w >= v.nb) return;
-  const uint32_t i = v.n0 + w, g = v.gid[i];
-  const double* s = gsum + (size_t)(g - v.g0) * CEN;
-  const double* sp = gsum_prev + (size_t)(g - v.g0) * CEN;
-  const double ms = s[NPROJ + 1 + c] / (double)(v.go[g + 1] - v.go[g]);
-  const float m = s[NPROJ] > 0.0 ? (float)(s[c] / s[NPROJ]) : 0.0f;
-  const float mp = sp[NPROJ] > 0.0 ? (float)(sp[c] / sp[NPROJ]) : 0.0f;
-  const float sc = ms > 0.0 ? (float)(1.0 / sqrt(ms)) : 1.0f;
-  P[(size_t)i * NPROJ + c] = __fmul_rn(__fsub_rn(P[(size_t)i * NPROJ + c], m), sc);
-  Pprev[(size_t)i * NPROJ + c] = __fmul_rn(__fsub_rn(Pprev[(size_t)i * NPROJ + c], mp), sc);
+  const uint32_t i = v.n0 + w;
+  const float4* cg = coef + (size_t)(v.gid[i] - v.g0) * NPROJ + 4 * h;
+  const float4 c0 = cg[0], c1 = cg[1], c2 = cg[2], c3 = cg[3];
+  float4* x = reinterpret_cast<float4*>(P) + 2 * (size_t)i + h;
+  const float4 a = *x;
+  *x = make_float4(__fmul_rn(__fsub_rn(a.x, c0.x), c0.y), __fmul_rn(__fsub_rn(a.y, c1.x), c1.y),
+                   __fmul_rn(__fsub_rn(a.z, c2.x), c2.y), __fmul_rn(__fsub_rn(a.w, c3.x), c3.y));
+  if (!Pprev) return;
+  float4* y = reinterpret_cast<float4*>(Pprev) + 2 * (size_t)i + h;
+  const float4 p = *y;
+  *y = make_float4(__fmul_rn(__fsub_rn(p.x, c0.z), c0.y), __fmul_rn(__fsub_rn(p.y, c1.z), c1.y),
+                   __fmul_rn(__fsub_rn(p.z, c2.z), c2.y), __fmul_rn(__fsub_rn(p.w, c3.z), c3.y));
 }
 
 // Feature columns 17..24: the smoothed, centred and scaled projections in bf16.
@@ -430,8 +535,8 @@ __global__ void k_proj_write(GView v, const float* __restrict__ P, bf16* __restr
 
 // ========================================================= reductions ==
 // Item = (graph, first node, end node): one warp sums V per-node doubles
-// (rows local to n0) over the item's nodes; then one thread per graph adds
-// its items in order. Fixed order throughout.
+// (rows local to n0) over the item's nodes; then one thread per graph and
+// value adds its items in order. Fixed order throughout.
 template <int V>
 __global__ void __launch_bounds__(256) k_item_reduce(const double* __restrict__ vals, uint32_t n0,
                                                      const int4* __restrict__ items, uint32_t n_items,
@@ -442,6 +547,7 @@ __global__ void __launch_bounds__(256) k_item_reduce(const double* __restrict__ 
   double acc[V];
 #pragma unroll
   for (int c = 0; c < V; ++c) acc[c] = 0.0;
+#pragma unroll 4
   for (uint32_t i = (uint32_t)it.y + lane; i < (uint32_t)it.z; i += 32) {
 #pragma unroll
     for (int c = 0; c < V; ++c) acc[c] += vals[(size_t)(i - n0) * V + c];
@@ -457,14 +563,14 @@ __global__ void __launch_bounds__(256) k_item_reduce(const double* __restrict__ 
 template <int V>
 __global__ void k_graph_sum(const double* __restrict__ part, const uint32_t* __restrict__ item_off, uint32_t g0,
                             uint32_t ng, uint32_t i0, double* __restrict__ gsum) {
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t g = t / V, c = t % V;
   if (g >= ng) return;
   const uint32_t a = item_off[g0 + g] - i0, b = item_off[g0 + g + 1] - i0;
-  for (int c = 0; c < V; ++c) {
-    double s = 0.0;
-    for (uint32_t it = a; it < b; ++it) s += part[(size_t)it * V + c];
-    gsum[(size_t)g * V + c] = s;
-  }
+  double s = 0.0;
+#pragma unroll 8
+  for (uint32_t it = a; it < b; ++it) s += part[(size_t)it * V + c];
+  gsum[(size_t)g * V + c] = s;
 }
 
 // out[col] = sum over z of part[z][col] in f64, one warp per column: lane l
@@ -482,58 +588,145 @@ __global__ void k_reduce_parts(const double* __restrict__ part, uint32_t chunks,
 }
 inline uint32_t reduce_parts_blocks(uint32_t width) { return cdiv(width * 32u, 256u); }
 
-__global__ void k_reduce_splits(const float* __restrict__ part, uint32_t splits, uint32_t width,
-                                float* __restrict__ out) {
-  const uint32_t col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= width) return;
+// out[col] = sum over z of part[z][col] in f64: thread (q, col) of a block adds
+// z = q, q + 8, ... (coalesced over 32 columns), then the eight in order.
+__global__ void __launch_bounds__(256) k_reduce_splits(const float* __restrict__ part, uint32_t splits,
+                                                       uint32_t width, float* __restrict__ out) {
+  __shared__ double sm[8][32];
+  const uint32_t c = threadIdx.x & 31, q = threadIdx.x >> 5, col = blockIdx.x * 32 + c;
   double s = 0.0;
-  for (uint32_t z = 0; z < splits; ++z) s += (double)part[(size_t)z * width + col];
+  if (col < width)
+#pragma unroll 8
+    for (uint32_t z = q; z < splits; z += 8) s += (double)part[(size_t)z * width + col];
+  sm[q][c] = s;
+  __syncthreads();
+  if (q != 0 || col >= width) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) s += sm[k][c];
   out[col] = (float)s;
 }
 
 // ============================================================ forward ==
 // Mean of the neighbours' rows (bf16, D columns of src) into dst[:, D:2D];
-// copy_self also copies the node's own row into dst[:, 0:D]. D/4 lanes per
-// node, 4 columns each, f32 sums in CSR order. src and dst may be the same
-// buffer (the halves are disjoint). Rows are local to the batch.
+// copy_self also copies the node's own row into dst[:, 0:D]. D/8 lanes per
+// node, 8 columns (one 16-byte load) each, f32 sums in CSR order. src and dst
+// may be the same buffer (the halves are disjoint). Rows are local to the
+// batch.
+//
+// Bound by the round trips of a node (its row bounds, ids, rows), so a node's
+// lanes read its neighbour ids together and take them from shuffles with 8
+// rows in flight, and 32 D/8 nodes share a warp. Long rows: a warp each in the
+// first blocks, 32 / (D/8) neighbours per load, the next ids in flight. Rows
+// past the count are zeros, added to sums that are never -0. Bound by issue (67
+// % of slots). Five blocks per SM cost a few spills and still win on large
+// sets. 128 columns, before (a warp per node, four rows in flight) and after:
+// 227,000 nodes 136 -> 121 us, 3.3 M nodes 1,468 -> 1,282; 32 columns 73 -> 35.
+// Eight f32 sums in four register pairs, added two at a time (each half
+// rounded as the scalar addition is).
+struct Sum8 {
+  unsigned long long p[4] = {0ull, 0ull, 0ull, 0ull};  // +0
+  __device__ __forceinline__ void add(int k, float lo, float hi) {
+    unsigned long long x;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(lo), "f"(hi));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p[k]) : "l"(p[k]), "l"(x));
+  }
+  __device__ __forceinline__ void get(float* a) const {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) asm("mov.b64 {%0, %1}, %2;" : "=f"(a[2 * k]), "=f"(a[2 * k + 1]) : "l"(p[k]));
+  }
+};
+
+// a += the row's 8 bf16 columns.
+__device__ __forceinline__ void add_row8(uint4 r, Sum8& a) {
+  const uint32_t q[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+  for (int k = 0; k < 4; ++k) a.add(k, __uint_as_float(q[k] << 16), __uint_as_float(q[k] & 0xFFFF0000u));
+}
+
 template <int D>
-__global__ void __launch_bounds__(256) k_agg(GView v, const bf16* src, int src_ld, bf16* dst, int dst_ld,
-                                             int copy_self) {
-  constexpr int LPN = D / 4;
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t w = t / LPN, c = (t % LPN) * 4;
-  if (w >= v.nb) return;
-  const uint32_t i = v.n0 + w, d = v.deg[i];
-  if (copy_self)
-    *reinterpret_cast<uint2*>(dst + (size_t)w * dst_ld + c) =
-        *reinterpret_cast<const uint2*>(src + (size_t)w * src_ld + c);
-  if (d > HUB_DEG) return;
-  const uint32_t* row = v.nbr + v.off[i];
-  float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  uint32_t e = 0;
-  for (; e + 4 <= d; e += 4) {
-    uint2 q[4];
+__global__ void __launch_bounds__(256, 5) k_agg(GView v, const bf16* src, int src_ld, bf16* dst, int dst_ld,
+                                             int copy_self, uint32_t lb) {
+  constexpr int LPN = D / 8, NPL = 32 / LPN, U = 8;
+  const uint32_t lane = threadIdx.x & 31, sub = lane % LPN, c = sub * 8;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  Sum8 a;
+  uint32_t w, d;
+  if (blockIdx.x < lb) {
+    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k >= v.n_long) return;
+    const uint32_t i = v.longs[k], q = lane / LPN;
+    d = v.deg[i];
+    w = i - v.n0;
+    const uint32_t* row = v.nbr + v.off[i];
+    uint32_t nx = lane < d ? row[lane] : i;
+    for (uint32_t base = 0; base < d; base += 32) {
+      const uint32_t id = nx - v.n0, cnt = min(32u, d - base);
+      nx = base + 32 + lane < d ? row[base + 32 + lane] : i;
+      for (uint32_t t = 0; t < cnt; t += U * NPL) {
+        uint4 r[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      q[u] = *reinterpret_cast<const uint2*>(src + (size_t)(row[e + u] - v.n0) * src_ld + c);
+        for (int u = 0; u < U; ++u) {
+          const uint32_t e = t + u * NPL + q, j = __shfl_sync(0xffffffffu, id, (int)(e & 31u));
+          r[u] = e < cnt ? *reinterpret_cast<const uint4*>(src + (size_t)j * src_ld + c) : zero;
+        }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      float f[4];
-      unpack4(q[u], f);
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) a[k] = __fadd_rn(a[k], f[k]);
+          for (int p = 0; p < NPL; ++p) {
+            if (t + u * NPL >= cnt) break;  // (the warp's: no shuffles for whole loads past the row)
+            const int from = (int)sub + p * LPN;
+            add_row8(make_uint4(__shfl_sync(0xffffffffu, r[u].x, from), __shfl_sync(0xffffffffu, r[u].y, from),
+                                __shfl_sync(0xffffffffu, r[u].z, from), __shfl_sync(0xffffffffu, r[u].w, from)), a);
+          }
+      }
+    }
+    if (q != 0) return;
+  } else {
+    const uint32_t t0 = (blockIdx.x - lb) * blockDim.x + threadIdx.x;
+    w = t0 / LPN;
+    if (w >= v.nb) return;
+    const uint32_t i = v.n0 + w;
+    d = v.deg[i];
+    if (copy_self)
+      *reinterpret_cast<uint4*>(dst + (size_t)w * dst_ld + c) =
+          *reinterpret_cast<const uint4*>(src + (size_t)w * src_ld + c);
+    if (d > LONG_DEG) return;
+    const uint32_t* row = v.nbr + v.off[i];
+    const uint32_t mask = ((1u << LPN) - 1u) << (lane - sub);
+    constexpr uint32_t CH = LPN < U ? LPN : U;
+    for (uint32_t base = 0; base < d; base += CH) {
+      const uint32_t cnt = min(CH, d - base);
+      const uint32_t id = sub < cnt ? row[base + sub] - v.n0 : w;
+      uint4 r[CH];
+#pragma unroll
+      for (uint32_t u = 0; u < CH; ++u) {
+        const uint32_t j = __shfl_sync(mask, id, (int)u, LPN);
+        r[u] = u < cnt ? *reinterpret_cast<const uint4*>(src + (size_t)j * src_ld + c) : zero;
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < CH; ++u)
+        add_row8(r[u], a);
     }
   }
-  for (; e < d; ++e) {
-    float f[4];
-    unpack4(*reinterpret_cast<const uint2*>(src + (size_t)(row[e] - v.n0) * src_ld + c), f);
+  // the mean: quotients by one divisor, in range unless a sum is tiny or huge
+  float m[8];
+  a.get(m);
+  const float fd = (float)d;
+  bool ok = true;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) a[k] = __fadd_rn(a[k], f[k]);
+  for (int k = 0; k < 8; ++k) ok = ok && (m[k] == 0.0f || (fabsf(m[k]) >= dev::DIV_LO && fabsf(m[k]) <= dev::DIV_HI));
+  if (d == 0) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m[k] = 0.0f;
+  } else if (ok) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m[k] = dev::div_in_range(m[k], fd);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m[k] = __fdiv_rn(m[k], fd);
   }
-  float m[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) m[k] = d ? __fdiv_rn(a[k], (float)d) : 0.0f;
-  *reinterpret_cast<uint2*>(dst + (size_t)w * dst_ld + D + c) = pack4(m);
+  const uint2 lo = pack4(m), hi = pack4(m + 4);
+  *reinterpret_cast<uint4*>(dst + (size_t)w * dst_ld + D + c) = make_uint4(lo.x, lo.y, hi.x, hi.y);
 }
 
 // Hub rows (deg > HUB_DEG): one block, warp s sums segment s, segments added in order.
@@ -623,15 +816,25 @@ __device__ __forceinline__ bool pair_at(const PairCtx& p, uint32_t i, uint32_t d
 
 __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf(x * x + y * y + z * z); }
 
+// Lanes per node of the pair passes: a node has about 14 pairs (its row and 8
+// partners), so a whole warp per node left more than half of its lanes idle.
+constexpr uint32_t PAIR_LANES = 16;
+__device__ __forceinline__ double pair_sum(double x) {
+  const uint32_t mask = 0xFFFFu << (threadIdx.x & 16u);
+#pragma unroll
+  for (int o = PAIR_LANES / 2; o; o >>= 1) x += __shfl_xor_sync(mask, x, o);
+  return x;
+}
+
 // Per node: sum q, sum q^2 and the pair count (target distances < 1e-6 skipped).
 __global__ void __launch_bounds__(256) k_loss_stats(PairCtx p, double* __restrict__ vals) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_LANES, lane = threadIdx.x % PAIR_LANES;
   if (w >= p.v.nb) return;
   const uint32_t i = p.v.n0 + w, d = p.v.deg[i], rowb = p.v.off[i], g = p.v.gid[i];
   const uint32_t gb = p.v.go[g], ng = p.v.go[g + 1] - gb;
   const float4 ti = p.T[i], yi = p.Y[w];
   double s1 = 0.0, s2 = 0.0, c = 0.0;
-  for (uint32_t q = lane; q < d + p.partners; q += 32) {
+  for (uint32_t q = lane; q < d + p.partners; q += PAIR_LANES) {
     uint32_t j;
     if (!pair_at(p, i, d, rowb, q, gb, ng, &j)) continue;
     const float4 tj = p.T[j], yj = p.Y[j - p.v.n0];
@@ -643,9 +846,9 @@ __global__ void __launch_bounds__(256) k_loss_stats(PairCtx p, double* __restric
     s2 += qq * qq;
     c += 1.0;
   }
-  s1 = warp_sum(s1);
-  s2 = warp_sum(s2);
-  c = warp_sum(c);
+  s1 = pair_sum(s1);
+  s2 = pair_sum(s2);
+  c = pair_sum(c);
   if (lane == 0) {
     vals[(size_t)w * 3] = s1;
     vals[(size_t)w * 3 + 1] = s2;
@@ -689,14 +892,14 @@ __global__ void __launch_bounds__(256) k_loss_finish(const double* __restrict__ 
 // dL/dY_i = sum over i's pairs of coef_g (alpha q - 1) alpha / d * (Y_i - Y_j) / r.
 __global__ void __launch_bounds__(256) k_loss_grad(PairCtx p, const double* __restrict__ galpha,
                                                    const double* __restrict__ gcoef, float4* __restrict__ dY) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_LANES, lane = threadIdx.x % PAIR_LANES;
   if (w >= p.v.nb) return;
   const uint32_t i = p.v.n0 + w, d = p.v.deg[i], rowb = p.v.off[i], g = p.v.gid[i];
   const uint32_t gb = p.v.go[g], ng = p.v.go[g + 1] - gb;
   const double a = galpha[g - p.v.g0], cf = gcoef[g - p.v.g0];
   const float4 ti = p.T[i], yi = p.Y[w];
   double gx = 0.0, gy = 0.0, gz = 0.0;
-  for (uint32_t q = lane; q < d + p.partners; q += 32) {
+  for (uint32_t q = lane; q < d + p.partners; q += PAIR_LANES) {
     uint32_t j;
     if (!pair_at(p, i, d, rowb, q, gb, ng, &j)) continue;
     const float4 tj = p.T[j], yj = p.Y[j - p.v.n0];
@@ -711,9 +914,9 @@ __global__ void __launch_bounds__(256) k_loss_grad(PairCtx p, const double* __re
     gy += wgt * dy;
     gz += wgt * dz;
   }
-  gx = warp_sum(gx);
-  gy = warp_sum(gy);
-  gz = warp_sum(gz);
+  gx = pair_sum(gx);
+  gy = pair_sum(gy);
+  gz = pair_sum(gz);
   if (lane == 0) dY[w] = make_float4((float)gx, (float)gy, (float)gz, 0.0f);
 }
 
@@ -752,83 +955,190 @@ __global__ void __launch_bounds__(256) k_head_bwd(uint32_t nb, const bf16* __res
 }
 
 // Head gradient partials per chunk of rows: [k*4 + c] = sum H3[r][k] dY[r][c],
-// [512 + c] = sum dY[r][c].
-__global__ void __launch_bounds__(HID) k_head_wgrad(uint32_t nb, uint32_t chunk, const bf16* __restrict__ H3,
-                                                    const float4* __restrict__ dY, double* __restrict__ part) {
-  const uint32_t k = threadIdx.x;
+// [512 + c] = sum dY[r][c]. Warp w of a block takes rows w, w + 8, ... of the
+// chunk, lane l the hidden columns 4l..4l+3, four rows in flight; the warps'
+// f64 sums are added in warp order. (A thread per column with one 2-byte load
+// in flight took 130 us on 158,000 rows, this 42; k_colsum 29 -> 12.)
+constexpr int CHUNK_WARPS = 8;
+__global__ void __launch_bounds__(32 * CHUNK_WARPS) k_head_wgrad(uint32_t nb, uint32_t chunk,
+                                                                 const bf16* __restrict__ H3,
+                                                                 const float4* __restrict__ dY,
+                                                                 double* __restrict__ part) {
+  __shared__ double sm[CHUNK_WARPS][3][HID];
+  __shared__ double sb[CHUNK_WARPS][3];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t r0 = blockIdx.x * chunk, r1 = min(nb, r0 + chunk);
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, bsum = 0.0;
-  for (uint32_t r = r0; r < r1; ++r) {
-    const double h = bf2f(H3[(size_t)r * HID + k]);
-    const float4 g = dY[r];
-    a0 += h * g.x;
-    a1 += h * g.y;
-    a2 += h * g.z;
-    if (k < 4) bsum += k == 0 ? g.x : k == 1 ? g.y : k == 2 ? g.z : 0.0f;
+  double acc[3][4] = {}, bs[3] = {};
+  constexpr int U = 4;
+  for (uint32_t r = r0 + w; r < r1; r += U * CHUNK_WARPS) {
+    uint2 hq[U];
+    float4 g[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t rr = r + u * CHUNK_WARPS;
+      const bool in = rr < r1;
+      hq[u] = in ? *reinterpret_cast<const uint2*>(H3 + (size_t)rr * HID + 4 * lane) : make_uint2(0u, 0u);
+      g[u] = in ? dY[rr] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float h[4];
+      unpack4(hq[u], h);
+      const double gx = g[u].x, gy = g[u].y, gz = g[u].z;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const double hk = h[k];
+        acc[0][k] += hk * gx;
+        acc[1][k] += hk * gy;
+        acc[2][k] += hk * gz;
+      }
+      bs[0] += gx;
+      bs[1] += gy;
+      bs[2] += gz;
+    }
   }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) sm[w][c][4 * lane + k] = acc[c][k];
+    if (lane == 0) sb[w][c] = bs[c];
+  }
+  __syncthreads();
   double* o = part + (size_t)blockIdx.x * HEAD_W;
-  o[k * 4] = a0;
-  o[k * 4 + 1] = a1;
-  o[k * 4 + 2] = a2;
-  o[k * 4 + 3] = 0.0;
-  if (k < 4) o[HID * 4 + k] = bsum;
+  for (uint32_t t = threadIdx.x; t < HEAD_W; t += blockDim.x) {
+    const uint32_t k = t >> 2, c = t & 3;
+    double s = 0.0;
+    if (c < 3)
+#pragma unroll
+      for (int q = 0; q < CHUNK_WARPS; ++q) s += k < HID ? sm[q][c][k] : sb[q][c];
+    o[t] = s;
+  }
 }
 
-// Bias gradient partials: column sums of dZ (bf16, 128 wide) per chunk of rows.
-__global__ void __launch_bounds__(HID) k_colsum(uint32_t nb, uint32_t chunk, const bf16* __restrict__ dZ,
-                                                double* __restrict__ part) {
-  const uint32_t c = threadIdx.x;
+// Bias gradient partials: column sums of dZ (bf16, 128 wide) per chunk of rows,
+// by warps as above.
+__global__ void __launch_bounds__(32 * CHUNK_WARPS) k_colsum(uint32_t nb, uint32_t chunk,
+                                                             const bf16* __restrict__ dZ, double* __restrict__ part) {
+  __shared__ double sm[CHUNK_WARPS][HID];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t r0 = blockIdx.x * chunk, r1 = min(nb, r0 + chunk);
-  double a = 0.0;
-  for (uint32_t r = r0; r < r1; ++r) a += bf2f(dZ[(size_t)r * HID + c]);
-  part[(size_t)blockIdx.x * HID + c] = a;
+  double acc[4] = {};
+  constexpr int U = 8;
+  for (uint32_t r = r0 + w; r < r1; r += U * CHUNK_WARPS) {
+    uint2 q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t rr = r + u * CHUNK_WARPS;
+      q[u] = rr < r1 ? *reinterpret_cast<const uint2*>(dZ + (size_t)rr * HID + 4 * lane) : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[4];
+      unpack4(q[u], f);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[k] += (double)f[k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) sm[w][4 * lane + k] = acc[k];
+  __syncthreads();
+  if (threadIdx.x < HID) {
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < CHUNK_WARPS; ++q) s += sm[q][threadIdx.x];
+    part[(size_t)blockIdx.x * HID + threadIdx.x] = s;
+  }
 }
 
 // dZ_{l-1}[j] = bf16((dA[j][0:128] + sum_{i in N(j)} dA[i][128:256] * (1 / deg_i)) * (H_l[j] > 0)):
 // the transpose of the mean aggregation (the CSR is symmetric), CSR order.
 // dA is the bf16 output of the activation-gradient GEMM (8 bytes per lane
 // and neighbour gathered).
-__global__ void __launch_bounds__(256) k_agg_bwd(GView v, const bf16* __restrict__ dA, const bf16* __restrict__ A,
-                                                 bf16* __restrict__ dZ) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= v.nb) return;
-  const uint32_t i = v.n0 + w, d = v.deg[i];
-  if (d > HUB_DEG) return;
-  const uint32_t c = lane * 4;
-  const uint32_t* row = v.nbr + v.off[i];
-  float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  // 32 neighbours at a time: lane k reads the k-th id and its neighbour's
-  // 1/degree (one round trip for all 32), then the warp gathers the rows
-  // four at a time, added in CSR order.
-  for (uint32_t base = 0; base < d; base += 32) {
-    const uint32_t cnt = min(32u, d - base);
-    uint32_t jl = 0;
-    float il = 0.0f;
-    if (lane < cnt) {
-      jl = row[base + lane];
-      il = __frcp_rn((float)v.deg[jl]);
-    }
-    for (uint32_t t = 0; t < cnt; t += 4) {
-      float q[4][4], inv[4];
+// 16 lanes per node, 8 columns each; long rows first, a warp each, two
+// neighbours per load (see k_agg). 158,000 nodes: 141 -> 79 us.
+__device__ __forceinline__ void add_row8_scaled(uint4 r, float s, float* a) {
+  float f[8];
+  unpack4(make_uint2(r.x, r.y), f);
+  unpack4(make_uint2(r.z, r.w), f + 4);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const uint32_t j = __shfl_sync(0xFFFFFFFFu, jl, (int)(t + u) & 31);
-        inv[u] = __shfl_sync(0xFFFFFFFFu, il, (int)(t + u) & 31);
-        if (t + u < cnt) unpack4(*reinterpret_cast<const uint2*>(dA + (size_t)(j - v.n0) * 2 * HID + HID + c), q[u]);
+  for (int k = 0; k < 8; ++k) a[k] = __fadd_rn(a[k], __fmul_rn(f[k], s));
+}
+
+__global__ void __launch_bounds__(256, 4) k_agg_bwd(GView v, const bf16* __restrict__ dA, const bf16* __restrict__ A,
+                                                 bf16* __restrict__ dZ, uint32_t lb) {
+  constexpr int LPN = HID / 8, U = 8;
+  const uint32_t lane = threadIdx.x & 31, sub = lane % LPN, c = sub * 8;
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  float a[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+  auto at = [&](uint32_t j) { return *reinterpret_cast<const uint4*>(dA + (size_t)(j - v.n0) * 2 * HID + HID + c); };
+  uint32_t w;
+  if (blockIdx.x < lb) {
+    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k >= v.n_long) return;
+    const uint32_t i = v.longs[k], d = v.deg[i], q = lane / LPN;
+    w = i - v.n0;
+    const uint32_t* row = v.nbr + v.off[i];
+    uint32_t nx = lane < d ? row[lane] : i;
+    for (uint32_t base = 0; base < d; base += 32) {
+      const uint32_t cnt = min(32u, d - base), jl = nx;
+      const float il = lane < cnt ? __frcp_rn((float)v.deg[jl]) : 0.0f;
+      nx = base + 32 + lane < d ? row[base + 32 + lane] : i;
+      for (uint32_t t = 0; t < cnt; t += 2 * U) {
+        uint4 r[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const uint32_t e = t + 2 * u + q, j = __shfl_sync(0xffffffffu, jl, (int)(e & 31u));
+          r[u] = e < cnt ? at(j) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int p = 0; p < 2; ++p) {
+            const int from = (int)sub + p * LPN;
+            const float inv = __shfl_sync(0xffffffffu, il, (int)((t + 2 * u + p) & 31u));
+            const uint4 x = make_uint4(__shfl_sync(0xffffffffu, r[u].x, from), __shfl_sync(0xffffffffu, r[u].y, from),
+                                       __shfl_sync(0xffffffffu, r[u].z, from), __shfl_sync(0xffffffffu, r[u].w, from));
+            if (t + 2 * u + p < cnt) add_row8_scaled(x, inv, a);
+          }
+      }
+    }
+    if (q != 0) return;
+  } else {
+    const uint32_t t0 = (blockIdx.x - lb) * blockDim.x + threadIdx.x;
+    w = t0 / LPN;
+    if (w >= v.nb) return;
+    const uint32_t i = v.n0 + w, d = v.deg[i];
+    if (d > LONG_DEG) return;
+    const uint32_t* row = v.nbr + v.off[i];
+    const uint32_t mask = ((1u << LPN) - 1u) << (lane - sub);
+    for (uint32_t base = 0; base < d; base += U) {
+      const uint32_t cnt = min((uint32_t)U, d - base);
+      const uint32_t jl = sub < cnt ? row[base + sub] : i;
+      const float il = sub < cnt ? __frcp_rn((float)v.deg[jl]) : 0.0f;
+      uint4 r[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        const uint32_t j = __shfl_sync(mask, jl, (int)u, LPN);
+        r[u] = u < cnt ? at(j) : zero;
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (t + u < cnt)
-#pragma unroll
-          for (int k = 0; k < 4; ++k) a[k] = __fadd_rn(a[k], __fmul_rn(q[u][k], inv[u]));
+      for (uint32_t u = 0; u < U; ++u) {
+        const float inv = __shfl_sync(mask, il, (int)u, LPN);
+        add_row8_scaled(r[u], inv, a);  // (a branch per row around it: 79 -> 102 us)
+      }
     }
   }
-  float h[4], o[4], sv[4];
-  unpack4(*reinterpret_cast<const uint2*>(dA + (size_t)w * 2 * HID + c), sv);
-  unpack4(*reinterpret_cast<const uint2*>(A + (size_t)w * 2 * HID + c), h);
+  float h[8], o[8], sv[8];
+  const uint4 s4 = *reinterpret_cast<const uint4*>(dA + (size_t)w * 2 * HID + c);
+  const uint4 h4 = *reinterpret_cast<const uint4*>(A + (size_t)w * 2 * HID + c);
+  unpack4(make_uint2(s4.x, s4.y), sv);
+  unpack4(make_uint2(s4.z, s4.w), sv + 4);
+  unpack4(make_uint2(h4.x, h4.y), h);
+  unpack4(make_uint2(h4.z, h4.w), h + 4);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) o[k] = h[k] > 0.0f ? __fadd_rn(sv[k], a[k]) : 0.0f;
-  *reinterpret_cast<uint2*>(dZ + (size_t)w * HID + c) = pack4(o);
+  for (int k = 0; k < 8; ++k) o[k] = h[k] > 0.0f ? __fadd_rn(sv[k], a[k]) : 0.0f;
+  const uint2 lo = pack4(o), hi = pack4(o + 4);
+  *reinterpret_cast<uint4*>(dZ + (size_t)w * HID + c) = make_uint4(lo.x, lo.y, hi.x, hi.y);
 }
 
 __global__ void __launch_bounds__(256) k_agg_bwd_hub(GView v, const uint32_t* __restrict__ hubs,
@@ -919,21 +1229,23 @@ __global__ void k_transpose_w(const bf16* __restrict__ w, ParamLayout L, bf16* _
 }
 
 // ============================================================ hand-off ==
-// Per node (one warp): Y.xyz, sum over row entries j > i of |Y_i - Y_j|^2, deg, deg^2.
+// Per node (eight lanes): Y.xyz, sum over row entries j > i of |Y_i - Y_j|^2, deg, deg^2.
 __global__ void __launch_bounds__(256) k_scale_vals(GView v, const float4* __restrict__ Y, double* __restrict__ vals) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, lane = threadIdx.x & 7;
   if (w >= v.nb) return;
   const uint32_t i = v.n0 + w, d = v.deg[i], rowb = v.off[i];
   const float4 yi = Y[w];
   double a = 0.0;
-  for (uint32_t q = lane; q < d; q += 32) {
+  for (uint32_t q = lane; q < d; q += 8) {
     const uint32_t j = v.nbr[rowb + q];
     if (j <= i) continue;
     const float4 yj = Y[j - v.n0];
     const double dx = (double)yi.x - yj.x, dy = (double)yi.y - yj.y, dz = (double)yi.z - yj.z;
     a += dx * dx + dy * dy + dz * dz;
   }
-  a = warp_sum(a);
+  const uint32_t mask = 0xFFu << (threadIdx.x & 24u);
+#pragma unroll
+  for (int o = 4; o; o >>= 1) a += __shfl_xor_sync(mask, a, o);
   if (lane == 0) {
     double* o = vals + (size_t)w * 6;
     o[0] = yi.x;
@@ -1093,7 +1405,7 @@ struct Buf {
 // global CSR plus the per-graph and per-item bookkeeping the kernels use.
 struct HostSet {
   uint32_t n = 0, G = 0;
-  std::vector<uint32_t> go, off, nbr, deg, gid, item_off, hubs;
+  std::vector<uint32_t> go, off, nbr, deg, gid, item_off, hubs, longs;
   std::vector<int4> items;
 };
 
@@ -1167,18 +1479,21 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
       h.items.push_back(make_int4((int)g, (int)b, (int)std::min(h.go[g + 1], b + ITEM_NODES), 0));
   }
   h.item_off[G] = (uint32_t)h.items.size();
-  for (uint32_t v = 0; v < n; ++v)
+  for (uint32_t v = 0; v < n; ++v) {
     if (h.deg[v] > HUB_DEG) h.hubs.push_back(v);
+    else if (h.deg[v] > LONG_DEG) h.longs.push_back(v);
+  }
   return h;
 }
 
 struct Batch {
   uint32_t g0, g1, n0, nb, i0, i1, h0, h1;
+  uint32_t l0, l1;  // its part of the long rows
 };
 
 struct DevSet {
   HostSet h;
-  Buf<uint32_t> go, off, nbr, deg, gid, item_off, hubs;
+  Buf<uint32_t> go, off, nbr, deg, gid, item_off, hubs, longs;
   Buf<int4> items;
   void upload(HostSet&& hs, cudaStream_t s) {
     h = std::move(hs);
@@ -1189,6 +1504,7 @@ struct DevSet {
     gid.upload(h.gid.data(), h.gid.size(), s);
     item_off.upload(h.item_off.data(), h.item_off.size(), s);
     hubs.upload(h.hubs.data(), h.hubs.size(), s);
+    longs.upload(h.longs.data(), h.longs.size(), s);
     items.upload(h.items.data(), h.items.size(), s);
     JC_CUDA_CHECK(cudaStreamSynchronize(s));  // host vectors stay owned by h
   }
@@ -1202,10 +1518,12 @@ struct DevSet {
     b.i1 = h.item_off[g1];
     b.h0 = (uint32_t)(std::lower_bound(h.hubs.begin(), h.hubs.end(), b.n0) - h.hubs.begin());
     b.h1 = (uint32_t)(std::lower_bound(h.hubs.begin(), h.hubs.end(), b.n0 + b.nb) - h.hubs.begin());
+    b.l0 = (uint32_t)(std::lower_bound(h.longs.begin(), h.longs.end(), b.n0) - h.longs.begin());
+    b.l1 = (uint32_t)(std::lower_bound(h.longs.begin(), h.longs.end(), b.n0 + b.nb) - h.longs.begin());
     return b;
   }
   GView view(const Batch& b) const {
-    return GView{off.p, nbr.p, deg.p, gid.p, go.p, b.n0, b.nb, b.g0};
+    return GView{off.p, nbr.p, deg.p, gid.p, go.p, b.n0, b.nb, b.g0, longs.p + b.l0, b.l1 - b.l0};
   }
 };
 
@@ -1316,6 +1634,8 @@ inline uint32_t warps_grid(uint64_t warps) { return cdiv(warps * 32, 256); }
 // Reduction scratch shared by features, loss, hand-off and evaluation.
 struct Reduce {
   Buf<double> vals, part, gsum, gsum2;
+  Buf<uint2> rows;
+  Buf<float4> coef;
   void ensure(uint32_t nodes, uint32_t items, uint32_t graphs) {
     vals.alloc((size_t)nodes * 8);
     part.alloc((size_t)items * CEN);
@@ -1327,7 +1647,7 @@ struct Reduce {
   void run(const DevSet& s, const Batch& b, double* out, cudaStream_t st) {
     const uint32_t ni = b.i1 - b.i0, ng = b.g1 - b.g0;
     if (ni) k_item_reduce<V><<<warps_grid(ni), 256, 0, st>>>(vals.p, b.n0, s.items.p + b.i0, ni, part.p);
-    if (ng) k_graph_sum<V><<<cdiv(ng, 128), 128, 0, st>>>(part.p, s.item_off.p, b.g0, ng, b.i0, out);
+    if (ng) k_graph_sum<V><<<cdiv((uint64_t)ng * V, 128), 128, 0, st>>>(part.p, s.item_off.p, b.g0, ng, b.i0, out);
   }
 };
 
@@ -1353,33 +1673,31 @@ void compute_features(const DevSet& s, uint64_t seed, uint32_t smooth_steps, uin
   red.ensure(n, (uint32_t)s.h.items.size(), s.h.G);
   if (cheb_steps) red2.ensure(n, (uint32_t)s.h.items.size(), s.h.G);
   if (n == 0) return;
-  k_features<<<warps_grid(n), 256, 0, st>>>(v, seed, X.p, P.p);
+  red.rows.alloc(n);
+  k_pack_rows<<<cdiv(n, 256), 256, 0, st>>>(s.off.p, s.deg.p, n, red.rows.p);
+  k_features<<<warps_grid(n), 256, 0, st>>>(v, red.rows.p, seed, X.p, P.p);
   const uint32_t ni = (uint32_t)s.h.items.size(), G = s.h.G;
-  auto sums = [&](const float* x, Reduce& r) {
-    k_proj_center_sums<<<warps_grid(ni), 256, 0, st>>>(x, s.deg.p, s.items.p, ni, r.part.p);
-    k_graph_sum<CEN><<<cdiv(G, 128), 128, 0, st>>>(r.part.p, s.item_off.p, 0, G, 0, r.gsum.p);
+  red.coef.alloc((size_t)G * NPROJ);
+  // centre and rescale x; with `prev` the Chebyshev pair (x, prev)
+  auto center = [&](float* x, float* prev) {
+    k_proj_center_sums<<<dim3(warps_grid(ni), prev ? 2 : 1), 256, 0, st>>>(x, prev, s.deg.p, s.items.p, ni, red.part.p,
+                                                                          red2.part.p);
+    k_center_coef<<<G, 256, 0, st>>>(red.part.p, prev ? red2.part.p : nullptr, s.item_off.p, s.go.p, red.coef.p);
+    k_proj_center<<<cdiv((uint64_t)n * 2, 256), 256, 0, st>>>(v, red.coef.p, x, prev);
   };
-  auto center = [&](float* x) {
-    sums(x, red);
-    k_proj_center<<<cdiv((uint64_t)n * 8, 256), 256, 0, st>>>(v, red.gsum.p, x);
-  };
-  const uint32_t n_hubs = (uint32_t)s.h.hubs.size();
+  const uint32_t n_hubs = (uint32_t)s.h.hubs.size(), lb = long_blocks(v.n_long);
   float* a = P.p;
   float* b = P2.p;
-  center(a);
+  center(a, nullptr);
   if (cheb_steps) {
     // a = y_{k-1}, b = y_k, c = y_{k+1}
     float* c = P3.p;
     const float c1_first = 2.0f / cheb_b, c1 = 4.0f / cheb_b;
-    k_smooth<1><<<cdiv(n, 256), 256, 0, st>>>(v, a, b, nullptr, c1_first);
+    k_smooth<1><<<lb + cdiv(n, 256), 256, 0, st>>>(v, a, b, nullptr, c1_first, lb);
     if (n_hubs) k_smooth_hub<1><<<n_hubs, 256, 0, st>>>(v, s.hubs.p, a, b, nullptr, c1_first);
     for (uint32_t r = 1; r < cheb_steps; ++r) {
-      if (r % RECENTER == 0) {
-        sums(b, red);
-        sums(a, red2);
-        k_proj_center_pair<<<cdiv((uint64_t)n * 8, 256), 256, 0, st>>>(v, red.gsum.p, red2.gsum.p, b, a);
-      }
-      k_smooth<2><<<cdiv(n, 256), 256, 0, st>>>(v, b, c, a, c1);
+      if (r % RECENTER == 0) center(b, a);
+      k_smooth<2><<<lb + cdiv(n, 256), 256, 0, st>>>(v, b, c, a, c1, lb);
       if (n_hubs) k_smooth_hub<2><<<n_hubs, 256, 0, st>>>(v, s.hubs.p, b, c, a, c1);
       float* t = a;
       a = b;
@@ -1387,15 +1705,15 @@ void compute_features(const DevSet& s, uint64_t seed, uint32_t smooth_steps, uin
       c = t;
     }
     std::swap(a, b);  // the last y_k is the input of the plain phase
-    center(a);
+    center(a, nullptr);
   }
   for (uint32_t r = 0; r < smooth_steps; ++r) {
-    k_smooth<0><<<cdiv(n, 256), 256, 0, st>>>(v, a, b, nullptr, 1.0f);
+    k_smooth<0><<<lb + cdiv(n, 256), 256, 0, st>>>(v, a, b, nullptr, 1.0f, lb);
     if (n_hubs) k_smooth_hub<0><<<n_hubs, 256, 0, st>>>(v, s.hubs.p, a, b, nullptr, 1.0f);
     std::swap(a, b);
-    if (r % RECENTER == RECENTER - 1) center(a);
+    if (r % RECENTER == RECENTER - 1) center(a, nullptr);
   }
-  center(a);
+  center(a, nullptr);
   k_proj_write<<<cdiv((uint64_t)n * 8, 256), 256, 0, st>>>(v, a, X.p);
   JC_CUDA_CHECK(cudaGetLastError());
 }
@@ -1724,12 +2042,12 @@ class Net {
 
   void forward(const DevSet& s, const Batch& b, const bf16* X) {
     const GView v = s.view(b);
-    const uint32_t nb = b.nb, nh = b.h1 - b.h0;
+    const uint32_t nb = b.nb, nh = b.h1 - b.h0, lb = long_blocks(v.n_long);
     const uint32_t* hubs = s.hubs.p + b.h0;
     const bf16* Xb = X + (size_t)b.n0 * FEAT;
     const size_t n_w = (size_t)(L_.kin[0] + L_.kin[1] + L_.kin[2]) * HID;
     k_transpose_w<<<cdiv(n_w, 256), 256, 0, st_>>>(theta_bf_.p, L_, wt_.p);
-    k_agg<FEAT><<<cdiv((uint64_t)nb * (FEAT / 4), 256), 256, 0, st_>>>(v, Xb, FEAT, A0_.p, 2 * FEAT, 1);
+    k_agg<FEAT><<<lb + cdiv((uint64_t)nb * (FEAT / 8), 256), 256, 0, st_>>>(v, Xb, FEAT, A0_.p, 2 * FEAT, 1, lb);
     if (nh) k_agg_hub<FEAT><<<nh, 256, 0, st_>>>(v, hubs, Xb, FEAT, A0_.p, 2 * FEAT);
     bf16* A[3] = {A0_.p, A1_.p, A2_.p};
     for (int l = 0; l < 3; ++l) {
@@ -1750,7 +2068,8 @@ class Net {
       g.bias = theta_.p + L_.b[l];
       gemm(g, 1, HID, st_);
       if (l < 2) {
-        k_agg<HID><<<cdiv((uint64_t)nb * (HID / 4), 256), 256, 0, st_>>>(v, A[l + 1], 2 * HID, A[l + 1], 2 * HID, 0);
+        k_agg<HID><<<lb + cdiv((uint64_t)nb * (HID / 8), 256), 256, 0, st_>>>(v, A[l + 1], 2 * HID, A[l + 1], 2 * HID,
+                                                                             0, lb);
         if (nh) k_agg_hub<HID><<<nh, 256, 0, st_>>>(v, hubs, A[l + 1], 2 * HID, A[l + 1], 2 * HID);
       }
     }
@@ -1769,19 +2088,19 @@ class Net {
     ensure_work(b, backward);
     red_.ensure(b.nb, b.i1 - b.i0, b.g1 - b.g0);
     const GView v = s.view(b);
-    const uint32_t nb = b.nb, ng = b.g1 - b.g0, nh = b.h1 - b.h0;
+    const uint32_t nb = b.nb, ng = b.g1 - b.g0, nh = b.h1 - b.h0, lb = long_blocks(v.n_long);
     const uint32_t* hubs = s.hubs.p + b.h0;
     forward(s, b, X);
     PairCtx pc{v, T_.p, Y_.p, hp_.partners, seed_, pair_step};
-    k_loss_stats<<<warps_grid(nb), 256, 0, st_>>>(pc, red_.vals.p);
+    k_loss_stats<<<cdiv((uint64_t)nb * PAIR_LANES, 256), 256, 0, st_>>>(pc, red_.vals.p);
     red_.run<3>(s, b, red_.gsum.p, st_);
     k_loss_finish<<<1, 256, 0, st_>>>(red_.gsum.p, ng, galpha_.p, gcoef_.p, loss_slot);
     if (!backward) return;
-    k_loss_grad<<<warps_grid(nb), 256, 0, st_>>>(pc, galpha_.p, gcoef_.p, dY_.p);
+    k_loss_grad<<<cdiv((uint64_t)nb * PAIR_LANES, 256), 256, 0, st_>>>(pc, galpha_.p, gcoef_.p, dY_.p);
     // head
     k_head_bwd<<<cdiv(nb, 256), 256, 0, st_>>>(nb, H3_.p, theta_bf_.p + L_.wh, dY_.p, dZ_.p);
     const uint32_t chunks = cdiv(nb, kChunk);
-    k_head_wgrad<<<chunks, HID, 0, st_>>>(nb, kChunk, H3_.p, dY_.p, cpart_.p);
+    k_head_wgrad<<<chunks, 32 * CHUNK_WARPS, 0, st_>>>(nb, kChunk, H3_.p, dY_.p, cpart_.p);
     k_reduce_parts<<<reduce_parts_blocks(HEAD_W), 256, 0, st_>>>(cpart_.p, chunks, HEAD_W, grad_.p + L_.wh);
     bf16* A[3] = {A0_.p, A1_.p, A2_.p};
     for (int l = 2; l >= 0; --l) {
@@ -1806,9 +2125,9 @@ class Net {
       g.c_split_stride = (long long)kin * HID;
       g.epilogue = tc::EPI_STORE_F32;
       gemm(g, splits, HID, st_);
-      k_reduce_splits<<<cdiv((uint64_t)kin * HID, 256), 256, 0, st_>>>(wpart_.p, (uint32_t)splits, kin * HID,
+      k_reduce_splits<<<cdiv((uint64_t)kin * HID, 32), 256, 0, st_>>>(wpart_.p, (uint32_t)splits, kin * HID,
                                                                        grad_.p + L_.w[l]);
-      k_colsum<<<chunks, HID, 0, st_>>>(nb, kChunk, dZ_.p, cpart_.p);
+      k_colsum<<<chunks, 32 * CHUNK_WARPS, 0, st_>>>(nb, kChunk, dZ_.p, cpart_.p);
       k_reduce_parts<<<reduce_parts_blocks(HID), 256, 0, st_>>>(cpart_.p, chunks, HID, grad_.p + L_.b[l]);
       if (l == 0) break;
       tc::GemmArgs h = gemm_args();
@@ -1827,7 +2146,7 @@ class Net {
       h.c_split_stride = 0;
       h.epilogue = tc::EPI_STORE_BF16;
       gemm(h, 1, 256, st_);
-      k_agg_bwd<<<warps_grid(nb), 256, 0, st_>>>(v, dA_.p, A[l], dZ_.p);
+      k_agg_bwd<<<lb + cdiv((uint64_t)nb * (HID / 8), 256), 256, 0, st_>>>(v, dA_.p, A[l], dZ_.p, lb);
       if (nh) k_agg_bwd_hub<<<nh, 256, 0, st_>>>(v, hubs, dA_.p, A[l], dZ_.p);
     }
     JC_CUDA_CHECK(cudaGetLastError());
@@ -1843,7 +2162,7 @@ class Net {
   void hand_off(const DevSet& s, const Batch& b) {
     const GView v = s.view(b);
     const uint32_t nb = b.nb, ng = b.g1 - b.g0;
-    k_scale_vals<<<warps_grid(nb), 256, 0, st_>>>(v, Y_.p, red_.vals.p);
+    k_scale_vals<<<cdiv((uint64_t)nb * 8, 256), 256, 0, st_>>>(v, Y_.p, red_.vals.p);
     red_.run<6>(s, b, red_.gsum.p, st_);
     k_scale_grav<<<cdiv(nb, 256), 256, 0, st_>>>(v, Y_.p, red_.gsum.p, red_.vals.p);
     red_.run<1>(s, b, red_.gsum2.p, st_);

@@ -62,3 +62,35 @@ def test_jacobi_forms_bit_exact(jc, orc, case):
     for _ in range(steps):
         assert np.array_equal(bits(e.step()), bits(o.step()))
     assert np.array_equal(bits(e.positions()), bits(o.positions()))
+
+
+def star(jc, leaves, extra):
+    """A star with a path through its first `extra` leaves."""
+    pairs = [(0, k) for k in range(1, leaves + 1)] + [(k, k + 1) for k in range(1, extra)]
+    return jc.csr_from_pairs(leaves + 1, np.array(pairs, np.uint32))
+
+
+# rows around the 32-entry rule of the long-row warps, their 16- and 32-entry
+# chunks and the 1,024-entry hub rule; the oracle sums every row in the device's
+# order and rounds to bf16 where the device stores bf16, so features may differ
+# by a bf16 step of a flipped rounding and the rest by the bars of a bf16 network
+@pytest.mark.parametrize("leaves", [31, 32, 33, 48, 63, 64, 65, 257, 1023, 1024, 1025])
+def test_mpnn_row_lengths(jc, orc, leaves):
+    graphs = [jc.gen_watts_strogatz(70, 6, 0.1, 3), star(jc, leaves, 20), jc.gen_scale_free(300, 3, 5)]
+    rng = np.random.default_rng(7)
+    targets = [rng.standard_normal(3 * g.n_nodes).astype(np.float32) for g in graphs]
+    for t in targets:
+        t[2::3] = 0.0
+    net = jc.Mpnn(2, 99)
+    net.set_params({"smooth_steps": 9, "cheb_steps": 17})
+    net.bind(graphs, targets)
+    gs = orc.GraphSet(graphs)
+    X, xo = net.features(), orc.mpnn_features(gs, 99, smooth_steps=9, cheb_steps=17)
+    assert np.array_equal(X[:, 1:17], xo[:, 1:17])
+    assert np.all(np.abs(X[:, 17:25] - xo[:, 17:25]) <= 2.0 ** -6 * np.abs(xo[:, 17:25]) + 1e-5)
+    loss, y, grad = net.grad(0, 3, pair_step=1)
+    t4 = np.concatenate([np.concatenate([t.reshape(-1, 3), np.zeros((len(t) // 3, 1), np.float32)], 1) for t in targets])
+    loss_o, y_o, grad_o = orc.mpnn_grad(gs, X, t4, 2, net.weights(), 8, 99, 1, 0, 3, emulate=True)
+    assert loss == pytest.approx(loss_o, rel=1e-3)
+    assert np.linalg.norm(y[:, :2] - y_o[:, :2]) <= 1e-2 * np.linalg.norm(y_o[:, :2])
+    assert np.linalg.norm(grad - grad_o) <= 3e-2 * np.linalg.norm(grad_o)
