@@ -94,3 +94,40 @@ def test_mpnn_row_lengths(jc, orc, leaves):
     assert loss == pytest.approx(loss_o, rel=1e-3)
     assert np.linalg.norm(y[:, :2] - y_o[:, :2]) <= 1e-2 * np.linalg.norm(y_o[:, :2])
     assert np.linalg.norm(grad - grad_o) <= 3e-2 * np.linalg.norm(grad_o)
+
+
+# the device check of predict and warm_start: what was refused stays refused and
+# what was accepted stays accepted, rows out of order (the host decides) and
+# duplicates included
+@pytest.mark.parametrize("case", ["ok", "unsorted", "duplicate", "self-loop", "one-sided", "one-sided-hub", "unsorted-one-sided"])
+def test_predict_undirected_check(jc, case):
+    rows = [sorted(set(jc.gen_grid(6).neighbors[o:e].tolist()))
+            for o, e in zip(jc.gen_grid(6).offsets[:-1], jc.gen_grid(6).offsets[1:])]
+    if case.startswith("unsorted"):
+        rows[7] = rows[7][::-1]
+    if case == "duplicate":
+        rows[0] = [rows[0][0]] + rows[0]
+    if case == "self-loop":
+        rows[3] = sorted(rows[3] + [3])
+    if case.endswith("one-sided"):
+        rows[35] = sorted(rows[35] + [0])
+    g = jc.Csr(36, np.cumsum([0] + [len(r) for r in rows]).astype(np.uint32), np.concatenate(rows).astype(np.uint32))
+    if case == "one-sided-hub":
+        s = star(jc, 1500, 3)
+        rows = [s.neighbors[o:e].tolist() for o, e in zip(s.offsets[:-1], s.offsets[1:])]
+        rows[700] = []  # the hub still lists 700
+        g = jc.Csr(1501, np.cumsum([0] + [len(r) for r in rows]).astype(np.uint32), np.concatenate(rows).astype(np.uint32))
+    graphs = [jc.gen_path(9), g, jc.gen_scale_free(50, 2, 1)]
+    net = jc.Mpnn(2, 5)
+    ev = jc.Evaluator(graphs)
+    seeds = [jc.seed_uniform(x.n_nodes, 2, 3) for x in graphs]
+    if case in ("ok", "unsorted", "duplicate"):
+        xyz, _ = net.predict(graphs)
+        assert all(np.all(np.isfinite(x)) for x in xyz)
+        net.warm_start(graphs, seeds, ev)
+    else:
+        for call in (lambda: net.predict(graphs), lambda: net.warm_start(graphs, seeds, ev)):
+            with pytest.raises(jc.JcError, match="undirected"):
+                call()
+        xyz, _ = net.predict(graphs[:1])  # the network stays usable
+        assert np.all(np.isfinite(xyz[0]))
