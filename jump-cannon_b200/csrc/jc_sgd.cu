@@ -8,8 +8,9 @@
 //   crates/graph-compute/src/engines/sgd_stress_gpu.rs   init :165-366, step :368-449
 //   crates/graph-compute/src/shaders/sgd_stress.wgsl     sgd_step :34-62
 //
-// Pivot selection and the per-pivot BFS stay on the host at init, as in the
-// reference (a device BFS is future work). Distances are stored pivot-major
+// The max-min pivot choice and its per-pivot BFS stay on the host at init, as in
+// the reference; random pivots take a device multi-source BFS. Distances are
+// stored pivot-major
 // (dist[t * n + i]) so that the threads of a warp, one node each, read one
 // contiguous row per pivot; u16 when every finite distance fits, else u32,
 // with the all-ones value as "unreachable".
@@ -36,6 +37,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "jc_common.h"
@@ -293,61 +295,138 @@ __global__ void k_pack(const float4* __restrict__ v, uint32_t n, float* __restri
 // previous level (the frontier). A level is one pull pass: node i ORs its
 // neighbours' frontier words, keeps the bits it has not seen, and records the
 // level as its distance to those pivots. Exact BFS distances, independent of
-// thread order. Words of 64 pivots, up to MS_WORDS per pass over a row.
-constexpr uint32_t MS_WORDS = 4;
+// thread order. A node holds `stride` words of 64 pivots, WB of them (one or
+// two 16-byte loads per neighbour) per pass over its row.
+//
+// A level is a few dependent round trips per node (row bounds, ids, frontier
+// words), so four neighbours' words are in flight, a node that every pivot has
+// reached gathers nothing, a gather ends once it holds every bit still wanted,
+// and blocks are small where nodes are few. Distances go straight into their
+// 16-bit rows (u32 from level 65,535 on). Levels are launched MS_CHUNK at a
+// time without waiting; one after the last growing level returns at once.
+// B200, random geometric graphs, us a level: 30,011 nodes with 100 pivots 16 -> 7,
+// 200,000 with 200 pivots 37 -> 22. A whole bind (host copies in it): 5.0 -> 1.7
+// ms and 27 -> 12; R-MAT scale 18 (hub rows, 6 levels) 310 -> 24.
+constexpr int MS_CHUNK = 32;
+using word_t = unsigned long long;
 
-__global__ void k_msbfs_seed(uint32_t n, uint32_t k, uint32_t W, const uint32_t* __restrict__ piv,
-                             unsigned long long* __restrict__ visited, unsigned long long* __restrict__ front,
-                             uint32_t* __restrict__ dist) {
+template <typename D>
+__global__ void k_msbfs_seed(uint32_t n, uint32_t k, uint32_t stride, const uint32_t* __restrict__ piv,
+                             word_t* __restrict__ visited, word_t* __restrict__ front, D* __restrict__ dist) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= k) return;
   const uint32_t v = piv[p];
-  const unsigned long long bit = 1ull << (p & 63u);
-  atomicOr(&visited[(size_t)v * W + (p >> 6)], bit);
-  atomicOr(&front[(size_t)v * W + (p >> 6)], bit);
-  dist[(size_t)p * n + v] = 0u;
+  const word_t bit = 1ull << (p & 63u);
+  atomicOr(&visited[(size_t)v * stride + (p >> 6)], bit);
+  atomicOr(&front[(size_t)v * stride + (p >> 6)], bit);
+  dist[(size_t)p * n + v] = 0;
 }
 
+template <int WB>
+struct Words {
+  word_t w[WB];
+};
+template <int WB>
+__device__ __forceinline__ Words<WB> load_words(const word_t* p) {
+  Words<WB> r;
+  if constexpr (WB == 1) {
+    r.w[0] = *p;
+  } else {
+#pragma unroll
+    for (int q = 0; q < WB / 2; ++q) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p + 2 * q);
+      r.w[2 * q] = v.x;
+      r.w[2 * q + 1] = v.y;
+    }
+  }
+  return r;
+}
+template <int WB>
+__device__ __forceinline__ void store_words(word_t* p, const Words<WB>& r) {
+  if constexpr (WB == 1) {
+    *p = r.w[0];
+  } else {
+#pragma unroll
+    for (int q = 0; q < WB / 2; ++q)
+      *reinterpret_cast<ulonglong2*>(p + 2 * q) = make_ulonglong2(r.w[2 * q], r.w[2 * q + 1]);
+  }
+}
+
+// *last: the highest level at which some node grew (0: the seeds).
+template <typename D, int WB>
 __global__ void __launch_bounds__(256)
-k_msbfs_level(uint32_t n, uint32_t W, const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
-              const unsigned long long* __restrict__ front, unsigned long long* __restrict__ next,
-              unsigned long long* __restrict__ visited, uint32_t* __restrict__ dist, uint32_t level,
-              uint32_t* __restrict__ progress) {
+k_msbfs_level(uint32_t n, uint32_t k, uint32_t stride, const uint32_t* __restrict__ off,
+              const uint32_t* __restrict__ nbr, const word_t* __restrict__ front, word_t* __restrict__ next,
+              word_t* __restrict__ visited, D* __restrict__ dist, uint32_t level, uint32_t* last) {
+  if (*(volatile uint32_t*)last + 1u < level) return;  // the level before added nothing
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   bool grew = false;
-  for (uint32_t w0 = 0; w0 < W; w0 += MS_WORDS) {
-    const uint32_t ww = min(MS_WORDS, W - w0);
-    unsigned long long acc[MS_WORDS] = {0ull, 0ull, 0ull, 0ull};
-    for (uint32_t e = off[i]; e < off[i + 1]; ++e) {
-      const unsigned long long* f = front + (size_t)nbr[e] * W + w0;
-      for (uint32_t w = 0; w < ww; ++w) acc[w] |= f[w];
-    }
-    for (uint32_t w = 0; w < ww; ++w) {
-      unsigned long long* vis = visited + (size_t)i * W + w0 + w;
-      unsigned long long nb = acc[w] & ~*vis;
-      next[(size_t)i * W + w0 + w] = nb;
-      if (!nb) continue;
-      *vis |= nb;
-      grew = true;
-      while (nb) {
-        const uint32_t b = (uint32_t)__ffsll((long long)nb) - 1u;
-        nb &= nb - 1ull;
-        dist[(size_t)((w0 + w) * 64u + b) * n + i] = level;
+  if (i < n) {
+    const uint32_t e0 = off[i], e1 = off[i + 1];
+    for (uint32_t w0 = 0; w0 < stride; w0 += WB) {
+      word_t* vis = visited + (size_t)i * stride + w0;
+      const Words<WB> seen = load_words<WB>(vis);
+      Words<WB> want, acc;
+      word_t missing = 0;
+#pragma unroll
+      for (int q = 0; q < WB; ++q) {
+        const uint32_t p0 = (w0 + q) * 64u;  // pivots [p0, p0 + 64) of this word
+        const word_t all = p0 + 64u <= k ? ~0ull : (p0 < k ? (1ull << (k - p0)) - 1ull : 0ull);
+        want.w[q] = all & ~seen.w[q];
+        acc.w[q] = 0ull;
+        missing |= want.w[q];
       }
+      uint32_t e = e0;
+      for (; missing && e + 4 <= e1; e += 4) {
+        uint32_t id[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) id[u] = __ldg(nbr + e + u);
+        Words<WB> f[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) f[u] = load_words<WB>(front + (size_t)id[u] * stride + w0);
+        missing = 0;
+#pragma unroll
+        for (int q = 0; q < WB; ++q) {
+          acc.w[q] |= f[0].w[q] | f[1].w[q] | f[2].w[q] | f[3].w[q];
+          missing |= want.w[q] & ~acc.w[q];
+        }
+      }
+      if (missing && e < e1) {  // one to three left, together
+        uint32_t id[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) id[u] = __ldg(nbr + min(e + u, e1 - 1u));
+        Words<WB> f[3];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) f[u] = load_words<WB>(front + (size_t)id[u] * stride + w0);
+#pragma unroll
+        for (int q = 0; q < WB; ++q) acc.w[q] |= f[0].w[q] | f[1].w[q] | f[2].w[q];
+      }
+      Words<WB> now;
+      word_t any = 0;
+#pragma unroll
+      for (int q = 0; q < WB; ++q) {
+        now.w[q] = acc.w[q] & want.w[q];
+        any |= now.w[q];
+      }
+      store_words<WB>(next + (size_t)i * stride + w0, now);
+      if (!any) continue;
+      grew = true;
+#pragma unroll
+      for (int q = 0; q < WB; ++q) {
+        acc.w[q] = seen.w[q] | now.w[q];
+        for (word_t nb = now.w[q]; nb; nb &= nb - 1ull)
+          dist[(size_t)((w0 + q) * 64u + (uint32_t)__ffsll((long long)nb) - 1u) * n + i] = (D)level;
+      }
+      store_words<WB>(vis, acc);
     }
   }
-  if (grew) {
-    atomicAdd(&progress[0], 1u);
-    atomicMax(&progress[1], level);
-  }
+  if (__syncthreads_or(grew) && threadIdx.x == 0) atomicMax(last, level);
 }
 
-__global__ void k_dist_to_u16(const uint32_t* __restrict__ d32, size_t count, uint16_t* __restrict__ d16) {
+__global__ void k_dist_widen(const uint16_t* __restrict__ d16, size_t count, uint32_t* __restrict__ d32) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
-  const uint32_t d = d32[t];
-  d16[t] = d == UNREACH ? (uint16_t)0xFFFFu : (uint16_t)d;
+  d32[t] = d16[t] == 0xFFFFu ? UNREACH : (uint32_t)d16[t];
 }
 
 // ============================================================== host ==
@@ -477,41 +556,57 @@ class SgdEngine : public Engine {
     for (uint32_t t = 0; t < k_; ++t) std::swap(idx[t], idx[t + (uint32_t)rng.below(n - t)]);
     pivots_.assign(idx.begin(), idx.begin() + k_);
     stream_state_ = rng.state;
-    const uint32_t W = (k_ + 63u) / 64u;
-    DBuf<uint32_t> doff, dnbr, dpiv, prog;
-    DBuf<unsigned long long> vis, fa, fb;
-    doff.alloc((size_t)n + 1);
-    dnbr.alloc(std::max<uint64_t>(nnz, 1));
-    dpiv.alloc(k_);
-    prog.alloc(2);
-    vis.alloc((size_t)n * W);
-    fa.alloc((size_t)n * W);
-    fb.alloc((size_t)n * W);
-    dist32_.alloc((size_t)k_ * n);
-    JC_CUDA_CHECK(cudaMemcpyAsync(doff.p, off, sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, stream_));
-    if (nnz) JC_CUDA_CHECK(cudaMemcpyAsync(dnbr.p, nbr, sizeof(uint32_t) * nnz, cudaMemcpyHostToDevice, stream_));
-    JC_CUDA_CHECK(cudaMemcpyAsync(dpiv.p, pivots_.data(), sizeof(uint32_t) * k_, cudaMemcpyHostToDevice, stream_));
-    JC_CUDA_CHECK(cudaMemsetAsync(vis.p, 0, sizeof(unsigned long long) * n * W, stream_));
-    JC_CUDA_CHECK(cudaMemsetAsync(fa.p, 0, sizeof(unsigned long long) * n * W, stream_));
-    JC_CUDA_CHECK(cudaMemsetAsync(dist32_.p, 0xFF, sizeof(uint32_t) * k_ * n, stream_));
-    JC_CUDA_CHECK(cudaMemsetAsync(prog.p, 0, 8, stream_));
-    k_msbfs_seed<<<cdiv(k_, 256), 256, 0, stream_>>>(n, k_, W, dpiv.p, vis.p, fa.p, dist32_.p);
-    // levels in chunks of 16; stop after a chunk in which no node grew (every
-    // level after the last growing one changes nothing)
+    // words per node: 1, 2 or a multiple of 4 (16-byte loads)
+    uint32_t W = (k_ + 63u) / 64u;
+    if (W > 2) W = (W + 3u) / 4u * 4u;
+    const size_t words = (size_t)n * W, cells = (size_t)k_ * n;
+    goff_.alloc((size_t)n + 1);
+    gnbr_.alloc(std::max<uint64_t>(nnz, 1));
+    piv_.alloc(k_);
+    last_.alloc(1);
+    vis_.alloc(words);
+    front_.alloc(2 * words);
+    dist16_.alloc(cells);
+    JC_CUDA_CHECK(cudaMemcpyAsync(goff_.p, off, sizeof(uint32_t) * ((size_t)n + 1), cudaMemcpyHostToDevice, stream_));
+    if (nnz) JC_CUDA_CHECK(cudaMemcpyAsync(gnbr_.p, nbr, sizeof(uint32_t) * nnz, cudaMemcpyHostToDevice, stream_));
+    JC_CUDA_CHECK(cudaMemcpyAsync(piv_.p, pivots_.data(), sizeof(uint32_t) * k_, cudaMemcpyHostToDevice, stream_));
+    word_t *fa = front_.p, *fb = front_.p + words;
+    JC_CUDA_CHECK(cudaMemsetAsync(vis_.p, 0, sizeof(word_t) * words, stream_));
+    JC_CUDA_CHECK(cudaMemsetAsync(fa, 0, sizeof(word_t) * words, stream_));
+    JC_CUDA_CHECK(cudaMemsetAsync(dist16_.p, 0xFF, sizeof(uint16_t) * cells, stream_));
+    JC_CUDA_CHECK(cudaMemsetAsync(last_.p, 0, 4, stream_));
+    k_msbfs_seed<uint16_t><<<cdiv(k_, 256), 256, 0, stream_>>>(n, k_, W, piv_.p, vis_.p, fa, dist16_.p);
+    const uint32_t threads = n <= JACOBI_SMALL_N ? 64u : 256u;
+    auto launch = [&](auto* dist, uint32_t level) {
+      using D = std::remove_pointer_t<decltype(dist)>;
+      const uint32_t blocks = cdiv(n, threads);
+      if (W == 1)
+        k_msbfs_level<D, 1><<<blocks, threads, 0, stream_>>>(n, k_, W, goff_.p, gnbr_.p, fa, fb, vis_.p, dist, level,
+                                                             last_.p);
+      else if (W == 2)
+        k_msbfs_level<D, 2><<<blocks, threads, 0, stream_>>>(n, k_, W, goff_.p, gnbr_.p, fa, fb, vis_.p, dist, level,
+                                                             last_.p);
+      else
+        k_msbfs_level<D, 4><<<blocks, threads, 0, stream_>>>(n, k_, W, goff_.p, gnbr_.p, fa, fb, vis_.p, dist, level,
+                                                             last_.p);
+      std::swap(fa, fb);
+    };
+    bool wide = false;
     uint32_t level = 1, maxd = 0;
     for (;;) {
-      uint32_t h[2] = {0, 0};
-      JC_CUDA_CHECK(cudaMemsetAsync(prog.p, 0, 4, stream_));
-      for (int c = 0; c < 16; ++c, ++level) {
-        k_msbfs_level<<<cdiv(n, 256), 256, 0, stream_>>>(n, W, doff.p, dnbr.p, fa.p, fb.p, vis.p, dist32_.p, level,
-                                                         prog.p);
-        std::swap(fa.p, fb.p);
+      for (int c = 0; c < MS_CHUNK; ++c, ++level) {
+        if (level == 0xFFFFu) {  // the first distance that 16 bits cannot hold
+          wide = true;
+          dist32_.alloc(cells);
+          k_dist_widen<<<(unsigned)((cells + 255) / 256), 256, 0, stream_>>>(dist16_.p, cells, dist32_.p);
+        }
+        if (wide) launch(dist32_.p, level);
+        else launch(dist16_.p, level);
       }
       JC_CUDA_CHECK(cudaGetLastError());
-      JC_CUDA_CHECK(cudaMemcpyAsync(h, prog.p, 8, cudaMemcpyDeviceToHost, stream_));
+      JC_CUDA_CHECK(cudaMemcpyAsync(&maxd, last_.p, 4, cudaMemcpyDeviceToHost, stream_));
       JC_CUDA_CHECK(cudaStreamSynchronize(stream_));
-      maxd = h[1];
-      if (h[0] == 0 || level > n + 16u) break;
+      if (maxd + 1 < level) break;  // the last level launched added nothing
     }
     host_dist_.clear();
     host_dist_valid_ = false;  // copied back on demand (stress and pivot read-outs)
@@ -519,7 +614,8 @@ class SgdEngine : public Engine {
   }
 
   // The rest of init, from the pivot distances: host rows (dist32 != null)
-  // or dist32_ already on the device.
+  // or rows already on the device (dist16_, or dist32_ when some distance does
+  // not fit 16 bits).
   void finish_init(uint32_t n, const float* xyz, uint32_t maxd, const std::vector<uint32_t>* dist32) {
     wide_ = maxd >= 0xFFFFu;
     // eta schedule, one entry per sweep up to the end of annealing
@@ -535,13 +631,8 @@ class SgdEngine : public Engine {
     // device buffers
     pos_a_.alloc(n); pos_b_.alloc(n); xyz_.alloc((size_t)3 * n); piv_.alloc(k_); eta_.alloc(n_eta_);
     ctr_.alloc(1);
-    if (!dist32) {  // distances on the device already (multi-source BFS)
-      if (!wide_ && k_ && n) {
-        dist16_.alloc((size_t)k_ * n);
-        const size_t cnt = (size_t)k_ * n;
-        k_dist_to_u16<<<(unsigned)((cnt + 255) / 256), 256, 0, stream_>>>(dist32_.p, cnt, dist16_.p);
-        JC_CUDA_CHECK(cudaGetLastError());
-      }
+    if (!dist32) {
+      // (on the device already: multi-source BFS)
     } else if (wide_) {
       dist32_.alloc((size_t)k_ * n);
       if (k_ && n)
@@ -775,6 +866,10 @@ class SgdEngine : public Engine {
   DBuf<float> xyz_, eta_;
   DBuf<uint32_t> piv_, ctr_, dist32_, cnt_;
   DBuf<uint16_t> dist16_;
+  // the multi-source BFS: the graph, and one bit per (node, pivot) seen, in the
+  // frontier and in the next one; kept for the next bind
+  DBuf<uint32_t> goff_, gnbr_, last_;
+  DBuf<word_t> vis_, front_;
   DBuf<long long> acc_;
 
   void ensure_stream() {

@@ -131,3 +131,30 @@ def test_predict_undirected_check(jc, case):
                 call()
         xyz, _ = net.predict(graphs[:1])  # the network stays usable
         assert np.all(np.isfinite(xyz[0]))
+
+
+# pivot words of 1, 2 and blocks of 4 (and their last, partial word), several
+# components, and hop distances on both sides of 65,535 (a path from its ends)
+@pytest.mark.parametrize("k", [1, 63, 64, 65, 128, 129, 256, 257])
+def test_multi_source_bfs_words(jc, orc, k):
+    a, b = jc.gen_scale_free(700, 2, 3), jc.gen_grid(17)
+    g = jc.csr_from_pairs(1000, np.concatenate([a.pairs(), b.pairs() + 700]))  # 11 isolated nodes
+    e = jc.LayoutEngine("sgd-stress-gpu")
+    e.set_params({"n_pivots": k, "random_pivots": True, "seed": 5})
+    for _ in range(2):  # the second bind reuses the first's workspace
+        e.init(g, jc.seed_uniform(1000, 2, 1))
+        piv, dist = e.pivots()
+        assert len(set(piv.tolist())) == k
+        for t in {0, k // 2, k - 1}:
+            assert np.array_equal(dist[t], orc.bfs(g, int(piv[t])))
+
+
+@pytest.mark.parametrize("n", [65000, 70000])
+def test_multi_source_bfs_long_path(jc, n):
+    g = jc.gen_path(n)
+    e = jc.LayoutEngine("sgd-stress-gpu")
+    e.set_params({"n_pivots": 3, "random_pivots": True, "seed": 1})
+    e.init(g, jc.seed_uniform(n, 2, 1))
+    piv, dist = e.pivots()
+    for t in range(3):
+        assert np.array_equal(dist[t], np.abs(np.arange(n) - int(piv[t])).astype(np.uint32))
