@@ -205,71 +205,122 @@ k_jacobi(const float4* __restrict__ pin, float4* __restrict__ pout, const uint32
 // Up to here 64-thread blocks, so that the nodes spread over every SM.
 constexpr uint32_t JACOBI_SMALL_N = 148u * 512u;
 
-// One batch of the per-pair scatter. Sample q = sweep * n + q0 + t.
+// A sweep's n samples, drawn in one pass: sample q = sweep * n + t is (node i,
+// pivot j, hop distance as f32 bits; 0 for a skipped pair: the node itself, or
+// unreachable). They do not depend on the positions, and drawing them inside a
+// batch put two 64-bit remainders and a cache-missing distance read into each
+// batch's chain of round trips.
 template <typename D>
 __global__ void __launch_bounds__(256)
-k_pairs(const float4* __restrict__ pos, long long* __restrict__ acc, uint32_t* __restrict__ cnt,
-        const uint32_t* __restrict__ pivots, const D* __restrict__ dist, uint32_t n, uint32_t k, uint64_t s0,
-        uint32_t q0, uint32_t count, const float* __restrict__ eta_table, uint32_t n_eta,
-        const uint32_t* __restrict__ sweep_ctr) {
+k_pairs_draw(uint4* __restrict__ samples, const uint32_t* __restrict__ pivots, const D* __restrict__ dist, uint32_t n,
+             uint32_t k, uint64_t s0, const uint32_t* __restrict__ sweep_ctr, uint32_t sweep) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  const uint32_t sw = *sweep_ctr;
-  const float eta = eta_table[sw < n_eta ? sw : n_eta - 1];
-  const uint64_t q = (uint64_t)sw * n + q0 + t;
+  if (t >= n) return;
+  const uint64_t q = (uint64_t)(*sweep_ctr + sweep) * n + t;
   const uint64_t G = 0x9E3779B97F4A7C15ull;
   const uint32_t i = (uint32_t)(smix(s0 + (2 * q + 1) * G) % n);
   const uint32_t pidx = (uint32_t)(smix(s0 + (2 * q + 2) * G) % k);
   const uint32_t j = pivots[pidx];
-  if (i == j) return;
   const D du = dist[(size_t)pidx * n + i];
-  const D sent = (D)~(D)0;
-  if (du == sent || du == 0) return;
-  const float d = (float)du;
-  const float4 a = pos[i], b = pos[j];
+  const float hop = (i == j || du == (D)~(D)0) ? 0.0f : (float)du;
+  samples[t] = make_uint4(i, j, __float_as_uint(hop), 0u);
+}
+
+// The pair update against positions a (node) and b (pivot): the pivot's move in
+// fixed point; the node's is its negative.
+__device__ __forceinline__ void pair_move(const float4 a, const float4 b, float d, float eta, long long* f) {
   const float dx = __fsub_rn(a.x, b.x), dy = __fsub_rn(a.y, b.y), dz = __fsub_rn(a.z, b.z);
   const float mag = fmaxf(len3(dx, dy, dz), 1e-6f);
   const float w = __fdiv_rn(1.0f, __fmul_rn(d, d));
   const float mu = fminf(__fmul_rn(w, eta), 1.0f);
   const float r = __fdiv_rn(__fmul_rn(__fmul_rn(0.5f, mu), __fsub_rn(mag, d)), mag);
-  const float rx = __fmul_rn(r, dx), ry = __fmul_rn(r, dy), rz = __fmul_rn(r, dz);
-  const long long fx = __double2ll_rn((double)rx * FIX_SCALE);
-  const long long fy = __double2ll_rn((double)ry * FIX_SCALE);
-  const long long fz = __double2ll_rn((double)rz * FIX_SCALE);
-  atomicAdd((unsigned long long*)&acc[3 * (size_t)i], (unsigned long long)(-fx));
-  atomicAdd((unsigned long long*)&acc[3 * (size_t)i + 1], (unsigned long long)(-fy));
-  atomicAdd((unsigned long long*)&acc[3 * (size_t)i + 2], (unsigned long long)(-fz));
-  atomicAdd((unsigned long long*)&acc[3 * (size_t)j], (unsigned long long)fx);
-  atomicAdd((unsigned long long*)&acc[3 * (size_t)j + 1], (unsigned long long)fy);
-  atomicAdd((unsigned long long*)&acc[3 * (size_t)j + 2], (unsigned long long)fz);
-  atomicAdd(&cnt[i], 1u);
-  atomicAdd(&cnt[j], 1u);
+  f[0] = __double2ll_rn((double)__fmul_rn(r, dx) * FIX_SCALE);
+  f[1] = __double2ll_rn((double)__fmul_rn(r, dy) * FIX_SCALE);
+  f[2] = __double2ll_rn((double)__fmul_rn(r, dz) * FIX_SCALE);
 }
 
-__global__ void __launch_bounds__(256)
-k_pairs_apply(float4* __restrict__ pos, long long* __restrict__ acc, uint32_t* __restrict__ cnt, uint32_t n) {
-  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n) return;
-  const uint32_t c = cnt[v];
-  if (c == 0) return;
+__device__ __forceinline__ void pair_add(long long* acc, uint32_t v, const long long* f, bool neg) {
+  unsigned long long* o = reinterpret_cast<unsigned long long*>(acc + 3 * (size_t)v);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) atomicAdd(o + c, (unsigned long long)(neg ? -f[c] : f[c]));
+}
+
+// Node v moves by the mean of its `c` accumulated moves.
+__device__ __forceinline__ float4 pair_moved(float4 p, const long long* a, uint32_t c) {
   const double inv = 1.0 / (FIX_SCALE * (double)c);
-  float4 p = pos[v];
-  p.x = __fadd_rn(p.x, (float)((double)acc[3 * (size_t)v] * inv));
-  p.y = __fadd_rn(p.y, (float)((double)acc[3 * (size_t)v + 1] * inv));
-  p.z = __fadd_rn(p.z, (float)((double)acc[3 * (size_t)v + 2] * inv));
-  pos[v] = p;
-  acc[3 * (size_t)v] = 0;
-  acc[3 * (size_t)v + 1] = 0;
-  acc[3 * (size_t)v + 2] = 0;
-  cnt[v] = 0;
+  p.x = __fadd_rn(p.x, (float)((double)a[0] * inv));
+  p.y = __fadd_rn(p.y, (float)((double)a[1] * inv));
+  p.z = __fadd_rn(p.z, (float)((double)a[2] * inv));
+  return p;
 }
 
-__global__ void k_add_counter(uint32_t* ctr, uint32_t by) { *ctr += by; }
+// A sweep is 64 batches of two short kernels, each a few dependent round trips,
+// so both are launched as programmatic dependents: a kernel is placed and reads
+// its samples while the one before drains, and waits for it (all of its writes)
+// before it touches positions or sums. At least one thread of each reaches the
+// wait, so completion passes down the chain; the draw and the step's end are
+// ordinary launches. (A cluster of eight CTAs that kept a whole sweep in one
+// launch with barriers between the phases was slower, 569 us a sweep at 200,000
+// nodes: every phase waits for the adds of 4,096 threads to drain.) B200, us a
+// sweep, before (samples drawn in the batch, a pass over all nodes to apply) and
+// after: 200,000 nodes 388 -> 238 (296 without the early placement), 30,000 382
+// -> 224, 1,000 27 -> 18, 1 M 599 -> 426.
+__device__ __forceinline__ void dependent_launch_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
-// The end of a step's Jacobi sweeps: the last sweep's output to the engine's
-// positions and the read-back array, and the sweep counter (one launch).
+// One batch: every pair against the batch-start positions, both moves added in
+// fixed point.
+__global__ void __launch_bounds__(128)
+k_pairs(const uint4* __restrict__ samples, uint32_t count, const float4* __restrict__ pos,
+        long long* __restrict__ acc, uint32_t* __restrict__ cnt, const float* __restrict__ eta_table, uint32_t n_eta,
+        const uint32_t* __restrict__ sweep_ctr, uint32_t sweep) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t sw = *sweep_ctr + sweep;
+  const float eta = eta_table[sw < n_eta ? sw : n_eta - 1];
+  const uint4 p = samples[t];
+  dependent_launch_wait();
+  const float hop = __uint_as_float(p.z);
+  if (!(hop > 0.0f)) return;
+  long long f[3];
+  pair_move(pos[p.x], pos[p.y], hop, eta, f);
+  pair_add(acc, p.x, f, true);
+  pair_add(acc, p.y, f, false);
+  atomicAdd(&cnt[p.x], 1u);
+  atomicAdd(&cnt[p.y], 1u);
+}
+
+// The batch's end: each node it touched moves by the mean of its moves and is
+// cleared. A thread per sample endpoint; the one that takes the node's count
+// owns it (the others find 0), so no pass over all n nodes looks for the few
+// that moved. Sums and position are read beside the count: only the owner
+// writes them, after its own reads.
+__global__ void __launch_bounds__(128)
+k_pairs_apply(const uint4* __restrict__ samples, uint32_t count, float4* __restrict__ pos, long long* __restrict__ acc,
+              uint32_t* __restrict__ cnt) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 2 * count) return;
+  const uint4 s = samples[t >> 1];
+  dependent_launch_wait();
+  if (!(__uint_as_float(s.z) > 0.0f)) return;
+  const uint32_t v = (t & 1u) ? s.y : s.x;
+  long long* m = acc + 3 * (size_t)v;
+  const long long f[3] = {__ldcg(m), __ldcg(m + 1), __ldcg(m + 2)};
+  const float4 p = __ldcg(pos + v);
+  const uint32_t c = atomicExch(cnt + v, 0u);
+  if (c == 0) return;
+  pos[v] = pair_moved(p, f, c);
+  m[0] = 0;
+  m[1] = 0;
+  m[2] = 0;
+}
+
+// The end of a step's sweeps: the last sweep's output to the engine's positions
+// and the read-back array, and the sweep counter (one launch).
 __global__ void __launch_bounds__(256)
-k_jacobi_end(const float4* v, uint32_t n, float4* pos, float* __restrict__ xyz, uint32_t* ctr, uint32_t sweeps) {
+k_step_end(const float4* v, uint32_t n, float4* pos, float* __restrict__ xyz, uint32_t* ctr, uint32_t sweeps) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *ctr += sweeps;
   if (i >= n) return;
@@ -648,6 +699,7 @@ class SgdEngine : public Engine {
     if (!jacobi_) {
       acc_.alloc((size_t)3 * std::max<uint32_t>(n, 1));
       cnt_.alloc(std::max<uint32_t>(n, 1));
+      samples_.alloc(n);
       JC_CUDA_CHECK(cudaMemsetAsync(acc_.p, 0, sizeof(long long) * 3 * std::max<uint32_t>(n, 1), stream_));
       JC_CUDA_CHECK(cudaMemsetAsync(cnt_.p, 0, sizeof(uint32_t) * std::max<uint32_t>(n, 1), stream_));
     }
@@ -871,6 +923,7 @@ class SgdEngine : public Engine {
   DBuf<uint32_t> goff_, gnbr_, last_;
   DBuf<word_t> vis_, front_;
   DBuf<long long> acc_;
+  DBuf<uint4> samples_;  // one sweep's pairs
 
   void ensure_stream() {
     if (!stream_) {
@@ -898,6 +951,21 @@ class SgdEngine : public Engine {
     if (!initialized_) fail(JC_ERR_STATE, std::string(desc_.id) + " step called before successful init");
   }
 
+  // k as an ordinary launch or as a programmatic dependent of the one before.
+  template <typename... P, typename... A>
+  void launch_pdl(bool pdl, uint32_t blocks, uint32_t threads, void (*k)(P...), A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream_;
+    cfg.attrs = &at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    JC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k, (P)args...));
+  }
+
   template <typename D>
   int enqueue_sweeps(const D* dist) {
     const uint32_t n = n_, k = k_;
@@ -922,10 +990,8 @@ class SgdEngine : public Engine {
         std::swap(in, out);
         ++L;
       }
-      k_jacobi_end<<<cdiv(n, 256), 256, 0, stream_>>>(in, n, pos_a_.p, xyz_.p, ctr_.p, sweeps);
+      k_step_end<<<cdiv(n, 256), 256, 0, stream_>>>(in, n, pos_a_.p, xyz_.p, ctr_.p, sweeps);
       ++L;
-      JC_CUDA_CHECK(cudaGetLastError());
-      return L;
     } else {
       // sgd_stress.rs:287-315: per sweep, eta(sweep), n samples, sweep += 1.
       // Default: batches of max(256, n/64) samples (at most 64 per sweep).
@@ -933,19 +999,20 @@ class SgdEngine : public Engine {
       batches = std::max(1u, std::min(batches, n));
       const uint32_t per = cdiv(n, batches);
       for (uint32_t s = 0; s < sweeps; ++s) {
+        k_pairs_draw<D><<<cdiv(n, 256), 256, 0, stream_>>>(samples_.p, piv_.p, dist, n, k, stream_state_, ctr_.p, s);
+        ++L;
         for (uint32_t q0 = 0; q0 < n; q0 += per) {
           const uint32_t cnt = std::min(per, n - q0);
-          k_pairs<D><<<cdiv(cnt, 256), 256, 0, stream_>>>(pos_a_.p, acc_.p, cnt_.p, piv_.p, dist, n, k,
-                                                          stream_state_, q0, cnt, eta_.p, n_eta_, ctr_.p);
-          k_pairs_apply<<<cdiv(n, 256), 256, 0, stream_>>>(pos_a_.p, acc_.p, cnt_.p, n);
+          launch_pdl(q0 > 0, cdiv(cnt, 128), 128, k_pairs, (const uint4*)samples_.p + q0, cnt, (const float4*)pos_a_.p,
+                     acc_.p, cnt_.p, (const float*)eta_.p, n_eta_, (const uint32_t*)ctr_.p, s);
+          launch_pdl(true, cdiv(2 * (uint64_t)cnt, 128), 128, k_pairs_apply, (const uint4*)samples_.p + q0, cnt,
+                     pos_a_.p, acc_.p, cnt_.p);
           L += 2;
         }
-        k_add_counter<<<1, 1, 0, stream_>>>(ctr_.p, 1u);
-        ++L;
       }
+      k_step_end<<<cdiv(n, 256), 256, 0, stream_>>>(pos_a_.p, n, pos_a_.p, xyz_.p, ctr_.p, sweeps);
+      ++L;
     }
-    k_pack<<<cdiv(n, 256), 256, 0, stream_>>>(pos_a_.p, n, xyz_.p);
-    ++L;
     JC_CUDA_CHECK(cudaGetLastError());
     return L;
   }

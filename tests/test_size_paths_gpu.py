@@ -158,3 +158,18 @@ def test_multi_source_bfs_long_path(jc, n):
     piv, dist = e.pivots()
     for t in range(3):
         assert np.array_equal(dist[t], np.abs(np.arange(n) - int(piv[t])).astype(np.uint32))
+
+
+# one batch, one sample a batch, block remainders, several sweeps a step
+@pytest.mark.parametrize("n,batches,sweeps", [(4096, 1, 1), (4097, 1, 2), (8192, 1, 1), (8193, 1, 1), (16384, 1, 2),
+                                              (16385, 1, 2), (20000, 3, 1), (700, 700, 1), (1501, 7, 3), (33000, 0, 1)])
+def test_pair_batches_bit_exact(jc, orc, n, batches, sweeps):
+    g = jc.gen_watts_strogatz(n, 4, 0.2, n)
+    pos = jc.seed_uniform(n, 3, 2) * np.float32(10.0)
+    s = {"n_pivots": 5, "eta_max": 4.0, "sweeps_per_step": sweeps}
+    e = jc.LayoutEngine("sgd-stress")
+    e.set_params({**s, "scatter_batches": batches})
+    e.init(g, pos)
+    o = orc.Sgd(g, pos, mode=2, scatter_batches=batches, **s)
+    for _ in range(3):
+        assert np.array_equal(bits(e.step()), bits(o.step()))
