@@ -87,7 +87,11 @@ constexpr uint32_t DEFAULT_HUB_THRESHOLD = 2048;
 // Lists at least this long (and below the hub threshold) are gathered by a
 // whole warp, 32 neighbours at a time, and summed in list order by lane 0: a
 // thread alone would wait on hundreds of dependent gather rounds.
-constexpr uint32_t DEFAULT_WARP_THRESHOLD = 512;
+// Where the graph does not fill the GPU the warps are free and a thread's list
+// only adds latency, so smaller graphs hand over shorter lists. B200, us a pass
+// at thresholds 512 / 128 / 32: Barabasi-Albert 10,000 nodes 35 / 22 / 17,
+// 100,000 55 / 33 / 38; R-MAT 262,144 nodes 102 / 112 / 129, 1 M 252 / 397 / 498.
+inline uint32_t default_warp_threshold(uint32_t n) { return n <= 32768u ? 32u : n <= 196608u ? 128u : 512u; }
 constexpr uint32_t DEFAULT_WALK_GROUP = 1;  // fastest in the B200 sweep (1, 2, 4, ..., 32)
 // The top of a single graph's tree (depth <= TOP_DEPTH, at most
 // 1 + 8 + 64 + 512 nodes) is staged in shared memory for the walk.
@@ -916,6 +920,54 @@ __device__ __forceinline__ void walk_counts_flush(uint32_t n_inter, uint32_t n_o
   }
 }
 
+// The same walk with the next node loaded before the current term is added: the
+// division no longer stands between a visit and the next load. It takes 38
+// registers, so it is for graphs that do not fill the SMs with warps, where a
+// walk is one latency chain. B200, us a walk, k_walk_rope and this: 400 nodes 58
+// -> 40, 10,000 102 -> 69, 65,537 75 -> 55; R-MAT 262,144 nodes 136 -> 153.
+// (Blocks of 64 spread 10,000 bodies over every SM but share fewer nodes in L1:
+// 74. Fewer bodies per warp: no gain from 16, slower below 8.)
+constexpr uint32_t WALK_AHEAD_N = 148u * 1024u;
+template <bool FAST>
+__global__ void __launch_bounds__(WALK_THREADS)
+k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, const float4* __restrict__ pos,
+             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep) {
+  const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t T = st->error ? 0u : st->n_tree;
+  uint32_t n_inter = 0, n_open = 0;
+  if (a < n) {
+    const uint32_t body = order[a];
+    if (!JC_IN_BOUNDS(body, n, &st->error)) return;
+    const float4 p = pos[body];
+    const float srd = __fmul_rn(P.scaling_ratio, degf[body]);
+    float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+    uint32_t idx = T > 0u ? 0u : END;
+    float4 c;
+    int4 m;
+    if (idx < T) load_node(nodes, c, m);
+    while (idx < T) {
+      const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
+      const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+      const bool leaf = m.y >= 0;
+      const bool use = leaf ? (uint32_t)m.y != body : __int_as_float(m.z) < __fmul_rn(P.theta2, r2);
+      const bool descend = !leaf && !use;
+      const uint32_t next = descend ? idx + 1u : (uint32_t)m.x;
+      const float mass = c.w;
+      if (next <= idx) break;
+      if (next < T) load_node(nodes + next, c, m);
+      if (use) {
+        rep_term<FAST>(dx, dy, dz, r2, srd, mass, fx, fy, fz);
+        ++n_inter;
+      }
+      n_open += descend ? 1u : 0u;
+      idx = next;
+    }
+    if (idx != END) set_error(st, JC_ERR_DEVICE_TIMEOUT);
+    frep[body] = make_float4(fx, fy, fz, 0.0f);
+  }
+  walk_counts_flush(n_inter, n_open, st);
+}
+
 // One thread per body, bodies in key order. Bounded to 32 registers, so
 // eight blocks (every warp slot of the SM) are resident: the walk waits on
 // its node loads, and full occupancy hides more of that (1M-node R-MAT walk
@@ -1477,9 +1529,12 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
         tr = r.tr;
       }
     } else if (blockIdx.x < P.n_hubs + (P.n_med + ATT_THREADS / 32 - 1) / (ATT_THREADS / 32)) {
-      // One warp per long list: the lanes gather 32 neighbours at a time (the
-      // next 32 are in flight while lane 0 adds the current ones in list
-      // order), so the sum is the same sequence of roundings as one thread's.
+      // One warp per long list: the lanes gather 32 neighbours at a time, and
+      // every lane adds them in list order from shuffles (unrolled: the
+      // shuffles do not wait for the additions), so the sum is the same sequence
+      // of roundings as one thread's. With one chunk of ids and positions in
+      // flight and a rolled loop a chunk took 1.1 us (R-MAT, 65,536 nodes: pass
+      // 73 us, now 49; 262,144 nodes 116 -> 102, 1 M 262 -> 252).
       const uint32_t mi = (blockIdx.x - P.n_hubs) * (ATT_THREADS / 32) + w;
       if (mi < P.n_med) {
         const uint32_t i0 = order[P.n_hubs + mi];
@@ -1488,25 +1543,28 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
         const float4 fr = frep[i];
         float fx = fr.x, fy = fr.y, fz = fr.z;
         const uint32_t e0 = off[i], e1 = off[i + 1];
-        auto gather = [&](uint32_t k) {
-          const uint32_t u = __ldg(nbr + k);
-          return JC_IN_BOUNDS(u, P.n, &st->error) ? __ldg(pos + u) : pi;
-        };
-        float4 q = e0 + lane < e1 ? gather(e0 + lane) : pi;
+        // ids two chunks ahead, positions one ahead of the chunk being added
+        auto id_at = [&](uint32_t k) { return k < e1 ? __ldg(nbr + k) : i; };
+        auto gather = [&](uint32_t u) { return JC_IN_BOUNDS(u, P.n, &st->error) ? __ldg(pos + u) : pi; };
+        uint32_t id = id_at(e0 + lane);
+        float4 q = gather(id);
+        id = id_at(e0 + 32 + lane);
         for (uint32_t base = e0; base < e1; base += 32) {
           const float4 cur = q;
-          const uint32_t nk = base + 32 + lane;
-          if (base + 32 < e1) q = nk < e1 ? gather(nk) : pi;
+          q = gather(id);
+          id = id_at(base + 64 + lane);
           float tx = -0.0f, ty = -0.0f, tz = -0.0f;  // -0 + term = term, signed zeros included
           att_term(cur, pi, P, tx, ty, tz);
-          const uint32_t cnt = min(32u, e1 - base);
-          for (uint32_t l = 0; l < cnt; ++l) {
-            const float ax = __shfl_sync(0xFFFFFFFFu, tx, l);
-            const float ay = __shfl_sync(0xFFFFFFFFu, ty, l);
-            const float az = __shfl_sync(0xFFFFFFFFu, tz, l);
-            fx = __fadd_rn(fx, ax);
-            fy = __fadd_rn(fy, ay);
-            fz = __fadd_rn(fz, az);
+          auto add = [&](uint32_t l) {
+            fx = __fadd_rn(fx, __shfl_sync(0xFFFFFFFFu, tx, l));
+            fy = __fadd_rn(fy, __shfl_sync(0xFFFFFFFFu, ty, l));
+            fz = __fadd_rn(fz, __shfl_sync(0xFFFFFFFFu, tz, l));
+          };
+          if (base + 32 <= e1) {
+#pragma unroll
+            for (uint32_t l = 0; l < 32; ++l) add(l);
+          } else {
+            for (uint32_t l = 0; l < e1 - base; ++l) add(l);
           }
         }
         if (lane == 0) {
@@ -1945,7 +2003,7 @@ class Fa2Engine : public Engine {
       n_hubs_ = 0;
       while (n_hubs_ < n && lo[order[n_hubs_] + 1] - lo[order[n_hubs_]] >= hub_threshold_) ++n_hubs_;
       n_med_ = 0;
-      const uint32_t warp_thr = s_.warp_threshold ? s_.warp_threshold : DEFAULT_WARP_THRESHOLD;
+      const uint32_t warp_thr = s_.warp_threshold ? s_.warp_threshold : default_warp_threshold(n);
       while (n_hubs_ + n_med_ < n && lo[order[n_hubs_ + n_med_] + 1] - lo[order[n_hubs_ + n_med_]] >= warp_thr)
         ++n_med_;
       n_att_ = lo[n];
@@ -2674,7 +2732,12 @@ class Fa2Engine : public Engine {
       return;
     }
     switch (walk_group_) {
-      case 1: k_walk_rope<FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
+      case 1:
+        if (forest_.n_graphs == 1 && n <= WALK_AHEAD_N) {
+          k_walk_ahead<FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p);
+          break;
+        }
+        k_walk_rope<FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
       case 2: k_walk<2, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
       case 4: k_walk<4, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
       case 8: k_walk<8, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
@@ -3175,7 +3238,7 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   k_clear<<<std::min<uint32_t>(cdiv(NOALLOC_TREE_CAP, 256), 1184), 256, 0, s>>>(first, n, P, st, nchild, arrive);
   k_fill<<<cdiv(n, 256), 256, 0, s>>>(hi, X, val, first, pos4, degf, n, P, st, nodes, parent, nchild, F1);
   k_com<<<cdiv(n, 256), 256, 0, s>>>(first, nodes, parent, nchild, arrive, n, st);
-  k_walk_rope<false><<<cdiv(n, WALK_THREADS), WALK_THREADS, 0, s>>>(nodes, val, pos4, degf, n, P, st, frep, F1);
+  k_walk_ahead<false><<<cdiv(n, WALK_THREADS), WALK_THREADS, 0, s>>>(nodes, val, pos4, degf, n, P, st, frep);
   k_att<<<cdiv(n, ATT_THREADS), ATT_THREADS, 0, s>>>(order, d_offsets, d_neighbors, pos4, frep, old4, degf, P, st,
                                                     force4, stats, partials, 1u);
   k_pack_xyz<<<cdiv(n, 256), 256, 0, s>>>(force4, n, d_forces_xyz);

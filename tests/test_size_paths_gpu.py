@@ -173,3 +173,37 @@ def test_pair_batches_bit_exact(jc, orc, n, batches, sweeps):
     o = orc.Sgd(g, pos, mode=2, scatter_batches=batches, **s)
     for _ in range(3):
         assert np.array_equal(bits(e.step()), bits(o.step()))
+
+
+def one_step(jc, orc, g, pos, **settings):
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params(settings)
+    e.init(g, pos)
+    e.step()
+    o = orc.Fa2(g, pos, bh=True, **{k: v for k, v in settings.items() if k not in ("hub_threshold", "warp_threshold")})
+    o.step()
+    return e, o.get()
+
+
+# attraction lists at the edges of the warp path (32 entries here, whole and
+# partial chunks of 32), as the graph's size chooses it
+@pytest.mark.parametrize("leaves,lin_log", [(k, False) for k in (30, 31, 32, 33, 63, 64, 65, 96, 97, 500)]
+                         + [(33, True), (97, True)])
+def test_attraction_list_lengths_bit_exact(jc, orc, leaves, lin_log):
+    g = star(jc, leaves, leaves // 2)
+    e, r = one_step(jc, orc, g, jc.seed_uniform(g.n_nodes, 3, leaves), theta=0.7, lin_log_mode=lin_log)
+    f, st = e.forces()
+    if lin_log:  # logf against the host's: one ulp of a term
+        assert np.linalg.norm(f - r["force"]) <= 1e-6 * np.linalg.norm(r["force"])
+    else:
+        assert np.array_equal(bits(f), bits(r["force"])) and np.array_equal(bits(st), bits(r["stats"]))
+
+
+# both sides of the walk's size rule (151,552) and of the list-length rule
+# (32,768 and 196,608)
+@pytest.mark.parametrize("n", [32768, 32769, 151552, 151553, 196608, 196609])
+def test_walk_and_list_size_rules_bit_exact(jc, orc, n):
+    g = jc.gen_scale_free(n, 2, n)
+    e, r = one_step(jc, orc, g, jc.seed_uniform(n, 3, 1), theta=0.9, hub_threshold=1 << 30)
+    f, _ = e.forces()
+    assert np.array_equal(bits(f), bits(r["force"]))
