@@ -17,9 +17,9 @@
 //               `c +/- half*0.5` (fa2_bh.rs:841-861). Packed as a 96-bit key
 //               (levels 0..20 in 63 bits, 21..31 in 33 bits). Bodies with a
 //               non-finite coordinate get bit 63 and sort last.
-//   radix sort  stable LSD over the 64-bit high key (8 passes). If two valid
-//               keys tie in those 21 levels, a device-gated re-sort by the
-//               low 33 bits then the high 64 bits restores full order.
+//   radix sort  stable LSD over the top 32 (batches 48) key bits; runs of equal
+//               tops are sorted one thread each, and if one is too long for
+//               that k_tie_resort restores the full 96-bit order.
 //   k_count     per sorted body: the number of octree nodes whose pre-order
 //               run starts at it. The reference's pointer octree (split a cell
 //               while it holds >= 2 bodies, one node per level, depth cap 32)
@@ -153,6 +153,7 @@ struct DevState {
   uint32_t bbox_done;
   uint32_t att_done;
   uint32_t steps_done;
+  uint32_t tie_bar;  // arrivals at the full re-sort's grid barriers this step
   uint32_t n_top;  // nodes of depth <= TOP_DEPTH listed this step (single graph)
   unsigned long long n_inter;
   unsigned long long n_open;
@@ -285,6 +286,7 @@ k_bbox(const float4* __restrict__ pos, uint32_t n, float* __restrict__ part, Dev
   st->n_top = 0;
   st->n_invalid = 0;
   st->tie = 0;
+  st->tie_bar = 0;
   st->max_depth = 0;
   st->dropped = 0;
   st->n_inter = 0;
@@ -418,6 +420,125 @@ k_seg_fix(uint64_t* __restrict__ hi, uint32_t* __restrict__ val, const uint64_t*
   for (uint32_t i = 0; i < len; ++i) {
     hi[a + i] = k[i];
     val[a + i] = v[i];
+  }
+}
+
+// The full 96-bit re-sort of the permutation, stable (equal keys keep their
+// order, which is body order), when k_seg_fix found a run it does not take: an
+// LSD radix sort of `val` by the low word's bytes and then the high word's,
+// keys read through the permutation, all passes in this one launch. A step
+// without ties (nearly every one) pays one launch that returns at once; as a
+// conditional graph node the passes cost 15 us of every step, and as gated
+// launches (no graph) 18 of them. Block b owns the b-th contiguous part of the
+// permutation; a pass counts its digits, a grid barrier later every block adds
+// up its offsets and scatters in order, and a second barrier ends the pass. The
+// barriers need every block resident (a cooperative launch) and their waits are
+// bounded: past the limit the error word is set and the block leaves. B200, us
+// a step against the conditional node: without ties 10,000 bodies 180 -> 166, 1 M
+// 1,194 -> 1,183; with them 10,000 377 -> 320, 100,000 507 -> 432, 1 M 1,843 -> 1,874.
+constexpr int TIE_THREADS = 1024;
+constexpr uint32_t TIE_PART = 2048;           // bodies per block, up to one block per SM
+constexpr uint32_t TIE_SPIN_LIMIT = 1u << 22;  // seconds of polling
+__device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target) {
+  __shared__ bool ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ok = true;
+    __threadfence();
+    atomicAdd(&st->tie_bar, 1u);
+    uint32_t spins = 0, seen;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&st->tie_bar) : "memory");
+      if (seen < target && ++spins > TIE_SPIN_LIMIT) {
+        set_error(st, JC_ERR_DEVICE_TIMEOUT);
+        ok = false;
+        break;
+      }
+    } while (seen < target);
+  }
+  __syncthreads();
+  return ok;
+}
+
+__global__ void __launch_bounds__(TIE_THREADS)
+k_tie_resort(const uint64_t* __restrict__ hi_orig, const uint64_t* __restrict__ lo_orig, uint32_t* val,
+             uint32_t* val_alt, uint64_t* __restrict__ hi_sorted, uint32_t n, int lo_passes, DevState* st,
+             uint32_t* table) {
+  if (st->tie == 0u) return;
+  __shared__ uint32_t wcnt[TIE_THREADS / 32][256];
+  __shared__ uint32_t base[256];
+  __shared__ uint32_t sh[32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, G = gridDim.x;
+  const uint32_t per = (n + G - 1) / G;
+  const uint32_t b0 = min(n, blockIdx.x * per), b1 = min(n, b0 + per);
+  const uint32_t lt = (1u << lane) - 1u;
+  uint32_t bars = 0;
+  uint32_t *src = val, *dst = val_alt;
+  for (int pass = 0; pass < lo_passes + 8; ++pass) {
+    const uint64_t* key = pass < lo_passes ? lo_orig : hi_orig;
+    const int shift = 8 * (pass < lo_passes ? pass : pass - lo_passes);
+    auto digit = [&](uint32_t v) { return JC_IN_BOUNDS(v, n, &st->error) ? (uint32_t)(key[v] >> shift) & 0xFFu : 0u; };
+    if (tid < 256) base[tid] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = b0 + tid; i < b1; i += TIE_THREADS) atomicAdd(&base[digit(__ldcg(src + i))], 1u);
+    __syncthreads();
+    if (tid < 256) __stcg(table + (size_t)tid * G + blockIdx.x, base[tid]);
+    bars += G;
+    if (!tie_barrier(st, bars)) return;
+    // four lanes per digit add up the blocks' counts, loads in flight
+    uint32_t tot = 0, pre = 0, all;
+    const uint32_t dg = tid >> 2;
+#pragma unroll 8
+    for (uint32_t g = tid & 3; g < G; g += 4) {
+      const uint32_t c = __ldcg(table + (size_t)dg * G + g);
+      pre += g < blockIdx.x ? c : 0u;
+      tot += c;
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      tot += __shfl_xor_sync(0xFFFFFFFFu, tot, o);
+      pre += __shfl_xor_sync(0xFFFFFFFFu, pre, o);
+    }
+    const uint32_t ex = dev::block_excl_scan((tid & 3) == 0 ? tot : 0u, &all, sh);
+    if ((tid & 3) == 0) base[dg] = ex + pre;
+    uint32_t nv = b0 + tid < b1 ? __ldcg(src + b0 + tid) : 0u, nd = b0 + tid < b1 ? digit(nv) : 256u;
+    for (uint32_t c0 = b0; c0 < b1; c0 += TIE_THREADS) {
+      const uint32_t i = c0 + tid, v = nv, d = nd;  // the next chunk's are in flight meanwhile
+      const bool in = i < b1, more = i + TIE_THREADS < b1;
+      nv = more ? __ldcg(src + i + TIE_THREADS) : 0u;
+      nd = more ? digit(nv) : 256u;
+      for (uint32_t k = tid; k < (TIE_THREADS / 32) * 256; k += TIE_THREADS) (&wcnt[0][0])[k] = 0;
+      __syncthreads();
+      const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+      if (in && (int)lane == __ffs(peers) - 1) wcnt[w][d] = (uint32_t)__popc(peers);
+      __syncthreads();
+      if (tid < 256) {
+        uint32_t run = base[tid];
+        for (int q = 0; q < TIE_THREADS / 32; ++q) {
+          const uint32_t c = wcnt[q][tid];
+          wcnt[q][tid] = run;
+          run += c;
+        }
+        base[tid] = run;
+      }
+      __syncthreads();
+      if (in) {
+        const uint32_t to = wcnt[w][d] + (uint32_t)__popc(peers & lt);
+        if (to < n) __stcg(dst + to, v);
+      }
+      __syncthreads();
+    }
+    bars += G;
+    if (!tie_barrier(st, bars)) return;
+    uint32_t* t = src;
+    src = dst;
+    dst = t;
+  }
+  for (uint32_t i = b0 + tid; i < b1; i += TIE_THREADS) {
+    const uint32_t v = __ldcg(src + i);
+    val[i] = v;
+    hi_sorted[i] = JC_IN_BOUNDS(v, n, &st->error) ? hi_orig[v] : 0ull;
   }
 }
 
@@ -1137,11 +1258,6 @@ k_walk_top(const TNode* __restrict__ nodes, const uint4* __restrict__ top, const
   walk_counts_flush(n_inter, n_open, st);
 }
 
-// Sets the graph condition that runs the full 96-bit re-sort.
-__global__ void k_set_tie_condition(cudaGraphConditionalHandle h, const DevState* st) {
-  cudaGraphSetConditional(h, st->tie ? 1u : 0u);
-}
-
 __device__ void speed_update(DevState* st, uint32_t n, float jitter_tolerance, double ts, double tt);
 
 // ------------------------------------------------------ batch kernels --
@@ -1230,6 +1346,7 @@ k_bbox_roots(Forest F, DevState* st) {
   if (g == 0) {
     st->n_invalid = 0;
     st->tie = 0;
+    st->tie_bar = 0;
     st->max_depth = 0;
     st->dropped = 0;
     st->n_inter = 0;
@@ -1850,6 +1967,24 @@ __global__ void k_csr_balance(const int* __restrict__ balance, uint32_t* ok) {
   }
 }
 
+inline uint32_t tie_blocks(uint32_t n, uint32_t sms) { return std::max(1u, std::min(sms, cdiv(n, TIE_PART))); }
+
+inline void launch_tie_resort(const uint64_t* hi_orig, const uint64_t* lo_orig, uint32_t* val, uint32_t* val_alt,
+                              uint64_t* hi_sorted, uint32_t n, int lo_passes, DevState* st, uint32_t* table,
+                              uint32_t sms, cudaStream_t s) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tie_blocks(n, sms));
+  cfg.blockDim = dim3(TIE_THREADS);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = cfg.gridDim.x > 1 ? 1 : 0;
+  JC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_tie_resort, hi_orig, lo_orig, val, val_alt, hi_sorted, n, lo_passes, st,
+                                   table));
+}
+
 class Fa2Engine : public Engine {
  public:
   explicit Fa2Engine(bool bh) : bh_(bh) {
@@ -2421,6 +2556,7 @@ class Fa2Engine : public Engine {
   jc_descriptor desc_{};
   Fa2Settings s_;
   uint32_t n_ = 0, n_att_ = 0, n_hubs_ = 0, n_med_ = 0, hub_threshold_ = DEFAULT_HUB_THRESHOLD, att_blocks_ = 0;
+  uint32_t sms_ = 1;
   uint32_t tree_cap_ = 0, sort_tiles_ = 0, scan_tiles_ = 0;
   uint32_t walk_group_ = DEFAULT_WALK_GROUP;
   uint32_t launches_ = 0;
@@ -2447,7 +2583,6 @@ class Fa2Engine : public Engine {
   // yet (the staged upload checks them); the other entry points validate first
   bool ids_checked_ = true;
   cudaStream_t stream_ = nullptr;
-  cudaStream_t side_ = nullptr;  // captures the conditional re-sort body
   cudaStream_t copy_ = nullptr;  // frame-stream copies (overlapping the steps)
   uint32_t* ok_host_ = nullptr;  // page-locked word: the device CSR check's verdict
   DevBuf<uint32_t> okb_;
@@ -2463,8 +2598,8 @@ class Fa2Engine : public Engine {
   DevBuf<DevState> state_;
   DevBuf<double2> partials_;
   // tree
-  DevBuf<uint64_t> hi_orig_, lo_orig_, hi_, hi_alt_, lo_, lo_alt_;
-  DevBuf<uint32_t> val_, val_alt_, sort_work_, sort_work2_, count_, first_, scan_sums_;
+  DevBuf<uint64_t> hi_orig_, lo_orig_, hi_, hi_alt_, lo_;
+  DevBuf<uint32_t> val_, val_alt_, sort_work_, tie_table_, count_, first_, scan_sums_;
   DevBuf<int8_t> lcp_;  // prefix-length index: L, m1, m2 back to back
   LcpIndex lcpx_{};
   DevBuf<TNode> nodes_;
@@ -2488,7 +2623,10 @@ class Fa2Engine : public Engine {
       if (cudaGetDeviceCount(&dev_count) != cudaSuccess || dev_count == 0)
         fail(JC_ERR_CUDA, "no CUDA device is available");
       stream_ = StreamCache::instance().take();
-      side_ = StreamCache::instance().take();
+      int dev = 0, sms = 0;
+      JC_CUDA_CHECK(cudaGetDevice(&dev));
+      JC_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      sms_ = (uint32_t)sms;
       copy_ = StreamCache::instance().take();
       for (auto& e : ev_) JC_CUDA_CHECK(cudaEventCreate(&e));
       static_assert(sizeof(DevState) <= SmallPinned::kSlot, "state mirror fits a small page-locked block");
@@ -2552,11 +2690,11 @@ class Fa2Engine : public Engine {
     // short of deep coincident clusters, which report JC_ERR_CAPACITY and
     // grow the buffers before the step is retried.
     tree_cap_ = std::max<uint32_t>(tree_cap_, 3 * n + 64);
-    hi_orig_.alloc(n); lo_orig_.alloc(n); hi_.alloc(n); hi_alt_.alloc(n); lo_.alloc(n); lo_alt_.alloc(n);
+    hi_orig_.alloc(n); lo_orig_.alloc(n); hi_.alloc(n); hi_alt_.alloc(n); lo_.alloc(n);
     val_.alloc(n); val_alt_.alloc(n);
     sort_tiles_ = dev::rs_tiles(std::max<uint32_t>(n, 1));
     sort_work_.alloc(dev::sort_work_words(std::max<uint32_t>(n, 1), 8));
-    sort_work2_.alloc(dev::sort_work_words(std::max<uint32_t>(n, 1), 8));
+    tie_table_.alloc(256 * (size_t)tie_blocks(n, sms_));
     count_.alloc((size_t)n + 1);
     first_.alloc((size_t)n + 2);
     scan_tiles_ = std::max<uint32_t>(1, cdiv(n, dev::SC_TILE));
@@ -2582,10 +2720,8 @@ class Fa2Engine : public Engine {
       for (auto& e : ev_)
         if (e) cudaEventDestroy(e);
       StreamCache::instance().give(stream_);
-      StreamCache::instance().give(side_);
       StreamCache::instance().give(copy_);
       stream_ = nullptr;
-      side_ = nullptr;
       copy_ = nullptr;
     }
     SmallPinned::instance().give(hst_);
@@ -2657,7 +2793,9 @@ class Fa2Engine : public Engine {
         k_seg_fix<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, lo_orig_.p, n, st, split);
         ++L;
       }
-      L += enqueue_tie_resort(st);
+      launch_tie_resort(hi_orig_.p, lo_orig_.p, val_.p, val_alt_.p, hi_.p, n, (3 * (32 - F.lh) + 7) / 8, st,
+                        tie_table_.p, sms_, stream_);
+      ++L;
       k_gather_u64<<<cdiv(n, 256), 256, 0, stream_>>>(lo_orig_.p, val_.p, lo_.p, st, nullptr, n);
       k_count<<<lcpx_.n2, COUNT_THREADS, 0, stream_>>>(hi_.p, lo_.p, n, st, count_.p, F, lcpx_);
       L += 2;
@@ -2749,60 +2887,6 @@ class Fa2Engine : public Engine {
   void launch_walk(const KParams& P, DevState* st) {
     if (s_.fast_repulsion) launch_walk_mode<true>(P, st);
     else launch_walk_mode<false>(P, st);
-  }
-
-  // Rare path (two valid keys tie in their first 21 levels): a conditional
-  // IF node whose body re-sorts by the low 33 bits and then the high 64 bits,
-  // giving the full 96-bit order. A one-thread kernel sets the condition
-  // from the device tie flag, so the body costs nothing when it is not taken.
-  int enqueue_tie_resort(DevState* st) {
-    const uint32_t n = n_;
-    if (!s_.use_graph) {
-      // Eager launches: the same kernels, each returning at once unless the
-      // device tie flag is set.
-      const uint32_t* gate = &st->tie;
-      const uint32_t* nvalid = &st->n_valid;
-      k_gather_u64<<<cdiv(n, 256), 256, 0, stream_>>>(lo_orig_.p, val_.p, lo_.p, st, gate, n);
-      int L = 1 + dev::radix_sort_pairs<uint64_t>(lo_.p, val_.p, lo_alt_.p, val_alt_.p, n, nvalid, 0, 33,
-                                                  sort_work2_.p, &st->error, gate, stream_);
-      k_gather_u64<<<cdiv(n, 256), 256, 0, stream_>>>(hi_orig_.p, val_.p, hi_.p, st, gate, n);
-      L += 1 + dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nvalid, 0, 64,
-                                               sort_work2_.p, &st->error, gate, stream_);
-      return L;
-    }
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t cg;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t nd = 0;
-    JC_CUDA_CHECK(cudaStreamGetCaptureInfo(stream_, &cs, nullptr, &cg, &deps, &nd));
-    if (cs != cudaStreamCaptureStatusActive) fail(JC_ERR_CUDA, "the step must be enqueued under stream capture");
-    cudaGraphConditionalHandle h;
-    JC_CUDA_CHECK(cudaGraphConditionalHandleCreate(&h, cg, 0, cudaGraphCondAssignDefault));
-    k_set_tie_condition<<<1, 1, 0, stream_>>>(h, st);
-    JC_CUDA_CHECK(cudaGetLastError());
-    JC_CUDA_CHECK(cudaStreamGetCaptureInfo(stream_, &cs, nullptr, &cg, &deps, &nd));
-    alignas(cudaGraphNodeParams) unsigned char cp_storage[sizeof(cudaGraphNodeParams)] = {};
-    cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(cp_storage);
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    JC_CUDA_CHECK(cudaGraphAddNode(&cnode, cg, deps, nd, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    JC_CUDA_CHECK(cudaStreamUpdateCaptureDependencies(stream_, &cnode, 1, cudaStreamSetCaptureDependencies));
-    JC_CUDA_CHECK(cudaStreamBeginCaptureToGraph(side_, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    const uint32_t* nvalid = &st->n_valid;
-    k_gather_u64<<<cdiv(n, 256), 256, 0, side_>>>(lo_orig_.p, val_.p, lo_.p, st, nullptr, n);
-    dev::radix_sort_pairs<uint64_t>(lo_.p, val_.p, lo_alt_.p, val_alt_.p, n, nvalid, 0, 33, sort_work2_.p,
-                                    &st->error, nullptr, side_);
-    k_gather_u64<<<cdiv(n, 256), 256, 0, side_>>>(hi_orig_.p, val_.p, hi_.p, st, nullptr, n);
-    dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nvalid, 0, 64, sort_work2_.p,
-                                    &st->error, nullptr, side_);
-    JC_CUDA_CHECK(cudaGetLastError());
-    cudaGraph_t captured;
-    JC_CUDA_CHECK(cudaStreamEndCapture(side_, &captured));
-    return 2;  // the condition kernel and the conditional node
   }
 
   // Phase boundary events: plain records when the kernels are launched one
@@ -3040,8 +3124,8 @@ constexpr uint32_t NOALLOC_LCP = NOALLOC_MAX_NODES;  // prefix-length index byte
 __host__ __device__ constexpr size_t na_round(size_t b) { return (b + 255) & ~(size_t)255; }
 
 struct NoAllocLayout {
-  size_t st, bbox, pos4, frep, force4, old4, degf, stats, order, hi_orig, lo_orig, hi, hi_alt, lo, lo_alt, val,
-      val_alt, count, first, sums, work, work2, partials, nodes, parent, nchild, arrive, lcp, total;
+  size_t st, bbox, pos4, frep, force4, old4, degf, stats, order, hi_orig, lo_orig, hi, hi_alt, lo, val,
+      val_alt, count, first, sums, work, table, partials, nodes, parent, nchild, arrive, lcp, total;
 };
 
 constexpr NoAllocLayout noalloc_layout() {
@@ -3062,14 +3146,13 @@ constexpr NoAllocLayout noalloc_layout() {
   L.hi = o; o += na_round(8 * N);
   L.hi_alt = o; o += na_round(8 * N);
   L.lo = o; o += na_round(8 * N);
-  L.lo_alt = o; o += na_round(8 * N);
   L.val = o; o += na_round(4 * N);
   L.val_alt = o; o += na_round(4 * N);
   L.count = o; o += na_round(4 * (N + 1));
   L.first = o; o += na_round(4 * (N + 2));
   L.sums = o; o += na_round(4 * (N / dev::SC_TILE + 2));
   L.work = o; o += na_round(4 * dev::sort_work_words((uint32_t)N, 8));
-  L.work2 = o; o += na_round(4 * dev::sort_work_words((uint32_t)N, 8));
+  L.table = o; o += na_round(4 * 256 * 16);
   L.partials = o; o += na_round(sizeof(double2) * (N / ATT_THREADS + 1));
   L.nodes = o; o += na_round(sizeof(TNode) * C);
   L.parent = o; o += na_round(4 * C);
@@ -3175,14 +3258,13 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   uint64_t* hi = (uint64_t*)(base + L.hi);
   uint64_t* hi_alt = (uint64_t*)(base + L.hi_alt);
   uint64_t* lo = (uint64_t*)(base + L.lo);
-  uint64_t* lo_alt = (uint64_t*)(base + L.lo_alt);
   uint32_t* val = (uint32_t*)(base + L.val);
   uint32_t* val_alt = (uint32_t*)(base + L.val_alt);
   uint32_t* count = (uint32_t*)(base + L.count);
   uint32_t* first = (uint32_t*)(base + L.first);
   uint32_t* sums = (uint32_t*)(base + L.sums);
   uint32_t* work = (uint32_t*)(base + L.work);
-  uint32_t* work2 = (uint32_t*)(base + L.work2);
+  uint32_t* table = (uint32_t*)(base + L.table);
   double2* partials = (double2*)(base + L.partials);
   TNode* nodes = (TNode*)(base + L.nodes);
   uint32_t* parent = (uint32_t*)(base + L.parent);
@@ -3226,12 +3308,12 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   k_keys<<<cdiv(n, 256), 256, 0, s>>>(pos4, n, st, hi_orig, lo_orig, hi, val, F1);
   dev::radix_sort_pairs<uint64_t>(hi, val, hi_alt, val_alt, n, nullptr, 32, 64, work, &st->error, nullptr, s);
   k_seg_fix<<<cdiv(n, 256), 256, 0, s>>>(hi, val, lo_orig, n, st, 32);
-  // ties in the first 21 levels: full 96-bit order, gated on the device flag
-  const uint32_t* gate = &st->tie;
-  k_gather_u64<<<cdiv(n, 256), 256, 0, s>>>(lo_orig, val, lo, st, gate, n);
-  dev::radix_sort_pairs<uint64_t>(lo, val, lo_alt, val_alt, n, &st->n_valid, 0, 33, work2, &st->error, gate, s);
-  k_gather_u64<<<cdiv(n, 256), 256, 0, s>>>(hi_orig, val, hi, st, gate, n);
-  dev::radix_sort_pairs<uint64_t>(hi, val, hi_alt, val_alt, n, &st->n_valid, 0, 64, work2, &st->error, gate, s);
+  // (at most 16 blocks: below the SM count of any device this library runs on)
+  try {
+    launch_tie_resort(hi_orig, lo_orig, val, val_alt, hi, n, 5, st, table, 16, s);
+  } catch (const Error&) {
+    return JC_ERR_CUDA;
+  }
   k_gather_u64<<<cdiv(n, 256), 256, 0, s>>>(lo_orig, val, lo, st, nullptr, n);
   k_count<<<X.n2, COUNT_THREADS, 0, s>>>(hi, lo, n, st, count, F1, X);
   dev::exclusive_scan(count, first, n, sums, s);

@@ -207,3 +207,51 @@ def test_walk_and_list_size_rules_bit_exact(jc, orc, n):
     e, r = one_step(jc, orc, g, jc.seed_uniform(n, 3, 1), theta=0.9, hub_threshold=1 << 30)
     f, _ = e.forces()
     assert np.array_equal(bits(f), bits(r["force"]))
+
+
+def crowded(jc, n, far, seed):
+    """A layout whose bodies share the first ten octant levels: a unit cube and
+    a body at distance `far`; every third body on a coarse lattice, so keys tie
+    in the high word too and whole keys repeat."""
+    pos = jc.seed_uniform(n, 3, seed)
+    k = np.arange(1, n, 3)
+    for c in range(3):
+        pos[3 * k + c] = np.round(pos[3 * k + c] * 16) / np.float32(16)
+    pos[:3] = far
+    return pos
+
+
+# the one-launch re-sort: a single block, one block's last part, several blocks
+# with barriers (2,048 bodies each), graph replays and plain launches
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("n", [40, 2048, 2049, 6143, 30001])
+def test_long_runs_resort_bit_exact(jc, orc, n, use_graph):
+    g = jc.gen_scale_free(n, 2, n)
+    pos = crowded(jc, n, 3.0e4, 5)
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params({"theta": 0.8, "use_graph": use_graph, "hub_threshold": 1 << 30})
+    e.init(g, pos)
+    o = orc.Fa2(g, pos, bh=True, theta=0.8)
+    for _ in range(2):
+        e.step()
+        o.step()
+        r = o.get()
+        assert e.tree_info()["nodes"] > 0
+        assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
+        assert np.array_equal(bits(e.positions()), bits(r["pos"]))
+
+
+def test_long_runs_resort_in_a_batch(jc):
+    graphs = [jc.gen_scale_free(n, 2, n) for n in (3000, 50, 2500)]
+    pos = [crowded(jc, g.n_nodes, 2.0e5, 9) for g in graphs]
+    b = jc.LayoutEngine("fa2-bh")
+    b.set_params({"theta": 0.8})
+    b.init_batch(graphs, pos)
+    out = b.step_many(3)
+    at = 0
+    for g, p in zip(graphs, pos):
+        e = jc.LayoutEngine("fa2-bh")
+        e.set_params({"theta": 0.8})
+        e.init(g, p)
+        assert np.array_equal(bits(out[at:at + 3 * g.n_nodes]), bits(e.step_many(3)))
+        at += 3 * g.n_nodes
