@@ -82,7 +82,8 @@ constexpr int ATT_THREADS = 256;
 
 constexpr int APPLY_THREADS = 256;
 constexpr int BBOX_THREADS = 256;
-constexpr int BBOX_BLOCKS = 296;  // 2 x 148 SMs
+constexpr int BBOX_BLOCKS = 296;  // 2 x 148 SMs, the most; small graphs take a block per 1,024 bodies
+inline uint32_t bbox_blocks(uint32_t n) { return std::min<uint32_t>(BBOX_BLOCKS, std::max(1u, (n + 1023u) / 1024u)); }
 constexpr uint32_t DEFAULT_HUB_THRESHOLD = 2048;
 // Lists at least this long (and below the hub threshold) are gathered by a
 // whole warp, 32 neighbours at a time, and summed in list order by lane 0: a
@@ -217,7 +218,11 @@ __device__ __forceinline__ void set_error(DevState* st, uint32_t code) { atomicC
 
 // --------------------------------------------------------------- bbox --
 __global__ void __launch_bounds__(BBOX_THREADS)
-k_bbox(const float4* __restrict__ pos, uint32_t n, float* __restrict__ part, DevState* st) {
+k_bbox(const float4* __restrict__ pos, uint32_t n, float* __restrict__ part, DevState* st,
+       uint32_t* __restrict__ sort_work, uint32_t sort_words) {
+  // (the sort's digit counts, tile counters and look-back words start at zero)
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < sort_words; i += gridDim.x * blockDim.x)
+    sort_work[i] = 0u;
   float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     float4 p = pos[i];
@@ -294,75 +299,120 @@ k_bbox(const float4* __restrict__ pos, uint32_t n, float* __restrict__ part, Dev
 }
 
 // --------------------------------------------------------------- keys --
-__global__ void __launch_bounds__(256)
-k_keys(const float4* __restrict__ pos, uint32_t n, DevState* st, uint64_t* __restrict__ hi_orig,
-       uint64_t* __restrict__ lo_orig, uint64_t* __restrict__ hi_sort, uint32_t* __restrict__ val, Forest F) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool invalid = false;
-  if (i < n) {
-    float4 p = pos[i];
-    uint64_t hi = 0, lo = 0;
-    if (isfinite(p.x) && isfinite(p.y) && isfinite(p.z)) {
-      const uint32_t g = F.node_graph ? F.node_graph[i] : 0u;
-      float cx, cy, cz, h;
-      uint64_t zf = 0;
-      if (F.n_graphs > 1) {
-        const float4 r = F.roots[g];
-        cx = r.x; cy = r.y; cz = r.z; h = r.w;
-        zf = F.zflat[g];
-      } else {
-        cx = st->root[0]; cy = st->root[1]; cz = st->root[2]; h = st->root[3];
-      }
-      const int lh = F.lh < 32 ? F.lh : 32;
-      if (zf >> 32) {
-        // every body of this graph has the same z: its z bits are the graph's
-        auto level = [&](uint64_t& w, int l) {
-          const uint32_t o = (p.x >= cx ? 1u : 0u) | (p.y >= cy ? 2u : 0u) | ((uint32_t)(zf >> l) & 1u) << 2;
-          w = (w << 3) | o;
-          const float hh = __fmul_rn(h, 0.5f);
-          cx = __fadd_rn(cx, (o & 1u) ? hh : -hh);
-          cy = __fadd_rn(cy, (o & 2u) ? hh : -hh);
-          h = hh;
-        };
-        int l = 0;
+// The octant digits of levels 0..31 of one finite position: levels [0, lh)
+// into hi, the rest into lo (two loops instead of a per-level choice of the
+// word). zf: the graph's z digits when all its bodies share them (see Forest).
+__device__ __forceinline__ void body_key(const float4 p, float cx, float cy, float cz, float h, uint64_t zf, int lh,
+                                         uint64_t& hi, uint64_t& lo) {
+  if (zf >> 32) {
+    // every body of this graph has the same z: its z bits are the graph's
+    auto level = [&](uint64_t& w, int l) {
+      const uint32_t o = (p.x >= cx ? 1u : 0u) | (p.y >= cy ? 2u : 0u) | ((uint32_t)(zf >> l) & 1u) << 2;
+      w = (w << 3) | o;
+      const float hh = __fmul_rn(h, 0.5f);
+      cx = __fadd_rn(cx, (o & 1u) ? hh : -hh);
+      cy = __fadd_rn(cy, (o & 2u) ? hh : -hh);
+      h = hh;
+    };
+    int l = 0;
 #pragma unroll 4
-        for (; l < lh; ++l) level(hi, l);
+    for (; l < lh; ++l) level(hi, l);
 #pragma unroll 4
-        for (; l < 32; ++l) level(lo, l);
-      } else {
-        // levels [0, lh) into the high word, the rest into the low word: two
-        // loops instead of a per-level choice of the destination word
-        auto level = [&](uint64_t& w) {
-          const uint32_t o = (p.x >= cx ? 1u : 0u) | (p.y >= cy ? 2u : 0u) | (p.z >= cz ? 4u : 0u);
-          w = (w << 3) | o;
-          const float hh = __fmul_rn(h, 0.5f);
-          cx = __fadd_rn(cx, (o & 1u) ? hh : -hh);
-          cy = __fadd_rn(cy, (o & 2u) ? hh : -hh);
-          cz = __fadd_rn(cz, (o & 4u) ? hh : -hh);
-          h = hh;
-        };
-        int l = 0;
+    for (; l < 32; ++l) level(lo, l);
+  } else {
+    auto level = [&](uint64_t& w) {
+      const uint32_t o = (p.x >= cx ? 1u : 0u) | (p.y >= cy ? 2u : 0u) | (p.z >= cz ? 4u : 0u);
+      w = (w << 3) | o;
+      const float hh = __fmul_rn(h, 0.5f);
+      cx = __fadd_rn(cx, (o & 1u) ? hh : -hh);
+      cy = __fadd_rn(cy, (o & 2u) ? hh : -hh);
+      cz = __fadd_rn(cz, (o & 4u) ? hh : -hh);
+      h = hh;
+    };
+    int l = 0;
 #pragma unroll 4
-        for (; l < lh; ++l) level(hi);
+    for (; l < lh; ++l) level(hi);
 #pragma unroll 4
-        for (; l < 32; ++l) level(lo);
-      }
-      hi <<= (63 - (int)F.gbits - 3 * F.lh);  // digits right under the graph id (no shift for one graph)
-      if (F.gbits) hi |= (uint64_t)g << (63 - F.gbits);
-    } else {
-      hi = 1ull << 63;
-      invalid = true;
-    }
-    hi_orig[i] = hi;
-    lo_orig[i] = lo;
-    hi_sort[i] = hi;
-    val[i] = i;
+    for (; l < 32; ++l) level(lo);
   }
-  uint32_t bal = __ballot_sync(0xFFFFFFFFu, invalid);
+}
+
+// Non-finite bodies of a warp into the counters.
+__device__ __forceinline__ void count_invalid(bool invalid, DevState* st) {
+  const uint32_t bal = __ballot_sync(0xFFFFFFFFu, invalid);
   if (bal && (threadIdx.x & 31) == 0) {
     atomicAdd(&st->n_invalid, (uint32_t)__popc(bal));
     atomicOr(&st->warn, JC_WARN_NONFINITE);
   }
+}
+
+// A single graph: the whole key (hi, lo) by body, its top 32 bits and the body
+// index for the sort, and the digit counts of the sort's four passes, which a
+// pass of its own read the keys again for. The sort moves 4-byte keys (8 bytes
+// a body and pass instead of 12, half the key registers). At most KEY_BLOCKS
+// blocks, so that few flush their counts.
+constexpr uint32_t KEY_BLOCKS = 148u * 8u;
+__global__ void __launch_bounds__(256)
+k_keys(const float4* __restrict__ pos, uint32_t n, DevState* st, ulonglong2* __restrict__ key,
+       uint32_t* __restrict__ top, uint32_t* __restrict__ val, uint32_t* __restrict__ counts) {
+  __shared__ uint32_t h[4][256];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) h[p][threadIdx.x] = 0;
+  __syncthreads();
+  const float cx = st->root[0], cy = st->root[1], cz = st->root[2], half = st->root[3];
+  for (uint32_t i0 = blockIdx.x * 256u; i0 < n; i0 += gridDim.x * 256u) {
+    const uint32_t i = i0 + threadIdx.x;
+    bool invalid = false;
+    if (i < n) {
+      const float4 p = pos[i];
+      uint64_t hi = 0, lo = 0;
+      if (isfinite(p.x) && isfinite(p.y) && isfinite(p.z)) {
+        body_key(p, cx, cy, cz, half, 0ull, 21, hi, lo);
+      } else {
+        hi = 1ull << 63;
+        invalid = true;
+      }
+      const uint32_t t = (uint32_t)(hi >> 32);
+      key[i] = make_ulonglong2(hi, lo);
+      top[i] = t;
+      val[i] = i;
+#pragma unroll
+      for (int p = 0; p < 4; ++p) atomicAdd(&h[p][(t >> (8 * p)) & 0xFFu], 1u);
+    }
+    count_invalid(invalid, st);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const uint32_t c = h[p][threadIdx.x];
+    if (c) atomicAdd(&counts[p * 256 + threadIdx.x], c);
+  }
+}
+
+// A batch: keys prefixed with the graph id.
+__global__ void __launch_bounds__(256)
+k_keys_batch(const float4* __restrict__ pos, uint32_t n, DevState* st, ulonglong2* __restrict__ key,
+             uint64_t* __restrict__ hi_sort, uint32_t* __restrict__ val, Forest F) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  bool invalid = false;
+  if (i < n) {
+    const float4 p = pos[i];
+    uint64_t hi = 0, lo = 0;
+    if (isfinite(p.x) && isfinite(p.y) && isfinite(p.z)) {
+      const uint32_t g = F.node_graph[i];
+      const float4 r = F.roots[g];
+      body_key(p, r.x, r.y, r.z, r.w, F.zflat[g], F.lh < 32 ? F.lh : 32, hi, lo);
+      hi <<= (63 - (int)F.gbits - 3 * F.lh);  // digits right under the graph id
+      hi |= (uint64_t)g << (63 - F.gbits);
+    } else {
+      hi = 1ull << 63;
+      invalid = true;
+    }
+    key[i] = make_ulonglong2(hi, lo);
+    hi_sort[i] = hi;
+    val[i] = i;
+  }
+  count_invalid(invalid, st);
 }
 
 // The tree sort orders the keys by their top bits only (a single graph: the
@@ -377,48 +427,67 @@ k_keys(const float4* __restrict__ pos, uint32_t n, DevState* st, uint64_t* __res
 // ordered without the full re-sort. A run longer than SEG_MAX sets the tie
 // flag instead, which sends the step through the full 96-bit re-sort.
 // Non-finite bodies (bit 63) sort last in any order.
+//
+// Sorted keys K: the top 32 bits alone (a single graph), or the high word (a
+// batch; its runs share the bits from `shift` up and are written back).
 constexpr uint32_t SEG_MAX = 32;
+__device__ __forceinline__ bool key_after(const ulonglong2 a, uint32_t va, const ulonglong2 b, uint32_t vb) {
+  return a.x > b.x || (a.x == b.x && (a.y > b.y || (a.y == b.y && va > vb)));
+}
+template <typename K>
 __global__ void __launch_bounds__(256)
-k_seg_fix(uint64_t* __restrict__ hi, uint32_t* __restrict__ val, const uint64_t* __restrict__ lo_orig, uint32_t n,
+k_seg_fix(K* __restrict__ sorted, uint32_t* __restrict__ val, const ulonglong2* __restrict__ key, uint32_t n,
           DevState* st, int shift) {
+  constexpr bool WORD = sizeof(K) == 8;
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a == 0) st->n_valid = n - st->n_invalid;  // valid bodies (the non-finite sort last)
   if (a >= n || st->error) return;
-  const uint64_t h = hi[a];
-  if (h >> 63) return;
-  const uint64_t top = h >> shift;
+  const K s = sorted[a];
+  if (s >> (8 * sizeof(K) - 1)) return;
+  const K top = s >> shift;
   // (runs only permute keys with equal top parts, so these reads are stable)
-  if (a > 0 && (hi[a - 1] >> shift) == top) return;  // not the first of its run
+  if (a > 0 && (sorted[a - 1] >> shift) == top) return;  // not the first of its run
   uint32_t len = 1;
-  while (a + len < n && len <= SEG_MAX && (hi[a + len] >> shift) == top) ++len;
+  while (a + len < n && len <= SEG_MAX && (sorted[a + len] >> shift) == top) ++len;
   if (len == 1) return;
   if (len > SEG_MAX) {
     st->tie = 1u;
     return;
   }
-  uint64_t k[SEG_MAX], l[SEG_MAX];
+  auto key_of = [&](uint32_t b) { return JC_IN_BOUNDS(b, n, &st->error) ? key[b] : make_ulonglong2(0ull, 0ull); };
+  if (len == 2) {  // most runs: no arrays
+    const uint32_t v0 = val[a], v1 = val[a + 1];
+    const ulonglong2 k0 = key_of(v0), k1 = key_of(v1);
+    if (key_after(k0, v0, k1, v1)) {
+      val[a] = v1;
+      val[a + 1] = v0;
+      if (WORD) {
+        sorted[a] = (K)k1.x;
+        sorted[a + 1] = (K)k0.x;
+      }
+    }
+    return;
+  }
+  ulonglong2 k[SEG_MAX];
   uint32_t v[SEG_MAX];
   for (uint32_t i = 0; i < len; ++i) {
-    k[i] = hi[a + i];
     v[i] = val[a + i];
-    l[i] = JC_IN_BOUNDS(v[i], n, &st->error) ? lo_orig[v[i]] : 0ull;
+    k[i] = key_of(v[i]);
   }
   for (uint32_t i = 1; i < len; ++i) {
-    const uint64_t kk = k[i], ll = l[i];
+    const ulonglong2 kk = k[i];
     const uint32_t vv = v[i];
     uint32_t j = i;
-    while (j > 0 && (k[j - 1] > kk || (k[j - 1] == kk && (l[j - 1] > ll || (l[j - 1] == ll && v[j - 1] > vv))))) {
+    while (j > 0 && key_after(k[j - 1], v[j - 1], kk, vv)) {
       k[j] = k[j - 1];
-      l[j] = l[j - 1];
       v[j] = v[j - 1];
       --j;
     }
     k[j] = kk;
-    l[j] = ll;
     v[j] = vv;
   }
   for (uint32_t i = 0; i < len; ++i) {
-    hi[a + i] = k[i];
+    if (WORD) sorted[a + i] = (K)k[i].x;
     val[a + i] = v[i];
   }
 }
@@ -461,9 +530,8 @@ __device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target) {
 }
 
 __global__ void __launch_bounds__(TIE_THREADS)
-k_tie_resort(const uint64_t* __restrict__ hi_orig, const uint64_t* __restrict__ lo_orig, uint32_t* val,
-             uint32_t* val_alt, uint64_t* __restrict__ hi_sorted, uint32_t n, int lo_passes, DevState* st,
-             uint32_t* table) {
+k_tie_resort(const ulonglong2* __restrict__ keys, uint32_t* val, uint32_t* val_alt,
+             uint64_t* __restrict__ hi_sorted, uint32_t n, int lo_passes, DevState* st, uint32_t* table) {
   if (st->tie == 0u) return;
   __shared__ uint32_t wcnt[TIE_THREADS / 32][256];
   __shared__ uint32_t base[256];
@@ -475,9 +543,12 @@ k_tie_resort(const uint64_t* __restrict__ hi_orig, const uint64_t* __restrict__ 
   uint32_t bars = 0;
   uint32_t *src = val, *dst = val_alt;
   for (int pass = 0; pass < lo_passes + 8; ++pass) {
-    const uint64_t* key = pass < lo_passes ? lo_orig : hi_orig;
+    // word 0 of a key is its high word, word 1 its low word
+    const uint64_t* key = reinterpret_cast<const uint64_t*>(keys) + (pass < lo_passes ? 1 : 0);
     const int shift = 8 * (pass < lo_passes ? pass : pass - lo_passes);
-    auto digit = [&](uint32_t v) { return JC_IN_BOUNDS(v, n, &st->error) ? (uint32_t)(key[v] >> shift) & 0xFFu : 0u; };
+    auto digit = [&](uint32_t v) {
+      return JC_IN_BOUNDS(v, n, &st->error) ? (uint32_t)(key[2 * (size_t)v] >> shift) & 0xFFu : 0u;
+    };
     if (tid < 256) base[tid] = 0;
     __syncthreads();
 #pragma unroll 4
@@ -538,20 +609,8 @@ k_tie_resort(const uint64_t* __restrict__ hi_orig, const uint64_t* __restrict__ 
   for (uint32_t i = b0 + tid; i < b1; i += TIE_THREADS) {
     const uint32_t v = __ldcg(src + i);
     val[i] = v;
-    hi_sorted[i] = JC_IN_BOUNDS(v, n, &st->error) ? hi_orig[v] : 0ull;
+    if (hi_sorted) hi_sorted[i] = JC_IN_BOUNDS(v, n, &st->error) ? keys[v].x : 0ull;
   }
-}
-
-__global__ void __launch_bounds__(256)
-k_gather_u64(const uint64_t* __restrict__ src, const uint32_t* __restrict__ val, uint64_t* __restrict__ dst,
-             DevState* st, const uint32_t* gate, uint32_t n) {
-  if (gate && *gate == 0) return;
-  uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a < st->n_valid) {
-    const uint32_t v = val[a];
-    if (JC_IN_BOUNDS(v, n, &st->error)) dst[a] = src[v];
-  }
-  (void)n;
 }
 
 // ---------------------------------------------------- prefix lengths --
@@ -661,57 +720,110 @@ __device__ __forceinline__ int64_t lcp_prev_below(const LcpIndex& X, uint32_t a,
 // ------------------------------------------------------------- count --
 // One block of 1024 threads per 1024 entries of L: its 32 warps write 32
 // first-level minima (m1) and the block their minimum (m2), so the whole
-// index is built in this pass.
+// index is built in this pass. The block reads its bodies' keys through the
+// permutation once (a pass of its own used to put the low words in order) and
+// scans its node counts: `first` holds each body's offset inside the block and
+// `totals` the block's sum until k_offsets adds the blocks before it.
 constexpr int COUNT_THREADS = 1024;
 __global__ void __launch_bounds__(COUNT_THREADS)
-k_count(const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo, uint32_t n, DevState* st,
-        uint32_t* __restrict__ count, Forest F, LcpIndex X) {
-  const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+k_count(const ulonglong2* __restrict__ key, const uint32_t* __restrict__ val, uint32_t n, DevState* st,
+        uint32_t* __restrict__ first, uint32_t* __restrict__ totals, Forest F, LcpIndex X) {
+  __shared__ ulonglong2 sk[COUNT_THREADS + 2];  // keys of bodies a - 1 .. a + 1 at sk[t .. t + 2]
+  __shared__ uint32_t sh[32];
+  __shared__ int wmin[COUNT_THREADS / 32];
+  const uint32_t t = threadIdx.x, a = blockIdx.x * COUNT_THREADS + t;
   const uint32_t N = st->n_valid;
+  auto load = [&](uint32_t b) {
+    const uint32_t v = b < N ? val[b] : n;
+    return v < n ? key[v] : make_ulonglong2(0ull, 0ull);
+  };
+  sk[t + 1] = load(a);
+  if (t == 0 && a > 0) sk[0] = load(a - 1);
+  if (t == COUNT_THREADS - 1) sk[COUNT_THREADS + 1] = load(a + 1);
+  __syncthreads();
   uint32_t c = 0;
   bool dup = false;
   int next = -1;  // lcp(a, a + 1), -1 at the last valid body and beyond
   if (a < N) {
-    uint64_t ha = hi[a], la = lo[a];
+    const ulonglong2 ka = sk[t + 1];
     int prev = -1;
     if (a > 0) {
-      prev = lcp_levels(hi[a - 1], lo[a - 1], ha, la, F.gbits, F.lh);
+      prev = lcp_levels(sk[t].x, sk[t].y, ka.x, ka.y, F.gbits, F.lh);
       dup = prev == 32;
     }
-    if (a + 1 < N) next = lcp_levels(ha, la, hi[a + 1], lo[a + 1], F.gbits, F.lh);
+    if (a + 1 < N) next = lcp_levels(ka.x, ka.y, sk[t + 2].x, sk[t + 2].y, F.gbits, F.lh);
     if (!dup) c = 1u + (uint32_t)max(0, max(0, next) - prev);
   }
-  if (a < n) count[a] = c;
+  uint32_t total;
+  const uint32_t local = dev::block_excl_scan(c, &total, sh);
+  if (a < n) first[a] = local;
+  if (t == 0) totals[blockIdx.x] = total;
   // the grid covers the index exactly: 32 * X.n1 = 1024 * X.n2 entries
-  __shared__ int wmin[COUNT_THREADS / 32];
   X.L[a] = (int8_t)next;
   int m = next;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-  if ((threadIdx.x & 31) == 0) {
+  if ((t & 31) == 0) {
     X.m1[a >> 5] = (int8_t)m;
-    wmin[threadIdx.x >> 5] = m;
+    wmin[t >> 5] = m;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    int v = wmin[threadIdx.x];
+  if (t < 32) {
+    int v = wmin[t];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    if (threadIdx.x == 0) X.m2[blockIdx.x] = (int8_t)v;
+    if (t == 0) X.m2[blockIdx.x] = (int8_t)v;
   }
   const uint32_t bal = __ballot_sync(0xFFFFFFFFu, dup);
-  if (bal && (threadIdx.x & 31) == 0) {
+  if (bal && (t & 31) == 0) {
     atomicAdd(&st->dropped, (uint32_t)__popc(bal));
     atomicOr(&st->warn, JC_WARN_DEPTH_CAP);
   }
 }
 
-// Capacity check + clearing of the per-node counters for this step.
-__global__ void __launch_bounds__(256)
-k_clear(const uint32_t* __restrict__ first, uint32_t n, KParams P, DevState* st,
-        uint32_t* __restrict__ nchild, uint32_t* __restrict__ arrive) {
-  uint32_t T = first[n];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+// The rest of the scan (one block per 1024 bodies, as k_count), the capacity
+// check and the clearing of the per-node counters for this step. Up to
+// OFFSET_BLOCKS blocks every block adds up the totals before its own; above,
+// `totals` comes scanned (`scanned`: with the sum in totals[gridDim.x]).
+constexpr uint32_t OFFSET_BLOCKS = 2048;
+__global__ void __launch_bounds__(COUNT_THREADS)
+k_offsets(const uint32_t* __restrict__ totals, int scanned, uint32_t* __restrict__ first, uint32_t n, KParams P,
+          DevState* st, uint32_t* __restrict__ nchild, uint32_t* __restrict__ arrive) {
+  __shared__ uint32_t sums[2][32];
+  __shared__ uint32_t s_before, s_all;
+  const uint32_t t = threadIdx.x;
+  if (scanned) {
+    if (t == 0) {
+      s_before = totals[blockIdx.x];
+      s_all = totals[gridDim.x];
+    }
+  } else {
+    uint32_t before = 0, all = 0;
+    for (uint32_t b = t; b < gridDim.x; b += COUNT_THREADS) {
+      const uint32_t c = totals[b];
+      all += c;
+      before += b < blockIdx.x ? c : 0u;
+    }
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    all = __reduce_add_sync(0xFFFFFFFFu, all);
+    if ((t & 31) == 0) {
+      sums[0][t >> 5] = before;
+      sums[1][t >> 5] = all;
+    }
+    __syncthreads();
+    if (t < 32) {
+      const uint32_t b = __reduce_add_sync(0xFFFFFFFFu, sums[0][t]), s = __reduce_add_sync(0xFFFFFFFFu, sums[1][t]);
+      if (t == 0) {
+        s_before = b;
+        s_all = s;
+      }
+    }
+  }
+  __syncthreads();
+  const uint32_t T = s_all, a = blockIdx.x * COUNT_THREADS + t;
+  if (a < n) first[a] += s_before;
+  if (blockIdx.x == 0 && t == 0) {
+    first[n] = T;
     if (T > P.tree_cap) {
       set_error(st, JC_ERR_CAPACITY);
       st->n_tree = 0;
@@ -720,11 +832,25 @@ k_clear(const uint32_t* __restrict__ first, uint32_t n, KParams P, DevState* st,
     }
     if (T > P.ref_cap) atomicOr(&st->warn, JC_WARN_REF_CAPACITY);
   }
-  uint32_t lim = min(T, P.tree_cap);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < lim; i += gridDim.x * blockDim.x) {
+  const uint32_t lim = min(T, P.tree_cap);
+  for (uint32_t i = a; i < lim; i += gridDim.x * COUNT_THREADS) {
     nchild[i] = 0;
     arrive[i] = 0;
   }
+}
+
+inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
+
+// k_count, the scan of its block totals where they are many, k_offsets.
+inline int launch_count(const ulonglong2* key, const uint32_t* val, uint32_t n, DevState* st, uint32_t* first,
+                        uint32_t* totals, uint32_t* scan_sums, const Forest& F, const LcpIndex& X, const KParams& P,
+                        uint32_t* nchild, uint32_t* arrive, cudaStream_t s) {
+  k_count<<<X.n2, COUNT_THREADS, 0, s>>>(key, val, n, st, first, totals, F, X);
+  int L = 2;
+  const bool scan = X.n2 > OFFSET_BLOCKS;
+  if (scan) L += dev::exclusive_scan(totals, totals, X.n2, scan_sums, s);
+  k_offsets<<<X.n2, COUNT_THREADS, 0, s>>>(totals, scan ? 1 : 0, first, n, P, st, nchild, arrive);
+  return L;
 }
 
 // ---------------------------------------------------------------- fill --
@@ -748,7 +874,7 @@ k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __rest
       const int prev = a > 0 ? (int)X.L[a - 1] : -1;
       const int top = max(0, (int)X.L[a]);
       const int n_int = max(0, top - prev);
-      const uint32_t g = key_graph(hi[a], F.gbits);
+      const uint32_t g = F.gbits ? key_graph(hi[a], F.gbits) : 0u;
       const uint32_t tend = F.n_graphs > 1 ? F.tree_end[g] : T;
       // root half extent halved once per level, as child_center does.
       float half = F.n_graphs > 1 ? F.roots[g].w : st->root[3];
@@ -1831,8 +1957,6 @@ struct DevBuf {
   ~DevBuf() { free(); }
 };
 
-inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
-
 // Mass of every body of a canonical CSR: 1 + its row length (the
 // non-self CSR entries, fa2_bh.rs:264-294), as the host computes it.
 __global__ void k_degf_from_offsets(const uint32_t* __restrict__ off, uint32_t n, float* __restrict__ degf) {
@@ -1969,9 +2093,8 @@ __global__ void k_csr_balance(const int* __restrict__ balance, uint32_t* ok) {
 
 inline uint32_t tie_blocks(uint32_t n, uint32_t sms) { return std::max(1u, std::min(sms, cdiv(n, TIE_PART))); }
 
-inline void launch_tie_resort(const uint64_t* hi_orig, const uint64_t* lo_orig, uint32_t* val, uint32_t* val_alt,
-                              uint64_t* hi_sorted, uint32_t n, int lo_passes, DevState* st, uint32_t* table,
-                              uint32_t sms, cudaStream_t s) {
+inline void launch_tie_resort(const ulonglong2* key, uint32_t* val, uint32_t* val_alt, uint64_t* hi_sorted, uint32_t n,
+                              int lo_passes, DevState* st, uint32_t* table, uint32_t sms, cudaStream_t s) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeCooperative;
   at.val.cooperative = 1;
@@ -1981,8 +2104,7 @@ inline void launch_tie_resort(const uint64_t* hi_orig, const uint64_t* lo_orig, 
   cfg.stream = s;
   cfg.attrs = &at;
   cfg.numAttrs = cfg.gridDim.x > 1 ? 1 : 0;
-  JC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_tie_resort, hi_orig, lo_orig, val, val_alt, hi_sorted, n, lo_passes, st,
-                                   table));
+  JC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_tie_resort, key, val, val_alt, hi_sorted, n, lo_passes, st, table));
 }
 
 class Fa2Engine : public Engine {
@@ -2557,7 +2679,7 @@ class Fa2Engine : public Engine {
   Fa2Settings s_;
   uint32_t n_ = 0, n_att_ = 0, n_hubs_ = 0, n_med_ = 0, hub_threshold_ = DEFAULT_HUB_THRESHOLD, att_blocks_ = 0;
   uint32_t sms_ = 1;
-  uint32_t tree_cap_ = 0, sort_tiles_ = 0, scan_tiles_ = 0;
+  uint32_t tree_cap_ = 0;
   uint32_t walk_group_ = DEFAULT_WALK_GROUP;
   uint32_t launches_ = 0;
   uint32_t warn_accum_ = 0;
@@ -2598,7 +2720,9 @@ class Fa2Engine : public Engine {
   DevBuf<DevState> state_;
   DevBuf<double2> partials_;
   // tree
-  DevBuf<uint64_t> hi_orig_, lo_orig_, hi_, hi_alt_, lo_;
+  DevBuf<ulonglong2> key_;  // (high, low) word by body
+  DevBuf<uint32_t> top_key_, top_alt_, totals_;
+  DevBuf<uint64_t> hi_, hi_alt_, lo_;
   DevBuf<uint32_t> val_, val_alt_, sort_work_, tie_table_, count_, first_, scan_sums_;
   DevBuf<int8_t> lcp_;  // prefix-length index: L, m1, m2 back to back
   LcpIndex lcpx_{};
@@ -2690,19 +2814,23 @@ class Fa2Engine : public Engine {
     // short of deep coincident clusters, which report JC_ERR_CAPACITY and
     // grow the buffers before the step is retried.
     tree_cap_ = std::max<uint32_t>(tree_cap_, 3 * n + 64);
-    hi_orig_.alloc(n); lo_orig_.alloc(n); hi_.alloc(n); hi_alt_.alloc(n); lo_.alloc(n);
+    key_.alloc(n);
+    if (graph_off_host_.size() > 2) {  // batches: sorted words, and the CTA-per-graph schedule's low words
+      hi_.alloc(n); hi_alt_.alloc(n); lo_.alloc(n);
+    } else {
+      top_key_.alloc(n); top_alt_.alloc(n);
+    }
     val_.alloc(n); val_alt_.alloc(n);
-    sort_tiles_ = dev::rs_tiles(std::max<uint32_t>(n, 1));
     sort_work_.alloc(dev::sort_work_words(std::max<uint32_t>(n, 1), 8));
     tie_table_.alloc(256 * (size_t)tie_blocks(n, sms_));
-    count_.alloc((size_t)n + 1);
+    if (graph_off_host_.size() > 2) count_.alloc((size_t)n + 1);
     first_.alloc((size_t)n + 2);
-    scan_tiles_ = std::max<uint32_t>(1, cdiv(n, dev::SC_TILE));
-    scan_sums_.alloc(scan_tiles_ + 1);
     nodes_.alloc(tree_cap_); parent_.alloc(tree_cap_); nchild_.alloc(tree_cap_);
     top_list_.alloc(TOP_MAX); top_.alloc(2 * TOP_MAX);
     arrive_.alloc(tree_cap_);
     const uint32_t nl = lcp_index_bytes(n), n2p = lcp_m2_bytes(nl);
+    totals_.alloc(nl / 1024 + 1);
+    scan_sums_.alloc(cdiv(nl / 1024, dev::SC_TILE) + 1);
     if (lcp_.n < (size_t)nl + nl / 32 + n2p || !lcp_.p) {
       lcp_.alloc((size_t)nl + nl / 32 + n2p);
       // entries past the bodies stay -1 ("run ends here") and the m2 padding
@@ -2780,28 +2908,29 @@ class Fa2Engine : public Engine {
         k_bbox_roots<<<cdiv(F.n_graphs, 8), 256, 0, stream_>>>(F, st);
         ++L;
       } else {
-        k_bbox<<<BBOX_BLOCKS, BBOX_THREADS, 0, stream_>>>(pos_.p, n, bbox_part_.p, st);
+        // (4 passes: digit counts, tile counters, look-back words)
+        k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, stream_>>>(pos_.p, n, bbox_part_.p, st, sort_work_.p,
+                                                             (uint32_t)dev::sort_work_words(n, 4));
       }
-      k_keys<<<cdiv(n, 256), 256, 0, stream_>>>(pos_.p, n, st, hi_orig_.p, lo_orig_.p, hi_.p, val_.p, F);
-      L += 2;
-      {
-        // a single graph: the top 32 bits (ten levels); a batch: the top 48
-        // (the graph id takes up to 16 of them), then the runs are fixed up
-        const int split = F.n_graphs > 1 ? 16 : 32;
-        L += dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nullptr, split, 64,
+      if (F.n_graphs > 1) {
+        // the top 48 bits (the graph id takes up to 16 of them), then the runs
+        k_keys_batch<<<cdiv(n, 256), 256, 0, stream_>>>(pos_.p, n, st, key_.p, hi_.p, val_.p, F);
+        L += dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nullptr, 16, 64,
                                              sort_work_.p, &st->error, nullptr, stream_);
-        k_seg_fix<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, lo_orig_.p, n, st, split);
-        ++L;
+        k_seg_fix<uint64_t><<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, key_.p, n, st, 16);
+      } else {
+        // the top 32 bits (ten levels), then the runs
+        k_keys<<<std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, stream_>>>(pos_.p, n, st, key_.p, top_key_.p, val_.p,
+                                                                        sort_work_.p);
+        L += dev::radix_passes<uint32_t>(top_key_.p, val_.p, top_alt_.p, val_alt_.p, n, nullptr, 0, 4, sort_work_.p,
+                                         &st->error, nullptr, stream_);
+        k_seg_fix<uint32_t><<<cdiv(n, 256), 256, 0, stream_>>>(top_key_.p, val_.p, key_.p, n, st, 0);
       }
-      launch_tie_resort(hi_orig_.p, lo_orig_.p, val_.p, val_alt_.p, hi_.p, n, (3 * (32 - F.lh) + 7) / 8, st,
+      launch_tie_resort(key_.p, val_.p, val_alt_.p, F.n_graphs > 1 ? hi_.p : nullptr, n, (3 * (32 - F.lh) + 7) / 8, st,
                         tie_table_.p, sms_, stream_);
-      ++L;
-      k_gather_u64<<<cdiv(n, 256), 256, 0, stream_>>>(lo_orig_.p, val_.p, lo_.p, st, nullptr, n);
-      k_count<<<lcpx_.n2, COUNT_THREADS, 0, stream_>>>(hi_.p, lo_.p, n, st, count_.p, F, lcpx_);
-      L += 2;
-      L += dev::exclusive_scan(count_.p, first_.p, n, scan_sums_.p, stream_);
-      k_clear<<<std::min<uint32_t>(cdiv(tree_cap_, 256), 1184), 256, 0, stream_>>>(first_.p, n, P, st, nchild_.p,
-                                                                                     arrive_.p);
+      L += 4;
+      L += launch_count(key_.p, val_.p, n, st, first_.p, totals_.p, scan_sums_.p, F, lcpx_, P, nchild_.p, arrive_.p,
+                        stream_);
       if (F.n_graphs > 1) {
         k_graph_trees<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, first_.p, st, F);
         ++L;
@@ -2810,7 +2939,7 @@ class Fa2Engine : public Engine {
       k_fill<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, lcpx_, val_.p, first_.p, pos_.p, degf_.p, n, P, st,
                                                  nodes_.p, parent_.p, nchild_.p, F, stage ? top_list_.p : nullptr);
       k_com<<<cdiv(n, 256), 256, 0, stream_>>>(first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p, n, st);
-      L += 3;
+      L += 2;
       if (stage) {
         k_top_build<<<1, 1024, 0, stream_>>>(nodes_.p, top_list_.p, st, top_.p);
         ++L;
@@ -3005,7 +3134,8 @@ class Fa2Engine : public Engine {
     TileBatch tb{G, graph_off_.p, t_work_.p, t_node_base_.p, t_cap_.p, t_lcp_base_.p, t_first_base_.p, t_gsteps_.p,
                  t_next_.p, gspeed_.p, t_nodes_.p, t_cells_.p, t_lcp_.p, t_first_.p};
     TileBufs tbufs{pos_.p, old_.p, force_.p, frep_.p, degf_.p, stats_.p, xyz_.p, aoff_.p, anbr_.p,
-                   hi_orig_.p, lo_orig_.p, hi_.p, lo_.p, val_.p, val_alt_.p, count_.p};
+                   reinterpret_cast<uint64_t*>(key_.p), reinterpret_cast<uint64_t*>(key_.p) + n_, hi_.p, lo_.p, val_.p,
+                   val_alt_.p, count_.p};
     const KParams P = kparams();
     k_tile_begin<<<1, 1, 0, stream_>>>(state_.p, t_next_.p);
     if (s_.fast_repulsion)
@@ -3124,8 +3254,8 @@ constexpr uint32_t NOALLOC_LCP = NOALLOC_MAX_NODES;  // prefix-length index byte
 __host__ __device__ constexpr size_t na_round(size_t b) { return (b + 255) & ~(size_t)255; }
 
 struct NoAllocLayout {
-  size_t st, bbox, pos4, frep, force4, old4, degf, stats, order, hi_orig, lo_orig, hi, hi_alt, lo, val,
-      val_alt, count, first, sums, work, table, partials, nodes, parent, nchild, arrive, lcp, total;
+  size_t st, bbox, pos4, frep, force4, old4, degf, stats, order, key, top_key, top_alt, val, val_alt,
+      first, totals, work, table, partials, nodes, parent, nchild, arrive, lcp, total;
 };
 
 constexpr NoAllocLayout noalloc_layout() {
@@ -3141,17 +3271,14 @@ constexpr NoAllocLayout noalloc_layout() {
   L.degf = o; o += na_round(4 * N);
   L.stats = o; o += na_round(8 * N);
   L.order = o; o += na_round(4 * N);
-  L.hi_orig = o; o += na_round(8 * N);
-  L.lo_orig = o; o += na_round(8 * N);
-  L.hi = o; o += na_round(8 * N);
-  L.hi_alt = o; o += na_round(8 * N);
-  L.lo = o; o += na_round(8 * N);
+  L.key = o; o += na_round(16 * N);
+  L.top_key = o; o += na_round(4 * N);
+  L.top_alt = o; o += na_round(4 * N);
   L.val = o; o += na_round(4 * N);
   L.val_alt = o; o += na_round(4 * N);
-  L.count = o; o += na_round(4 * (N + 1));
   L.first = o; o += na_round(4 * (N + 2));
-  L.sums = o; o += na_round(4 * (N / dev::SC_TILE + 2));
-  L.work = o; o += na_round(4 * dev::sort_work_words((uint32_t)N, 8));
+  L.totals = o; o += na_round(4 * (N / 1024 + 1));
+  L.work = o; o += na_round(4 * dev::sort_work_words((uint32_t)N, 4));
   L.table = o; o += na_round(4 * 256 * 16);
   L.partials = o; o += na_round(sizeof(double2) * (N / ATT_THREADS + 1));
   L.nodes = o; o += na_round(sizeof(TNode) * C);
@@ -3253,16 +3380,13 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   float* degf = (float*)(base + L.degf);
   float2* stats = (float2*)(base + L.stats);
   uint32_t* order = (uint32_t*)(base + L.order);
-  uint64_t* hi_orig = (uint64_t*)(base + L.hi_orig);
-  uint64_t* lo_orig = (uint64_t*)(base + L.lo_orig);
-  uint64_t* hi = (uint64_t*)(base + L.hi);
-  uint64_t* hi_alt = (uint64_t*)(base + L.hi_alt);
-  uint64_t* lo = (uint64_t*)(base + L.lo);
+  ulonglong2* key = (ulonglong2*)(base + L.key);
+  uint32_t* top_key = (uint32_t*)(base + L.top_key);
+  uint32_t* top_alt = (uint32_t*)(base + L.top_alt);
   uint32_t* val = (uint32_t*)(base + L.val);
   uint32_t* val_alt = (uint32_t*)(base + L.val_alt);
-  uint32_t* count = (uint32_t*)(base + L.count);
   uint32_t* first = (uint32_t*)(base + L.first);
-  uint32_t* sums = (uint32_t*)(base + L.sums);
+  uint32_t* totals = (uint32_t*)(base + L.totals);
   uint32_t* work = (uint32_t*)(base + L.work);
   uint32_t* table = (uint32_t*)(base + L.table);
   double2* partials = (double2*)(base + L.partials);
@@ -3304,21 +3428,19 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   }
   k_noalloc_prepare<<<cdiv(n, 256), 256, 0, s>>>(d_offsets, d_neighbors, n, degf, order, st);
   k_unpack_xyz<<<cdiv(n, 256), 256, 0, s>>>(d_positions_xyz, n, pos4);
-  k_bbox<<<BBOX_BLOCKS, BBOX_THREADS, 0, s>>>(pos4, n, (float*)(base + L.bbox), st);
-  k_keys<<<cdiv(n, 256), 256, 0, s>>>(pos4, n, st, hi_orig, lo_orig, hi, val, F1);
-  dev::radix_sort_pairs<uint64_t>(hi, val, hi_alt, val_alt, n, nullptr, 32, 64, work, &st->error, nullptr, s);
-  k_seg_fix<<<cdiv(n, 256), 256, 0, s>>>(hi, val, lo_orig, n, st, 32);
+  k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, s>>>(pos4, n, (float*)(base + L.bbox), st, work,
+                                                  (uint32_t)dev::sort_work_words(n, 4));
+  k_keys<<<std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, s>>>(pos4, n, st, key, top_key, val, work);
+  dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, nullptr, 0, 4, work, &st->error, nullptr, s);
+  k_seg_fix<uint32_t><<<cdiv(n, 256), 256, 0, s>>>(top_key, val, key, n, st, 0);
   // (at most 16 blocks: below the SM count of any device this library runs on)
   try {
-    launch_tie_resort(hi_orig, lo_orig, val, val_alt, hi, n, 5, st, table, 16, s);
+    launch_tie_resort(key, val, val_alt, nullptr, n, 5, st, table, 16, s);
   } catch (const Error&) {
     return JC_ERR_CUDA;
   }
-  k_gather_u64<<<cdiv(n, 256), 256, 0, s>>>(lo_orig, val, lo, st, nullptr, n);
-  k_count<<<X.n2, COUNT_THREADS, 0, s>>>(hi, lo, n, st, count, F1, X);
-  dev::exclusive_scan(count, first, n, sums, s);
-  k_clear<<<std::min<uint32_t>(cdiv(NOALLOC_TREE_CAP, 256), 1184), 256, 0, s>>>(first, n, P, st, nchild, arrive);
-  k_fill<<<cdiv(n, 256), 256, 0, s>>>(hi, X, val, first, pos4, degf, n, P, st, nodes, parent, nchild, F1);
+  launch_count(key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
+  k_fill<<<cdiv(n, 256), 256, 0, s>>>(nullptr, X, val, first, pos4, degf, n, P, st, nodes, parent, nchild, F1);
   k_com<<<cdiv(n, 256), 256, 0, s>>>(first, nodes, parent, nchild, arrive, n, st);
   k_walk_ahead<false><<<cdiv(n, WALK_THREADS), WALK_THREADS, 0, s>>>(nodes, val, pos4, degf, n, P, st, frep);
   k_att<<<cdiv(n, ATT_THREADS), ATT_THREADS, 0, s>>>(order, d_offsets, d_neighbors, pos4, frep, old4, degf, P, st,

@@ -248,24 +248,17 @@ __host__ __device__ constexpr size_t sort_work_words(uint32_t n_max, int passes)
   return (size_t)passes * RS_RADIX + passes + (size_t)passes * rs_tiles(n_max) * RS_RADIX;
 }
 
-// Sorts (keys, vals) by bits [bit_begin, bit_end) with an even number of
-// passes (the result ends in keys/vals). `work` holds sort_work_words words.
-// Returns the number of nodes (kernels + memsets) issued.
+// The passes alone: the digit counts are in `work` already and the words after
+// them are zero. Returns the number of kernels issued.
 template <typename K>
-inline int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, uint32_t n_max,
-                            const uint32_t* d_count, int bit_begin, int bit_end, uint32_t* work,
-                            uint32_t* err, const uint32_t* gate, cudaStream_t s) {
-  if (n_max == 0) return 0;
+inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, uint32_t n_max,
+                        const uint32_t* d_count, int bit_begin, int passes, uint32_t* work, uint32_t* err,
+                        const uint32_t* gate, cudaStream_t s) {
   const uint32_t tiles = rs_tiles(n_max);
   const bool small = rs_rounds(n_max) == RS_ROUNDS_SMALL;
-  int passes = (bit_end - bit_begin + 7) / 8;
-  if (passes & 1) ++passes;
   uint32_t* counts = work;
   uint32_t* tile_ctr = counts + passes * RS_RADIX;
   uint32_t* status = tile_ctr + passes;
-  cudaMemsetAsync(work, 0, sizeof(uint32_t) * sort_work_words(n_max, passes), s);
-  const uint32_t hist_blocks = tiles < 592u ? tiles : 592u;
-  os_hist<K><<<hist_blocks, RS_THREADS, 0, s>>>(keys, n_max, d_count, bit_begin, passes, counts, gate);
   K* kin = keys;
   uint32_t* vin = vals;
   K* kout = keys_alt;
@@ -285,7 +278,24 @@ inline int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
   }
-  return 2 + passes;
+  return passes;
+}
+
+// Sorts (keys, vals) by bits [bit_begin, bit_end) with an even number of
+// passes (the result ends in keys/vals). `work` holds sort_work_words words.
+// Returns the number of nodes (kernels + memsets) issued.
+template <typename K>
+inline int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, uint32_t n_max,
+                            const uint32_t* d_count, int bit_begin, int bit_end, uint32_t* work,
+                            uint32_t* err, const uint32_t* gate, cudaStream_t s) {
+  if (n_max == 0) return 0;
+  const uint32_t tiles = rs_tiles(n_max);
+  int passes = (bit_end - bit_begin + 7) / 8;
+  if (passes & 1) ++passes;
+  cudaMemsetAsync(work, 0, sizeof(uint32_t) * sort_work_words(n_max, passes), s);
+  const uint32_t hist_blocks = tiles < 592u ? tiles : 592u;
+  os_hist<K><<<hist_blocks, RS_THREADS, 0, s>>>(keys, n_max, d_count, bit_begin, passes, work, gate);
+  return 2 + radix_passes(keys, vals, keys_alt, vals_alt, n_max, d_count, bit_begin, passes, work, err, gate, s);
 }
 
 // ---------------------------------------------------------------- scan --
