@@ -68,6 +68,7 @@
 #include "jc_common.h"
 #include "jc_engine.h"
 #include "jc_exact.cuh"
+#include "jc_launch.cuh"
 #include "jc_params.h"
 #include "jc_sort.cuh"
 #include "jc_pool.h"
@@ -220,6 +221,7 @@ __device__ __forceinline__ void set_error(DevState* st, uint32_t code) { atomicC
 __global__ void __launch_bounds__(BBOX_THREADS)
 k_bbox(const float4* __restrict__ pos, uint32_t n, float* __restrict__ part, DevState* st,
        uint32_t* __restrict__ sort_work, uint32_t sort_words) {
+  dev::dependent_launch_wait();
   // (the sort's digit counts, tile counters and look-back words start at zero)
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < sort_words; i += gridDim.x * blockDim.x)
     sort_work[i] = 0u;
@@ -355,6 +357,7 @@ constexpr uint32_t KEY_BLOCKS = 148u * 8u;
 __global__ void __launch_bounds__(256)
 k_keys(const float4* __restrict__ pos, uint32_t n, DevState* st, ulonglong2* __restrict__ key,
        uint32_t* __restrict__ top, uint32_t* __restrict__ val, uint32_t* __restrict__ counts) {
+  dev::dependent_launch_wait();
   __shared__ uint32_t h[4][256];
 #pragma unroll
   for (int p = 0; p < 4; ++p) h[p][threadIdx.x] = 0;
@@ -438,6 +441,7 @@ template <typename K>
 __global__ void __launch_bounds__(256)
 k_seg_fix(K* __restrict__ sorted, uint32_t* __restrict__ val, const ulonglong2* __restrict__ key, uint32_t n,
           DevState* st, int shift) {
+  dev::dependent_launch_wait();
   constexpr bool WORD = sizeof(K) == 8;
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a == 0) st->n_valid = n - st->n_invalid;  // valid bodies (the non-finite sort last)
@@ -532,6 +536,7 @@ __device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target) {
 __global__ void __launch_bounds__(TIE_THREADS)
 k_tie_resort(const ulonglong2* __restrict__ keys, uint32_t* val, uint32_t* val_alt,
              uint64_t* __restrict__ hi_sorted, uint32_t n, int lo_passes, DevState* st, uint32_t* table) {
+  dev::dependent_launch_wait();
   if (st->tie == 0u) return;
   __shared__ uint32_t wcnt[TIE_THREADS / 32][256];
   __shared__ uint32_t base[256];
@@ -728,6 +733,7 @@ constexpr int COUNT_THREADS = 1024;
 __global__ void __launch_bounds__(COUNT_THREADS)
 k_count(const ulonglong2* __restrict__ key, const uint32_t* __restrict__ val, uint32_t n, DevState* st,
         uint32_t* __restrict__ first, uint32_t* __restrict__ totals, Forest F, LcpIndex X) {
+  dev::dependent_launch_wait();
   __shared__ ulonglong2 sk[COUNT_THREADS + 2];  // keys of bodies a - 1 .. a + 1 at sk[t .. t + 2]
   __shared__ uint32_t sh[32];
   __shared__ int wmin[COUNT_THREADS / 32];
@@ -789,6 +795,7 @@ constexpr uint32_t OFFSET_BLOCKS = 2048;
 __global__ void __launch_bounds__(COUNT_THREADS)
 k_offsets(const uint32_t* __restrict__ totals, int scanned, uint32_t* __restrict__ first, uint32_t n, KParams P,
           DevState* st, uint32_t* __restrict__ nchild, uint32_t* __restrict__ arrive) {
+  dev::dependent_launch_wait();
   __shared__ uint32_t sums[2][32];
   __shared__ uint32_t s_before, s_all;
   const uint32_t t = threadIdx.x;
@@ -842,14 +849,15 @@ k_offsets(const uint32_t* __restrict__ totals, int scanned, uint32_t* __restrict
 inline uint32_t cdiv(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 // k_count, the scan of its block totals where they are many, k_offsets.
-inline int launch_count(const ulonglong2* key, const uint32_t* val, uint32_t n, DevState* st, uint32_t* first,
+inline int launch_count(bool chained, const ulonglong2* key, const uint32_t* val, uint32_t n, DevState* st, uint32_t* first,
                         uint32_t* totals, uint32_t* scan_sums, const Forest& F, const LcpIndex& X, const KParams& P,
                         uint32_t* nchild, uint32_t* arrive, cudaStream_t s) {
-  k_count<<<X.n2, COUNT_THREADS, 0, s>>>(key, val, n, st, first, totals, F, X);
+  launch_chained(chained, s, X.n2, COUNT_THREADS, 0, k_count, key, val, n, st, first, totals, F, X);
   int L = 2;
   const bool scan = X.n2 > OFFSET_BLOCKS;
   if (scan) L += dev::exclusive_scan(totals, totals, X.n2, scan_sums, s);
-  k_offsets<<<X.n2, COUNT_THREADS, 0, s>>>(totals, scan ? 1 : 0, first, n, P, st, nchild, arrive);
+  launch_chained(chained && !scan, s, X.n2, COUNT_THREADS, 0, k_offsets, totals, scan ? 1 : 0, first, n, P, st, nchild,
+                 arrive);
   return L;
 }
 
@@ -863,6 +871,7 @@ k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __rest
        uint32_t n, KParams P, DevState* st, TNode* __restrict__ nodes,
        uint32_t* __restrict__ parent, uint32_t* __restrict__ nchild, Forest F,
        uint32_t* __restrict__ top_list = nullptr) {
+  dev::dependent_launch_wait();
   uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t N = st->n_valid;
   if (st->error) return;
@@ -943,6 +952,7 @@ k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __rest
 __global__ void __launch_bounds__(256)
 k_com(const uint32_t* __restrict__ first, TNode* nodes, const uint32_t* __restrict__ parent,
       const uint32_t* __restrict__ nchild, uint32_t* __restrict__ arrive, uint32_t n, DevState* st) {
+  dev::dependent_launch_wait();
   uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   if (st->error) return;
   const uint32_t N = st->n_valid;
@@ -1045,6 +1055,7 @@ template <int G, bool FAST>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_walk(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, const float4* __restrict__ pos,
        const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep, Forest F) {
+  dev::dependent_launch_wait();
   const int lane = threadIdx.x & 31;
   const uint32_t a = blockIdx.x * WALK_THREADS + threadIdx.x;
   const uint32_t body0 = a < n ? order[a] : 0u;
@@ -1179,6 +1190,7 @@ template <bool FAST>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, const float4* __restrict__ pos,
              const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep) {
+  dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t T = st->error ? 0u : st->n_tree;
   uint32_t n_inter = 0, n_open = 0;
@@ -1223,6 +1235,7 @@ template <bool FAST>
 __global__ void __launch_bounds__(WALK_THREADS, 2048 / WALK_THREADS)
 k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, const float4* __restrict__ pos,
             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep, Forest F) {
+  dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * WALK_THREADS + threadIdx.x;
   const uint32_t T = st->error ? 0u : st->n_tree;
   uint32_t n_inter = 0, n_open = 0;
@@ -1251,6 +1264,7 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
 __global__ void __launch_bounds__(1024)
 k_top_build(const TNode* __restrict__ nodes, const uint32_t* __restrict__ top_list, DevState* st,
             uint4* __restrict__ top) {
+  dev::dependent_launch_wait();
   __shared__ uint32_t key[1024];
   const uint32_t t = threadIdx.x;
   const uint32_t listed = st->n_top;
@@ -1302,6 +1316,7 @@ __global__ void __launch_bounds__(WALK_THREADS)
 k_walk_top(const TNode* __restrict__ nodes, const uint4* __restrict__ top, const uint32_t* __restrict__ order,
            const float4* __restrict__ pos, const float* __restrict__ degf, uint32_t n, KParams P, DevState* st,
            float4* __restrict__ frep) {
+  dev::dependent_launch_wait();
   __shared__ uint4 tsm[2 * TOP_MAX];
   const uint32_t T = st->error ? 0u : st->n_tree;
   const uint32_t nt = min(st->n_top, TOP_MAX);
@@ -1588,6 +1603,7 @@ template <int I>
 __global__ void __launch_bounds__(brute_threads(I))
 k_brute(const float4* __restrict__ pos, const float* __restrict__ degf, uint32_t n, KParams P,
         float4* __restrict__ frep) {
+  dev::dependent_launch_wait();
   extern __shared__ float4 brute_sm[];  // float4: 16-byte aligned rows
   float* term = reinterpret_cast<float*>(brute_sm);  // [2][3][I][BRUTE_ROW]
   __shared__ float4 body[I];
@@ -1733,6 +1749,7 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
       const float4* __restrict__ pos, const float4* __restrict__ frep, const float4* __restrict__ old_force,
       const float* __restrict__ degf, KParams P, DevState* st, float4* __restrict__ force,
       float2* __restrict__ stats, double2* __restrict__ partials, uint32_t n_graphs) {
+  dev::dependent_launch_wait();
   __shared__ double red_sw[ATT_THREADS / 32], red_tr[ATT_THREADS / 32];
   __shared__ float hub_sum[3][ATT_THREADS / 32];
   __shared__ bool last;
@@ -1896,6 +1913,7 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
 __global__ void __launch_bounds__(APPLY_THREADS)
 k_apply(float4* __restrict__ pos, float4* __restrict__ old_force, const float4* __restrict__ force,
         const float* __restrict__ degf, KParams P, const DevState* st, float* __restrict__ xyz, Forest F) {
+  dev::dependent_launch_wait();
   if (st->error) return;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= P.n) return;
@@ -2899,6 +2917,7 @@ class Fa2Engine : public Engine {
     const KParams P = kparams();
     const uint32_t n = n_;
     DevState* st = state_.p;
+    const bool chain = chained();
     int L = 0;
     record_phase(0);
     if (bh_) {
@@ -2920,25 +2939,26 @@ class Fa2Engine : public Engine {
         k_seg_fix<uint64_t><<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, key_.p, n, st, 16);
       } else {
         // the top 32 bits (ten levels), then the runs
-        k_keys<<<std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, stream_>>>(pos_.p, n, st, key_.p, top_key_.p, val_.p,
-                                                                        sort_work_.p);
+        launch_chained(chain, stream_, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos_.p, n, st, key_.p,
+                       top_key_.p, val_.p, sort_work_.p);
         L += dev::radix_passes<uint32_t>(top_key_.p, val_.p, top_alt_.p, val_alt_.p, n, nullptr, 0, 4, sort_work_.p,
-                                         &st->error, nullptr, stream_);
-        k_seg_fix<uint32_t><<<cdiv(n, 256), 256, 0, stream_>>>(top_key_.p, val_.p, key_.p, n, st, 0);
+                                         &st->error, nullptr, stream_, chain);
+        launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key_.p, val_.p, key_.p, n, st, 0);
       }
       launch_tie_resort(key_.p, val_.p, val_alt_.p, F.n_graphs > 1 ? hi_.p : nullptr, n, (3 * (32 - F.lh) + 7) / 8, st,
                         tie_table_.p, sms_, stream_);
       L += 4;
-      L += launch_count(key_.p, val_.p, n, st, first_.p, totals_.p, scan_sums_.p, F, lcpx_, P, nchild_.p, arrive_.p,
+      L += launch_count(chain, key_.p, val_.p, n, st, first_.p, totals_.p, scan_sums_.p, F, lcpx_, P, nchild_.p, arrive_.p,
                         stream_);
       if (F.n_graphs > 1) {
         k_graph_trees<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, first_.p, st, F);
         ++L;
       }
       const bool stage = stage_top();
-      k_fill<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, lcpx_, val_.p, first_.p, pos_.p, degf_.p, n, P, st,
-                                                 nodes_.p, parent_.p, nchild_.p, F, stage ? top_list_.p : nullptr);
-      k_com<<<cdiv(n, 256), 256, 0, stream_>>>(first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p, n, st);
+      launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_fill, hi_.p, lcpx_, val_.p, first_.p, pos_.p, degf_.p, n, P,
+                     st, nodes_.p, parent_.p, nchild_.p, F, stage ? top_list_.p : nullptr);
+      launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_com, first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p, n,
+                     st);
       L += 2;
       if (stage) {
         k_top_build<<<1, 1024, 0, stream_>>>(nodes_.p, top_list_.p, st, top_.p);
@@ -2953,8 +2973,8 @@ class Fa2Engine : public Engine {
       L += 1;
     }
     record_phase(2);
-    k_att<<<att_blocks_, ATT_THREADS, 0, stream_>>>(aorder_.p, aoff_.p, anbr_.p, pos_.p, frep_.p, old_.p, degf_.p, P,
-                                                    st, force_.p, stats_.p, partials_.p, forest_.n_graphs);
+    launch_chained(chain, stream_, att_blocks_, ATT_THREADS, 0, k_att, aorder_.p, aoff_.p, anbr_.p, pos_.p, frep_.p,
+                   old_.p, degf_.p, P, st, force_.p, stats_.p, partials_.p, forest_.n_graphs);
     if (forest_.n_graphs > 1) {
       k_speed_slices<<<forest_.n_slices, 256, 0, stream_>>>(stats_.p, forest_, st);
       k_speed_graphs<<<cdiv(forest_.n_graphs, 256), 256, 0, stream_>>>(forest_, s_.jitter_tolerance, st);
@@ -2962,8 +2982,8 @@ class Fa2Engine : public Engine {
       ++L;
     }
     record_phase(3);
-    k_apply<<<cdiv(n, APPLY_THREADS), APPLY_THREADS, 0, stream_>>>(pos_.p, old_.p, force_.p, degf_.p, P, st, xyz_.p,
-                                                                   forest_);
+    launch_chained(chain, stream_, cdiv(n, APPLY_THREADS), APPLY_THREADS, 0, k_apply, pos_.p, old_.p, force_.p, degf_.p,
+                   P, st, xyz_.p, forest_);
     record_phase(4);
     L += 2;
     JC_CUDA_CHECK(cudaGetLastError());
@@ -2974,6 +2994,7 @@ class Fa2Engine : public Engine {
   void launch_brute_as(const KParams& P) {
     if (brute_smem(I) > 48 * 1024)
       JC_CUDA_CHECK(cudaFuncSetAttribute(k_brute<I>, cudaFuncAttributeMaxDynamicSharedMemorySize, brute_smem(I)));
+    // (the step's first launch: ordinary)
     k_brute<I><<<cdiv(n_, I), brute_threads(I), brute_smem(I), stream_>>>(pos_.p, degf_.p, n_, P, frep_.p);
   }
 
@@ -2984,6 +3005,17 @@ class Fa2Engine : public Engine {
     if (n_ > 8u * 148u) launch_brute_as<16>(P);
     else if (n_ > 4u * 148u) launch_brute_as<8>(P);
     else launch_brute_as<4>(P);
+  }
+
+  // A small single graph's step chains its kernels as programmatic dependents
+  // where nothing but kernels stands between them (no phase events). B200, us a
+  // replayed step without and with: 400 nodes 104 -> 102, 2,000 134 -> 131, 10,000
+  // 156 -> 154, but 65,537 180 -> 205 and 1 M 1,155 -> 1,161. (The pass of
+  // jc_fa2_bh_forces_noalloc, launched one by one: 300 nodes 155 -> 137 us, 20,000
+  // 292 -> 273.)
+  static constexpr uint32_t CHAIN_MAX_N = 32768;
+  bool chained() const {
+    return n_ <= CHAIN_MAX_N && s_.use_graph && !capture_phases_ && forest_.n_graphs == 1 && !stage_top();
   }
 
   // The staged-top walk: a single graph, walk group 1.
@@ -3001,10 +3033,13 @@ class Fa2Engine : public Engine {
     switch (walk_group_) {
       case 1:
         if (forest_.n_graphs == 1 && n <= WALK_AHEAD_N) {
-          k_walk_ahead<FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p);
+          launch_chained(chained(), stream_, grid.x, WALK_THREADS, 0, k_walk_ahead<FAST>, nodes_.p, val_.p, pos_.p,
+                         degf_.p, n, P, st, frep_.p);
           break;
         }
-        k_walk_rope<FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
+        launch_chained(chained(), stream_, grid.x, WALK_THREADS, 0, k_walk_rope<FAST>, nodes_.p, val_.p, pos_.p, degf_.p, n,
+                       P, st, frep_.p, forest_);
+        break;
       case 2: k_walk<2, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
       case 4: k_walk<4, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
       case 8: k_walk<8, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
@@ -3430,21 +3465,24 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   k_unpack_xyz<<<cdiv(n, 256), 256, 0, s>>>(d_positions_xyz, n, pos4);
   k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, s>>>(pos4, n, (float*)(base + L.bbox), st, work,
                                                   (uint32_t)dev::sort_work_words(n, 4));
-  k_keys<<<std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, s>>>(pos4, n, st, key, top_key, val, work);
-  dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, nullptr, 0, 4, work, &st->error, nullptr, s);
-  k_seg_fix<uint32_t><<<cdiv(n, 256), 256, 0, s>>>(top_key, val, key, n, st, 0);
-  // (at most 16 blocks: below the SM count of any device this library runs on)
+  // (chained as programmatic dependents from here on; at most 16 blocks for
+  // the re-sort: below the SM count of any device this library runs on)
   try {
+    launch_chained(true, s, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos4, n, st, key, top_key, val, work);
+    dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, nullptr, 0, 4, work, &st->error, nullptr, s, true);
+    launch_chained(true, s, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key, val, key, n, st, 0);
     launch_tie_resort(key, val, val_alt, nullptr, n, 5, st, table, 16, s);
+    launch_count(true, key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
+    launch_chained(true, s, cdiv(n, 256), 256, 0, k_fill, nullptr, X, val, first, pos4, degf, n, P, st, nodes, parent,
+                   nchild, F1, nullptr);
+    launch_chained(true, s, cdiv(n, 256), 256, 0, k_com, first, nodes, parent, nchild, arrive, n, st);
+    launch_chained(true, s, cdiv(n, WALK_THREADS), WALK_THREADS, 0, k_walk_ahead<false>, nodes, val, pos4, degf, n, P, st,
+                   frep);
+    launch_chained(true, s, cdiv(n, ATT_THREADS), ATT_THREADS, 0, k_att, order, d_offsets, d_neighbors, pos4, frep, old4,
+                   degf, P, st, force4, stats, partials, 1u);
   } catch (const Error&) {
     return JC_ERR_CUDA;
   }
-  launch_count(key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
-  k_fill<<<cdiv(n, 256), 256, 0, s>>>(nullptr, X, val, first, pos4, degf, n, P, st, nodes, parent, nchild, F1);
-  k_com<<<cdiv(n, 256), 256, 0, s>>>(first, nodes, parent, nchild, arrive, n, st);
-  k_walk_ahead<false><<<cdiv(n, WALK_THREADS), WALK_THREADS, 0, s>>>(nodes, val, pos4, degf, n, P, st, frep);
-  k_att<<<cdiv(n, ATT_THREADS), ATT_THREADS, 0, s>>>(order, d_offsets, d_neighbors, pos4, frep, old4, degf, P, st,
-                                                    force4, stats, partials, 1u);
   k_pack_xyz<<<cdiv(n, 256), 256, 0, s>>>(force4, n, d_forces_xyz);
   if (cudaGetLastError() != cudaSuccess) return JC_ERR_CUDA;
   uint32_t err = 0;

@@ -43,6 +43,7 @@
 #include "jc_common.h"
 #include "jc_engine.h"
 #include "jc_exact.cuh"
+#include "jc_launch.cuh"
 #include "jc_params.h"
 
 namespace jc {
@@ -257,18 +258,13 @@ __device__ __forceinline__ float4 pair_moved(float4 p, const long long* a, uint3
 // A sweep is 64 batches of two short kernels, each a few dependent round trips,
 // so both are launched as programmatic dependents: a kernel is placed and reads
 // its samples while the one before drains, and waits for it (all of its writes)
-// before it touches positions or sums. At least one thread of each reaches the
-// wait, so completion passes down the chain; the draw and the step's end are
-// ordinary launches. (A cluster of eight CTAs that kept a whole sweep in one
+// before it touches positions or sums; the draw and the step's end are ordinary
+// launches. (A cluster of eight CTAs that kept a whole sweep in one
 // launch with barriers between the phases was slower, 569 us a sweep at 200,000
 // nodes: every phase waits for the adds of 4,096 threads to drain.) B200, us a
 // sweep, before (samples drawn in the batch, a pass over all nodes to apply) and
 // after: 200,000 nodes 388 -> 238 (296 without the early placement), 30,000 382
 // -> 224, 1,000 27 -> 18, 1 M 599 -> 426.
-__device__ __forceinline__ void dependent_launch_wait() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 // One batch: every pair against the batch-start positions, both moves added in
 // fixed point.
@@ -281,7 +277,7 @@ k_pairs(const uint4* __restrict__ samples, uint32_t count, const float4* __restr
   const uint32_t sw = *sweep_ctr + sweep;
   const float eta = eta_table[sw < n_eta ? sw : n_eta - 1];
   const uint4 p = samples[t];
-  dependent_launch_wait();
+  dev::dependent_launch_wait();
   const float hop = __uint_as_float(p.z);
   if (!(hop > 0.0f)) return;
   long long f[3];
@@ -303,7 +299,7 @@ k_pairs_apply(const uint4* __restrict__ samples, uint32_t count, float4* __restr
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * count) return;
   const uint4 s = samples[t >> 1];
-  dependent_launch_wait();
+  dev::dependent_launch_wait();
   if (!(__uint_as_float(s.z) > 0.0f)) return;
   const uint32_t v = (t & 1u) ? s.y : s.x;
   long long* m = acc + 3 * (size_t)v;
@@ -951,21 +947,6 @@ class SgdEngine : public Engine {
     if (!initialized_) fail(JC_ERR_STATE, std::string(desc_.id) + " step called before successful init");
   }
 
-  // k as an ordinary launch or as a programmatic dependent of the one before.
-  template <typename... P, typename... A>
-  void launch_pdl(bool pdl, uint32_t blocks, uint32_t threads, void (*k)(P...), A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(threads);
-    cfg.stream = stream_;
-    cfg.attrs = &at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    JC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k, (P)args...));
-  }
-
   template <typename D>
   int enqueue_sweeps(const D* dist) {
     const uint32_t n = n_, k = k_;
@@ -1003,9 +984,9 @@ class SgdEngine : public Engine {
         ++L;
         for (uint32_t q0 = 0; q0 < n; q0 += per) {
           const uint32_t cnt = std::min(per, n - q0);
-          launch_pdl(q0 > 0, cdiv(cnt, 128), 128, k_pairs, (const uint4*)samples_.p + q0, cnt, (const float4*)pos_a_.p,
+          launch_chained(q0 > 0, stream_, cdiv(cnt, 128), 128, 0, k_pairs, (const uint4*)samples_.p + q0, cnt, (const float4*)pos_a_.p,
                      acc_.p, cnt_.p, (const float*)eta_.p, n_eta_, (const uint32_t*)ctr_.p, s);
-          launch_pdl(true, cdiv(2 * (uint64_t)cnt, 128), 128, k_pairs_apply, (const uint4*)samples_.p + q0, cnt,
+          launch_chained(true, stream_, cdiv(2 * (uint64_t)cnt, 128), 128, 0, k_pairs_apply, (const uint4*)samples_.p + q0, cnt,
                      pos_a_.p, acc_.p, cnt_.p);
           L += 2;
         }

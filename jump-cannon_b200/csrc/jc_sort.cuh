@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "jc_check.cuh"
+#include "jc_launch.cuh"
 
 namespace jc {
 namespace dev {
@@ -133,6 +134,7 @@ os_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restri
         uint32_t* __restrict__ vout, uint32_t n_max, const uint32_t* d_count, int shift,
         const uint32_t* __restrict__ gcount, uint32_t* status, uint32_t* tile_ctr, const uint32_t* gate,
         uint32_t* err) {
+  dependent_launch_wait();
   if (gate && *gate == 0) return;
   __shared__ uint32_t wcnt[RS_WARPS][RS_RADIX];
   __shared__ uint32_t base[RS_RADIX];
@@ -253,7 +255,7 @@ __host__ __device__ constexpr size_t sort_work_words(uint32_t n_max, int passes)
 template <typename K>
 inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, uint32_t n_max,
                         const uint32_t* d_count, int bit_begin, int passes, uint32_t* work, uint32_t* err,
-                        const uint32_t* gate, cudaStream_t s) {
+                        const uint32_t* gate, cudaStream_t s, bool chained = false) {
   const uint32_t tiles = rs_tiles(n_max);
   const bool small = rs_rounds(n_max) == RS_ROUNDS_SMALL;
   uint32_t* counts = work;
@@ -266,15 +268,9 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
   for (int p = 0; p < passes; ++p) {
     int shift = bit_begin + 8 * p;
     if (shift >= (int)(8 * sizeof(K))) shift = 8 * (int)sizeof(K) - 8;
-    if (small)
-      os_pass<K, RS_ROUNDS_SMALL><<<tiles, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n_max, d_count, shift,
-                                                               counts + p * RS_RADIX,
-                                                               status + (size_t)p * tiles * RS_RADIX, tile_ctr + p,
-                                                               gate, err);
-    else
-      os_pass<K, RS_ROUNDS><<<tiles, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n_max, d_count, shift,
-                                                         counts + p * RS_RADIX, status + (size_t)p * tiles * RS_RADIX,
-                                                         tile_ctr + p, gate, err);
+    launch_chained(chained, s, tiles, RS_THREADS, 0, small ? os_pass<K, RS_ROUNDS_SMALL> : os_pass<K, RS_ROUNDS>, kin,
+                   vin, kout, vout, n_max, d_count, shift, counts + p * RS_RADIX,
+                   status + (size_t)p * tiles * RS_RADIX, tile_ctr + p, gate, err);
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
   }
