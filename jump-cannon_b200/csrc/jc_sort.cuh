@@ -27,15 +27,14 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_ROUNDS = 16;                        // items per lane
 constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;      // 4096 items per block
 constexpr int RS_RADIX = 256;
-// Below RS_SMALL_N items a tile holds 8 items per lane (2048 per block): a
-// tile's ranking is a serial chain of rounds, so where the tiles would not
-// fill the GPU shorter tiles finish sooner (B200: a 10,000-body step 0.274 ->
-// 0.261 ms); above it 16 per lane keep the look-back chains short (1M bodies:
-// tree build 0.446 ms against 0.471 with 8).
-constexpr int RS_ROUNDS_SMALL = 8;
-constexpr uint32_t RS_SMALL_N = 296u * 2048u;
+// Items per lane by size: a tile's ranking is a serial chain of rounds, so where
+// the tiles would not fill the GPU shorter tiles finish sooner; many tiles make
+// the look-back chains long. B200, tree build in us with 4-byte keys at 2 / 4 /
+// 8 / 16 items: 400 bodies 57 / 59 / 63 / 71, 10,000 92 / 95 / 97 / 109, 150,000
+// 145 / 138 / 140 / 149, 262,144 185 / 172 / 168 / 174, 600,000 335 / 279 / 259 /
+// 255, 1 M 541 / 552 / 426 / 399.
 __host__ __device__ constexpr int rs_rounds(uint32_t n_max) {
-  return n_max <= RS_SMALL_N ? RS_ROUNDS_SMALL : RS_ROUNDS;
+  return n_max <= 32768u ? 2 : n_max <= 196608u ? 4 : n_max <= 400000u ? 8 : RS_ROUNDS;
 }
 __host__ __device__ constexpr uint32_t rs_tiles(uint32_t n_max) {
   return (n_max + (uint32_t)(RS_THREADS * rs_rounds(n_max)) - 1) / (uint32_t)(RS_THREADS * rs_rounds(n_max));
@@ -257,7 +256,9 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
                         const uint32_t* d_count, int bit_begin, int passes, uint32_t* work, uint32_t* err,
                         const uint32_t* gate, cudaStream_t s, bool chained = false) {
   const uint32_t tiles = rs_tiles(n_max);
-  const bool small = rs_rounds(n_max) == RS_ROUNDS_SMALL;
+  const int rounds = rs_rounds(n_max);
+  const auto pass = rounds == 2 ? os_pass<K, 2> : rounds == 4 ? os_pass<K, 4> : rounds == 8 ? os_pass<K, 8>
+                                                                                           : os_pass<K, RS_ROUNDS>;
   uint32_t* counts = work;
   uint32_t* tile_ctr = counts + passes * RS_RADIX;
   uint32_t* status = tile_ctr + passes;
@@ -268,8 +269,7 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
   for (int p = 0; p < passes; ++p) {
     int shift = bit_begin + 8 * p;
     if (shift >= (int)(8 * sizeof(K))) shift = 8 * (int)sizeof(K) - 8;
-    launch_chained(chained, s, tiles, RS_THREADS, 0, small ? os_pass<K, RS_ROUNDS_SMALL> : os_pass<K, RS_ROUNDS>, kin,
-                   vin, kout, vout, n_max, d_count, shift, counts + p * RS_RADIX,
+    launch_chained(chained, s, tiles, RS_THREADS, 0, pass, kin, vin, kout, vout, n_max, d_count, shift, counts + p * RS_RADIX,
                    status + (size_t)p * tiles * RS_RADIX, tile_ctr + p, gate, err);
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;

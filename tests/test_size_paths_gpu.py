@@ -255,3 +255,12 @@ def test_long_runs_resort_in_a_batch(jc):
         e.init(g, p)
         assert np.array_equal(bits(out[at:at + 3 * g.n_nodes]), bits(e.step_many(3)))
         at += 3 * g.n_nodes
+
+
+# both sides of the sort's tile-size rules and of the walk chain's rule
+@pytest.mark.parametrize("n", [511, 512, 513, 32767, 32768, 32769, 196607, 400000, 400001])
+def test_sort_tile_rules_bit_exact(jc, orc, n):
+    g = jc.gen_watts_strogatz(n, 4, 0.05, n) if n < 100000 else jc.gen_path(n)
+    e, r = one_step(jc, orc, g, jc.seed_uniform(n, 3, 7), theta=1.2)
+    assert e.tree_info()["nodes"] == r["n_octree"]
+    assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
