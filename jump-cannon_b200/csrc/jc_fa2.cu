@@ -864,13 +864,15 @@ inline int launch_count(bool chained, const ulonglong2* key, const uint32_t* val
 // ---------------------------------------------------------------- fill --
 // Bounded to 32 registers (eight blocks per SM, no spills): the fill waits on
 // its prefix-length searches and position gathers (tree build 0.443 -> 0.440 ms
-// on the 1M-node R-MAT against 40 registers).
+// on the 1M-node R-MAT against 40 registers). KIDS: every node also enters its
+// parent's list of children (eight slots per cell, in order of arrival).
+template <bool KIDS>
 __global__ void __launch_bounds__(256, 8)
 k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __restrict__ val,
        const uint32_t* __restrict__ first, const float4* __restrict__ pos, const float* __restrict__ degf,
        uint32_t n, KParams P, DevState* st, TNode* __restrict__ nodes,
        uint32_t* __restrict__ parent, uint32_t* __restrict__ nchild, Forest F,
-       uint32_t* __restrict__ top_list = nullptr) {
+       uint32_t* __restrict__ top_list, uint32_t* __restrict__ kids) {
   dev::dependent_launch_wait();
   uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t N = st->n_valid;
@@ -919,7 +921,10 @@ k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __rest
         nodes[idx].cm = make_float4(0.f, 0.f, 0.f, 0.f);
         uint32_t par = j == 0 ? first_parent : idx - 1;
         parent[idx] = par;
-        if (par != END && JC_IN_BOUNDS(par, P.tree_cap, &st->error)) atomicAdd(&nchild[par], 1u);
+        if (par != END && JC_IN_BOUNDS(par, P.tree_cap, &st->error)) {
+          const uint32_t slot = atomicAdd(&nchild[par], 1u) & 0xFFFFu;
+          if (KIDS && slot < 8u) kids[8 * (size_t)par + slot] = idx;
+        }
         if (top_list && d <= TOP_DEPTH) {
           const uint32_t slot = atomicAdd(&st->n_top, 1u);
           if (slot < TOP_MAX) top_list[slot] = idx;
@@ -937,7 +942,10 @@ k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __rest
       nodes[leaf].cm = make_float4(p.x, p.y, p.z, fmaxf(degf[body], 1e-3f));
       uint32_t par = n_int > 0 ? leaf - 1 : first_parent;
       parent[leaf] = par;
-      if (par != END && JC_IN_BOUNDS(par, P.tree_cap, &st->error)) atomicAdd(&nchild[par], 1u + (1u << 16));  // leaves also count in the high half
+      if (par != END && JC_IN_BOUNDS(par, P.tree_cap, &st->error)) {
+        const uint32_t slot = atomicAdd(&nchild[par], 1u + (1u << 16)) & 0xFFFFu;  // leaves also count in the high half
+        if (KIDS && slot < 8u) kids[8 * (size_t)par + slot] = leaf;
+      }
       if (top_list && (int)leaf_depth <= TOP_DEPTH) {
         const uint32_t slot = atomicAdd(&st->n_top, 1u);
         if (slot < TOP_MAX) top_list[slot] = leaf;
@@ -1014,6 +1022,105 @@ k_com(const uint32_t* __restrict__ first, TNode* nodes, const uint32_t* __restri
     uint32_t up = parent[node];
     if (up != END && up >= node) { set_error(st, JC_ERR_DEVICE_TIMEOUT); return; }
     node = up;
+  }
+}
+
+// The same climb where the tree is small and a cell's chain of child loads sets
+// the time: a cell's children come from its list (k_fill, any order), sorted
+// here by index, which is octant order, and all their centres are loaded at
+// once; the next cell's counts, list and parent load while this one is summed.
+// The sorted lists (END past the last child) are left for k_walk_warp. Large
+// trees keep k_com: they have climbs enough to hide the chains, and the lists
+// cost traffic. B200, tree build in us with k_com and with this (the
+// lists' writing in it): 400 bodies 56 -> 50, 10,000 91 -> 82, 65,537 119 -> 112,
+// 150,000 137 -> 132, R-MAT 262,144 168 -> 170, 1 M 400 -> 408.
+constexpr uint32_t KIDS_MAX_N = 196608u;
+__device__ __forceinline__ void sort8(uint32_t* k) {
+  // Batcher's odd-even merge network, 19 comparators
+  auto cx = [&](int a, int b) {
+    const uint32_t lo = min(k[a], k[b]), hi = max(k[a], k[b]);
+    k[a] = lo;
+    k[b] = hi;
+  };
+  cx(0, 1); cx(2, 3); cx(4, 5); cx(6, 7);
+  cx(0, 2); cx(1, 3); cx(4, 6); cx(5, 7);
+  cx(1, 2); cx(5, 6);
+  cx(0, 4); cx(1, 5); cx(2, 6); cx(3, 7);
+  cx(2, 4); cx(3, 5);
+  cx(1, 2); cx(3, 4); cx(5, 6);
+}
+
+__global__ void __launch_bounds__(128)
+k_com_kids(const uint32_t* __restrict__ first, TNode* nodes, const uint32_t* __restrict__ parent,
+           const uint32_t* __restrict__ nchild, uint32_t* __restrict__ kids, uint32_t* __restrict__ arrive, uint32_t n,
+           DevState* st) {
+  dev::dependent_launch_wait();
+  const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (st->error) return;
+  const uint32_t N = st->n_valid;
+  if (a >= N) return;
+  const uint32_t stop = first[a + 1];
+  if (stop == first[a]) return;
+  const uint32_t T = first[n];
+  // (who climbs: as in k_com)
+  const uint32_t leaf = stop - 1;
+  if (!JC_IN_BOUNDS(leaf, T, &st->error)) return;
+  uint32_t node = parent[leaf];
+  if (node == END || !JC_IN_BOUNDS(node, T, &st->error)) return;
+  uint32_t nc = nchild[node];
+  if ((nc >> 16) != (nc & 0xFFFFu) || leaf != node + 1u) return;
+  uint32_t up = parent[node];
+  uint4 l0 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)node);
+  uint4 l1 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)node + 4);
+  bool first_cell = true;
+  uint32_t guard = 0;
+  for (;;) {
+    if (++guard > 64u) { set_error(st, JC_ERR_DEVICE_TIMEOUT); return; }
+    if (!first_cell) {
+      const uint32_t cells = (nc & 0xFFFFu) - (nc >> 16);
+      if (cells != 1u) {
+        uint32_t old;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(arrive + node) : "memory");
+        if (old + 1u != cells) return;
+      }
+    }
+    first_cell = false;
+    const uint32_t cnt = nc & 0xFFFFu;
+    if (cnt > 8u || (up != END && up >= node)) { set_error(st, JC_ERR_DEVICE_TIMEOUT); return; }
+    uint32_t k[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if ((uint32_t)q >= cnt || k[q] >= T) k[q] = END;
+    sort8(k);
+    float4 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = k[q] != END ? __ldcg(&nodes[k[q]].cm) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t self = node, nxt = up;
+    if (nxt != END) {  // the next cell's words, behind the centres
+      nc = nchild[nxt];
+      up = parent[nxt];
+      l0 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)nxt);
+      l1 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)nxt + 4);
+    }
+    float tot = 0.0f, sx = 0.0f, sy = 0.0f, sz = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (k[q] != END) {
+        tot = __fadd_rn(tot, v[q].w);
+        sx = __fadd_rn(sx, __fmul_rn(v[q].x, v[q].w));
+        sy = __fadd_rn(sy, __fmul_rn(v[q].y, v[q].w));
+        sz = __fadd_rn(sz, __fmul_rn(v[q].z, v[q].w));
+      }
+    if (tot > 0.0f) {
+      sx = __fdiv_rn(sx, tot);
+      sy = __fdiv_rn(sy, tot);
+      sz = __fdiv_rn(sz, tot);
+    }
+    __stcg(&nodes[self].cm, make_float4(sx, sy, sz, tot));
+    *reinterpret_cast<uint4*>(kids + 8 * (size_t)self) = make_uint4(k[0], k[1], k[2], k[3]);
+    *reinterpret_cast<uint4*>(kids + 8 * (size_t)self + 4) = make_uint4(k[4], k[5], k[6], k[7]);
+    if (nxt == END) return;
+    node = nxt;
   }
 }
 
@@ -1250,6 +1357,178 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
     if (JC_IN_BOUNDS(body, n, &st->error)) frep[body] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   walk_counts_flush(n_inter, n_open, st);
+}
+
+// A warp per body, for graphs of so few bodies that a walk's chain of visits
+// (hundreds of node loads, one after another) is the whole cost. The nodes a
+// body meets are the root and the children of every cell it opens, whatever
+// order they are tested in; only the terms have to be added in pre-order, and a
+// node's index is its place in pre-order. So the warp tests the tree level by
+// level, 32 nodes at a time: opened cells put their children (k_com_kids's
+// lists) into the next level's queue, accepted nodes go into a list and a bitmap
+// over node indices. A population count of the bitmap below a node is its
+// term's rank; the lanes compute the terms into rank order, WW_TERMS at a time,
+// and one lane per axis adds them. Same terms, same roundings, same order as the
+// rope walk. A body that outgrows the queue or the list (or a tree past the
+// bitmap) is walked along the ropes by one lane. (Exact mode only: the tolerance
+// mode's fused accumulation has no separate terms.) Bound by instruction issue from
+// about 10,000 bodies on (it issues three times the rope walk's instructions).
+// B200, us a walk, k_walk_ahead and this, theta 0.8: 400 bodies (0.7) 39 -> 12,
+// 2,000 54 -> 18, 5,000 66 -> 34, 10,000 70 -> 61 (0.7: 89 -> 75), 15,000 69 -> 89.
+constexpr uint32_t WW_QUEUE = 512, WW_LIST = 1024, WW_TERMS = 256, WW_WARPS = 4;
+constexpr uint32_t WW_ROW = WW_TERMS + 4;  // axes 4 banks apart
+constexpr uint32_t WW_MAX_N = 10240u;
+constexpr float WW_MIN_THETA2 = 0.4f;      // below, lists outgrow their arrays
+inline uint32_t ww_words(uint32_t n) { return std::min(1024u, (2u * n + 8u + 63u) / 64u); }  // 64 nodes each
+constexpr size_t ww_warp_bytes(uint32_t words) {
+  // bitmap, ranks, list, then the two queues or the terms
+  const size_t q = 2 * 2 * (size_t)WW_QUEUE, t = 3 * 4 * (size_t)WW_ROW;
+  return ((8 * (size_t)words + 2 * (size_t)words + 15) / 16) * 16 + 2 * (size_t)WW_LIST + (q > t ? q : t);
+}
+
+__global__ void __launch_bounds__(32 * WW_WARPS)
+k_walk_warp(const TNode* __restrict__ nodes, const uint32_t* __restrict__ kids, const uint32_t* __restrict__ order,
+            const float4* __restrict__ pos, const float* __restrict__ degf, uint32_t n, KParams P, DevState* st,
+            float4* __restrict__ frep, uint32_t words) {
+  dev::dependent_launch_wait();
+  extern __shared__ uint4 ww_smem[];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  unsigned char* base = reinterpret_cast<unsigned char*>(ww_smem) + w * ww_warp_bytes(words);
+  unsigned long long* bits = reinterpret_cast<unsigned long long*>(base);
+  uint16_t* ranks = reinterpret_cast<uint16_t*>(base + 8 * (size_t)words);
+  uint16_t* list = reinterpret_cast<uint16_t*>(base + ((10 * (size_t)words + 15) / 16) * 16);
+  uint16_t* queue = list + WW_LIST;                       // two of WW_QUEUE
+  float* terms = reinterpret_cast<float*>(queue);         // [3][WW_ROW], after the traversal
+  const uint32_t T = st->error ? 0u : st->n_tree;
+  const uint32_t a = blockIdx.x * WW_WARPS + w;
+  if (a >= n) return;
+  const uint32_t body = order[a];
+  if (!JC_IN_BOUNDS(body, n, &st->error)) return;
+  if (T == 0u) {
+    if (lane == 0) frep[body] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
+  const float4 p = pos[body];
+  const float srd = __fmul_rn(P.scaling_ratio, degf[body]);
+  uint32_t n_acc = 0, n_open = 0;
+  bool ok = T <= 64u * words;
+  const uint32_t used = (T + 63u) / 64u;
+  if (ok) {
+    for (uint32_t k = lane; k < used; k += 32) bits[k] = 0ull;
+    if (lane == 0) queue[0] = 0;
+    __syncwarp();
+    uint16_t *cur = queue, *nxt = queue + WW_QUEUE;
+    uint32_t n_cur = 1, levels = 0;
+    while (n_cur && ok) {
+      uint32_t n_nxt = 0;
+      for (uint32_t k0 = 0; k0 < n_cur; k0 += 32) {
+        const bool have = k0 + lane < n_cur;
+        const uint32_t idx = have ? cur[k0 + lane] : 0u;
+        float4 c;
+        int4 m;
+        load_node(nodes + idx, c, m);
+        const uint4 l0 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)idx);
+        const uint4 l1 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)idx + 4);
+        const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
+        const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+        const bool leaf = m.y >= 0;
+        const bool use = have && (leaf ? (uint32_t)m.y != body : __int_as_float(m.z) < __fmul_rn(P.theta2, r2));
+        const bool open = have && !leaf && !use;
+        const uint32_t um = __ballot_sync(0xFFFFFFFFu, use), om = __ballot_sync(0xFFFFFFFFu, open);
+        if (use) {
+          const uint32_t at = n_acc + __popc(um & lt);
+          if (at < WW_LIST) list[at] = (uint16_t)idx;
+          atomicOr(reinterpret_cast<uint32_t*>(bits) + (idx >> 5), 1u << (idx & 31u));
+        }
+        n_acc += __popc(um);
+        n_open += __popc(om);
+        if (om) {
+          const uint32_t k[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+          uint32_t nc = 0;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) nc += (open && k[q] < T) ? 1u : 0u;
+          // children of the lanes below: nc <= 8 in four bit planes
+          uint32_t at = n_nxt, tot = 0;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const uint32_t bm = __ballot_sync(0xFFFFFFFFu, (nc >> b) & 1u);
+            at += __popc(bm & lt) << b;
+            tot += __popc(bm) << b;
+          }
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if ((uint32_t)q < nc && at + q < WW_QUEUE) nxt[at + q] = (uint16_t)k[q];
+          n_nxt += tot;
+        }
+      }
+      // (a level deeper than any octree's: a malformed tree)
+      ok = n_nxt <= WW_QUEUE && n_acc <= WW_LIST && ++levels <= 64u;
+      __syncwarp();
+      uint16_t* t = cur;
+      cur = nxt;
+      nxt = t;
+      n_cur = n_nxt;
+    }
+  }
+  if (!ok) {
+    // along the ropes, one lane
+    if (lane == 0) {
+      uint32_t ni = 0, no = 0;
+      walk_one<false>(nodes, body, p, srd, 0u, T, P.theta2, st, frep, ni, no);
+      atomicAdd(&st->n_inter, (unsigned long long)ni);
+      atomicAdd(&st->n_open, (unsigned long long)no);
+    }
+    return;
+  }
+  // ranks: accepted nodes before each word
+  uint32_t run = 0;
+  for (uint32_t k0 = 0; k0 < used; k0 += 32) {
+    const uint32_t c = k0 + lane < used ? (uint32_t)__popcll(bits[k0 + lane]) : 0u;
+    uint32_t v = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+      if ((int)lane >= o) v += y;
+    }
+    if (k0 + lane < used) ranks[k0 + lane] = (uint16_t)(run + v - c);
+    run += __shfl_sync(0xFFFFFFFFu, v, 31);
+  }
+  __syncwarp();
+  float sum = 0.0f;
+  for (uint32_t r0 = 0; r0 < n_acc; r0 += WW_TERMS) {
+    const uint32_t cnt = min(WW_TERMS, n_acc - r0);
+    for (uint32_t k = lane; k < n_acc; k += 32) {
+      const uint32_t idx = list[k];
+      const uint32_t r = ranks[idx >> 6] + (uint32_t)__popcll(bits[idx >> 6] & ((1ull << (idx & 63u)) - 1ull)) - r0;
+      if (r >= WW_TERMS) continue;
+      const float4 c = nodes[idx].cm;
+      const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
+      const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+      float fx = -0.0f, fy = -0.0f, fz = -0.0f;  // -0 + term = term, signed zeros included
+      rep_term<false>(dx, dy, dz, r2, srd, c.w, fx, fy, fz);
+      terms[r] = fx;
+      terms[WW_ROW + r] = fy;
+      terms[2 * WW_ROW + r] = fz;
+    }
+    if (lane < 3)  // whole groups of four: -0 leaves a sum as it is
+      for (uint32_t q = cnt; q < ((cnt + 3u) & ~3u); ++q) terms[lane * WW_ROW + q] = -0.0f;
+    __syncwarp();
+    if (lane < 3) {
+      const float4* t4 = reinterpret_cast<const float4*>(terms + lane * WW_ROW);
+#pragma unroll 8
+      for (uint32_t q = 0; q < (cnt + 3u) / 4u; ++q) {
+        const float4 v = t4[q];
+        sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
+      }
+    }
+    __syncwarp();
+  }
+  const float sy = __shfl_sync(0xFFFFFFFFu, sum, 1), sz = __shfl_sync(0xFFFFFFFFu, sum, 2);
+  if (lane == 0) {
+    frep[body] = make_float4(sum, sy, sz, 0.0f);
+    atomicAdd(&st->n_inter, (unsigned long long)n_acc);
+    atomicAdd(&st->n_open, (unsigned long long)n_open);
+  }
 }
 
 // ------------------------------------------------------ staged top --
@@ -2109,6 +2388,17 @@ __global__ void k_csr_balance(const int* __restrict__ balance, uint32_t* ok) {
   }
 }
 
+inline void launch_walk_warp(bool chained, const TNode* nodes, const uint32_t* kids, const uint32_t* order,
+                             const float4* pos, const float* degf, uint32_t n, const KParams& P, DevState* st,
+                             float4* frep, cudaStream_t s) {
+  const uint32_t words = ww_words(n);
+  const size_t smem = WW_WARPS * ww_warp_bytes(words);
+  if (smem > 48 * 1024)
+    JC_CUDA_CHECK(cudaFuncSetAttribute(k_walk_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  launch_chained(chained, s, cdiv(n, WW_WARPS), 32 * WW_WARPS, smem, k_walk_warp, nodes, kids, order, pos, degf, n,
+                 P, st, frep, words);
+}
+
 inline uint32_t tie_blocks(uint32_t n, uint32_t sms) { return std::max(1u, std::min(sms, cdiv(n, TIE_PART))); }
 
 inline void launch_tie_resort(const ulonglong2* key, uint32_t* val, uint32_t* val_alt, uint64_t* hi_sorted, uint32_t n,
@@ -2745,7 +3035,7 @@ class Fa2Engine : public Engine {
   DevBuf<int8_t> lcp_;  // prefix-length index: L, m1, m2 back to back
   LcpIndex lcpx_{};
   DevBuf<TNode> nodes_;
-  DevBuf<uint32_t> parent_, nchild_, arrive_, top_list_;
+  DevBuf<uint32_t> parent_, nchild_, arrive_, top_list_, kids_;
   DevBuf<uint4> top_;
   // batch (forest) layout
   std::vector<uint32_t> graph_off_host_{0u, 0u};
@@ -2844,6 +3134,7 @@ class Fa2Engine : public Engine {
     if (graph_off_host_.size() > 2) count_.alloc((size_t)n + 1);
     first_.alloc((size_t)n + 2);
     nodes_.alloc(tree_cap_); parent_.alloc(tree_cap_); nchild_.alloc(tree_cap_);
+    if (n <= KIDS_MAX_N && graph_off_host_.size() <= 2) kids_.alloc(8 * (size_t)tree_cap_);
     top_list_.alloc(TOP_MAX); top_.alloc(2 * TOP_MAX);
     arrive_.alloc(tree_cap_);
     const uint32_t nl = lcp_index_bytes(n), n2p = lcp_m2_bytes(nl);
@@ -2955,10 +3246,16 @@ class Fa2Engine : public Engine {
         ++L;
       }
       const bool stage = stage_top();
-      launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_fill, hi_.p, lcpx_, val_.p, first_.p, pos_.p, degf_.p, n, P,
-                     st, nodes_.p, parent_.p, nchild_.p, F, stage ? top_list_.p : nullptr);
-      launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_com, first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p, n,
-                     st);
+      const bool kl = kid_lists();
+      launch_chained(chain, stream_, cdiv(n, 256), 256, 0, kl ? k_fill<true> : k_fill<false>, hi_.p, lcpx_, val_.p,
+                     first_.p, pos_.p, degf_.p, n, P, st, nodes_.p, parent_.p, nchild_.p, F,
+                     stage ? top_list_.p : nullptr, kids_.p);
+      if (kl)
+        launch_chained(chain, stream_, cdiv(n, 128), 128, 0, k_com_kids, first_.p, nodes_.p, parent_.p, nchild_.p,
+                       kids_.p, arrive_.p, n, st);
+      else
+        launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_com, first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p,
+                       n, st);
       L += 2;
       if (stage) {
         k_top_build<<<1, 1024, 0, stream_>>>(nodes_.p, top_list_.p, st, top_.p);
@@ -3007,6 +3304,9 @@ class Fa2Engine : public Engine {
     else launch_brute_as<4>(P);
   }
 
+  // Child lists (k_com_kids, k_walk_warp): a single graph of few bodies.
+  bool kid_lists() const { return forest_.n_graphs == 1 && n_ <= KIDS_MAX_N; }
+
   // A small single graph's step chains its kernels as programmatic dependents
   // where nothing but kernels stands between them (no phase events). B200, us a
   // replayed step without and with: 400 nodes 104 -> 102, 2,000 134 -> 131, 10,000
@@ -3032,6 +3332,10 @@ class Fa2Engine : public Engine {
     }
     switch (walk_group_) {
       case 1:
+        if (!FAST && kid_lists() && n <= WW_MAX_N && P.theta2 >= WW_MIN_THETA2) {
+          launch_walk_warp(chained(), nodes_.p, kids_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, stream_);
+          break;
+        }
         if (forest_.n_graphs == 1 && n <= WALK_AHEAD_N) {
           launch_chained(chained(), stream_, grid.x, WALK_THREADS, 0, k_walk_ahead<FAST>, nodes_.p, val_.p, pos_.p,
                          degf_.p, n, P, st, frep_.p);
@@ -3253,7 +3557,7 @@ class Fa2Engine : public Engine {
     uint32_t need = 0;
     JC_CUDA_CHECK(cudaMemcpy(&need, first_.p + n_, sizeof(uint32_t), cudaMemcpyDeviceToHost));
     tree_cap_ = std::max<uint32_t>(need + need / 4 + 64, tree_cap_ * 2);
-    nodes_.free(); parent_.free(); nchild_.free(); arrive_.free();
+    nodes_.free(); parent_.free(); nchild_.free(); arrive_.free(); kids_.free();
     alloc_tree(n_);
     warn_accum_ |= hst_->warn;
     uint32_t zero = 0;
@@ -3290,7 +3594,7 @@ __host__ __device__ constexpr size_t na_round(size_t b) { return (b + 255) & ~(s
 
 struct NoAllocLayout {
   size_t st, bbox, pos4, frep, force4, old4, degf, stats, order, key, top_key, top_alt, val, val_alt,
-      first, totals, work, table, partials, nodes, parent, nchild, arrive, lcp, total;
+      first, totals, work, table, partials, nodes, parent, nchild, arrive, kids, lcp, total;
 };
 
 constexpr NoAllocLayout noalloc_layout() {
@@ -3320,6 +3624,7 @@ constexpr NoAllocLayout noalloc_layout() {
   L.parent = o; o += na_round(4 * C);
   L.nchild = o; o += na_round(4 * C);
   L.arrive = o; o += na_round(4 * C);
+  L.kids = o; o += na_round(32 * C);
   L.lcp = o; o += na_round(NOALLOC_LCP + NOALLOC_LCP / 32 + 32);
   L.total = o;
   return L;
@@ -3429,6 +3734,7 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   uint32_t* parent = (uint32_t*)(base + L.parent);
   uint32_t* nchild = (uint32_t*)(base + L.nchild);
   uint32_t* arrive = (uint32_t*)(base + L.arrive);
+  uint32_t* kids = (uint32_t*)(base + L.kids);
   int8_t* lcp = (int8_t*)(base + L.lcp);
   const LcpIndex X{lcp, lcp + NOALLOC_LCP, lcp + NOALLOC_LCP + NOALLOC_LCP / 32, NOALLOC_LCP / 32,
                    NOALLOC_LCP / 1024};
@@ -3473,11 +3779,14 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
     launch_chained(true, s, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key, val, key, n, st, 0);
     launch_tie_resort(key, val, val_alt, nullptr, n, 5, st, table, 16, s);
     launch_count(true, key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
-    launch_chained(true, s, cdiv(n, 256), 256, 0, k_fill, nullptr, X, val, first, pos4, degf, n, P, st, nodes, parent,
-                   nchild, F1, nullptr);
-    launch_chained(true, s, cdiv(n, 256), 256, 0, k_com, first, nodes, parent, nchild, arrive, n, st);
-    launch_chained(true, s, cdiv(n, WALK_THREADS), WALK_THREADS, 0, k_walk_ahead<false>, nodes, val, pos4, degf, n, P, st,
-                   frep);
+    launch_chained(true, s, cdiv(n, 256), 256, 0, k_fill<true>, nullptr, X, val, first, pos4, degf, n, P, st, nodes,
+                   parent, nchild, F1, nullptr, kids);
+    launch_chained(true, s, cdiv(n, 128), 128, 0, k_com_kids, first, nodes, parent, nchild, kids, arrive, n, st);
+    if (n <= WW_MAX_N && P.theta2 >= WW_MIN_THETA2)
+      launch_walk_warp(true, nodes, kids, val, pos4, degf, n, P, st, frep, s);
+    else
+      launch_chained(true, s, cdiv(n, WALK_THREADS), WALK_THREADS, 0, k_walk_ahead<false>, nodes, val, pos4, degf, n, P,
+                     st, frep);
     launch_chained(true, s, cdiv(n, ATT_THREADS), ATT_THREADS, 0, k_att, order, d_offsets, d_neighbors, pos4, frep, old4,
                    degf, P, st, force4, stats, partials, 1u);
   } catch (const Error&) {

@@ -264,3 +264,36 @@ def test_sort_tile_rules_bit_exact(jc, orc, n):
     e, r = one_step(jc, orc, g, jc.seed_uniform(n, 3, 7), theta=1.2)
     assert e.tree_info()["nodes"] == r["n_octree"]
     assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
+
+
+# the warp walk: its smallest graphs, whole and partial blocks of four warps,
+# both sides of its size rule (10,240) and of its theta rule (0.632), lists longer
+# than one batch of 256 terms; trees past its bitmap and queues it does not hold
+# (chains of close pairs, a dense ball at a small theta) go along the ropes
+@pytest.mark.parametrize("case", ["n1", "n2", "n3", "n7", "n8", "n9", "n1000", "n10240", "n10241", "theta0.63", "theta0.64",
+                                  "2d", "chains", "dense"])
+def test_warp_walk_bit_exact(jc, orc, case):
+    theta, n = 0.8, 3000
+    if case[0] == "n":
+        n = int(case[1:])
+    if case.startswith("theta"):
+        theta = float(case[5:])
+    if case == "dense":
+        theta, n = 0.64, 9000
+    pos = jc.seed_uniform(n, 2 if case == "2d" else 3, n)
+    if case == "chains":
+        p = pos.reshape(n, 3)
+        p[1:2001:2] = p[0:2000:2] + np.array([3e-6, -2e-6, 1e-6], np.float32)
+    g = jc.gen_scale_free(n, 2, n) if n > 3 else jc.gen_path(n)
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params({"theta": theta})
+    e.init(g, pos)
+    o = orc.Fa2(g, pos, bh=True, theta=theta)
+    o.set_tree_capacity(1 << 20)
+    for _ in range(3):
+        e.step()
+        o.step()
+        r = o.get()
+        assert e.tree_info()["nodes"] == r["n_octree"]
+        assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
+        assert e.walk_counts() == (r["n_inter"], r["n_open"])
