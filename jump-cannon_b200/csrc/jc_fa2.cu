@@ -339,6 +339,22 @@ __device__ __forceinline__ void body_key(const float4 p, float cx, float cy, flo
   }
 }
 
+// (1 << 32) | the 32 z octant bits of every body of a graph whose finite bodies
+// share one z (lo == hi), else 0: the keys' z tests, once.
+__device__ __forceinline__ uint64_t flat_z_bits(float lo, float hi, const float4 root) {
+  if (!(lo == hi && isfinite(lo))) return 0;
+  float cz = root.z, h = root.w;
+  uint32_t bits = 0;
+  for (int l = 0; l < 32; ++l) {
+    const bool up = lo >= cz;
+    bits |= (up ? 1u : 0u) << l;
+    const float hh = __fmul_rn(h, 0.5f);
+    cz = __fadd_rn(cz, up ? hh : -hh);
+    h = hh;
+  }
+  return (1ull << 32) | bits;
+}
+
 // Non-finite bodies of a warp into the counters.
 __device__ __forceinline__ void count_invalid(bool invalid, DevState* st) {
   const uint32_t bal = __ballot_sync(0xFFFFFFFFu, invalid);
@@ -1749,20 +1765,7 @@ k_bbox_roots(Forest F, DevState* st) {
                                   __fmul_rn(0.5f, __fadd_rn(r[2], r[5])), __fmul_rn(half, 1.05f));
   F.roots[g] = root;
   F.tree_root[g] = END;
-  uint64_t zf = 0;
-  if (r[2] == r[5] && isfinite(r[2])) {  // one z for every finite body: k_keys' z tests, once
-    float cz = root.z, h = root.w;
-    uint32_t bits = 0;
-    for (int l = 0; l < 32; ++l) {
-      const bool up = r[2] >= cz;
-      bits |= (up ? 1u : 0u) << l;
-      const float hh = __fmul_rn(h, 0.5f);
-      cz = __fadd_rn(cz, up ? hh : -hh);
-      h = hh;
-    }
-    zf = (1ull << 32) | bits;
-  }
-  F.zflat[g] = zf;
+  F.zflat[g] = flat_z_bits(r[2], r[5], root);
   if (g == 0) {
     st->n_invalid = 0;
     st->tie = 0;
@@ -2233,6 +2236,7 @@ __global__ void k_unpack_xyz(const float* __restrict__ xyz, uint32_t n, float4* 
 }
 
 #include "jc_fa2_tile.cuh"
+#include "jc_fa2_graph.cuh"
 
 // ============================================================== host ==
 template <typename T>
@@ -3042,6 +3046,9 @@ class Fa2Engine : public Engine {
   Forest forest_{1, 0, 21, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
                  nullptr};
   DevBuf<uint32_t> node_graph_, graph_off_, tree_root_, tree_end_;
+  uint32_t biggest_ = 0;              // bodies of a batch's largest graph
+  DevBuf<uint32_t> graph_order_;      // graph ids, largest first
+  DevBuf<GraphTally> graph_tally_;
   DevBuf<float4> roots_;
   DevBuf<float2> gspeed_;
   DevBuf<uint64_t> zflat_;
@@ -3073,7 +3080,18 @@ class Fa2Engine : public Engine {
     forest_.n_graphs = G;
     forest_.gbits = 0;
     forest_.lh = 21;
+    biggest_ = 0;
     if (G <= 1) return;
+    std::vector<uint32_t> order(G);
+    auto size = [&](uint32_t g) { return graph_off_host_[g + 1] - graph_off_host_[g]; };
+    for (uint32_t g = 0; g < G; ++g) {
+      order[g] = g;
+      biggest_ = std::max(biggest_, size(g));
+    }
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return size(a) > size(b); });
+    graph_order_.alloc(G); graph_tally_.alloc(1);
+    JC_CUDA_CHECK(cudaMemcpyAsync(graph_order_.p, order.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, stream_));
+    JC_CUDA_CHECK(cudaMemsetAsync(graph_tally_.p, 0, sizeof(GraphTally), stream_));
     uint32_t gb = 1;
     while ((1u << gb) < G) ++gb;
     forest_.gbits = gb;
@@ -3213,53 +3231,58 @@ class Fa2Engine : public Engine {
     record_phase(0);
     if (bh_) {
       const Forest F = forest_;
-      if (F.n_graphs > 1) {
-        k_bbox_slices<<<F.n_slices, 256, 0, stream_>>>(pos_.p, F);
-        k_bbox_roots<<<cdiv(F.n_graphs, 8), 256, 0, stream_>>>(F, st);
+      if (graph_build()) {
+        launch_graph_build(P);
         ++L;
       } else {
-        // (4 passes: digit counts, tile counters, look-back words)
-        k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, stream_>>>(pos_.p, n, bbox_part_.p, st, sort_work_.p,
-                                                             (uint32_t)dev::sort_work_words(n, 4));
-      }
-      if (F.n_graphs > 1) {
-        // the top 48 bits (the graph id takes up to 16 of them), then the runs
-        k_keys_batch<<<cdiv(n, 256), 256, 0, stream_>>>(pos_.p, n, st, key_.p, hi_.p, val_.p, F);
-        L += dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nullptr, 16, 64,
-                                             sort_work_.p, &st->error, nullptr, stream_);
-        k_seg_fix<uint64_t><<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, key_.p, n, st, 16);
-      } else {
-        // the top 32 bits (ten levels), then the runs
-        launch_chained(chain, stream_, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos_.p, n, st, key_.p,
-                       top_key_.p, val_.p, sort_work_.p);
-        L += dev::radix_passes<uint32_t>(top_key_.p, val_.p, top_alt_.p, val_alt_.p, n, nullptr, 0, 4, sort_work_.p,
-                                         &st->error, nullptr, stream_, chain);
-        launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key_.p, val_.p, key_.p, n, st, 0);
-      }
-      launch_tie_resort(key_.p, val_.p, val_alt_.p, F.n_graphs > 1 ? hi_.p : nullptr, n, (3 * (32 - F.lh) + 7) / 8, st,
-                        tie_table_.p, sms_, stream_);
-      L += 4;
-      L += launch_count(chain, key_.p, val_.p, n, st, first_.p, totals_.p, scan_sums_.p, F, lcpx_, P, nchild_.p, arrive_.p,
-                        stream_);
-      if (F.n_graphs > 1) {
-        k_graph_trees<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, first_.p, st, F);
-        ++L;
-      }
-      const bool stage = stage_top();
-      const bool kl = kid_lists();
-      launch_chained(chain, stream_, cdiv(n, 256), 256, 0, kl ? k_fill<true> : k_fill<false>, hi_.p, lcpx_, val_.p,
-                     first_.p, pos_.p, degf_.p, n, P, st, nodes_.p, parent_.p, nchild_.p, F,
-                     stage ? top_list_.p : nullptr, kids_.p);
-      if (kl)
-        launch_chained(chain, stream_, cdiv(n, 128), 128, 0, k_com_kids, first_.p, nodes_.p, parent_.p, nchild_.p,
-                       kids_.p, arrive_.p, n, st);
-      else
-        launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_com, first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p,
-                       n, st);
-      L += 2;
-      if (stage) {
-        k_top_build<<<1, 1024, 0, stream_>>>(nodes_.p, top_list_.p, st, top_.p);
-        ++L;
+        if (F.n_graphs > 1) {
+          k_bbox_slices<<<F.n_slices, 256, 0, stream_>>>(pos_.p, F);
+          k_bbox_roots<<<cdiv(F.n_graphs, 8), 256, 0, stream_>>>(F, st);
+          ++L;
+        } else {
+          // (4 passes: digit counts, tile counters, look-back words)
+          k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, stream_>>>(pos_.p, n, bbox_part_.p, st, sort_work_.p,
+                                                               (uint32_t)dev::sort_work_words(n, 4));
+        }
+        if (F.n_graphs > 1) {
+          // the top 48 bits (the graph id takes up to 16 of them), then the runs
+          k_keys_batch<<<cdiv(n, 256), 256, 0, stream_>>>(pos_.p, n, st, key_.p, hi_.p, val_.p, F);
+          L += dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nullptr, 16, 64,
+                                               sort_work_.p, &st->error, nullptr, stream_);
+          k_seg_fix<uint64_t><<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, key_.p, n, st, 16);
+        } else {
+          // the top 32 bits (ten levels), then the runs
+          launch_chained(chain, stream_, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos_.p, n, st, key_.p,
+                         top_key_.p, val_.p, sort_work_.p);
+          L += dev::radix_passes<uint32_t>(top_key_.p, val_.p, top_alt_.p, val_alt_.p, n, nullptr, 0, 4, sort_work_.p,
+                                           &st->error, nullptr, stream_, chain);
+          launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key_.p, val_.p, key_.p, n, st, 0);
+        }
+        launch_tie_resort(key_.p, val_.p, val_alt_.p, F.n_graphs > 1 ? hi_.p : nullptr, n, (3 * (32 - F.lh) + 7) / 8, st,
+                          tie_table_.p, sms_, stream_);
+        L += 4;
+        L += launch_count(chain, key_.p, val_.p, n, st, first_.p, totals_.p, scan_sums_.p, F, lcpx_, P, nchild_.p, arrive_.p,
+                          stream_);
+        if (F.n_graphs > 1) {
+          k_graph_trees<<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, first_.p, st, F);
+          ++L;
+        }
+        const bool stage = stage_top();
+        const bool kl = kid_lists();
+        launch_chained(chain, stream_, cdiv(n, 256), 256, 0, kl ? k_fill<true> : k_fill<false>, hi_.p, lcpx_, val_.p,
+                       first_.p, pos_.p, degf_.p, n, P, st, nodes_.p, parent_.p, nchild_.p, F,
+                       stage ? top_list_.p : nullptr, kids_.p);
+        if (kl)
+          launch_chained(chain, stream_, cdiv(n, 128), 128, 0, k_com_kids, first_.p, nodes_.p, parent_.p, nchild_.p,
+                         kids_.p, arrive_.p, n, st);
+        else
+          launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_com, first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p,
+                         n, st);
+        L += 2;
+        if (stage) {
+          k_top_build<<<1, 1024, 0, stream_>>>(nodes_.p, top_list_.p, st, top_.p);
+          ++L;
+        }
       }
       record_phase(1);
       launch_walk(P, st);
@@ -3285,6 +3308,26 @@ class Fa2Engine : public Engine {
     L += 2;
     JC_CUDA_CHECK(cudaGetLastError());
     return L;
+  }
+
+  // A batch whose largest graph a CTA can sort in shared memory.
+  bool graph_build() const { return forest_.n_graphs > 1 && biggest_ <= GB_MAX_N; }
+
+  template <int T>
+  void launch_graph_build_as(const KParams& P) {
+    const uint32_t items = gb_items(biggest_);
+    const size_t smem = gb_smem(items, T);
+    if (smem > 32 * 1024)
+      JC_CUDA_CHECK(cudaFuncSetAttribute(k_graph_build<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_graph_build<T><<<forest_.n_graphs, T, smem, stream_>>>(pos_.p, degf_.p, forest_, graph_order_.p, key_.p, val_.p,
+                                                             first_.p + n_, nodes_.p, parent_.p, P, state_.p,
+                                                             graph_tally_.p, items);
+  }
+
+  void launch_graph_build(const KParams& P) {
+    if (biggest_ > GB_MIDDLE) launch_graph_build_as<1024>(P);
+    else if (biggest_ > GB_SMALL) launch_graph_build_as<512>(P);
+    else launch_graph_build_as<256>(P);
   }
 
   template <int I>

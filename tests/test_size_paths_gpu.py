@@ -297,3 +297,46 @@ def test_warp_walk_bit_exact(jc, orc, case):
         assert e.tree_info()["nodes"] == r["n_octree"]
         assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
         assert e.walk_counts() == (r["n_inter"], r["n_open"])
+
+
+# a batch's trees built one CTA a graph: graphs around the blocks of 32, 256 and
+# 1,024 bodies, each largest size on both sides of the thread and size rules (past
+# 8,192 the forest's kernels), one body and none; runs of equal tops that need the
+# whole key; close pairs whose chains of cells outgrow the shared lists, the ropes
+# and the tree's first capacity; whole keys repeated; bodies at no position
+@pytest.mark.parametrize("case", ["edges", "2048", "2049", "4096", "4097", "8192", "8193", "2d", "runs", "runs8193", "chains",
+                                  "repeats", "nan", "nan8193"])
+def test_batch_trees_equal_single_engines(jc, case):
+    big = int(case[-4:]) if case[-4:].isdigit() else 2000
+    sizes = [1, 2, 3, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025] if case == "edges" else [50, big, 1, 700, min(big, 2000)]
+    graphs = [jc.gen_scale_free(n, 2, n) if n > 3 else jc.gen_path(n) for n in sizes]
+    pos = [jc.seed_uniform(n, 2 if case == "2d" else 3, 3 * n) for n in sizes]
+    if case.startswith("runs"):
+        pos = [crowded(jc, n, 3.0e4, 11) if n > 40 else p for n, p in zip(sizes, pos)]
+    for n, p in zip(sizes, pos):
+        p = p.reshape(n, 3)
+        if case == "chains" and n > 40:
+            p[1:n - 1:2] = p[0:n - 2:2] + np.array([3e-6, -2e-6, 1e-6], np.float32)
+        if case == "repeats" and n > 40:
+            p[40:80 if n > 80 else n] = p[:min(n, 80) - 40]
+        if case.startswith("nan"):
+            p[0 if n < 40 else 7, 1] = np.nan
+    b = jc.LayoutEngine("fa2-bh")
+    b.set_params({"theta": 0.8})
+    b.init_batch(graphs, pos)
+    es = []
+    for g, p in zip(graphs, pos):
+        e = jc.LayoutEngine("fa2-bh")
+        e.set_params({"theta": 0.8, "hub_threshold": 1 << 30, "warp_threshold": 1 << 30})
+        e.init(g, p)
+        es.append(e)
+    for _ in range(3):
+        b.step_many(1)
+        for e in es:
+            e.step_many(1)
+        for x, y in ((b.forces()[0], [e.forces()[0] for e in es]), (b.positions(), [e.positions() for e in es])):
+            y = np.concatenate(y)
+            assert np.array_equal(np.isnan(x), np.isnan(y))
+            assert np.array_equal(bits(x)[~np.isnan(x)], bits(y)[~np.isnan(y)])
+        assert b.tree_info()["nodes"] == sum(e.tree_info()["nodes"] for e in es)
+        assert b.walk_counts() == tuple(sum(c) for c in zip(*(e.walk_counts() for e in es)))
