@@ -1305,14 +1305,15 @@ __device__ __forceinline__ void walk_counts_flush(uint32_t n_inter, uint32_t n_o
 // division no longer stands between a visit and the next load. It takes 38
 // registers, so it is for graphs that do not fill the SMs with warps, where a
 // walk is one latency chain. B200, us a walk, k_walk_rope and this: 400 nodes 58
-// -> 40, 10,000 102 -> 69, 65,537 75 -> 55; R-MAT 262,144 nodes 136 -> 153.
+// -> 40, 10,000 102 -> 69, 65,537 75 -> 55; R-MAT 262,144 nodes 136 -> 153. A batch's
+// step, us: 100 graphs, 52,671 bodies 122 -> 112, 500 graphs, 74,429 bodies 89 -> 80.
 // (Blocks of 64 spread 10,000 bodies over every SM but share fewer nodes in L1:
 // 74. Fewer bodies per warp: no gain from 16, slower below 8.)
 constexpr uint32_t WALK_AHEAD_N = 148u * 1024u;
 template <bool FAST>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, const float4* __restrict__ pos,
-             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep) {
+             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep, Forest F) {
   dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t T = st->error ? 0u : st->n_tree;
@@ -1323,10 +1324,10 @@ k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order
     const float4 p = pos[body];
     const float srd = __fmul_rn(P.scaling_ratio, degf[body]);
     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-    uint32_t idx = T > 0u ? 0u : END;
+    uint32_t idx = T == 0u ? END : F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
     float4 c;
     int4 m;
-    if (idx < T) load_node(nodes, c, m);
+    if (idx < T) load_node(nodes + idx, c, m);
     while (idx < T) {
       const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
       const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
@@ -3379,9 +3380,9 @@ class Fa2Engine : public Engine {
           launch_walk_warp(chained(), nodes_.p, kids_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, stream_);
           break;
         }
-        if (forest_.n_graphs == 1 && n <= WALK_AHEAD_N) {
+        if (n <= WALK_AHEAD_N) {
           launch_chained(chained(), stream_, grid.x, WALK_THREADS, 0, k_walk_ahead<FAST>, nodes_.p, val_.p, pos_.p,
-                         degf_.p, n, P, st, frep_.p);
+                         degf_.p, n, P, st, frep_.p, forest_);
           break;
         }
         launch_chained(chained(), stream_, grid.x, WALK_THREADS, 0, k_walk_rope<FAST>, nodes_.p, val_.p, pos_.p, degf_.p, n,
@@ -3829,7 +3830,7 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
       launch_walk_warp(true, nodes, kids, val, pos4, degf, n, P, st, frep, s);
     else
       launch_chained(true, s, cdiv(n, WALK_THREADS), WALK_THREADS, 0, k_walk_ahead<false>, nodes, val, pos4, degf, n, P,
-                     st, frep);
+                     st, frep, F1);
     launch_chained(true, s, cdiv(n, ATT_THREADS), ATT_THREADS, 0, k_att, order, d_offsets, d_neighbors, pos4, frep, old4,
                    degf, P, st, force4, stats, partials, 1u);
   } catch (const Error&) {

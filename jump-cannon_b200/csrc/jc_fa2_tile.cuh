@@ -81,29 +81,34 @@ __device__ __forceinline__ void load_node_c(const TNode* p, float4& cm, int4& me
 }
 
 // The rope walk of one body over its graph's tree (local node indices,
-// root 0, T nodes); the same visit sequence and terms as walk_one.
+// root 0, T nodes); the same visit sequence and terms as walk_one. The next node
+// loads before the current term is added (k_walk_ahead); the kernel's 64 registers
+// hold it. B200, us a step of this schedule: 1,000 graphs of 50 to 2,000 bodies 457 ->
+// 408, 2,000 of 100 to 1,000 341 -> 309, 4,000 of 100 to 4,000 1,737 -> 1,543.
 template <bool FAST>
 __device__ __forceinline__ float4 tile_walk(const TNode* __restrict__ nodes, uint32_t body, const float4 p, float srd,
                                             uint32_t T, float theta2, bool& bad, uint32_t& n_inter,
                                             uint32_t& n_open) {
   float fx = 0.0f, fy = 0.0f, fz = 0.0f;
   uint32_t idx = 0;
+  float4 c;
+  int4 m;
+  load_node_c(nodes, c, m);  // (T > 0)
   while (idx < T) {
-    float4 c;
-    int4 m;
-    load_node_c(nodes + idx, c, m);
     const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
     const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
     const bool leaf = m.y >= 0;
     const bool use = leaf ? (uint32_t)m.y != body : __int_as_float(m.z) < __fmul_rn(theta2, r2);
+    const bool descend = !leaf && !use;
+    const uint32_t next = descend ? idx + 1u : (uint32_t)m.x;
+    const float mass = c.w;
+    if (next <= idx) break;
+    if (next < T) load_node_c(nodes + next, c, m);  // before the term: see k_walk_ahead
     if (use) {
-      rep_term<FAST>(dx, dy, dz, r2, srd, c.w, fx, fy, fz);
+      rep_term<FAST>(dx, dy, dz, r2, srd, mass, fx, fy, fz);
       ++n_inter;
     }
-    const bool descend = !leaf && !use;
     n_open += descend ? 1u : 0u;
-    const uint32_t next = descend ? idx + 1u : (uint32_t)m.x;
-    if (next <= idx) break;
     idx = next;
   }
   if (idx != END) bad = true;

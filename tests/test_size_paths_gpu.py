@@ -305,10 +305,12 @@ def test_warp_walk_bit_exact(jc, orc, case):
 # whole key; close pairs whose chains of cells outgrow the shared lists, the ropes
 # and the tree's first capacity; whole keys repeated; bodies at no position
 @pytest.mark.parametrize("case", ["edges", "2048", "2049", "4096", "4097", "8192", "8193", "2d", "runs", "runs8193", "chains",
-                                  "repeats", "nan", "nan8193"])
+                                  "repeats", "nan", "nan8193", "many"])
 def test_batch_trees_equal_single_engines(jc, case):
     big = int(case[-4:]) if case[-4:].isdigit() else 2000
     sizes = [1, 2, 3, 31, 32, 33, 255, 256, 257, 1023, 1024, 1025] if case == "edges" else [50, big, 1, 700, min(big, 2000)]
+    if case == "many":  # more bodies than the walk's size rule (151,552)
+        sizes = [8000 - k for k in range(20)]
     graphs = [jc.gen_scale_free(n, 2, n) if n > 3 else jc.gen_path(n) for n in sizes]
     pos = [jc.seed_uniform(n, 2 if case == "2d" else 3, 3 * n) for n in sizes]
     if case.startswith("runs"):
