@@ -1048,7 +1048,7 @@ k_com(const uint32_t* __restrict__ first, TNode* nodes, const uint32_t* __restri
 // The sorted lists (END past the last child) are left for k_walk_warp. Large
 // trees keep k_com: they have climbs enough to hide the chains, and the lists
 // cost traffic. B200, tree build in us with k_com and with this (the
-// lists' writing in it): 400 bodies 56 -> 50, 10,000 91 -> 82, 65,537 119 -> 112,
+// lists' writing in it): 10,000 bodies 91 -> 82, 65,537 119 -> 112,
 // 150,000 137 -> 132, R-MAT 262,144 168 -> 170, 1 M 400 -> 408.
 constexpr uint32_t KIDS_MAX_N = 196608u;
 __device__ __forceinline__ void sort8(uint32_t* k) {
@@ -1381,8 +1381,8 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
 // body meets are the root and the children of every cell it opens, whatever
 // order they are tested in; only the terms have to be added in pre-order, and a
 // node's index is its place in pre-order. So the warp tests the tree level by
-// level, 32 nodes at a time: opened cells put their children (k_com_kids's
-// lists) into the next level's queue, accepted nodes go into a list and a bitmap
+// level, 32 nodes at a time: opened cells put their children (the lists of
+// k_com_kids or k_graph_build) into the next level's queue, accepted nodes go into a list and a bitmap
 // over node indices. A population count of the bitmap below a node is its
 // term's rank; the lanes compute the terms into rank order, WW_TERMS at a time,
 // and one lane per axis adds them. Same terms, same roundings, same order as the
@@ -2393,6 +2393,30 @@ __global__ void k_csr_balance(const int* __restrict__ balance, uint32_t* ok) {
   }
 }
 
+template <int T>
+inline void launch_graph_build_as(const float4* pos, const float* degf, const Forest& F, uint32_t biggest,
+                                  const uint32_t* order, ulonglong2* key, uint32_t* val, uint32_t* first_total, TNode* nodes,
+                                  uint32_t* cells, const KParams& P, DevState* st, GraphTally* tally, uint32_t* kids,
+                                  cudaStream_t s) {
+  const uint32_t items = gb_items(biggest);
+  const size_t smem = gb_smem(items, T);
+  if (smem > 32 * 1024)
+    JC_CUDA_CHECK(cudaFuncSetAttribute(k_graph_build<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_graph_build<T><<<F.n_graphs, T, smem, s>>>(pos, degf, F, order, key, val, first_total, nodes, cells, P, st, tally, items,
+                                               kids);
+}
+
+// The trees of a batch, or of one small graph (kids: the child lists its walk reads).
+inline void launch_graph_build_kernel(const float4* pos, const float* degf, const Forest& F, uint32_t biggest,
+                                      const uint32_t* order, ulonglong2* key, uint32_t* val, uint32_t* first_total,
+                                      TNode* nodes, uint32_t* cells, const KParams& P, DevState* st, GraphTally* tally,
+                                      uint32_t* kids, cudaStream_t s) {
+  auto launch = launch_graph_build_as<256>;
+  if (F.n_graphs == 1 ? biggest > GB_SINGLE_256 : biggest > GB_SMALL) launch = launch_graph_build_as<512>;
+  if (F.n_graphs == 1 ? biggest > GB_SINGLE_512 : biggest > GB_MIDDLE) launch = launch_graph_build_as<1024>;
+  launch(pos, degf, F, biggest, order, key, val, first_total, nodes, cells, P, st, tally, kids, s);
+}
+
 inline void launch_walk_warp(bool chained, const TNode* nodes, const uint32_t* kids, const uint32_t* order,
                              const float4* pos, const float* degf, uint32_t n, const KParams& P, DevState* st,
                              float4* frep, cudaStream_t s) {
@@ -3082,6 +3106,8 @@ class Fa2Engine : public Engine {
     forest_.gbits = 0;
     forest_.lh = 21;
     biggest_ = 0;
+    graph_tally_.alloc(1);
+    JC_CUDA_CHECK(cudaMemsetAsync(graph_tally_.p, 0, sizeof(GraphTally), stream_));
     if (G <= 1) return;
     std::vector<uint32_t> order(G);
     auto size = [&](uint32_t g) { return graph_off_host_[g + 1] - graph_off_host_[g]; };
@@ -3090,9 +3116,8 @@ class Fa2Engine : public Engine {
       biggest_ = std::max(biggest_, size(g));
     }
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return size(a) > size(b); });
-    graph_order_.alloc(G); graph_tally_.alloc(1);
+    graph_order_.alloc(G);
     JC_CUDA_CHECK(cudaMemcpyAsync(graph_order_.p, order.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, stream_));
-    JC_CUDA_CHECK(cudaMemsetAsync(graph_tally_.p, 0, sizeof(GraphTally), stream_));
     uint32_t gb = 1;
     while ((1u << gb) < G) ++gb;
     forest_.gbits = gb;
@@ -3311,24 +3336,16 @@ class Fa2Engine : public Engine {
     return L;
   }
 
-  // A batch whose largest graph a CTA can sort in shared memory.
-  bool graph_build() const { return forest_.n_graphs > 1 && biggest_ <= GB_MAX_N; }
-
-  template <int T>
-  void launch_graph_build_as(const KParams& P) {
-    const uint32_t items = gb_items(biggest_);
-    const size_t smem = gb_smem(items, T);
-    if (smem > 32 * 1024)
-      JC_CUDA_CHECK(cudaFuncSetAttribute(k_graph_build<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_graph_build<T><<<forest_.n_graphs, T, smem, stream_>>>(pos_.p, degf_.p, forest_, graph_order_.p, key_.p, val_.p,
-                                                             first_.p + n_, nodes_.p, parent_.p, P, state_.p,
-                                                             graph_tally_.p, items);
+  // A batch whose largest graph a CTA can sort in shared memory; a single graph
+  // of so few bodies that one CTA is done before the device-wide passes are.
+  bool graph_build() const {
+    return forest_.n_graphs > 1 ? biggest_ <= GB_MAX_N : n_ <= GB_SINGLE_N && !stage_top();
   }
 
   void launch_graph_build(const KParams& P) {
-    if (biggest_ > GB_MIDDLE) launch_graph_build_as<1024>(P);
-    else if (biggest_ > GB_SMALL) launch_graph_build_as<512>(P);
-    else launch_graph_build_as<256>(P);
+    const bool one = forest_.n_graphs == 1;
+    launch_graph_build_kernel(pos_.p, degf_.p, forest_, one ? n_ : biggest_, graph_order_.p, key_.p, val_.p, first_.p + n_,
+                              nodes_.p, parent_.p, P, state_.p, graph_tally_.p, one ? kids_.p : nullptr, stream_);
   }
 
   template <int I>

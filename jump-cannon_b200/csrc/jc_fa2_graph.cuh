@@ -1,4 +1,4 @@
-// Octrees of a batch of small graphs, one CTA per graph.
+// Octrees of a batch of small graphs, one CTA per graph, or of one small graph.
 //
 // Included by jc_fa2.cu after the device helpers it reuses (TNode, DevState,
 // KParams, Forest, body_key, key_after, lcp_levels, the prefix-length index). A
@@ -40,6 +40,11 @@ constexpr uint32_t GB_MAX_N = 8192;   // bodies of the largest graph
 // 8,000 379 with 512, 307 with 1,024.
 constexpr uint32_t GB_SMALL = 2048;
 constexpr uint32_t GB_MIDDLE = 4096;
+// A single graph: one launch on one SM instead of eleven over all of them. B200, us a
+// step, those and this with 256, 512 and 1,024 threads: 20 bodies 47, 29, 31, 37; 400
+// 66, 41, 40, 45; 1,000 78, 53, 51, 55; 2,000 86, 78, 70, 72; 3,000 97, 125, 89, 91;
+// 4,000 103, 154, 109, 108.
+constexpr uint32_t GB_SINGLE_N = 3072, GB_SINGLE_256 = 256, GB_SINGLE_512 = GB_SINGLE_N;
 constexpr int GB_DEPTHS = 33;        // cell depths 0..32
 
 template <int T>
@@ -136,7 +141,7 @@ __global__ void __launch_bounds__(T, 1024 / T)
 k_graph_build(const float4* __restrict__ pos, const float* __restrict__ degf, Forest F,
               const uint32_t* __restrict__ order, ulonglong2* key, uint32_t* __restrict__ val,
               uint32_t* __restrict__ first_total, TNode* nodes, uint32_t* cells, KParams P, DevState* st,
-              GraphTally* tally, uint32_t items) {
+              GraphTally* tally, uint32_t items, uint32_t* kids) {
   extern __shared__ __align__(1024) unsigned char gb_raw[];
   __shared__ GraphShared<T> S;
   uint32_t* k0 = reinterpret_cast<uint32_t*>(gb_raw);
@@ -146,9 +151,10 @@ k_graph_build(const float4* __restrict__ pos, const float* __restrict__ degf, Fo
   uint16_t* v1 = v0 + items;
   const uint32_t tid = threadIdx.x;
   const int lane = tid & 31, w = tid >> 5;
-  const uint32_t g = order[blockIdx.x];
-  const uint32_t B = F.graph_off[g];
-  const uint32_t n = F.graph_off[g + 1] - B;
+  const bool single = F.n_graphs == 1;
+  const uint32_t g = single ? 0u : order[blockIdx.x];
+  const uint32_t B = single ? 0u : F.graph_off[g];
+  const uint32_t n = single ? P.n : F.graph_off[g + 1] - B;
   key += B;
   val += B;
   pos += B;
@@ -332,7 +338,7 @@ k_graph_build(const float4* __restrict__ pos, const float* __restrict__ degf, Fo
     if (tid == 0) {
       first[n] = tot;
       S.base = atomicAdd(&tally->cursor, tot);
-      F.tree_root[g] = tot ? S.base : END;
+      if (!single) F.tree_root[g] = tot ? S.base : END;
     }
   }
   __syncthreads();
@@ -454,26 +460,33 @@ k_graph_build(const float4* __restrict__ pos, const float* __restrict__ degf, Fo
           if (linked) {
             const uint32_t end = link[v];
             uint32_t c = v + 1;
-            for (int half = 0; half < 2 && c < end; ++half) {
+            for (int half = 0; half < 2 && (kids || c < end); ++half) {
               float4 kid[4];
-              int k = 0;
+              uint32_t id[4];
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
+              for (int i = 0; i < 4; ++i) {
+                id[i] = END;
                 if (c < end) {
+                  id[i] = c;
                   kid[i] = t[c].cm;
                   c = link[c];
-                  k = i + 1;
                 }
+              }
+              if (kids) reinterpret_cast<uint4*>(kids)[2 * (size_t)v + half] = make_uint4(id[0], id[1], id[2], id[3]);
 #pragma unroll
               for (int i = 0; i < 4; ++i)
-                if (i < k) add(kid[i]);
+                if (id[i] != END) add(kid[i]);
             }
             if (c != end) bad = true;
           } else {
             const uint32_t end = (uint32_t)t[v].meta.x;
-            uint32_t c = v + 1, kids = 0;
+            uint32_t c = v + 1, k = 0;
+            if (kids)
+              for (int i = 0; i < 8; ++i) kids[8 * (size_t)v + i] = END;
             while (base + c != end) {
-              if (c >= tot || ++kids > 8u) { bad = true; break; }
+              if (c >= tot || k >= 8u) { bad = true; break; }
+              if (kids) kids[8 * (size_t)v + k] = c;
+              ++k;
               add(t[c].cm);
               const uint32_t nx = (uint32_t)t[c].meta.x;
               if (nx == END && end == END) break;

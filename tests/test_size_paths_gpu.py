@@ -342,3 +342,33 @@ def test_batch_trees_equal_single_engines(jc, case):
             assert np.array_equal(bits(x)[~np.isnan(x)], bits(y)[~np.isnan(y)])
         assert b.tree_info()["nodes"] == sum(e.tree_info()["nodes"] for e in es)
         assert b.walk_counts() == tuple(sum(c) for c in zip(*(e.walk_counts() for e in es)))
+
+
+# a single graph's tree in one launch: both sides of its thread and size rules
+# (256, 3,072), the rope walks on its tree, bodies at no position and whole keys
+# repeated
+@pytest.mark.parametrize("case", ["256", "257", "1024", "1025", "3072", "3073", "rope", "nan", "repeats"])
+def test_single_graph_trees_bit_exact(jc, orc, case):
+    n = int(case) if case.isdigit() else 500
+    pos = jc.seed_uniform(n, 3, n)
+    p = pos.reshape(n, 3)
+    if case == "nan":
+        p[[3, 499], 1] = np.nan
+    if case == "repeats":
+        p[40:80] = p[:40]
+    g = jc.gen_scale_free(n, 2, n)
+    theta = 0.5 if case == "rope" else 0.8
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params({"theta": theta})
+    e.init(g, pos)
+    e.step()
+    o = orc.Fa2(g, pos, bh=True, theta=theta)
+    o.set_tree_capacity(1 << 20)  # repeated keys reach the depth cap
+    o.step()
+    r = o.get()
+    assert e.tree_info()["nodes"] == r["n_octree"]
+    f, _ = e.forces()
+    nan = np.isnan(r["force"])
+    assert np.array_equal(np.isnan(f), nan)
+    assert np.array_equal(bits(f)[~nan], bits(r["force"])[~nan])
+    assert e.walk_counts() == (r["n_inter"], r["n_open"])
