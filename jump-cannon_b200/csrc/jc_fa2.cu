@@ -2027,6 +2027,48 @@ __device__ void speed_update(DevState* st, uint32_t n, float jitter_tolerance, d
   st->speed_eff = eff;
 }
 
+// Row i's terms [e0, e1) added to f by a warp: the lanes gather 32 neighbours at a
+// time, and every lane adds them in list order from shuffles (unrolled: the
+// shuffles do not wait for the additions), so the sum is the same sequence of
+// roundings as one thread's. With one chunk of ids and positions in flight and a
+// rolled loop a chunk took 1.1 us (R-MAT, 65,536 nodes: pass 73 us, now 49; 262,144
+// nodes 116 -> 102, 1 M 262 -> 252).
+__device__ __forceinline__ void att_row_warp(uint32_t e0, uint32_t e1, const uint32_t* __restrict__ nbr,
+                                             const float4* __restrict__ pos, uint32_t i, const float4 pi, const KParams& P,
+                                             DevState* st, float& fx, float& fy, float& fz) {
+  const int lane = threadIdx.x & 31;
+  // ids two chunks ahead, positions one ahead of the chunk being added
+  auto id_at = [&](uint32_t k) { return k < e1 ? __ldg(nbr + k) : i; };
+  auto gather = [&](uint32_t u) { return JC_IN_BOUNDS(u, P.n, &st->error) ? __ldg(pos + u) : pi; };
+  uint32_t id = id_at(e0 + lane);
+  float4 q = gather(id);
+  id = id_at(e0 + 32 + lane);
+  for (uint32_t base = e0; base < e1; base += 32) {
+    const float4 cur = q;
+    q = gather(id);
+    id = id_at(base + 64 + lane);
+    float tx = -0.0f, ty = -0.0f, tz = -0.0f;  // -0 + term = term, signed zeros included
+    att_term(cur, pi, P, tx, ty, tz);
+    auto add = [&](uint32_t l) {
+      fx = __fadd_rn(fx, __shfl_sync(0xFFFFFFFFu, tx, l));
+      fy = __fadd_rn(fy, __shfl_sync(0xFFFFFFFFu, ty, l));
+      fz = __fadd_rn(fz, __shfl_sync(0xFFFFFFFFu, tz, l));
+    };
+    if (base + 32 <= e1) {
+#pragma unroll
+      for (uint32_t l = 0; l < 32; ++l) add(l);
+    } else {
+      for (uint32_t l = 0; l < e1 - base; ++l) add(l);
+    }
+  }
+}
+
+// UNSORTED: no schedule was made for the rows (the no-allocation pass, which sees
+// the CSR on the device only), so a warp first takes its lanes' rows of
+// UNSORTED_ROW entries or more together, one after another (20,000 nodes of a
+// scale-free graph: 55 -> 22 us).
+constexpr uint32_t UNSORTED_ROW = 32;
+template <bool UNSORTED>
 __global__ void __launch_bounds__(ATT_THREADS)
 k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
       const float4* __restrict__ pos, const float4* __restrict__ frep, const float4* __restrict__ old_force,
@@ -2072,12 +2114,7 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
         tr = r.tr;
       }
     } else if (blockIdx.x < P.n_hubs + (P.n_med + ATT_THREADS / 32 - 1) / (ATT_THREADS / 32)) {
-      // One warp per long list: the lanes gather 32 neighbours at a time, and
-      // every lane adds them in list order from shuffles (unrolled: the
-      // shuffles do not wait for the additions), so the sum is the same sequence
-      // of roundings as one thread's. With one chunk of ids and positions in
-      // flight and a rolled loop a chunk took 1.1 us (R-MAT, 65,536 nodes: pass
-      // 73 us, now 49; 262,144 nodes 116 -> 102, 1 M 262 -> 252).
+      // One warp per long list.
       const uint32_t mi = (blockIdx.x - P.n_hubs) * (ATT_THREADS / 32) + w;
       if (mi < P.n_med) {
         const uint32_t i0 = order[P.n_hubs + mi];
@@ -2085,31 +2122,7 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
         const float4 pi = pos[i];
         const float4 fr = frep[i];
         float fx = fr.x, fy = fr.y, fz = fr.z;
-        const uint32_t e0 = off[i], e1 = off[i + 1];
-        // ids two chunks ahead, positions one ahead of the chunk being added
-        auto id_at = [&](uint32_t k) { return k < e1 ? __ldg(nbr + k) : i; };
-        auto gather = [&](uint32_t u) { return JC_IN_BOUNDS(u, P.n, &st->error) ? __ldg(pos + u) : pi; };
-        uint32_t id = id_at(e0 + lane);
-        float4 q = gather(id);
-        id = id_at(e0 + 32 + lane);
-        for (uint32_t base = e0; base < e1; base += 32) {
-          const float4 cur = q;
-          q = gather(id);
-          id = id_at(base + 64 + lane);
-          float tx = -0.0f, ty = -0.0f, tz = -0.0f;  // -0 + term = term, signed zeros included
-          att_term(cur, pi, P, tx, ty, tz);
-          auto add = [&](uint32_t l) {
-            fx = __fadd_rn(fx, __shfl_sync(0xFFFFFFFFu, tx, l));
-            fy = __fadd_rn(fy, __shfl_sync(0xFFFFFFFFu, ty, l));
-            fz = __fadd_rn(fz, __shfl_sync(0xFFFFFFFFu, tz, l));
-          };
-          if (base + 32 <= e1) {
-#pragma unroll
-            for (uint32_t l = 0; l < 32; ++l) add(l);
-          } else {
-            for (uint32_t l = 0; l < e1 - base; ++l) add(l);
-          }
-        }
+        att_row_warp(off[i], off[i + 1], nbr, pos, i, pi, P, st, fx, fy, fz);
         if (lane == 0) {
           NodeOut r = finish_node(i, fx, fy, fz, pi, degf[i], P, old_force, force, stats);
           sw = r.sw;
@@ -2126,7 +2139,23 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
       const float4 fr = have ? frep[i] : make_float4(0.f, 0.f, 0.f, 0.f);
       float fx = fr.x, fy = fr.y, fz = fr.z;
       const uint32_t e0 = have ? off[i] : 0u, e1 = have ? off[i + 1] : 0u;
-      if (have) {
+      const bool together = UNSORTED && e1 - e0 >= UNSORTED_ROW;
+      if (UNSORTED) {
+        for (uint32_t m = __ballot_sync(0xFFFFFFFFu, together); m; m &= m - 1u) {
+          const int l = __ffs(m) - 1;
+          auto from = [&](float v) { return __shfl_sync(0xFFFFFFFFu, v, l); };
+          const float4 pl = make_float4(from(pi.x), from(pi.y), from(pi.z), from(pi.w));
+          float gx = from(fx), gy = from(fy), gz = from(fz);
+          att_row_warp(__shfl_sync(0xFFFFFFFFu, e0, l), __shfl_sync(0xFFFFFFFFu, e1, l), nbr, pos,
+                       __shfl_sync(0xFFFFFFFFu, i, l), pl, P, st, gx, gy, gz);
+          if (lane == l) {
+            fx = gx;
+            fy = gy;
+            fz = gz;
+          }
+        }
+      }
+      if (have && !together) {
         uint32_t k = e0;
         // ids up to a 16-byte boundary one by one, then eight ids in two
         // vector loads and eight gathers in flight, terms always in list order
@@ -3319,7 +3348,7 @@ class Fa2Engine : public Engine {
       L += 1;
     }
     record_phase(2);
-    launch_chained(chain, stream_, att_blocks_, ATT_THREADS, 0, k_att, aorder_.p, aoff_.p, anbr_.p, pos_.p, frep_.p,
+    launch_chained(chain, stream_, att_blocks_, ATT_THREADS, 0, k_att<false>, aorder_.p, aoff_.p, anbr_.p, pos_.p, frep_.p,
                    old_.p, degf_.p, P, st, force_.p, stats_.p, partials_.p, forest_.n_graphs);
     if (forest_.n_graphs > 1) {
       k_speed_slices<<<forest_.n_slices, 256, 0, stream_>>>(stats_.p, forest_, st);
@@ -3654,7 +3683,7 @@ constexpr uint32_t NOALLOC_LCP = NOALLOC_MAX_NODES;  // prefix-length index byte
 __host__ __device__ constexpr size_t na_round(size_t b) { return (b + 255) & ~(size_t)255; }
 
 struct NoAllocLayout {
-  size_t st, bbox, pos4, frep, force4, old4, degf, stats, order, key, top_key, top_alt, val, val_alt,
+  size_t st, tally, bbox, pos4, frep, force4, old4, degf, stats, order, key, top_key, top_alt, val, val_alt,
       first, totals, work, table, partials, nodes, parent, nchild, arrive, kids, lcp, total;
 };
 
@@ -3663,6 +3692,7 @@ constexpr NoAllocLayout noalloc_layout() {
   const size_t N = NOALLOC_MAX_NODES, C = NOALLOC_TREE_CAP;
   size_t o = 0;
   L.st = o; o += na_round(sizeof(DevState));
+  L.tally = o; o += na_round(sizeof(GraphTally));
   L.bbox = o; o += na_round(sizeof(float) * 6 * BBOX_BLOCKS);
   L.pos4 = o; o += na_round(16 * N);
   L.frep = o; o += na_round(16 * N);
@@ -3698,35 +3728,53 @@ constexpr NoAllocLayout kNoAlloc = noalloc_layout();
 // cudaGetSymbolAddress, once per device.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAlloc.total];
 
-// Degrees, identity order and the CSR check of the no-allocation pass. The
-// caller's CSR never went through the host validation of jc_engine_init, so
-// every row is checked here before anything gathers through it: decreasing
-// offsets, a non-empty row with no neighbour array, or a neighbour id >= n
-// records JC_ERR_ARG in the error word and skips the row's reads; every later
-// kernel of the pass (k_walk_rope, k_att, ...) then does no work.
-__global__ void k_noalloc_prepare(const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr, uint32_t n,
-                                  float* __restrict__ degf, uint32_t* __restrict__ order, DevState* st) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) {
+// Degrees, row order, widened positions, zeroed forces and the CSR check of the
+// no-allocation pass. The caller's CSR never went through the host validation of
+// jc_engine_init, so every row is checked here before anything gathers through it:
+// decreasing offsets, a non-empty row with no neighbour array, or a neighbour id
+// >= n records JC_ERR_ARG in the error word and skips the row's reads; every later
+// kernel of the pass that reads rows then does no work. Eight lanes a row: a thread
+// a row waited for its longest row's chain of loads (20,000 nodes of a scale-free
+// graph 22 us, now 11 with the widening, 3 us on its own, in it).
+//
+// The order deals the rows to the warps like cards, n / 32 apart in a warp, since
+// the longest rows of a growing graph are its first: the attraction pass would
+// give them all to one warp.
+constexpr uint32_t PREPARE_LANES = 8;
+__global__ void __launch_bounds__(256)
+k_noalloc_prepare(const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr, const float* __restrict__ xyz,
+                  uint32_t n, float* __restrict__ degf, uint32_t* __restrict__ order, float4* __restrict__ pos,
+                  float4* __restrict__ old_force, DevState* st) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0) {
     st->speed = 1.0f;
     st->speed_eff = 1.0f;
   }
-  if (i >= n) return;
-  order[i] = i;
-  const uint32_t e0 = off[i], e1 = off[i + 1];
-  uint32_t d = 0;
-  if (e1 < e0 || (e1 > e0 && nbr == nullptr)) {
-    set_error(st, JC_ERR_ARG);
-  } else {
-    bool bad = false;
-    for (uint32_t e = e0; e < e1; ++e) {
-      const uint32_t u = nbr[e];
-      bad |= u >= n;
-      d += u != i ? 1u : 0u;
-    }
-    if (bad) set_error(st, JC_ERR_ARG);
+  if (t < n) {
+    pos[t] = make_float4(xyz[3 * (size_t)t], xyz[3 * (size_t)t + 1], xyz[3 * (size_t)t + 2], 0.0f);
+    old_force[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t l = t & 31u, q = n / 32u, rem = n & 31u;
+    order[t] = l * q + min(l, rem) + (t >> 5);
   }
-  degf[i] = (float)d + 1.0f;  // fa2_bh.rs:264-294: non-self CSR entries, mass = deg + 1
+  const uint32_t i = t / PREPARE_LANES, sub = t % PREPARE_LANES;
+  uint32_t d = 0;
+  bool bad = false;
+  if (i < n) {
+    const uint32_t e0 = off[i], e1 = off[i + 1];
+    bad = e1 < e0 || (e1 > e0 && nbr == nullptr);
+    if (!bad) {
+#pragma unroll 4
+      for (uint32_t e = e0 + sub; e < e1; e += PREPARE_LANES) {
+        const uint32_t u = nbr[e];
+        bad |= u >= n;
+        d += u != i ? 1u : 0u;
+      }
+    }
+  }
+#pragma unroll
+  for (uint32_t o = PREPARE_LANES / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xFFFFFFFFu, d, o);
+  if (bad) set_error(st, JC_ERR_ARG);
+  if (i < n && sub == 0) degf[i] = (float)d + 1.0f;  // fa2_bh.rs:264-294: non-self CSR entries, mass = deg + 1
 }
 
 }  // namespace fa2
@@ -3774,6 +3822,7 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
   const NoAllocLayout& L = kNoAlloc;
   cudaStream_t s = (cudaStream_t)cuda_stream;
   DevState* st = (DevState*)(base + L.st);
+  GraphTally* tally = (GraphTally*)(base + L.tally);
   float4* pos4 = (float4*)(base + L.pos4);
   float4* frep = (float4*)(base + L.frep);
   float4* force4 = (float4*)(base + L.force4);
@@ -3820,35 +3869,39 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
 
   const uint32_t n = n_nodes;
   const Forest F1{1, 0, 21, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  // The array keeps the previous call's contents: zero what must start at 0.
-  if (cudaMemsetAsync(st, 0, sizeof(DevState), s) != cudaSuccess ||
-      cudaMemsetAsync(old4, 0, sizeof(float4) * n, s) != cudaSuccess ||
-      cudaMemsetAsync(lcp, 0xFF, NOALLOC_LCP + NOALLOC_LCP / 32, s) != cudaSuccess ||  // -1: run ends
-      cudaMemsetAsync(lcp + NOALLOC_LCP + NOALLOC_LCP / 32, 0x7F, 32, s) != cudaSuccess) {  // m2 padding: never
+  // The array keeps the previous call's contents: zero what must start at 0. (The
+  // prefix-length index is written whole by k_count: it is sized for all
+  // NOALLOC_MAX_NODES bodies and needs no padding.)
+  static_assert(NOALLOC_LCP % (32 * 1024) == 0, "whole rows of m2");
+  if (cudaMemsetAsync(st, 0, kNoAlloc.tally - kNoAlloc.st + sizeof(GraphTally), s) != cudaSuccess) {
     (void)cudaGetLastError();
     return JC_ERR_CUDA;
   }
-  k_noalloc_prepare<<<cdiv(n, 256), 256, 0, s>>>(d_offsets, d_neighbors, n, degf, order, st);
-  k_unpack_xyz<<<cdiv(n, 256), 256, 0, s>>>(d_positions_xyz, n, pos4);
-  k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, s>>>(pos4, n, (float*)(base + L.bbox), st, work,
-                                                  (uint32_t)dev::sort_work_words(n, 4));
-  // (chained as programmatic dependents from here on; at most 16 blocks for
+  k_noalloc_prepare<<<cdiv((uint64_t)PREPARE_LANES * n, 256), 256, 0, s>>>(d_offsets, d_neighbors, d_positions_xyz, n, degf,
+                                                                          order, pos4, old4, st);
+  // (chained as programmatic dependents from the tree on; at most 16 blocks for
   // the re-sort: below the SM count of any device this library runs on)
   try {
-    launch_chained(true, s, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos4, n, st, key, top_key, val, work);
-    dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, nullptr, 0, 4, work, &st->error, nullptr, s, true);
-    launch_chained(true, s, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key, val, key, n, st, 0);
-    launch_tie_resort(key, val, val_alt, nullptr, n, 5, st, table, 16, s);
-    launch_count(true, key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
-    launch_chained(true, s, cdiv(n, 256), 256, 0, k_fill<true>, nullptr, X, val, first, pos4, degf, n, P, st, nodes,
-                   parent, nchild, F1, nullptr, kids);
-    launch_chained(true, s, cdiv(n, 128), 128, 0, k_com_kids, first, nodes, parent, nchild, kids, arrive, n, st);
+    if (n <= GB_SINGLE_N) {
+      launch_graph_build_kernel(pos4, degf, F1, n, nullptr, key, val, first + n, nodes, parent, P, st, tally, kids, s);
+    } else {
+      k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, s>>>(pos4, n, (float*)(base + L.bbox), st, work,
+                                                      (uint32_t)dev::sort_work_words(n, 4));
+      launch_chained(true, s, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos4, n, st, key, top_key, val, work);
+      dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, nullptr, 0, 4, work, &st->error, nullptr, s, true);
+      launch_chained(true, s, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key, val, key, n, st, 0);
+      launch_tie_resort(key, val, val_alt, nullptr, n, 5, st, table, 16, s);
+      launch_count(true, key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
+      launch_chained(true, s, cdiv(n, 256), 256, 0, k_fill<true>, nullptr, X, val, first, pos4, degf, n, P, st, nodes,
+                     parent, nchild, F1, nullptr, kids);
+      launch_chained(true, s, cdiv(n, 128), 128, 0, k_com_kids, first, nodes, parent, nchild, kids, arrive, n, st);
+    }
     if (n <= WW_MAX_N && P.theta2 >= WW_MIN_THETA2)
       launch_walk_warp(true, nodes, kids, val, pos4, degf, n, P, st, frep, s);
     else
       launch_chained(true, s, cdiv(n, WALK_THREADS), WALK_THREADS, 0, k_walk_ahead<false>, nodes, val, pos4, degf, n, P,
                      st, frep, F1);
-    launch_chained(true, s, cdiv(n, ATT_THREADS), ATT_THREADS, 0, k_att, order, d_offsets, d_neighbors, pos4, frep, old4,
+    launch_chained(true, s, cdiv(n, ATT_THREADS), ATT_THREADS, 0, k_att<true>, order, d_offsets, d_neighbors, pos4, frep, old4,
                    degf, P, st, force4, stats, partials, 1u);
   } catch (const Error&) {
     return JC_ERR_CUDA;

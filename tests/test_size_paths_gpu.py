@@ -372,3 +372,27 @@ def test_single_graph_trees_bit_exact(jc, orc, case):
     assert np.array_equal(np.isnan(f), nan)
     assert np.array_equal(bits(f)[~nan], bits(r["force"])[~nan])
     assert e.walk_counts() == (r["n_inter"], r["n_open"])
+
+
+# the no-allocation pass: rows around the 32 entries a warp takes together (whole
+# and partial chunks), 40 such rows in two warps, row orders of whole and partial
+# warps, one body, both sides of the tree's size rule (3,072)
+@pytest.mark.parametrize("case", ["star31", "star32", "star33", "star64", "star97", "clique40", "1", "2", "31", "32", "33",
+                                  "3072", "3073"])
+def test_noalloc_rows_bit_exact(jc, orc, case):
+    torch = pytest.importorskip("torch")
+    if case.startswith("star"):
+        g = star(jc, int(case[4:]), int(case[4:]))
+    elif case == "clique40":
+        g = jc.csr_from_pairs(40, np.array([(a, b) for a in range(40) for b in range(a + 1, 40)], np.uint32))
+    else:
+        g = jc.gen_scale_free(int(case), 2, 3) if int(case) > 3 else jc.gen_path(int(case))
+    pos = jc.seed_uniform(g.n_nodes, 3, 21)
+    off, nbr = (torch.from_numpy(a.view(np.int32).copy()).cuda() for a in (g.offsets, g.neighbors))
+    p, out = torch.from_numpy(pos).cuda(), torch.full((3 * g.n_nodes,), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        jc.fa2_bh_forces_noalloc(g.n_nodes, off.data_ptr(), nbr.data_ptr(), p.data_ptr(), out.data_ptr(), theta=0.7)
+        o = orc.Fa2(g, pos, bh=True, theta=0.7)
+        o.step()
+        assert np.array_equal(bits(out.cpu().numpy()), bits(o.get()["force"]))
