@@ -23,13 +23,13 @@ __device__ __forceinline__ void dependent_launch_wait() {
 // k as a programmatic dependent of the launch before it on `s` (a kernel), or
 // as an ordinary launch.
 template <typename... P, typename... A>
-inline void launch_chained(bool dependent, cudaStream_t s, uint32_t blocks, uint32_t threads, size_t smem,
+inline void launch_chained(bool dependent, cudaStream_t s, dim3 blocks, uint32_t threads, size_t smem,
                            void (*k)(P...), A... args) {
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(blocks);
+  cfg.gridDim = blocks;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
