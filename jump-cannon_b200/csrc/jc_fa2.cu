@@ -10,6 +10,8 @@
 // One step is a fixed sequence of kernels on the engine's stream, captured
 // once into a CUDA graph and replayed (no host round trip inside a step):
 //
+//   k_graph_build  (jc_fa2_graph.cuh) everything up to the walk in one launch, for
+//               a small graph or a batch of small graphs; else:
 //   k_bbox      finite-coordinate bounding box -> root centre / half extent
 //               (fa2_bh.rs:768-799), last block finalises.
 //   k_keys      per body, the octant digits of levels 0..31 computed with the
@@ -27,19 +29,21 @@
 //               sorted neighbours; bodies whose 32 digits equal their
 //               predecessor's are the ones the reference drops at the depth
 //               cap (fa2_bh.rs:874-922) and get zero nodes.
-//   scan        node index of each body's first node (pre-order == DFS order
+//   k_offsets   node index of each body's first node (pre-order == DFS order
 //               with children in octant order 0..7, as assign_ropes walks).
 //   k_fill      writes every node: pre-order makes `next` = index + 1 and
-//               `skip` = first node after the subtree (found by a binary
-//               search over the sorted keys); parent links; child counts.
+//               `skip` = first node after the subtree (found through the
+//               prefix-length index); parent links; child counts or lists.
 //   k_com       bottom-up centre of mass with arrival counters; the last child
 //               to arrive sums the children in octant order in f32, as
-//               aggregate_com_postorder does (fa2_bh.rs:927-967).
-//   k_walk      theta-criterion walk. A warp takes 32 consecutive bodies in
-//               key order and walks the union of their paths node by node in
-//               pre-order; every lane keeps its own accept/open decision via
-//               per-depth ballot masks, so each body sees exactly the node
-//               sequence of the reference's rope walk (wgsl:114-156).
+//               aggregate_com_postorder does (fa2_bh.rs:927-967). k_com_kids:
+//               the same from child lists, for smaller trees.
+//   k_walk_*    theta-criterion walk: a lane per body along the ropes
+//               (k_walk_rope; k_walk_ahead where the graph does not fill the
+//               GPU), a warp per body on the smallest graphs (k_walk_warp), or
+//               lanes sharing a node stream (k_walk<G>, by setting). Each body
+//               meets exactly the nodes of the reference's rope walk, its terms
+//               added in the same order (wgsl:114-156).
 //   k_att       attraction over the per-node edge list in the shader's edge
 //               order, gravity, swing/traction, per-block f64 partial sums;
 //               the last block finishes the reduction and runs the adaptive
@@ -3302,15 +3306,15 @@ class Fa2Engine : public Engine {
         if (F.n_graphs > 1) {
           // the top 48 bits (the graph id takes up to 16 of them), then the runs
           k_keys_batch<<<cdiv(n, 256), 256, 0, stream_>>>(pos_.p, n, st, key_.p, hi_.p, val_.p, F);
-          L += dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, nullptr, 16, 64,
-                                               sort_work_.p, &st->error, nullptr, stream_);
+          L += dev::radix_sort_pairs<uint64_t>(hi_.p, val_.p, hi_alt_.p, val_alt_.p, n, 16, 64,
+                                               sort_work_.p, &st->error, stream_);
           k_seg_fix<uint64_t><<<cdiv(n, 256), 256, 0, stream_>>>(hi_.p, val_.p, key_.p, n, st, 16);
         } else {
           // the top 32 bits (ten levels), then the runs
           launch_chained(chain, stream_, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos_.p, n, st, key_.p,
                          top_key_.p, val_.p, sort_work_.p);
-          L += dev::radix_passes<uint32_t>(top_key_.p, val_.p, top_alt_.p, val_alt_.p, n, nullptr, 0, 4, sort_work_.p,
-                                           &st->error, nullptr, stream_, chain);
+          L += dev::radix_passes<uint32_t>(top_key_.p, val_.p, top_alt_.p, val_alt_.p, n, 0, 4, sort_work_.p,
+                                           &st->error, stream_, chain);
           launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key_.p, val_.p, key_.p, n, st, 0);
         }
         launch_tie_resort(key_.p, val_.p, val_alt_.p, F.n_graphs > 1 ? hi_.p : nullptr, n, (3 * (32 - F.lh) + 7) / 8, st,
@@ -3888,7 +3892,7 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
       k_bbox<<<bbox_blocks(n), BBOX_THREADS, 0, s>>>(pos4, n, (float*)(base + L.bbox), st, work,
                                                       (uint32_t)dev::sort_work_words(n, 4));
       launch_chained(true, s, std::min(cdiv(n, 256), KEY_BLOCKS), 256, 0, k_keys, pos4, n, st, key, top_key, val, work);
-      dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, nullptr, 0, 4, work, &st->error, nullptr, s, true);
+      dev::radix_passes<uint32_t>(top_key, val, top_alt, val_alt, n, 0, 4, work, &st->error, s, true);
       launch_chained(true, s, cdiv(n, 256), 256, 0, k_seg_fix<uint32_t>, top_key, val, key, n, st, 0);
       launch_tie_resort(key, val, val_alt, nullptr, n, 5, st, table, 16, s);
       launch_count(true, key, val, n, st, first, totals, nullptr, F1, X, P, nchild, arrive, s);
@@ -3956,15 +3960,15 @@ extern "C" jc_status jc_selftest_sort_wait(uint32_t* device_status, float* wait_
     uint32_t* counts = work;
     uint32_t* tile_ctr = work + dev::RS_RADIX;
     uint32_t* status = tile_ctr + 1;
-    dev::os_hist<uint64_t><<<2, dev::RS_THREADS, 0, s>>>(keys, n, nullptr, 0, 1, counts, nullptr);
+    dev::os_hist<uint64_t><<<2, dev::RS_THREADS, 0, s>>>(keys, n, 0, 1, counts);
     const uint32_t one = 1u;
     JC_CUDA_CHECK(cudaMemcpyAsync(tile_ctr, &one, 4, cudaMemcpyHostToDevice, s));
     JC_CUDA_CHECK(cudaEventCreate(&e0));
     JC_CUDA_CHECK(cudaEventCreate(&e1));
     JC_CUDA_CHECK(cudaEventRecord(e0, s));
-    dev::os_pass<uint64_t, dev::RS_ROUNDS><<<1, dev::RS_THREADS, 0, s>>>(keys, vals, keys_out, vals_out, n, nullptr, 0,
+    dev::os_pass<uint64_t, dev::RS_ROUNDS><<<1, dev::RS_THREADS, 0, s>>>(keys, vals, keys_out, vals_out, n, 0,
                                                                         counts, status,
-                                                        tile_ctr, nullptr, err);
+                                                        tile_ctr, err);
     JC_CUDA_CHECK(cudaGetLastError());
     JC_CUDA_CHECK(cudaEventRecord(e1, s));
     JC_CUDA_CHECK(cudaMemcpyAsync(device_status, err, 4, cudaMemcpyDeviceToHost, s));

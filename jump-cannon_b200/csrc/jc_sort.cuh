@@ -1,13 +1,8 @@
 // Device-wide primitives for the octree build: a stable LSD radix sort of
 // (key, u32 value) pairs with 8-bit digits, and an exclusive scan of u32.
 //
-// Both read their item count from device memory (so they can sit inside a
-// captured CUDA graph while the count changes from step to step) and accept
-// an optional device "gate" word: when the gate is 0 every kernel returns at
-// once, which is how the rare tie-breaking re-sort is made conditional
-// without a host round trip.
-//
-// Radix sort: one histogram kernel for all passes, then one kernel per
+// Radix sort: the digit counts of all passes (os_hist, or the kernel that makes
+// the keys), then one kernel per
 // 8-bit pass (os_pass): per-tile stable ranking with warp ballots and
 // per-warp digit counters (item order in a tile = warp, round, lane = input
 // order) and decoupled look-back across tiles for the output offsets.
@@ -38,12 +33,6 @@ __host__ __device__ constexpr int rs_rounds(uint32_t n_max) {
 }
 __host__ __device__ constexpr uint32_t rs_tiles(uint32_t n_max) {
   return (n_max + (uint32_t)(RS_THREADS * rs_rounds(n_max)) - 1) / (uint32_t)(RS_THREADS * rs_rounds(n_max));
-}
-
-__device__ __forceinline__ uint32_t rs_count(uint32_t n_max, const uint32_t* d_count) {
-  if (d_count == nullptr) return n_max;
-  uint32_t c = *d_count;
-  return c < n_max ? c : n_max;
 }
 
 // Exclusive scan across a 256-thread block (one value per thread).
@@ -105,13 +94,10 @@ constexpr int OS_WINDOW = 8;  // predecessors' status words read per round trip
 // bit_begin + 8p .. +8). counts must be zeroed first.
 template <typename K>
 __global__ void __launch_bounds__(RS_THREADS)
-os_hist(const K* __restrict__ keys, uint32_t n_max, const uint32_t* d_count, int bit_begin, int passes,
-        uint32_t* __restrict__ counts, const uint32_t* gate) {
-  if (gate && *gate == 0) return;
+os_hist(const K* __restrict__ keys, uint32_t n, int bit_begin, int passes, uint32_t* __restrict__ counts) {
   __shared__ uint32_t h[8][RS_RADIX];
   for (int i = threadIdx.x; i < 8 * RS_RADIX; i += RS_THREADS) (&h[0][0])[i] = 0;
   __syncthreads();
-  const uint32_t n = rs_count(n_max, d_count);
   for (uint32_t i = blockIdx.x * RS_THREADS + threadIdx.x; i < n; i += gridDim.x * RS_THREADS) {
     const K k = keys[i];
     for (int p = 0; p < passes; ++p) {
@@ -130,16 +116,13 @@ os_hist(const K* __restrict__ keys, uint32_t n_max, const uint32_t* d_count, int
 template <typename K, int ROUNDS = RS_ROUNDS>
 __global__ void __launch_bounds__(RS_THREADS)
 os_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
-        uint32_t* __restrict__ vout, uint32_t n_max, const uint32_t* d_count, int shift,
-        const uint32_t* __restrict__ gcount, uint32_t* status, uint32_t* tile_ctr, const uint32_t* gate,
-        uint32_t* err) {
+        uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* __restrict__ gcount, uint32_t* status,
+        uint32_t* tile_ctr, uint32_t* err) {
   dependent_launch_wait();
-  if (gate && *gate == 0) return;
   __shared__ uint32_t wcnt[RS_WARPS][RS_RADIX];
   __shared__ uint32_t base[RS_RADIX];
   __shared__ uint32_t sh_scan[32];
   __shared__ uint32_t s_tile;
-  const uint32_t n = rs_count(n_max, d_count);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
   for (int i = threadIdx.x; i < RS_WARPS * RS_RADIX; i += RS_THREADS) (&wcnt[0][0])[i] = 0;
@@ -253,8 +236,7 @@ __host__ __device__ constexpr size_t sort_work_words(uint32_t n_max, int passes)
 // them are zero. Returns the number of kernels issued.
 template <typename K>
 inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, uint32_t n_max,
-                        const uint32_t* d_count, int bit_begin, int passes, uint32_t* work, uint32_t* err,
-                        const uint32_t* gate, cudaStream_t s, bool chained = false) {
+                        int bit_begin, int passes, uint32_t* work, uint32_t* err, cudaStream_t s, bool chained = false) {
   const uint32_t tiles = rs_tiles(n_max);
   const int rounds = rs_rounds(n_max);
   const auto pass = rounds == 2 ? os_pass<K, 2> : rounds == 4 ? os_pass<K, 4> : rounds == 8 ? os_pass<K, 8>
@@ -269,8 +251,8 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
   for (int p = 0; p < passes; ++p) {
     int shift = bit_begin + 8 * p;
     if (shift >= (int)(8 * sizeof(K))) shift = 8 * (int)sizeof(K) - 8;
-    launch_chained(chained, s, tiles, RS_THREADS, 0, pass, kin, vin, kout, vout, n_max, d_count, shift, counts + p * RS_RADIX,
-                   status + (size_t)p * tiles * RS_RADIX, tile_ctr + p, gate, err);
+    launch_chained(chained, s, tiles, RS_THREADS, 0, pass, kin, vin, kout, vout, n_max, shift,
+                   counts + p * RS_RADIX, status + (size_t)p * tiles * RS_RADIX, tile_ctr + p, err);
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
   }
@@ -282,16 +264,15 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
 // Returns the number of nodes (kernels + memsets) issued.
 template <typename K>
 inline int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, uint32_t n_max,
-                            const uint32_t* d_count, int bit_begin, int bit_end, uint32_t* work,
-                            uint32_t* err, const uint32_t* gate, cudaStream_t s) {
+                            int bit_begin, int bit_end, uint32_t* work, uint32_t* err, cudaStream_t s) {
   if (n_max == 0) return 0;
   const uint32_t tiles = rs_tiles(n_max);
   int passes = (bit_end - bit_begin + 7) / 8;
   if (passes & 1) ++passes;
   cudaMemsetAsync(work, 0, sizeof(uint32_t) * sort_work_words(n_max, passes), s);
   const uint32_t hist_blocks = tiles < 592u ? tiles : 592u;
-  os_hist<K><<<hist_blocks, RS_THREADS, 0, s>>>(keys, n_max, d_count, bit_begin, passes, work, gate);
-  return 2 + radix_passes(keys, vals, keys_alt, vals_alt, n_max, d_count, bit_begin, passes, work, err, gate, s);
+  os_hist<K><<<hist_blocks, RS_THREADS, 0, s>>>(keys, n_max, bit_begin, passes, work);
+  return 2 + radix_passes(keys, vals, keys_alt, vals_alt, n_max, bit_begin, passes, work, err, s);
 }
 
 // ---------------------------------------------------------------- scan --

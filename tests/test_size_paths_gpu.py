@@ -396,3 +396,21 @@ def test_noalloc_rows_bit_exact(jc, orc, case):
         o = orc.Fa2(g, pos, bh=True, theta=0.7)
         o.step()
         assert np.array_equal(bits(out.cpu().numpy()), bits(o.get()["force"]))
+
+
+# graphs of no bodies in a batch, on both of its tree paths
+@pytest.mark.parametrize("big", [300, 8193])
+def test_empty_graphs_in_a_batch(jc, big):
+    none = jc.Csr(0, np.zeros(1, np.uint32), np.zeros(0, np.uint32))
+    g = [jc.gen_scale_free(big, 2, 1), jc.gen_scale_free(40, 2, 2)]
+    p = [jc.seed_uniform(big, 3, 3), jc.seed_uniform(40, 3, 4)]
+    b = jc.LayoutEngine("fa2-bh")
+    b.init_batch([none, g[0], none, g[1], none], [np.zeros(0, np.float32), p[0], np.zeros(0, np.float32), p[1],
+                                                  np.zeros(0, np.float32)])
+    out = b.step_many(3)
+    alone = []
+    for x, y in zip(g, p):
+        e = jc.LayoutEngine("fa2-bh")
+        e.init(x, y)
+        alone.append(e.step_many(3))
+    assert np.array_equal(bits(out), bits(np.concatenate(alone)))
