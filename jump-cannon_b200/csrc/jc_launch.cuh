@@ -21,21 +21,35 @@ __device__ __forceinline__ void dependent_launch_wait() {
 }  // namespace dev
 
 // k as a programmatic dependent of the launch before it on `s` (a kernel), or
-// as an ordinary launch.
+// as an ordinary launch. carveout: the shared memory to set aside on an SM, in
+// percent, or -1 for the driver's choice.
 template <typename... P, typename... A>
-inline void launch_chained(bool dependent, cudaStream_t s, dim3 blocks, uint32_t threads, size_t smem,
+inline void launch_chained(bool dependent, int carveout, cudaStream_t s, dim3 blocks, uint32_t threads, size_t smem,
                            void (*k)(P...), A... args) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute at[2]{};
+  unsigned n = 0;
+  if (dependent) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (carveout >= 0) {
+    at[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[n++].val.sharedMemCarveout = (unsigned)carveout;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = blocks;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = dependent ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = n;
   JC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k, (P)args...));
+}
+
+template <typename... P, typename... A>
+inline void launch_chained(bool dependent, cudaStream_t s, dim3 blocks, uint32_t threads, size_t smem, void (*k)(P...),
+                           A... args) {
+  launch_chained(dependent, -1, s, blocks, threads, smem, k, args...);
 }
 
 }  // namespace jc

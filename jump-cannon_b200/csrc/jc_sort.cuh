@@ -22,12 +22,14 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_ROUNDS = 16;                        // items per lane
 constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;      // 4096 items per block
 constexpr int RS_RADIX = 256;
+constexpr int RS_CHAIN_CARVEOUT = 7;                 // percent of an SM: 16 KB
 // Items per lane by size: a tile's ranking is a serial chain of rounds, so where
 // the tiles would not fill the GPU shorter tiles finish sooner; many tiles make
 // the look-back chains long. B200, tree build in us with 4-byte keys at 2 / 4 /
-// 8 / 16 items: 400 bodies 57 / 59 / 63 / 71, 10,000 92 / 95 / 97 / 109, 150,000
-// 145 / 138 / 140 / 149, 262,144 185 / 172 / 168 / 174, 600,000 335 / 279 / 259 /
-// 255, 1 M 541 / 552 / 426 / 399.
+// 8 / 16 items: 4,000 bodies 65 / 67 / 72 / 79, 10,000 74 / 76 / 79 / 90, 32,768
+// 85 / 85 / 88 / 95, 150,000 120 / 114 / 113 / 119, 262,144 167 / 155 / 150 / 155,
+// 400,000 333 / 205 / 198 / 197, 600,000 293 / 247 / 228 / 224, 1 M 548 / 590 / 519 /
+// 361.
 __host__ __device__ constexpr int rs_rounds(uint32_t n_max) {
   return n_max <= 32768u ? 2 : n_max <= 196608u ? 4 : n_max <= 400000u ? 8 : RS_ROUNDS;
 }
@@ -76,13 +78,14 @@ constexpr uint32_t OS_VAL = (1u << 30) - 1;
 constexpr uint32_t OS_SPIN_LIMIT = 1u << 20;  // about a second of waiting
 constexpr uint32_t OS_ERR_TIMEOUT = 4u;    // JC_ERR_DEVICE_TIMEOUT
 
-__device__ __forceinline__ void st_release_u32(uint32_t* p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // A status word carries everything it publishes (flag + count in one 32-bit
-// word), so the look-back reads need no acquire ordering: relaxed loads, of
-// which a window can be in flight at once (acquire loads would complete one
-// after another).
+// word), so the look-back needs no ordering: relaxed stores (a release store
+// waits for the block's earlier accesses: 1 M bodies, tree build 399 -> 393 us,
+// 150,000 125 -> 117) and relaxed loads, of which a window can be in flight at
+// once (acquire loads would complete one after another).
 __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -123,6 +126,13 @@ os_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restri
   __shared__ uint32_t base[RS_RADIX];
   __shared__ uint32_t sh_scan[32];
   __shared__ uint32_t s_tile;
+  // 4-byte keys leave through shared memory in digit order, so that a digit's run
+  // is written in whole sectors (8-byte keys would need more than 48 KB at 16
+  // items a lane). B200, tree build in us: 10,000 bodies 81 -> 76, 65,537 101 -> 96,
+  // 262,144 161 -> 151, 1 M 393 -> 360, 4.2 M 1,459 -> 1,383.
+  constexpr bool STAGED = sizeof(K) == 4;
+  __shared__ K skey[STAGED ? RS_THREADS * ROUNDS : 1];
+  __shared__ uint32_t sval[STAGED ? RS_THREADS * ROUNDS : 1];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
   for (int i = threadIdx.x; i < RS_WARPS * RS_RADIX; i += RS_THREADS) (&wcnt[0][0])[i] = 0;
@@ -172,10 +182,30 @@ os_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restri
   }
   uint32_t* my = status + (size_t)tile * RS_RADIX + d;
   uint32_t excl = 0;
+  if constexpr (STAGED) {
+    st_relaxed_u32(my, (tile == 0 ? OS_INC : OS_AGG) | tot);
+    // the tile in digit order in shared memory, so that a digit's run leaves in
+    // whole sectors; the predecessors publish meanwhile
+    uint32_t unused;
+    const uint32_t local = block_excl_scan_256(tot, &unused, sh_scan);
+    base[d] = local;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      if (chunk + r * 32 + lane < n) {
+        const uint32_t dg = (uint32_t)(key[r] >> shift) & 0xFFu;
+        const uint32_t at = base[dg] + wcnt[w][dg] + rank[r];
+        if (JC_IN_BOUNDS(at, RS_THREADS * ROUNDS, err)) {
+          skey[at] = key[r];
+          sval[at] = val[r];
+        }
+      }
+    }
+  }
   if (tile == 0) {
-    st_release_u32(my, OS_INC | tot);
+    if constexpr (!STAGED) st_relaxed_u32(my, OS_INC | tot);
   } else {
-    st_release_u32(my, OS_AGG | tot);
+    if constexpr (!STAGED) st_relaxed_u32(my, OS_AGG | tot);
     // All tiles run at once and publish their aggregates early, so the chain
     // back to the nearest inclusive prefix can be long: read OS_WINDOW
     // predecessors per round trip, add them in order, stop at the first
@@ -206,10 +236,28 @@ os_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restri
         __nanosleep(32);
       }
     }
-    st_release_u32(my, OS_INC | (excl + tot));
+    st_relaxed_u32(my, OS_INC | (excl + tot));
   }
   uint32_t total_dummy;
   const uint32_t start = block_excl_scan_256(gcount[d], &total_dummy, sh_scan);
+  if constexpr (STAGED) {
+    base[d] = start + excl - base[d];  // (modulo 2^32)
+    __syncthreads();
+    const uint32_t t0 = tile * (RS_THREADS * ROUNDS);
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      const uint32_t i = r * RS_THREADS + threadIdx.x;
+      if (t0 + i < n) {
+        const K k = skey[i];
+        const uint32_t dst = base[(uint32_t)(k >> shift) & 0xFFu] + i;
+        if (JC_IN_BOUNDS(dst, n, err)) {
+          kout[dst] = k;
+          vout[dst] = sval[i];
+        }
+      }
+    }
+    return;
+  }
   base[d] = start + excl;
   __syncthreads();
 #pragma unroll
@@ -251,7 +299,10 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
   for (int p = 0; p < passes; ++p) {
     int shift = bit_begin + 8 * p;
     if (shift >= (int)(8 * sizeof(K))) shift = 8 * (int)sizeof(K) - 8;
-    launch_chained(chained, s, tiles, RS_THREADS, 0, pass, kin, vin, kout, vout, n_max, shift,
+    // (a chain leaves no SM idle between kernels, so none can change its split of
+    // shared memory and L1 in it: one block's share here, or the walk at the chain's
+    // end keeps a small L1: 32,768 bodies 188 us a step, now 174)
+    launch_chained(chained, chained ? RS_CHAIN_CARVEOUT : -1, s, tiles, RS_THREADS, 0, pass, kin, vin, kout, vout, n_max, shift,
                    counts + p * RS_RADIX, status + (size_t)p * tiles * RS_RADIX, tile_ctr + p, err);
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
