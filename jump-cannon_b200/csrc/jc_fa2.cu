@@ -3403,11 +3403,11 @@ class Fa2Engine : public Engine {
 
   // A small single graph's step chains its kernels as programmatic dependents
   // where nothing but kernels stands between them (no phase events). B200, us a
-  // replayed step without and with: 400 nodes 104 -> 102, 2,000 134 -> 131, 10,000
-  // 156 -> 154, but 65,537 180 -> 205 and 1 M 1,155 -> 1,161. (The pass of
-  // jc_fa2_bh_forces_noalloc, launched one by one: 300 nodes 155 -> 137 us, 20,000
-  // 292 -> 273.)
-  static constexpr uint32_t CHAIN_MAX_N = 32768;
+  // replayed step without and with: 400 nodes 43.0 -> 41.5, 2,000 69.7 -> 71.5, 4,000
+  // 96.3 -> 95.1, 10,000 141.8 -> 139.4, 20,000 164.6 -> 160.5, but 32,768 175.0 ->
+  // 176.5, 65,537 177 -> 225. (The pass of jc_fa2_bh_forces_noalloc, launched one by
+  // one, is chained at all its sizes: 300 nodes 155 -> 137 us, 20,000 292 -> 273.)
+  static constexpr uint32_t CHAIN_MAX_N = 24576;
   bool chained() const {
     return n_ <= CHAIN_MAX_N && s_.use_graph && !capture_phases_ && forest_.n_graphs == 1 && !stage_top();
   }

@@ -301,7 +301,8 @@ inline int radix_passes(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt
     if (shift >= (int)(8 * sizeof(K))) shift = 8 * (int)sizeof(K) - 8;
     // (a chain leaves no SM idle between kernels, so none can change its split of
     // shared memory and L1 in it: one block's share here, or the walk at the chain's
-    // end keeps a small L1: 32,768 bodies 188 us a step, now 174)
+    // end keeps a small L1: jc_fa2_bh_forces_noalloc at 32,768 bodies 280 us and more,
+    // 228 with this)
     launch_chained(chained, chained ? RS_CHAIN_CARVEOUT : -1, s, tiles, RS_THREADS, 0, pass, kin, vin, kout, vout, n_max, shift,
                    counts + p * RS_RADIX, status + (size_t)p * tiles * RS_RADIX, tile_ctr + p, err);
     K* tk = kin; kin = kout; kout = tk;

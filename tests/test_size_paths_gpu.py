@@ -258,7 +258,7 @@ def test_long_runs_resort_in_a_batch(jc):
 
 
 # both sides of the sort's tile-size rules and of the walk chain's rule
-@pytest.mark.parametrize("n", [511, 512, 513, 32767, 32768, 32769, 196607, 400000, 400001])
+@pytest.mark.parametrize("n", [511, 512, 513, 24576, 24577, 32767, 32768, 32769, 196607, 400000, 400001])
 def test_sort_tile_rules_bit_exact(jc, orc, n):
     g = jc.gen_watts_strogatz(n, 4, 0.05, n) if n < 100000 else jc.gen_path(n)
     e, r = one_step(jc, orc, g, jc.seed_uniform(n, 3, 7), theta=1.2)
