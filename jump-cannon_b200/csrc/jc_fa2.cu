@@ -132,8 +132,21 @@ struct __align__(32) TNode {
 };
 static_assert(sizeof(TNode) == 32, "a node is one 32-byte sector");
 
-// One node in a single 256-bit load (read-only path): the walk is bound by
-// L1 request throughput, and one 32-byte request per visit replaces two.
+// One node in a single 256-bit load: the walk is bound by L1 request
+// throughput, and one 32-byte request per visit replaces two. load_node takes
+// the read-only path, so it is for launches that begin after the tree is
+// written; load_node_c is coherent, for kernels chained behind the tree's
+// (jc_launch.cuh) and for trees written earlier in the same launch.
+__device__ __forceinline__ void load_node_c(const TNode* p, float4& cm, int4& meta) {
+  uint32_t r0, r1, r2, r3, r4, r5, r6, r7;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3), "=r"(r4), "=r"(r5), "=r"(r6), "=r"(r7)
+               : "l"(p)
+               : "memory");
+  cm = make_float4(__uint_as_float(r0), __uint_as_float(r1), __uint_as_float(r2), __uint_as_float(r3));
+  meta = make_int4((int)r4, (int)r5, (int)r6, (int)r7);
+}
+
 __device__ __forceinline__ void load_node(const TNode* p, float4& cm, int4& meta) {
   uint32_t r0, r1, r2, r3, r4, r5, r6, r7;
   asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -375,8 +388,8 @@ __device__ __forceinline__ void count_invalid(bool invalid, DevState* st) {
 // blocks, so that few flush their counts.
 constexpr uint32_t KEY_BLOCKS = 148u * 8u;
 __global__ void __launch_bounds__(256)
-k_keys(const float4* __restrict__ pos, uint32_t n, DevState* st, ulonglong2* __restrict__ key,
-       uint32_t* __restrict__ top, uint32_t* __restrict__ val, uint32_t* __restrict__ counts) {
+k_keys(const float4* __restrict__ pos, uint32_t n, DevState* st, ulonglong2* key, uint32_t* top, uint32_t* val,
+       uint32_t* counts) {
   dev::dependent_launch_wait();
   __shared__ uint32_t h[4][256];
 #pragma unroll
@@ -459,8 +472,7 @@ __device__ __forceinline__ bool key_after(const ulonglong2 a, uint32_t va, const
 }
 template <typename K>
 __global__ void __launch_bounds__(256)
-k_seg_fix(K* __restrict__ sorted, uint32_t* __restrict__ val, const ulonglong2* __restrict__ key, uint32_t n,
-          DevState* st, int shift) {
+k_seg_fix(K* sorted, uint32_t* val, const ulonglong2* key, uint32_t n, DevState* st, int shift) {
   dev::dependent_launch_wait();
   constexpr bool WORD = sizeof(K) == 8;
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -751,8 +763,8 @@ __device__ __forceinline__ int64_t lcp_prev_below(const LcpIndex& X, uint32_t a,
 // `totals` the block's sum until k_offsets adds the blocks before it.
 constexpr int COUNT_THREADS = 1024;
 __global__ void __launch_bounds__(COUNT_THREADS)
-k_count(const ulonglong2* __restrict__ key, const uint32_t* __restrict__ val, uint32_t n, DevState* st,
-        uint32_t* __restrict__ first, uint32_t* __restrict__ totals, Forest F, LcpIndex X) {
+k_count(const ulonglong2* key, const uint32_t* val, uint32_t n, DevState* st, uint32_t* first, uint32_t* totals,
+        Forest F, LcpIndex X) {
   dev::dependent_launch_wait();
   __shared__ ulonglong2 sk[COUNT_THREADS + 2];  // keys of bodies a - 1 .. a + 1 at sk[t .. t + 2]
   __shared__ uint32_t sh[32];
@@ -813,8 +825,8 @@ k_count(const ulonglong2* __restrict__ key, const uint32_t* __restrict__ val, ui
 // `totals` comes scanned (`scanned`: with the sum in totals[gridDim.x]).
 constexpr uint32_t OFFSET_BLOCKS = 2048;
 __global__ void __launch_bounds__(COUNT_THREADS)
-k_offsets(const uint32_t* __restrict__ totals, int scanned, uint32_t* __restrict__ first, uint32_t n, KParams P,
-          DevState* st, uint32_t* __restrict__ nchild, uint32_t* __restrict__ arrive) {
+k_offsets(const uint32_t* totals, int scanned, uint32_t* first, uint32_t n, KParams P, DevState* st,
+          uint32_t* nchild, uint32_t* arrive) {
   dev::dependent_launch_wait();
   __shared__ uint32_t sums[2][32];
   __shared__ uint32_t s_before, s_all;
@@ -888,11 +900,9 @@ inline int launch_count(bool chained, const ulonglong2* key, const uint32_t* val
 // parent's list of children (eight slots per cell, in order of arrival).
 template <bool KIDS>
 __global__ void __launch_bounds__(256, 8)
-k_fill(const uint64_t* __restrict__ hi, const LcpIndex X, const uint32_t* __restrict__ val,
-       const uint32_t* __restrict__ first, const float4* __restrict__ pos, const float* __restrict__ degf,
-       uint32_t n, KParams P, DevState* st, TNode* __restrict__ nodes,
-       uint32_t* __restrict__ parent, uint32_t* __restrict__ nchild, Forest F,
-       uint32_t* __restrict__ top_list, uint32_t* __restrict__ kids) {
+k_fill(const uint64_t* hi, const LcpIndex X, const uint32_t* val, const uint32_t* first,
+       const float4* __restrict__ pos, const float* __restrict__ degf, uint32_t n, KParams P, DevState* st,
+       TNode* nodes, uint32_t* parent, uint32_t* nchild, Forest F, uint32_t* top_list, uint32_t* kids) {
   dev::dependent_launch_wait();
   uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t N = st->n_valid;
@@ -1071,9 +1081,8 @@ __device__ __forceinline__ void sort8(uint32_t* k) {
 }
 
 __global__ void __launch_bounds__(128)
-k_com_kids(const uint32_t* __restrict__ first, TNode* nodes, const uint32_t* __restrict__ parent,
-           const uint32_t* __restrict__ nchild, uint32_t* __restrict__ kids, uint32_t* __restrict__ arrive, uint32_t n,
-           DevState* st) {
+k_com_kids(const uint32_t* first, TNode* nodes, const uint32_t* parent, const uint32_t* nchild, uint32_t* kids,
+           uint32_t* arrive, uint32_t n, DevState* st) {
   dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   if (st->error) return;
@@ -1257,10 +1266,11 @@ k_walk(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, cons
 // (wgsl:114-156) with nothing shared between lanes, so no masks or votes.
 // Adds this body's repulsion terms in the reference's visit order and writes
 // frep[body]; returns false (error set) on a malformed rope.
-template <bool FAST>
-__device__ __forceinline__ void walk_one(const TNode* __restrict__ nodes, uint32_t body, const float4 p, float srd,
-                                         uint32_t root, uint32_t T, float theta2, DevState* st,
-                                         float4* __restrict__ frep, uint32_t& n_inter, uint32_t& n_open) {
+// CHAINED: the nodes may be written by a kernel this launch is chained behind.
+template <bool FAST, bool CHAINED>
+__device__ __forceinline__ void walk_one(const TNode* nodes, uint32_t body, const float4 p, float srd, uint32_t root,
+                                         uint32_t T, float theta2, DevState* st, float4* frep, uint32_t& n_inter,
+                                         uint32_t& n_open) {
   float fx = 0.0f, fy = 0.0f, fz = 0.0f;
   uint32_t idx = root;
   // Ropes strictly increase, so the walk ends; it leaves the loop at END or at
@@ -1269,7 +1279,8 @@ __device__ __forceinline__ void walk_one(const TNode* __restrict__ nodes, uint32
   while (idx < T) {
     float4 c;
     int4 m;
-    load_node(nodes + idx, c, m);
+    if (CHAINED) load_node_c(nodes + idx, c, m);
+    else load_node(nodes + idx, c, m);
     const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
     const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
     const bool leaf = m.y >= 0;
@@ -1316,8 +1327,8 @@ __device__ __forceinline__ void walk_counts_flush(uint32_t n_inter, uint32_t n_o
 constexpr uint32_t WALK_AHEAD_N = 148u * 1024u;
 template <bool FAST>
 __global__ void __launch_bounds__(WALK_THREADS)
-k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, const float4* __restrict__ pos,
-             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep, Forest F) {
+k_walk_ahead(const TNode* nodes, const uint32_t* order, const float4* __restrict__ pos,
+             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* frep, Forest F) {
   dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t T = st->error ? 0u : st->n_tree;
@@ -1331,7 +1342,7 @@ k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order
     uint32_t idx = T == 0u ? END : F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
     float4 c;
     int4 m;
-    if (idx < T) load_node(nodes + idx, c, m);
+    if (idx < T) load_node_c(nodes + idx, c, m);
     while (idx < T) {
       const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
       const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
@@ -1341,7 +1352,7 @@ k_walk_ahead(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order
       const uint32_t next = descend ? idx + 1u : (uint32_t)m.x;
       const float mass = c.w;
       if (next <= idx) break;
-      if (next < T) load_node(nodes + next, c, m);
+      if (next < T) load_node_c(nodes + next, c, m);
       if (use) {
         rep_term<FAST>(dx, dy, dz, r2, srd, mass, fx, fy, fz);
         ++n_inter;
@@ -1371,7 +1382,7 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
     const uint32_t body = order[a];
     if (!JC_IN_BOUNDS(body, n, &st->error)) return;
     const uint32_t root = F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
-    walk_one<FAST>(nodes, body, pos[body], __fmul_rn(P.scaling_ratio, degf[body]), root, T, P.theta2, st, frep,
+    walk_one<FAST, false>(nodes, body, pos[body], __fmul_rn(P.scaling_ratio, degf[body]), root, T, P.theta2, st, frep,
                    n_inter, n_open);
   } else if (a < n) {
     const uint32_t body = order[a];
@@ -1408,9 +1419,8 @@ constexpr size_t ww_warp_bytes(uint32_t words) {
 }
 
 __global__ void __launch_bounds__(32 * WW_WARPS)
-k_walk_warp(const TNode* __restrict__ nodes, const uint32_t* __restrict__ kids, const uint32_t* __restrict__ order,
-            const float4* __restrict__ pos, const float* __restrict__ degf, uint32_t n, KParams P, DevState* st,
-            float4* __restrict__ frep, uint32_t words) {
+k_walk_warp(const TNode* nodes, const uint32_t* kids, const uint32_t* order, const float4* __restrict__ pos,
+            const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* frep, uint32_t words) {
   dev::dependent_launch_wait();
   extern __shared__ uint4 ww_smem[];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
@@ -1447,7 +1457,7 @@ k_walk_warp(const TNode* __restrict__ nodes, const uint32_t* __restrict__ kids, 
         const uint32_t idx = have ? cur[k0 + lane] : 0u;
         float4 c;
         int4 m;
-        load_node(nodes + idx, c, m);
+        load_node_c(nodes + idx, c, m);
         const uint4 l0 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)idx);
         const uint4 l1 = *reinterpret_cast<const uint4*>(kids + 8 * (size_t)idx + 4);
         const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
@@ -1495,7 +1505,7 @@ k_walk_warp(const TNode* __restrict__ nodes, const uint32_t* __restrict__ kids, 
     // along the ropes, one lane
     if (lane == 0) {
       uint32_t ni = 0, no = 0;
-      walk_one<false>(nodes, body, p, srd, 0u, T, P.theta2, st, frep, ni, no);
+      walk_one<false, true>(nodes, body, p, srd, 0u, T, P.theta2, st, frep, ni, no);
       atomicAdd(&st->n_inter, (unsigned long long)ni);
       atomicAdd(&st->n_open, (unsigned long long)no);
     }
@@ -2075,9 +2085,9 @@ constexpr uint32_t UNSORTED_ROW = 32;
 template <bool UNSORTED>
 __global__ void __launch_bounds__(ATT_THREADS)
 k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr,
-      const float4* __restrict__ pos, const float4* __restrict__ frep, const float4* __restrict__ old_force,
-      const float* __restrict__ degf, KParams P, DevState* st, float4* __restrict__ force,
-      float2* __restrict__ stats, double2* __restrict__ partials, uint32_t n_graphs) {
+      const float4* __restrict__ pos, const float4* frep, const float4* __restrict__ old_force,
+      const float* __restrict__ degf, KParams P, DevState* st, float4* force, float2* stats, double2* partials,
+      uint32_t n_graphs) {
   dev::dependent_launch_wait();
   __shared__ double red_sw[ATT_THREADS / 32], red_tr[ATT_THREADS / 32];
   __shared__ float hub_sum[3][ATT_THREADS / 32];
@@ -2227,8 +2237,8 @@ k_att(const uint32_t* __restrict__ order, const uint32_t* __restrict__ off, cons
 
 // --------------------------------------------------------------- apply --
 __global__ void __launch_bounds__(APPLY_THREADS)
-k_apply(float4* __restrict__ pos, float4* __restrict__ old_force, const float4* __restrict__ force,
-        const float* __restrict__ degf, KParams P, const DevState* st, float* __restrict__ xyz, Forest F) {
+k_apply(float4* pos, float4* old_force, const float4* force, const float* __restrict__ degf, KParams P,
+        const DevState* st, float* xyz, Forest F) {
   dev::dependent_launch_wait();
   if (st->error) return;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3335,8 +3345,7 @@ class Fa2Engine : public Engine {
           launch_chained(chain, stream_, cdiv(n, 128), 128, 0, k_com_kids, first_.p, nodes_.p, parent_.p, nchild_.p,
                          kids_.p, arrive_.p, n, st);
         else
-          launch_chained(chain, stream_, cdiv(n, 256), 256, 0, k_com, first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p,
-                         n, st);
+          k_com<<<cdiv(n, 256), 256, 0, stream_>>>(first_.p, nodes_.p, parent_.p, nchild_.p, arrive_.p, n, st);
         L += 2;
         if (stage) {
           k_top_build<<<1, 1024, 0, stream_>>>(nodes_.p, top_list_.p, st, top_.p);
@@ -3435,8 +3444,8 @@ class Fa2Engine : public Engine {
                          degf_.p, n, P, st, frep_.p, forest_);
           break;
         }
-        launch_chained(chained(), stream_, grid.x, WALK_THREADS, 0, k_walk_rope<FAST>, nodes_.p, val_.p, pos_.p, degf_.p, n,
-                       P, st, frep_.p, forest_);
+        // (never chained: it reads the nodes through the read-only path)
+        k_walk_rope<FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_);
         break;
       case 2: k_walk<2, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;
       case 4: k_walk<4, FAST><<<grid, WALK_THREADS, 0, stream_>>>(nodes_.p, val_.p, pos_.p, degf_.p, n, P, st, frep_.p, forest_); break;

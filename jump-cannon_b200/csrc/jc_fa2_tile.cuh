@@ -69,17 +69,6 @@ struct TileBufs {
   uint32_t* count;
 };
 
-// Coherent 256-bit node load: the tile kernel reads nodes written earlier in
-// the same launch, so the non-coherent read-only path cannot be used.
-__device__ __forceinline__ void load_node_c(const TNode* p, float4& cm, int4& meta) {
-  uint32_t r0, r1, r2, r3, r4, r5, r6, r7;
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3), "=r"(r4), "=r"(r5), "=r"(r6), "=r"(r7)
-               : "l"(p));
-  cm = make_float4(__uint_as_float(r0), __uint_as_float(r1), __uint_as_float(r2), __uint_as_float(r3));
-  meta = make_int4((int)r4, (int)r5, (int)r6, (int)r7);
-}
-
 // The rope walk of one body over its graph's tree (local node indices,
 // root 0, T nodes); the same visit sequence and terms as walk_one. The next node
 // loads before the current term is added (k_walk_ahead); the kernel's 64 registers

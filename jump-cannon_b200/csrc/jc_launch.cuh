@@ -4,6 +4,13 @@
 // writes, in every thread that does so and in at least one thread whatever the
 // input, so completion passes down the chain. In an ordinary launch both
 // instructions do nothing.
+//
+// A dependent lives while the kernels before it still store, so for it their
+// output is not read-only data: it is read by ordinary loads (never __ldg or
+// ld.global.nc) and through pointers without __restrict__, which would allow
+// the compiler both, and a load moved above the wait. Only what the chain does not
+// write before the kernel (graphs, degrees, the positions until the last kernel
+// moves them) goes through the read-only path.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -226,11 +226,13 @@ __global__ void __launch_bounds__(256) k_features(GView v, const uint2* __restri
 
 // A neighbour's 8 projection columns: one 32-byte row, fetched as one
 // 256-bit load (one L1 request instead of two; the rows are 32-byte aligned).
+// Coherent: the step before wrote them, and the steps are chained.
 __device__ __forceinline__ void load_row8(const float* p, float4& q0, float4& q1) {
   uint32_t r0, r1, r2, r3, r4, r5, r6, r7;
-  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3), "=r"(r4), "=r"(r5), "=r"(r6), "=r"(r7)
-      : "l"(p));
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3), "=r"(r4), "=r"(r5), "=r"(r6), "=r"(r7)
+               : "l"(p)
+               : "memory");
   q0 = make_float4(__uint_as_float(r0), __uint_as_float(r1), __uint_as_float(r2), __uint_as_float(r3));
   q1 = make_float4(__uint_as_float(r4), __uint_as_float(r5), __uint_as_float(r6), __uint_as_float(r7));
 }
@@ -262,8 +264,8 @@ __device__ __forceinline__ float filter_out(float px, float x, float xp, float c
 // entries outlasted the rest of the step: 227,000 nodes 78 -> 18 us, 3.3 M
 // nodes 248 -> 142.
 template <int MODE>
-__device__ __forceinline__ void smooth_long(const GView& v, uint32_t i, const float* __restrict__ pin,
-                                            float* __restrict__ pout, const float* __restrict__ pprev, float c1) {
+__device__ __forceinline__ void smooth_long(const GView& v, uint32_t i, const float* pin, float* pout,
+                                            const float* pprev, float c1) {
   constexpr int K = 4;  // chunk: 4 K neighbours
   const uint32_t lane = threadIdx.x & 31, q = lane >> 3, c = lane & 7, d = v.deg[i];
   const uint32_t* row = v.nbr + v.off[i];
@@ -275,7 +277,7 @@ __device__ __forceinline__ void smooth_long(const GView& v, uint32_t i, const fl
   };
   auto vals = [&](uint32_t base) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) val[k] = base + 4 * k + q < d ? __ldg(pin + 8 * (size_t)id[k] + c) : 0.0f;
+    for (int k = 0; k < K; ++k) val[k] = base + 4 * k + q < d ? pin[8 * (size_t)id[k] + c] : 0.0f;
   };
   ids(0);
   vals(0);
@@ -303,8 +305,8 @@ __device__ __forceinline__ void smooth_long(const GView& v, uint32_t i, const fl
 inline uint32_t long_blocks(uint32_t n_long) { return cdiv(n_long, 8); }  // a warp per long row
 
 template <int MODE>
-__global__ void __launch_bounds__(256, 6) k_smooth(GView v, const float* __restrict__ pin, float* __restrict__ pout,
-                                                const float* __restrict__ pprev, float c1, uint32_t lb) {
+__global__ void __launch_bounds__(256, 6) k_smooth(GView v, const float* pin, float* pout, const float* pprev,
+                                                float c1, uint32_t lb) {
   dev::dependent_launch_wait();
   if (blockIdx.x < lb) {
     const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -400,9 +402,8 @@ __global__ void __launch_bounds__(256, 6) k_smooth(GView v, const float* __restr
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(256) k_smooth_hub(GView v, const uint32_t* __restrict__ hubs,
-                                                    const float* __restrict__ pin, float* __restrict__ pout,
-                                                    const float* __restrict__ pprev, float c1) {
+__global__ void __launch_bounds__(256) k_smooth_hub(GView v, const uint32_t* __restrict__ hubs, const float* pin,
+                                                    float* pout, const float* pprev, float c1) {
   dev::dependent_launch_wait();
   __shared__ float part[HUB_SEGS][NPROJ];
   const uint32_t i = hubs[blockIdx.x], d = v.deg[i];
@@ -434,15 +435,15 @@ __global__ void __launch_bounds__(256) k_smooth_hub(GView v, const uint32_t* __r
 // to unit mean square at the same time so the decaying modes never underflow.
 constexpr int CEN = 2 * NPROJ + 1;
 // blockIdx.y picks the array (x, or the Chebyshev pair's x_prev).
-__global__ void __launch_bounds__(256) k_proj_center_sums(const float* __restrict__ P0, const float* __restrict__ P1,
+__global__ void __launch_bounds__(256) k_proj_center_sums(const float* P0, const float* P1,
                                                           const uint32_t* __restrict__ deg,
                                                           const int4* __restrict__ items, uint32_t n_items,
-                                                          double* __restrict__ part0, double* __restrict__ part1) {
+                                                          double* part0, double* part1) {
   dev::dependent_launch_wait();
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= n_items) return;
-  const float* __restrict__ P = blockIdx.y ? P1 : P0;
-  double* __restrict__ part = blockIdx.y ? part1 : part0;
+  const float* P = blockIdx.y ? P1 : P0;
+  double* part = blockIdx.y ? part1 : part0;
   const int4 it = items[w];
   double acc[CEN];
 #pragma unroll
@@ -472,10 +473,9 @@ __global__ void __launch_bounds__(256) k_proj_center_sums(const float* __restric
 // w + 8, ..., then the warps' sums in order (one shape on every run). Every
 // node recomputing them from the sums spent its pass on f64 divisions
 // (227,000 nodes: 15 us a pass and 21 for the pair, now 6 with 6 here).
-__global__ void __launch_bounds__(256) k_center_coef(const double* __restrict__ part, const double* __restrict__ part_prev,
+__global__ void __launch_bounds__(256) k_center_coef(const double* part, const double* part_prev,
                                                      const uint32_t* __restrict__ item_off,
-                                                     const uint32_t* __restrict__ go,
-                                                     float4* __restrict__ coef) {
+                                                     const uint32_t* __restrict__ go, float4* coef) {
   dev::dependent_launch_wait();
   __shared__ double sm[8][2][32];
   const uint32_t g = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -510,8 +510,7 @@ __global__ void __launch_bounds__(256) k_center_coef(const double* __restrict__ 
 // the three-term recurrence intact (the constant vector is an eigenvector of
 // the walk and the projection that removes it commutes with the walk). Four
 // columns per thread.
-__global__ void __launch_bounds__(256) k_proj_center(GView v, const float4* __restrict__ coef,
-                                                     float* __restrict__ P, float* __restrict__ Pprev) {
+__global__ void __launch_bounds__(256) k_proj_center(GView v, const float4* coef, float* P, float* Pprev) {
   dev::dependent_launch_wait();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t w = t >> 1, h = t & 1;

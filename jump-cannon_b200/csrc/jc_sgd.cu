@@ -269,9 +269,8 @@ __device__ __forceinline__ float4 pair_moved(float4 p, const long long* a, uint3
 // One batch: every pair against the batch-start positions, both moves added in
 // fixed point.
 __global__ void __launch_bounds__(128)
-k_pairs(const uint4* __restrict__ samples, uint32_t count, const float4* __restrict__ pos,
-        long long* __restrict__ acc, uint32_t* __restrict__ cnt, const float* __restrict__ eta_table, uint32_t n_eta,
-        const uint32_t* __restrict__ sweep_ctr, uint32_t sweep) {
+k_pairs(const uint4* __restrict__ samples, uint32_t count, const float4* pos, long long* acc, uint32_t* cnt,
+        const float* __restrict__ eta_table, uint32_t n_eta, const uint32_t* __restrict__ sweep_ctr, uint32_t sweep) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= count) return;
   const uint32_t sw = *sweep_ctr + sweep;
@@ -294,8 +293,7 @@ k_pairs(const uint4* __restrict__ samples, uint32_t count, const float4* __restr
 // that moved. Sums and position are read beside the count: only the owner
 // writes them, after its own reads.
 __global__ void __launch_bounds__(128)
-k_pairs_apply(const uint4* __restrict__ samples, uint32_t count, float4* __restrict__ pos, long long* __restrict__ acc,
-              uint32_t* __restrict__ cnt) {
+k_pairs_apply(const uint4* __restrict__ samples, uint32_t count, float4* pos, long long* acc, uint32_t* cnt) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 2 * count) return;
   const uint4 s = samples[t >> 1];

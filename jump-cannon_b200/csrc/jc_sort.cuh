@@ -118,9 +118,8 @@ os_hist(const K* __restrict__ keys, uint32_t n, int bit_begin, int passes, uint3
 
 template <typename K, int ROUNDS = RS_ROUNDS>
 __global__ void __launch_bounds__(RS_THREADS)
-os_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
-        uint32_t* __restrict__ vout, uint32_t n, int shift, const uint32_t* __restrict__ gcount, uint32_t* status,
-        uint32_t* tile_ctr, uint32_t* err) {
+os_pass(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, uint32_t n, int shift, const uint32_t* gcount,
+        uint32_t* status, uint32_t* tile_ctr, uint32_t* err) {
   dependent_launch_wait();
   __shared__ uint32_t wcnt[RS_WARPS][RS_RADIX];
   __shared__ uint32_t base[RS_RADIX];
