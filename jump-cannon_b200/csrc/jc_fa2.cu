@@ -1411,7 +1411,7 @@ constexpr uint32_t WW_QUEUE = 512, WW_LIST = 1024, WW_TERMS = 256, WW_WARPS = 4;
 constexpr uint32_t WW_ROW = WW_TERMS + 4;  // axes 4 banks apart
 constexpr uint32_t WW_MAX_N = 10240u;
 constexpr float WW_MIN_THETA2 = 0.4f;      // below, lists outgrow their arrays
-inline uint32_t ww_words(uint32_t n) { return std::min(1024u, (2u * n + 8u + 63u) / 64u); }  // 64 nodes each
+constexpr uint32_t ww_words(uint32_t n) { return std::min(1024u, (2u * n + 8u + 63u) / 64u); }  // 64 nodes each
 constexpr size_t ww_warp_bytes(uint32_t words) {
   // bitmap, ranks, list, then the two queues or the terms
   const size_t q = 2 * 2 * (size_t)WW_QUEUE, t = 3 * 4 * (size_t)WW_ROW;
@@ -2443,8 +2443,9 @@ inline void launch_graph_build_as(const float4* pos, const float* degf, const Fo
                                   cudaStream_t s) {
   const uint32_t items = gb_items(biggest);
   const size_t smem = gb_smem(items, T);
-  if (smem > 32 * 1024)
-    JC_CUDA_CHECK(cudaFuncSetAttribute(k_graph_build<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (the limit belongs to the kernel, not to one engine: always the most any launch takes)
+  JC_CUDA_CHECK(cudaFuncSetAttribute(k_graph_build<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)gb_smem(gb_items(gb_max_n(T)), T)));
   k_graph_build<T><<<F.n_graphs, T, smem, s>>>(pos, degf, F, order, key, val, first_total, nodes, cells, P, st, tally, items,
                                                kids);
 }
@@ -2465,8 +2466,7 @@ inline void launch_walk_warp(bool chained, const TNode* nodes, const uint32_t* k
                              float4* frep, cudaStream_t s) {
   const uint32_t words = ww_words(n);
   const size_t smem = WW_WARPS * ww_warp_bytes(words);
-  if (smem > 48 * 1024)
-    JC_CUDA_CHECK(cudaFuncSetAttribute(k_walk_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static_assert(WW_WARPS * ww_warp_bytes(ww_words(WW_MAX_N)) <= 48 * 1024, "needs no opt-in");
   launch_chained(chained, s, cdiv(n, WW_WARPS), 32 * WW_WARPS, smem, k_walk_warp, nodes, kids, order, pos, degf, n,
                  P, st, frep, words);
 }

@@ -45,6 +45,9 @@ constexpr uint32_t GB_MIDDLE = 4096;
 // 66, 41, 40, 45; 1,000 78, 53, 51, 55; 2,000 86, 78, 70, 72; 3,000 97, 125, 89, 91;
 // 4,000 103, 154, 109, 108.
 constexpr uint32_t GB_SINGLE_N = 3072, GB_SINGLE_256 = 256, GB_SINGLE_512 = GB_SINGLE_N;
+// The largest graph that T threads take.
+constexpr uint32_t gb_max_n(int T) { return T == 256 ? GB_SMALL : T == 512 ? GB_MIDDLE : GB_MAX_N; }
+static_assert(GB_SINGLE_256 <= GB_SMALL && GB_SINGLE_N <= GB_MIDDLE, "a single graph's sizes too");
 constexpr int GB_DEPTHS = 33;        // cell depths 0..32
 
 template <int T>

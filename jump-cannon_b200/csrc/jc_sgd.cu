@@ -958,8 +958,10 @@ class SgdEngine : public Engine {
       const size_t smem = sizeof(float4) * k + sizeof(float2) * mu_len;
       if (sizeof(float4) * k + sizeof(float) * mu_len > 200 * 1024)
         fail(JC_ERR_ARG, "too many pivots for the shared-memory pivot stage");
+      // (the limit belongs to the kernel, not to one engine: always the most any launch takes)
       if (smem > 48 * 1024)
-        JC_CUDA_CHECK(cudaFuncSetAttribute(k_jacobi<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        JC_CUDA_CHECK(cudaFuncSetAttribute(k_jacobi<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           200 * 1024 + (int)(sizeof(float) * JACOBI_MU_MAX)));
       float4* in = pos_a_.p;
       float4* out = pos_b_.p;
       const uint32_t threads = n <= JACOBI_SMALL_N ? 64u : 256u;
