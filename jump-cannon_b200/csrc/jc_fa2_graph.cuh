@@ -34,6 +34,14 @@ struct GraphTally {
 };
 
 constexpr uint32_t GB_MAX_N = 8192;   // bodies of the largest graph
+// Runs of keys with equal top words up to this long are ordered by counting, each entry
+// against its run; a longer one, or one where GB_TIES others share an entry's next 32
+// bits too (each such pair reads a whole key), sends the graph through the sort of whole
+// keys. B200, us of this phase in one CTA, a thread a run of up to 32 and now: clusters of
+// 100 bodies, 2,000 bodies 44 -> 13, 8,000 229 -> 51 (a batch's step 639 -> 294, and 350
+// by the forest's kernels); uniform layouts of 8,000 2.8 -> 2.3. (A bitonic network over
+// whole keys in place of the sixteen passes: 85 us for 8,000 bodies, where these take 80.)
+constexpr uint32_t GB_RUN = 128, GB_TIES = 16;
 // Threads a graph by the largest one: 256, from 2,048 bodies 512, from 4,096 1,024.
 // us a step: 1,000 graphs to 2,000 bodies 233 with 256 threads, 269 with 512; 300 to
 // 4,000 379 with 256, 319 with 512; 1,000 to 4,096 421 with 512, 520 with 1,024; 60 to
@@ -60,7 +68,9 @@ struct GraphShared {
   float size2[GB_DEPTHS];  // (cell side)^2 by depth
   unsigned long long zf;
   uint32_t n_invalid;
-  uint32_t long_run;
+  uint32_t n_run;
+  uint32_t long_run;  // a run past GB_RUN (set before the counting)
+  uint32_t tied;      // an entry with GB_TIES ties (set by it)
   uint32_t dropped;
   uint32_t leaf_depth;
   uint32_t base;
@@ -210,7 +220,9 @@ k_graph_build(const float4* __restrict__ pos, const float* __restrict__ degf, Fo
       S.root = root;
       S.zf = flat_z_bits(r[2], r[5], root);
       S.n_invalid = 0;
+      S.n_run = 0;
       S.long_run = 0;
+      S.tied = 0;
       S.dropped = 0;
       S.leaf_depth = 0;
     }
@@ -241,38 +253,66 @@ k_graph_build(const float4* __restrict__ pos, const float* __restrict__ degf, Fo
   // ---- sort: the top 32 bits, then the runs of equal tops (k_seg_fix) ----
   for (int p = 0; p < 4; ++p)
     gb_pass<T>(p & 1 ? k1 : k0, p & 1 ? v1 : v0, p & 1 ? k0 : k1, p & 1 ? v0 : v1, n, 8 * p, wcnt, S.scan, &st->error);
-  for (uint32_t a = tid; a < N; a += T) {
-    const uint32_t top = k0[a];
-    if (a > 0 && k0[a - 1] == top) continue;  // not the first of its run
-    uint32_t len = 1;
-    while (a + len < N && len <= SEG_MAX && k0[a + len] == top) ++len;
-    if (len == 1) continue;
-    if (len > SEG_MAX) {
-      S.long_run = 1u;
-      continue;
+  // A thread an entry: its place in its run is the number of the run's entries
+  // before it, by the key's next 32 bits in shared memory (whole keys only where
+  // those tie). A thread a run, sorting up to 32 entries, kept the CTA waiting for
+  // its longest runs (see GB_RUN).
+  auto whole = [&](uint32_t a) {
+    const uint32_t v = v0[a];
+    return JC_IN_BOUNDS(v, n, &st->error) ? key[v] : make_ulonglong2(0ull, 0ull);
+  };
+  uint16_t* const entry = reinterpret_cast<uint16_t*>(wcnt);  // the entries in runs, in any order
+  for (uint32_t a0 = 0; a0 < N; a0 += T) {
+    const uint32_t a = a0 + tid, top = a < N ? k0[a] : 0u;
+    const bool in = a < N && ((a > 0 && k0[a - 1] == top) || (a + 1 < N && k0[a + 1] == top));
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+    if (m == 0u) continue;  // (the warp's)
+    if (a + GB_RUN < N && k0[a + GB_RUN] == top) S.long_run = 1u;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&S.n_run, (uint32_t)__popc(m));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+    if (in) {
+      entry[at] = (uint16_t)a;
+      k1[a] = (uint32_t)whole(a).x;
     }
-    ulonglong2 k[SEG_MAX];
-    uint32_t v[SEG_MAX];
-    for (uint32_t q = 0; q < len; ++q) {
-      v[q] = v0[a + q];
-      k[q] = JC_IN_BOUNDS(v[q], n, &st->error) ? key[v[q]] : make_ulonglong2(0ull, 0ull);
-    }
-    for (uint32_t q = 1; q < len; ++q) {
-      const ulonglong2 kk = k[q];
-      const uint32_t vv = v[q];
-      uint32_t j = q;
-      while (j > 0 && key_after(k[j - 1], v[j - 1], kk, vv)) {
-        k[j] = k[j - 1];
-        v[j] = v[j - 1];
-        --j;
-      }
-      k[j] = kk;
-      v[j] = vv;
-    }
-    for (uint32_t q = 0; q < len; ++q) v0[a + q] = (uint16_t)v[q];
   }
   __syncthreads();
-  if (S.long_run) {
+  const uint32_t n_run = S.n_run;
+  if (n_run && !S.long_run) {
+    for (uint32_t q = tid; q < n_run; q += T) {
+      const uint32_t a = entry[q], top = k0[a], low = k1[a], body = v0[a];
+      const ulonglong2 own = whole(a);
+      uint32_t left = 0, right = 0, before = 0, ties = 0;
+      while (ties < GB_TIES && left < a && k0[a - left - 1] == top) {
+        ++left;
+        const uint32_t x = k1[a - left];
+        before += x < low ? 1u : 0u;
+        if (x == low) {
+          ++ties;
+          before += key_after(whole(a - left), v0[a - left], own, body) ? 0u : 1u;
+        }
+      }
+      while (ties < GB_TIES && a + right + 1 < N && k0[a + right + 1] == top) {
+        ++right;
+        const uint32_t x = k1[a + right];
+        before += x < low ? 1u : 0u;
+        if (x == low) {
+          ++ties;
+          before += key_after(own, body, whole(a + right), v0[a + right]) ? 1u : 0u;
+        }
+      }
+      if (ties >= GB_TIES) {
+        S.tied = 1u;
+        break;
+      }
+      v1[a - left + before] = (uint16_t)body;
+    }
+    __syncthreads();
+    if (!S.tied)
+      for (uint32_t q = tid; q < n_run; q += T) v0[entry[q]] = v1[entry[q]];
+    __syncthreads();
+  }
+  if (S.long_run || S.tied) {
     // the whole order, stably by the four words of the key from body order
     for (int word = 0; word < 4; ++word) {
       for (uint32_t i = tid; i < n; i += T) {

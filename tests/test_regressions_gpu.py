@@ -1,5 +1,6 @@
 """Faults that were found in use, each held by the smallest call that shows it."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -57,3 +58,67 @@ def test_shared_memory_limit_is_no_engines_own(jc, kind):
         return go
 
     assert _concurrently([work(8000, 6000), work(4200, 3500)]) == []
+
+
+def _best(f, reps=7):
+    ts = []
+    for _ in range(reps):
+        t = time.perf_counter()
+        f()
+        ts.append(time.perf_counter() - t)
+    return min(ts)
+
+
+def _clustered(jc, n, dim, seed):
+    """Tight clusters of about 100 bodies: long runs share the first ten octant levels."""
+    r = np.random.RandomState(seed)
+    c = max(1, n // 100)
+    p = np.zeros((n, 3), np.float32)
+    p[:, :dim] = r.uniform(-1, 1, (c, dim))[np.arange(n) % c] + r.normal(0, 1e-3, (n, dim))
+    return p.reshape(-1)
+
+
+# One CTA a graph, runs of equal first levels on both sides of the longest that is
+# ordered by counting (128; `far` has one of n - 1) and of the ties it takes (16 of an
+# entry: `ties`), distinct keys, whole keys repeated, a body at no position
+@pytest.mark.parametrize("case", ["far", "lattice", "ties16", "ties17", "nan"])
+@pytest.mark.parametrize("n", [34, 128, 129, 130, 256, 257, 1000, 2048, 3072])
+def test_long_runs_of_one_graph_bit_exact(jc, orc, n, case):
+    pos = jc.seed_uniform(n, 3, n)
+    if case == "lattice":
+        pos = (np.round(pos * 4) / 4).astype(np.float32)
+    pos[:3] = 3.0e4
+    if case.startswith("ties"):  # groups that share 64 bits of the key and differ below
+        pos[:3] = 1.0
+        q, k = pos.reshape(n, 3), int(case[4:])
+        q[1:] = q[1 + (np.arange(n - 1) // k) * k] + np.float32(1e-6) * (np.arange(n - 1) % k)[:, None]
+    if case == "nan":
+        pos[3 * (n // 2) + 1] = np.nan
+    g = jc.gen_scale_free(n, 2, n)
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params({"theta": 0.8})
+    e.init(g, pos)
+    o = orc.Fa2(g, pos, bh=True, theta=0.8)
+    o.set_tree_capacity(1 << 20)
+    for _ in range(2):
+        e.step()
+        o.step()
+        f, r = e.forces()[0], o.get()["force"]
+        assert np.array_equal(np.isnan(f), np.isnan(r))
+        assert np.array_equal(bits(f)[~np.isnan(f)], bits(r)[~np.isnan(r)])
+
+
+# A batch of clustered layouts took 2.6 to 3.1 times a uniform one's step (sixteen
+# radix passes a graph in place of four); the forest's kernels 1.1 times
+@pytest.mark.parametrize("lo,hi", [(50, 2000), (1000, 4000), (4000, 8000)])
+def test_clustered_batch_costs_no_multiple(jc, lo, hi):
+    sizes = np.linspace(lo, hi, 40).astype(int)
+    graphs = [jc.gen_scale_free(int(n), 3, int(n)) for n in sizes]
+    t = []
+    for make in (lambda n: jc.seed_uniform(n, 2, n), lambda n: _clustered(jc, n, 2, n)):
+        e = jc.LayoutEngine("fa2-bh")
+        e.set_params({"theta": 0.8, "max_displacement": 1e-9})
+        e.init_batch(graphs, [make(int(n)) for n in sizes])
+        e.step_many(5, readback=False)
+        t.append(_best(lambda: e.step_many(50, readback=False)))
+    assert t[1] < 1.8 * t[0]
