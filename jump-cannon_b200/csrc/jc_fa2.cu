@@ -1326,6 +1326,36 @@ __device__ __forceinline__ void walk_counts_flush(uint32_t n_inter, uint32_t n_o
 // 74. Fewer bodies per warp: no gain from 16, slower below 8.)
 constexpr uint32_t WALK_AHEAD_N = 148u * 1024u;
 template <bool FAST>
+__device__ __forceinline__ void walk_one_ahead(const TNode* nodes, uint32_t body, const float4 p, float srd,
+                                               uint32_t root, uint32_t T, float theta2, DevState* st, float4* frep,
+                                               uint32_t& n_inter, uint32_t& n_open) {
+  float fx = 0.0f, fy = 0.0f, fz = 0.0f;
+  uint32_t idx = root;
+  float4 c;
+  int4 m;
+  if (idx < T) load_node_c(nodes + idx, c, m);
+  while (idx < T) {
+    const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
+    const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    const bool leaf = m.y >= 0;
+    const bool use = leaf ? (uint32_t)m.y != body : __int_as_float(m.z) < __fmul_rn(theta2, r2);
+    const bool descend = !leaf && !use;
+    const uint32_t next = descend ? idx + 1u : (uint32_t)m.x;
+    const float mass = c.w;
+    if (next <= idx) break;
+    if (next < T) load_node_c(nodes + next, c, m);
+    if (use) {
+      rep_term<FAST>(dx, dy, dz, r2, srd, mass, fx, fy, fz);
+      ++n_inter;
+    }
+    n_open += descend ? 1u : 0u;
+    idx = next;
+  }
+  if (idx != END) set_error(st, JC_ERR_DEVICE_TIMEOUT);
+  frep[body] = make_float4(fx, fy, fz, 0.0f);
+}
+
+template <bool FAST>
 __global__ void __launch_bounds__(WALK_THREADS)
 k_walk_ahead(const TNode* nodes, const uint32_t* order, const float4* __restrict__ pos,
              const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* frep, Forest F) {
@@ -1336,32 +1366,9 @@ k_walk_ahead(const TNode* nodes, const uint32_t* order, const float4* __restrict
   if (a < n) {
     const uint32_t body = order[a];
     if (!JC_IN_BOUNDS(body, n, &st->error)) return;
-    const float4 p = pos[body];
-    const float srd = __fmul_rn(P.scaling_ratio, degf[body]);
-    float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-    uint32_t idx = T == 0u ? END : F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
-    float4 c;
-    int4 m;
-    if (idx < T) load_node_c(nodes + idx, c, m);
-    while (idx < T) {
-      const float dx = __fsub_rn(p.x, c.x), dy = __fsub_rn(p.y, c.y), dz = __fsub_rn(p.z, c.z);
-      const float r2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-      const bool leaf = m.y >= 0;
-      const bool use = leaf ? (uint32_t)m.y != body : __int_as_float(m.z) < __fmul_rn(P.theta2, r2);
-      const bool descend = !leaf && !use;
-      const uint32_t next = descend ? idx + 1u : (uint32_t)m.x;
-      const float mass = c.w;
-      if (next <= idx) break;
-      if (next < T) load_node_c(nodes + next, c, m);
-      if (use) {
-        rep_term<FAST>(dx, dy, dz, r2, srd, mass, fx, fy, fz);
-        ++n_inter;
-      }
-      n_open += descend ? 1u : 0u;
-      idx = next;
-    }
-    if (idx != END) set_error(st, JC_ERR_DEVICE_TIMEOUT);
-    frep[body] = make_float4(fx, fy, fz, 0.0f);
+    const uint32_t root = T == 0u ? END : F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
+    walk_one_ahead<FAST>(nodes, body, pos[body], __fmul_rn(P.scaling_ratio, degf[body]), root, T, P.theta2, st, frep,
+                         n_inter, n_open);
   }
   walk_counts_flush(n_inter, n_open, st);
 }
@@ -1401,8 +1408,11 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
 // over node indices. A population count of the bitmap below a node is its
 // term's rank; the lanes compute the terms into rank order, WW_TERMS at a time,
 // and one lane per axis adds them. Same terms, same roundings, same order as the
-// rope walk. A body that outgrows the queue or the list (or a tree past the
-// bitmap) is walked along the ropes by one lane. (Exact mode only: the tolerance
+// rope walk. A body that outgrows the queue or the list is walked along the ropes
+// by one lane, as all are where the tree outgrows the bitmaps (close pairs, each
+// under a chain of cells); past WW_LANES_N bodies the first blocks then walk a body a
+// lane, as k_walk_ahead does, and the rest leave (us a walk, a lane a warp and this:
+// 3,000 bodies 54 and 56, 5,000 71 -> 65, 10,000 147 -> 70). (Exact mode only: the tolerance
 // mode's fused accumulation has no separate terms.) Bound by instruction issue from
 // about 10,000 bodies on (it issues three times the rope walk's instructions).
 // B200, us a walk, k_walk_ahead and this, theta 0.8: 400 bodies (0.7) 39 -> 12,
@@ -1410,6 +1420,7 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
 constexpr uint32_t WW_QUEUE = 512, WW_LIST = 1024, WW_TERMS = 256, WW_WARPS = 4;
 constexpr uint32_t WW_ROW = WW_TERMS + 4;  // axes 4 banks apart
 constexpr uint32_t WW_MAX_N = 10240u;
+constexpr uint32_t WW_LANES_N = 4096u;
 constexpr float WW_MIN_THETA2 = 0.4f;      // below, lists outgrow their arrays
 constexpr uint32_t ww_words(uint32_t n) { return std::min(1024u, (2u * n + 8u + 63u) / 64u); }  // 64 nodes each
 constexpr size_t ww_warp_bytes(uint32_t words) {
@@ -1431,6 +1442,17 @@ k_walk_warp(const TNode* nodes, const uint32_t* kids, const uint32_t* order, con
   uint16_t* queue = list + WW_LIST;                       // two of WW_QUEUE
   float* terms = reinterpret_cast<float*>(queue);         // [3][WW_ROW], after the traversal
   const uint32_t T = st->error ? 0u : st->n_tree;
+  if (T > 64u * words && n > WW_LANES_N) {  // (the whole grid)
+    const uint32_t a = blockIdx.x * (32 * WW_WARPS) + threadIdx.x;
+    if (blockIdx.x * (32 * WW_WARPS) >= n) return;
+    uint32_t ni = 0, no = 0;
+    const uint32_t body = a < n ? order[a] : n;
+    if (a < n && JC_IN_BOUNDS(body, n, &st->error))
+      walk_one_ahead<false>(nodes, body, pos[body], __fmul_rn(P.scaling_ratio, degf[body]), 0u, T, P.theta2, st, frep, ni,
+                            no);
+    walk_counts_flush(ni, no, st);
+    return;
+  }
   const uint32_t a = blockIdx.x * WW_WARPS + w;
   if (a >= n) return;
   const uint32_t body = order[a];

@@ -147,3 +147,26 @@ def test_tree_of_close_pairs_is_no_slower_in_one_launch(jc):
     one, _ = _step_and_phases(jc, 2000)
     passes, _ = _step_and_phases(jc, 2000, walk_stage_top=True)
     assert one < 1.03 * passes
+
+
+# A tree past the warp walk's bitmaps: 147 us a walk of 10,000 bodies (one lane a warp)
+# beside 121 of the staged walk, now 70
+def test_walk_past_the_bitmaps_is_no_slower(jc):
+    assert _step_and_phases(jc, 10000)[1][1] < _step_and_phases(jc, 10000, walk_stage_top=True)[1][1]
+
+
+# ... whose bodies then go a lane each (past 4,096 bodies): partial blocks and warps
+@pytest.mark.parametrize("n", [4096, 4097, 5003, 10240])
+def test_walk_past_the_bitmaps_bit_exact(jc, orc, n):
+    g, pos = jc.gen_scale_free(n, 2, n), _close_pairs(jc, n)
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params({"theta": 0.8, "hub_threshold": 1 << 30})
+    e.init(g, pos)
+    o = orc.Fa2(g, pos, bh=True, theta=0.8)
+    o.set_tree_capacity(1 << 20)
+    for _ in range(2):
+        e.step()
+        o.step()
+        r = o.get()
+        assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
+        assert e.walk_counts() == (r["n_inter"], r["n_open"])
