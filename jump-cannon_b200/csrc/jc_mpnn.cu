@@ -823,23 +823,75 @@ __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf(
 
 // Lanes per node of the pair passes: a node has about 14 pairs (its row and 8
 // partners), so a whole warp per node left more than half of its lanes idle.
-constexpr uint32_t PAIR_LANES = 16;
-__device__ __forceinline__ double pair_sum(double x) {
-  const uint32_t mask = 0xFFFFu << (threadIdx.x & 16u);
+constexpr int PAIR_LANES = 16;
+constexpr int SCALE_LANES = 8;
+
+// A pass over rows by their length: a block for a hub row (blocks [0, nh)), a warp
+// for a long row (the next long_blocks), LANES lanes for any other node. With LANES
+// for every row a hub's entries outlasted the pass: R-MAT of 262,144 nodes, us a pass,
+// a warp for every row / LANES for every row / this: k_loss_stats 836 / 1,526 / 157,
+// k_loss_grad 928 / 1,696 / 208, k_scale_vals 564 / 1,665 / 79.
+struct RowShare {
+  uint32_t w, lane, lanes;  // node (batch row), and this thread's place among those on it
+};
+template <int LANES>
+__device__ __forceinline__ bool row_share(const GView& v, const uint32_t* hubs, uint32_t nh, RowShare& r) {
+  const uint32_t lb = (v.n_long + 7u) / 8u;
+  if (blockIdx.x < nh) {
+    r = {hubs[blockIdx.x] - v.n0, threadIdx.x, 256u};
+    return true;
+  }
+  if (blockIdx.x < nh + lb) {
+    const uint32_t k = (blockIdx.x - nh) * 8 + (threadIdx.x >> 5);
+    if (k >= v.n_long) return false;
+    r = {v.longs[k] - v.n0, threadIdx.x & 31u, 32u};
+    return true;
+  }
+  r = {((blockIdx.x - nh - lb) * 256u + threadIdx.x) / LANES, threadIdx.x % LANES, (uint32_t)LANES};
+  return r.w < v.nb && v.deg[v.n0 + r.w] <= LONG_DEG;
+}
+template <int LANES>
+inline uint32_t row_blocks(const GView& v, uint32_t nh) {
+  return nh + long_blocks(v.n_long) + cdiv((uint64_t)v.nb * LANES, 256);
+}
+
+// The sums of x over the threads on a node, in its first thread (true there).
+template <int LANES, int V>
+__device__ __forceinline__ bool row_sum(const RowShare& r, double (&x)[V]) {
+  if (r.lanes == (uint32_t)LANES) {
+    const uint32_t mask = (uint32_t)((1ull << LANES) - 1ull) << (threadIdx.x & 31u & ~(uint32_t)(LANES - 1));
 #pragma unroll
-  for (int o = PAIR_LANES / 2; o; o >>= 1) x += __shfl_xor_sync(mask, x, o);
-  return x;
+    for (int k = 0; k < V; ++k)
+#pragma unroll
+      for (int o = LANES / 2; o; o >>= 1) x[k] += __shfl_xor_sync(mask, x[k], o);
+    return r.lane == 0;
+  }
+#pragma unroll
+  for (int k = 0; k < V; ++k) x[k] = warp_sum(x[k]);
+  if (r.lanes == 32u) return r.lane == 0;
+  __shared__ double part[8][V];  // a hub: the whole block
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < V; ++k) part[threadIdx.x >> 5][k] = x[k];
+  __syncthreads();
+  if (threadIdx.x != 0) return false;
+#pragma unroll
+  for (int k = 0; k < V; ++k)
+    for (int q = 1; q < 8; ++q) x[k] += part[q][k];
+  return true;
 }
 
 // Per node: sum q, sum q^2 and the pair count (target distances < 1e-6 skipped).
-__global__ void __launch_bounds__(256) k_loss_stats(PairCtx p, double* __restrict__ vals) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_LANES, lane = threadIdx.x % PAIR_LANES;
-  if (w >= p.v.nb) return;
+__global__ void __launch_bounds__(256) k_loss_stats(PairCtx p, const uint32_t* __restrict__ hubs, uint32_t nh,
+                                                    double* __restrict__ vals) {
+  RowShare share;
+  if (!row_share<PAIR_LANES>(p.v, hubs, nh, share)) return;
+  const uint32_t w = share.w;
   const uint32_t i = p.v.n0 + w, d = p.v.deg[i], rowb = p.v.off[i], g = p.v.gid[i];
   const uint32_t gb = p.v.go[g], ng = p.v.go[g + 1] - gb;
   const float4 ti = p.T[i], yi = p.Y[w];
-  double s1 = 0.0, s2 = 0.0, c = 0.0;
-  for (uint32_t q = lane; q < d + p.partners; q += PAIR_LANES) {
+  double s[3] = {};  // sum q, sum q^2, count
+  for (uint32_t q = share.lane; q < d + p.partners; q += share.lanes) {
     uint32_t j;
     if (!pair_at(p, i, d, rowb, q, gb, ng, &j)) continue;
     const float4 tj = p.T[j], yj = p.Y[j - p.v.n0];
@@ -847,17 +899,14 @@ __global__ void __launch_bounds__(256) k_loss_stats(PairCtx p, double* __restric
     if (!(dt >= 1e-6f)) continue;
     const float r = len3(yi.x - yj.x, yi.y - yj.y, yi.z - yj.z);
     const double qq = (double)r / (double)dt;
-    s1 += qq;
-    s2 += qq * qq;
-    c += 1.0;
+    s[0] += qq;
+    s[1] += qq * qq;
+    s[2] += 1.0;
   }
-  s1 = pair_sum(s1);
-  s2 = pair_sum(s2);
-  c = pair_sum(c);
-  if (lane == 0) {
-    vals[(size_t)w * 3] = s1;
-    vals[(size_t)w * 3 + 1] = s2;
-    vals[(size_t)w * 3 + 2] = c;
+  if (row_sum<PAIR_LANES>(share, s)) {
+    vals[(size_t)w * 3] = s[0];
+    vals[(size_t)w * 3 + 1] = s[1];
+    vals[(size_t)w * 3 + 2] = s[2];
   }
 }
 
@@ -895,16 +944,18 @@ __global__ void __launch_bounds__(256) k_loss_finish(const double* __restrict__ 
 }
 
 // dL/dY_i = sum over i's pairs of coef_g (alpha q - 1) alpha / d * (Y_i - Y_j) / r.
-__global__ void __launch_bounds__(256) k_loss_grad(PairCtx p, const double* __restrict__ galpha,
+__global__ void __launch_bounds__(256) k_loss_grad(PairCtx p, const uint32_t* __restrict__ hubs, uint32_t nh,
+                                                   const double* __restrict__ galpha,
                                                    const double* __restrict__ gcoef, float4* __restrict__ dY) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / PAIR_LANES, lane = threadIdx.x % PAIR_LANES;
-  if (w >= p.v.nb) return;
+  RowShare share;
+  if (!row_share<PAIR_LANES>(p.v, hubs, nh, share)) return;
+  const uint32_t w = share.w;
   const uint32_t i = p.v.n0 + w, d = p.v.deg[i], rowb = p.v.off[i], g = p.v.gid[i];
   const uint32_t gb = p.v.go[g], ng = p.v.go[g + 1] - gb;
   const double a = galpha[g - p.v.g0], cf = gcoef[g - p.v.g0];
   const float4 ti = p.T[i], yi = p.Y[w];
-  double gx = 0.0, gy = 0.0, gz = 0.0;
-  for (uint32_t q = lane; q < d + p.partners; q += PAIR_LANES) {
+  double s[3] = {};
+  for (uint32_t q = share.lane; q < d + p.partners; q += share.lanes) {
     uint32_t j;
     if (!pair_at(p, i, d, rowb, q, gb, ng, &j)) continue;
     const float4 tj = p.T[j], yj = p.Y[j - p.v.n0];
@@ -915,14 +966,11 @@ __global__ void __launch_bounds__(256) k_loss_grad(PairCtx p, const double* __re
     if (!(r > 1e-12f)) continue;
     const double qq = (double)r / (double)dt;
     const double wgt = cf * (a * qq - 1.0) * a / ((double)dt * (double)r);
-    gx += wgt * dx;
-    gy += wgt * dy;
-    gz += wgt * dz;
+    s[0] += wgt * dx;
+    s[1] += wgt * dy;
+    s[2] += wgt * dz;
   }
-  gx = pair_sum(gx);
-  gy = pair_sum(gy);
-  gz = pair_sum(gz);
-  if (lane == 0) dY[w] = make_float4((float)gx, (float)gy, (float)gz, 0.0f);
+  if (row_sum<PAIR_LANES>(share, s)) dY[w] = make_float4((float)s[0], (float)s[1], (float)s[2], 0.0f);
 }
 
 // =========================================================== backward ==
@@ -1234,29 +1282,28 @@ __global__ void k_transpose_w(const bf16* __restrict__ w, ParamLayout L, bf16* _
 }
 
 // ============================================================ hand-off ==
-// Per node (eight lanes): Y.xyz, sum over row entries j > i of |Y_i - Y_j|^2, deg, deg^2.
-__global__ void __launch_bounds__(256) k_scale_vals(GView v, const float4* __restrict__ Y, double* __restrict__ vals) {
-  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, lane = threadIdx.x & 7;
-  if (w >= v.nb) return;
+// Per node: Y.xyz, sum over row entries j > i of |Y_i - Y_j|^2, deg, deg^2.
+__global__ void __launch_bounds__(256) k_scale_vals(GView v, const uint32_t* __restrict__ hubs, uint32_t nh,
+                                                    const float4* __restrict__ Y, double* __restrict__ vals) {
+  RowShare share;
+  if (!row_share<SCALE_LANES>(v, hubs, nh, share)) return;
+  const uint32_t w = share.w;
   const uint32_t i = v.n0 + w, d = v.deg[i], rowb = v.off[i];
   const float4 yi = Y[w];
-  double a = 0.0;
-  for (uint32_t q = lane; q < d; q += 8) {
+  double s[1] = {};
+  for (uint32_t q = share.lane; q < d; q += share.lanes) {
     const uint32_t j = v.nbr[rowb + q];
     if (j <= i) continue;
     const float4 yj = Y[j - v.n0];
     const double dx = (double)yi.x - yj.x, dy = (double)yi.y - yj.y, dz = (double)yi.z - yj.z;
-    a += dx * dx + dy * dy + dz * dz;
+    s[0] += dx * dx + dy * dy + dz * dz;
   }
-  const uint32_t mask = 0xFFu << (threadIdx.x & 24u);
-#pragma unroll
-  for (int o = 4; o; o >>= 1) a += __shfl_xor_sync(mask, a, o);
-  if (lane == 0) {
+  if (row_sum<SCALE_LANES>(share, s)) {
     double* o = vals + (size_t)w * 6;
     o[0] = yi.x;
     o[1] = yi.y;
     o[2] = yi.z;
-    o[3] = a;
+    o[3] = s[0];
     o[4] = (double)d;
     o[5] = (double)d * (double)d;
   }
@@ -2204,11 +2251,11 @@ class Net {
     const uint32_t* hubs = s.hubs.p + b.h0;
     forward(s, b, X);
     PairCtx pc{v, T_.p, Y_.p, hp_.partners, seed_, pair_step};
-    k_loss_stats<<<cdiv((uint64_t)nb * PAIR_LANES, 256), 256, 0, st_>>>(pc, red_.vals.p);
+    k_loss_stats<<<row_blocks<PAIR_LANES>(v, nh), 256, 0, st_>>>(pc, hubs, nh, red_.vals.p);
     red_.run<3>(s, b, red_.gsum.p, st_);
     k_loss_finish<<<1, 256, 0, st_>>>(red_.gsum.p, ng, galpha_.p, gcoef_.p, loss_slot);
     if (!backward) return;
-    k_loss_grad<<<cdiv((uint64_t)nb * PAIR_LANES, 256), 256, 0, st_>>>(pc, galpha_.p, gcoef_.p, dY_.p);
+    k_loss_grad<<<row_blocks<PAIR_LANES>(v, nh), 256, 0, st_>>>(pc, hubs, nh, galpha_.p, gcoef_.p, dY_.p);
     // head
     k_head_bwd<<<cdiv(nb, 256), 256, 0, st_>>>(nb, H3_.p, theta_bf_.p + L_.wh, dY_.p, dZ_.p);
     const uint32_t chunks = cdiv(nb, kChunk);
@@ -2274,7 +2321,8 @@ class Net {
   void hand_off(const DevSet& s, const Batch& b) {
     const GView v = s.view(b);
     const uint32_t nb = b.nb, ng = b.g1 - b.g0;
-    k_scale_vals<<<cdiv((uint64_t)nb * 8, 256), 256, 0, st_>>>(v, Y_.p, red_.vals.p);
+    const uint32_t nh = b.h1 - b.h0;
+    k_scale_vals<<<row_blocks<SCALE_LANES>(v, nh), 256, 0, st_>>>(v, s.hubs.p + b.h0, nh, Y_.p, red_.vals.p);
     red_.run<6>(s, b, red_.gsum.p, st_);
     k_scale_grav<<<cdiv(nb, 256), 256, 0, st_>>>(v, Y_.p, red_.gsum.p, red_.vals.p);
     red_.run<1>(s, b, red_.gsum2.p, st_);

@@ -170,3 +170,24 @@ def test_walk_past_the_bitmaps_bit_exact(jc, orc, n):
         r = o.get()
         assert np.array_equal(bits(e.forces()[0]), bits(r["force"]))
         assert e.walk_counts() == (r["n_inter"], r["n_open"])
+
+
+def _star(jc, leaves):
+    return jc.csr_from_pairs(leaves + 1, np.stack([np.zeros(leaves, np.uint32), np.arange(1, leaves + 1, dtype=np.uint32)], 1).reshape(-1))
+
+
+# The passes over a node's pairs and over its row give a hub's row a block: a fixed few
+# lanes took 12 times a path's hand-off, and most of the gradient
+def test_hub_rows_do_not_outlast_the_passes(jc):
+    n = 60001
+    t = []
+    for g in (_star(jc, n - 1), jc.gen_path(n)):
+        net = jc.Mpnn(2, 7)
+        net.set_params({"smooth_steps": 1, "cheb_steps": 0})
+        pos = jc.seed_uniform(n, 2, 1)
+        hand_off = min((net.predict([g]), net.predict_stages()[2])[1] for _ in range(5))
+        net.bind([g], [pos * np.float32(100)])
+        net.grad(0, 1)
+        t.append((hand_off, _best(lambda: net.grad(0, 1))))
+    assert t[0][0] < 4 * t[1][0]
+    assert t[0][1] < 14 * t[1][1]  # (18 before; most of the rest is the hub aggregation)
