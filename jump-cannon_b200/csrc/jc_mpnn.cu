@@ -540,8 +540,8 @@ __global__ void k_proj_write(GView v, const float* __restrict__ P, bf16* __restr
 
 // ========================================================= reductions ==
 // Item = (graph, first node, end node): one warp sums V per-node doubles
-// (rows local to n0) over the item's nodes; then one thread per graph and
-// value adds its items in order. Fixed order throughout.
+// (rows local to n0) over the item's nodes; then a block per graph adds its
+// items. Fixed shape throughout.
 template <int V>
 __global__ void __launch_bounds__(256) k_item_reduce(const double* __restrict__ vals, uint32_t n0,
                                                      const int4* __restrict__ items, uint32_t n_items,
@@ -565,17 +565,32 @@ __global__ void __launch_bounds__(256) k_item_reduce(const double* __restrict__ 
   }
 }
 
+// One block per graph: thread t adds items t, t + 256, ..., then warps and block.
+// (One thread per graph and value went through a large graph's items one after
+// another: R-MAT of 262,144 nodes, 1,024 items, 67 us for six values, now 5.)
 template <int V>
-__global__ void k_graph_sum(const double* __restrict__ part, const uint32_t* __restrict__ item_off, uint32_t g0,
-                            uint32_t ng, uint32_t i0, double* __restrict__ gsum) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t g = t / V, c = t % V;
-  if (g >= ng) return;
+__global__ void __launch_bounds__(256) k_graph_sum(const double* __restrict__ part,
+                                                   const uint32_t* __restrict__ item_off, uint32_t g0, uint32_t i0,
+                                                   double* __restrict__ gsum) {
+  __shared__ double sm[8][V];
+  const uint32_t g = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t a = item_off[g0 + g] - i0, b = item_off[g0 + g + 1] - i0;
-  double s = 0.0;
-#pragma unroll 8
-  for (uint32_t it = a; it < b; ++it) s += part[(size_t)it * V + c];
-  gsum[(size_t)g * V + c] = s;
+  double s[V] = {};
+#pragma unroll 2
+  for (uint32_t it = a + threadIdx.x; it < b; it += 256)
+#pragma unroll
+    for (int c = 0; c < V; ++c) s[c] += part[(size_t)it * V + c];
+#pragma unroll
+  for (int c = 0; c < V; ++c) {
+    s[c] = warp_sum(s[c]);
+    if (lane == 0) sm[w][c] = s[c];
+  }
+  __syncthreads();
+  if (threadIdx.x >= V) return;
+  double t = sm[0][threadIdx.x];
+#pragma unroll
+  for (int q = 1; q < 8; ++q) t += sm[q][threadIdx.x];
+  gsum[(size_t)g * V + threadIdx.x] = t;
 }
 
 // out[col] = sum over z of part[z][col] in f64, one warp per column: lane l
@@ -1789,7 +1804,7 @@ struct Reduce {
   void run(const DevSet& s, const Batch& b, double* out, cudaStream_t st) {
     const uint32_t ni = b.i1 - b.i0, ng = b.g1 - b.g0;
     if (ni) k_item_reduce<V><<<warps_grid(ni), 256, 0, st>>>(vals.p, b.n0, s.items.p + b.i0, ni, part.p);
-    if (ng) k_graph_sum<V><<<cdiv((uint64_t)ng * V, 128), 128, 0, st>>>(part.p, s.item_off.p, b.g0, ng, b.i0, out);
+    if (ng) k_graph_sum<V><<<ng, 256, 0, st>>>(part.p, s.item_off.p, b.g0, b.i0, out);
   }
 };
 

@@ -191,3 +191,17 @@ def test_hub_rows_do_not_outlast_the_passes(jc):
         t.append((hand_off, _best(lambda: net.grad(0, 1))))
     assert t[0][0] < 4 * t[1][0]
     assert t[0][1] < 14 * t[1][1]  # (18 before; most of the rest is the hub aggregation)
+
+
+# A large graph's partial sums are added by a block, not by one thread for each value
+# (with items of 256 nodes that chain is 4,096 long here). The evaluator's time over
+# one graph beside the same nodes as 64 graphs: 1.11 times before, 0.99 now.
+def test_one_large_graph_sums_like_many(jc):
+    n = 1 << 20
+    t = []
+    for graphs in ([jc.gen_grid(1024)], [jc.gen_grid(128)] * 64):
+        ev = jc.Evaluator(graphs, 8)
+        x = jc.seed_uniform(n, 2, 1)
+        ev(x)
+        t.append(_best(lambda: ev(x), 15))
+    assert t[0] < 1.06 * t[1]
