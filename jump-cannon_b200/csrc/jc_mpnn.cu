@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(256) k_reduce_splits(const float* __restrict__
 // Bound by the round trips of a node (its row bounds, ids, rows), so a node's
 // lanes read its neighbour ids together and take them from shuffles with 8
 // rows in flight, and 32 D/8 nodes share a warp. Long rows: a warp each in the
-// first blocks, 32 / (D/8) neighbours per load, the next ids in flight. Rows
+// first blocks (agg_long), the next ids in flight. Rows
 // past the count are zeros, added to sums that are never -0. Bound by issue (67
 // % of slots). Five blocks per SM cost a few spills and still win on large
 // sets. 128 columns, before (a warp per node, four rows in flight) and after:
@@ -663,45 +663,96 @@ __device__ __forceinline__ void add_row8(uint4 r, Sum8& a) {
   for (int k = 0; k < 4; ++k) a.add(k, __uint_as_float(q[k] << 16), __uint_as_float(q[k] & 0xFFFF0000u));
 }
 
+// The mean's quotients by one divisor, in range unless a sum is tiny or huge.
+template <int N>
+__device__ __forceinline__ void row_mean(float (&m)[N], uint32_t d) {
+  const float fd = (float)d;
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < N; ++k) ok = ok && (m[k] == 0.0f || (fabsf(m[k]) >= dev::DIV_LO && fabsf(m[k]) <= dev::DIV_HI));
+  if (d == 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) m[k] = 0.0f;
+  } else if (ok) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) m[k] = dev::div_in_range(m[k], fd);
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; ++k) m[k] = __fdiv_rn(m[k], fd);
+  }
+}
+
+// A long row's mean by a warp, ids from a shuffle, f32 sums in CSR order: 128 columns
+// four a lane, 32 columns two a lane and two neighbours a load (the sums take the
+// second one's from a shuffle). Sixteen bytes a lane meant up to eight neighbours a
+// load, all handed round by shuffles and added by every lane. us a pass, a warp a row
+// with four rows in flight / sixteen bytes a lane / this: R-MAT of 262,144 nodes, 128
+// columns 258 / 357 / 261, 32 columns 163 / 182 / 154, backward 403 / 425 / 314; rows of
+// 64 only, 4 M entries, network of a prediction 312 / 566 / 355, whole gradient 1,370 /
+// 1,580 / 1,240. (A launch of its own: the 64 graphs' network 364 -> 576, no overlap with
+// the short rows. Columns one a lane: 32 columns, rows of 64, 80 where this takes 65.)
+template <int D>
+__device__ __forceinline__ void agg_long(const GView& v, uint32_t i, const bf16* src, int src_ld, bf16* dst, int dst_ld) {
+  constexpr int C = D == 128 ? 4 : 2, LPR = D / C, NPL = 32 / LPR;
+  constexpr uint32_t U = 8;
+  const uint32_t lane = threadIdx.x & 31, q = lane / LPR, c = C * (lane % LPR), d = v.deg[i];
+  const uint32_t* row = v.nbr + v.off[i];
+  float m[C] = {};
+  uint32_t nx = lane < d ? row[lane] : i;
+  for (uint32_t base = 0; base < d; base += 32) {
+    const uint32_t id = nx - v.n0, cnt = min(32u, d - base);
+    nx = base + 32 + lane < d ? row[base + 32 + lane] : i;
+    for (uint32_t t = 0; t < cnt; t += U * NPL) {
+      uint2 f[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        const uint32_t e = t + u * NPL + q;
+        const bf16* p = src + (size_t)__shfl_sync(0xffffffffu, id, (int)(e & 31u)) * src_ld + c;
+        if constexpr (C == 4) f[u] = e < cnt ? *reinterpret_cast<const uint2*>(p) : make_uint2(0u, 0u);
+        else f[u].x = e < cnt ? *reinterpret_cast<const uint32_t*>(p) : 0u;
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u)
+#pragma unroll
+        for (int p = 0; p < NPL; ++p) {
+          float x[4];
+          if constexpr (NPL > 1) {
+            const uint32_t r = __shfl_sync(0xffffffffu, f[u].x, (int)(lane % LPR) + p * LPR);
+            x[0] = __uint_as_float(r << 16);
+            x[1] = __uint_as_float(r & 0xFFFF0000u);
+          } else {
+            unpack4(f[u], x);
+          }
+#pragma unroll
+          for (int k = 0; k < C; ++k) m[k] = __fadd_rn(m[k], x[k]);
+        }
+    }
+  }
+  if (q != 0) return;
+  row_mean<C>(m, d);
+  bf16* o = dst + (size_t)(i - v.n0) * dst_ld + D + c;
+  if constexpr (C == 4) {
+    *reinterpret_cast<uint2*>(o) = pack4(m);
+  } else {
+    const float x[4] = {m[0], m[1], 0.0f, 0.0f};
+    *reinterpret_cast<uint32_t*>(o) = pack4(x).x;
+  }
+}
+
 template <int D>
 __global__ void __launch_bounds__(256, 5) k_agg(GView v, const bf16* src, int src_ld, bf16* dst, int dst_ld,
                                              int copy_self, uint32_t lb) {
-  constexpr int LPN = D / 8, NPL = 32 / LPN, U = 8;
+  constexpr int LPN = D / 8, U = 8;
   const uint32_t lane = threadIdx.x & 31, sub = lane % LPN, c = sub * 8;
+  if (blockIdx.x < lb) {
+    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k < v.n_long) agg_long<D>(v, v.longs[k], src, src_ld, dst, dst_ld);
+    return;
+  }
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   Sum8 a;
   uint32_t w, d;
-  if (blockIdx.x < lb) {
-    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (k >= v.n_long) return;
-    const uint32_t i = v.longs[k], q = lane / LPN;
-    d = v.deg[i];
-    w = i - v.n0;
-    const uint32_t* row = v.nbr + v.off[i];
-    uint32_t nx = lane < d ? row[lane] : i;
-    for (uint32_t base = 0; base < d; base += 32) {
-      const uint32_t id = nx - v.n0, cnt = min(32u, d - base);
-      nx = base + 32 + lane < d ? row[base + 32 + lane] : i;
-      for (uint32_t t = 0; t < cnt; t += U * NPL) {
-        uint4 r[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint32_t e = t + u * NPL + q, j = __shfl_sync(0xffffffffu, id, (int)(e & 31u));
-          r[u] = e < cnt ? *reinterpret_cast<const uint4*>(src + (size_t)j * src_ld + c) : zero;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int p = 0; p < NPL; ++p) {
-            if (t + u * NPL >= cnt) break;  // (the warp's: no shuffles for whole loads past the row)
-            const int from = (int)sub + p * LPN;
-            add_row8(make_uint4(__shfl_sync(0xffffffffu, r[u].x, from), __shfl_sync(0xffffffffu, r[u].y, from),
-                                __shfl_sync(0xffffffffu, r[u].z, from), __shfl_sync(0xffffffffu, r[u].w, from)), a);
-          }
-      }
-    }
-    if (q != 0) return;
-  } else {
+  {
     const uint32_t t0 = (blockIdx.x - lb) * blockDim.x + threadIdx.x;
     w = t0 / LPN;
     if (w >= v.nb) return;
@@ -728,23 +779,9 @@ __global__ void __launch_bounds__(256, 5) k_agg(GView v, const bf16* src, int sr
         add_row8(r[u], a);
     }
   }
-  // the mean: quotients by one divisor, in range unless a sum is tiny or huge
   float m[8];
   a.get(m);
-  const float fd = (float)d;
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) ok = ok && (m[k] == 0.0f || (fabsf(m[k]) >= dev::DIV_LO && fabsf(m[k]) <= dev::DIV_HI));
-  if (d == 0) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) m[k] = 0.0f;
-  } else if (ok) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) m[k] = dev::div_in_range(m[k], fd);
-  } else {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) m[k] = __fdiv_rn(m[k], fd);
-  }
+  row_mean<8>(m, d);
   const uint2 lo = pack4(m), hi = pack4(m + 4);
   *reinterpret_cast<uint4*>(dst + (size_t)w * dst_ld + D + c) = make_uint4(lo.x, lo.y, hi.x, hi.y);
 }
@@ -1122,8 +1159,8 @@ __global__ void __launch_bounds__(32 * CHUNK_WARPS) k_colsum(uint32_t nb, uint32
 // the transpose of the mean aggregation (the CSR is symmetric), CSR order.
 // dA is the bf16 output of the activation-gradient GEMM (8 bytes per lane
 // and neighbour gathered).
-// 16 lanes per node, 8 columns each; long rows first, a warp each, two
-// neighbours per load (see k_agg). 158,000 nodes: 141 -> 79 us.
+// 16 lanes per node, 8 columns each; long rows first, a warp each (see
+// agg_long). 158,000 nodes: 141 -> 79 us.
 __device__ __forceinline__ void add_row8_scaled(uint4 r, float s, float* a) {
   float f[8];
   unpack4(make_uint2(r.x, r.y), f);
@@ -1132,46 +1169,57 @@ __device__ __forceinline__ void add_row8_scaled(uint4 r, float s, float* a) {
   for (int k = 0; k < 8; ++k) a[k] = __fadd_rn(a[k], __fmul_rn(f[k], s));
 }
 
+// A long row by a warp, four columns a lane (see agg_long).
+__device__ __forceinline__ void agg_bwd_long(const GView& v, uint32_t i, const bf16* __restrict__ dA,
+                                             const bf16* __restrict__ A, bf16* __restrict__ dZ) {
+  constexpr uint32_t U = 8;
+  const uint32_t lane = threadIdx.x & 31, d = v.deg[i], c = 4 * lane, w = i - v.n0;
+  const uint32_t* row = v.nbr + v.off[i];
+  float a[4] = {};
+  uint32_t nx = lane < d ? row[lane] : i;
+  for (uint32_t base = 0; base < d; base += 32) {
+    const uint32_t jl = nx, cnt = min(32u, d - base);
+    const float il = lane < cnt ? __frcp_rn((float)v.deg[jl]) : 0.0f;
+    nx = base + 32 + lane < d ? row[base + 32 + lane] : i;
+    for (uint32_t t = 0; t < cnt; t += U) {
+      uint2 r[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        const uint32_t j = __shfl_sync(0xffffffffu, jl, (int)(t + u)) - v.n0;
+        r[u] = t + u < cnt ? *reinterpret_cast<const uint2*>(dA + (size_t)j * 2 * HID + HID + c) : make_uint2(0u, 0u);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        const float inv = __shfl_sync(0xffffffffu, il, (int)(t + u));
+        float f[4];
+        unpack4(r[u], f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = __fadd_rn(a[k], __fmul_rn(f[k], inv));
+      }
+    }
+  }
+  float h[4], o[4], sv[4];
+  unpack4(*reinterpret_cast<const uint2*>(dA + (size_t)w * 2 * HID + c), sv);
+  unpack4(*reinterpret_cast<const uint2*>(A + (size_t)w * 2 * HID + c), h);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) o[k] = h[k] > 0.0f ? __fadd_rn(sv[k], a[k]) : 0.0f;
+  *reinterpret_cast<uint2*>(dZ + (size_t)w * HID + c) = pack4(o);
+}
+
 __global__ void __launch_bounds__(256, 4) k_agg_bwd(GView v, const bf16* __restrict__ dA, const bf16* __restrict__ A,
                                                  bf16* __restrict__ dZ, uint32_t lb) {
   constexpr int LPN = HID / 8, U = 8;
   const uint32_t lane = threadIdx.x & 31, sub = lane % LPN, c = sub * 8;
+  if (blockIdx.x < lb) {
+    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (k < v.n_long) agg_bwd_long(v, v.longs[k], dA, A, dZ);
+    return;
+  }
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   float a[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   auto at = [&](uint32_t j) { return *reinterpret_cast<const uint4*>(dA + (size_t)(j - v.n0) * 2 * HID + HID + c); };
   uint32_t w;
-  if (blockIdx.x < lb) {
-    const uint32_t k = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (k >= v.n_long) return;
-    const uint32_t i = v.longs[k], d = v.deg[i], q = lane / LPN;
-    w = i - v.n0;
-    const uint32_t* row = v.nbr + v.off[i];
-    uint32_t nx = lane < d ? row[lane] : i;
-    for (uint32_t base = 0; base < d; base += 32) {
-      const uint32_t cnt = min(32u, d - base), jl = nx;
-      const float il = lane < cnt ? __frcp_rn((float)v.deg[jl]) : 0.0f;
-      nx = base + 32 + lane < d ? row[base + 32 + lane] : i;
-      for (uint32_t t = 0; t < cnt; t += 2 * U) {
-        uint4 r[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const uint32_t e = t + 2 * u + q, j = __shfl_sync(0xffffffffu, jl, (int)(e & 31u));
-          r[u] = e < cnt ? at(j) : zero;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            const int from = (int)sub + p * LPN;
-            const float inv = __shfl_sync(0xffffffffu, il, (int)((t + 2 * u + p) & 31u));
-            const uint4 x = make_uint4(__shfl_sync(0xffffffffu, r[u].x, from), __shfl_sync(0xffffffffu, r[u].y, from),
-                                       __shfl_sync(0xffffffffu, r[u].z, from), __shfl_sync(0xffffffffu, r[u].w, from));
-            if (t + 2 * u + p < cnt) add_row8_scaled(x, inv, a);
-          }
-      }
-    }
-    if (q != 0) return;
-  } else {
+  {
     const uint32_t t0 = (blockIdx.x - lb) * blockDim.x + threadIdx.x;
     w = t0 / LPN;
     if (w >= v.nb) return;
