@@ -1613,19 +1613,20 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
   h.deg.resize(n);
   h.gid.resize(n);
   // Pieces of at most PIECE nodes of one graph, on all host threads: first the
-  // offsets of every piece, then (with every range known to be sound) its ids.
+  // offsets of every piece, then (with every range known to be sound) its ids. No
+  // memory is taken on those threads: an exception there would end the process.
   // The first fault in graph order is the one reported.
   constexpr uint32_t PIECE = 16384;
   struct Piece {
     uint32_t g, v0, v1;
     uint32_t fault = 0;  // 1: first offset, 2: decreasing offsets, 3: id out of range
     uint32_t id = 0;
-    std::vector<uint32_t> hubs, longs;
+    uint32_t hubs = 0, longs = 0;  // how many, then where its first goes
   };
   std::vector<Piece> pieces;
   for (uint32_t g = 0; g < G; ++g)
     for (uint32_t v = 0; v == 0 || v < graph_nodes[g]; v += PIECE)
-      pieces.push_back({g, v, std::min(graph_nodes[g], v + PIECE), 0, 0, {}, {}});
+      pieces.push_back({g, v, std::min(graph_nodes[g], v + PIECE)});
   auto report = [&]() {
     for (const Piece& p : pieces) {
       const std::string name = "graph " + std::to_string(p.g);
@@ -1653,11 +1654,20 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
       h.off[b + v] = (uint32_t)(e0 + o[v]);
       h.deg[b + v] = d;
       h.gid[b + v] = p.g;
-      if (d > HUB_DEG) p.hubs.push_back(b + v);
-      else if (d > LONG_DEG) p.longs.push_back(b + v);
+      if (d > HUB_DEG) ++p.hubs;
+      else if (d > LONG_DEG) ++p.longs;
     }
   }
   report();
+  uint32_t n_hubs = 0, n_longs = 0;
+  for (Piece& p : pieces) {
+    std::swap(p.hubs, n_hubs);
+    std::swap(p.longs, n_longs);
+    n_hubs += p.hubs;
+    n_longs += p.longs;
+  }
+  h.hubs.resize(n_hubs);
+  h.longs.resize(n_longs);
 #pragma omp parallel for schedule(dynamic, 1)
   for (int64_t k = 0; k < (int64_t)pieces.size(); ++k) {
     Piece& p = pieces[k];
@@ -1665,6 +1675,10 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
     const uint64_t e0 = ebase[p.g];
     const uint32_t* o = offsets + b + p.g;
     const uint32_t* nb = neighbors + e0;
+    for (uint32_t v = p.v0, hub = p.hubs, lng = p.longs; v < p.v1; ++v) {
+      if (h.deg[b + v] > HUB_DEG) h.hubs[hub++] = b + v;
+      else if (h.deg[b + v] > LONG_DEG) h.longs[lng++] = b + v;
+    }
     for (uint32_t e = o[p.v0]; e < o[p.v1]; ++e) {
       if (nb[e] >= ng) {
         p.fault = 3;
@@ -1676,10 +1690,6 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
   }
   report();
   h.off[n] = (uint32_t)nnz;
-  for (const Piece& p : pieces) {
-    h.hubs.insert(h.hubs.end(), p.hubs.begin(), p.hubs.end());
-    h.longs.insert(h.longs.end(), p.longs.begin(), p.longs.end());
-  }
   if (undirected) check_undirected(h);
   h.item_off.resize(G + 1);
   for (uint32_t g = 0; g < G; ++g) {
