@@ -1613,9 +1613,10 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
   h.deg.resize(n);
   h.gid.resize(n);
   // Pieces of at most PIECE nodes of one graph, on all host threads: first the
-  // offsets of every piece, then (with every range known to be sound) its ids. No
-  // memory is taken on those threads: an exception there would end the process.
-  // The first fault in graph order is the one reported.
+  // offsets of every piece, then the ids of the graphs before the first fault (their
+  // ranges are known to be sound), so the first fault in graph order is the one
+  // reported. No memory is taken on those threads: an exception there would end the
+  // process.
   constexpr uint32_t PIECE = 16384;
   struct Piece {
     uint32_t g, v0, v1;
@@ -1627,14 +1628,6 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
   for (uint32_t g = 0; g < G; ++g)
     for (uint32_t v = 0; v == 0 || v < graph_nodes[g]; v += PIECE)
       pieces.push_back({g, v, std::min(graph_nodes[g], v + PIECE)});
-  auto report = [&]() {
-    for (const Piece& p : pieces) {
-      const std::string name = "graph " + std::to_string(p.g);
-      if (p.fault == 1) fail(JC_ERR_ARG, name + ": offsets[0] must be 0");
-      if (p.fault == 2) fail(JC_ERR_ARG, name + ": offsets must be non-decreasing");
-      if (p.fault == 3) fail(JC_ERR_ARG, name + ": neighbor id " + std::to_string(p.id) + " out of range");
-    }
-  };
 #pragma omp parallel for schedule(dynamic, 1)
   for (int64_t k = 0; k < (int64_t)pieces.size(); ++k) {
     Piece& p = pieces[k];
@@ -1658,9 +1651,9 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
       else if (d > LONG_DEG) ++p.longs;
     }
   }
-  report();
-  uint32_t n_hubs = 0, n_longs = 0;
+  uint32_t n_hubs = 0, n_longs = 0, sound = G;  // graphs before the first fault
   for (Piece& p : pieces) {
+    if (p.fault) sound = std::min(sound, p.g);
     std::swap(p.hubs, n_hubs);
     std::swap(p.longs, n_longs);
     n_hubs += p.hubs;
@@ -1671,6 +1664,7 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
 #pragma omp parallel for schedule(dynamic, 1)
   for (int64_t k = 0; k < (int64_t)pieces.size(); ++k) {
     Piece& p = pieces[k];
+    if (p.g >= sound) continue;
     const uint32_t b = h.go[p.g], ng = graph_nodes[p.g];
     const uint64_t e0 = ebase[p.g];
     const uint32_t* o = offsets + b + p.g;
@@ -1688,7 +1682,12 @@ HostSet assemble(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offset
       h.nbr[e0 + e] = b + nb[e];
     }
   }
-  report();
+  for (const Piece& p : pieces) {
+    const std::string name = "graph " + std::to_string(p.g);
+    if (p.fault == 1) fail(JC_ERR_ARG, name + ": offsets[0] must be 0");
+    if (p.fault == 2) fail(JC_ERR_ARG, name + ": offsets must be non-decreasing");
+    if (p.fault == 3) fail(JC_ERR_ARG, name + ": neighbor id " + std::to_string(p.id) + " out of range");
+  }
   h.off[n] = (uint32_t)nnz;
   if (undirected) check_undirected(h);
   h.item_off.resize(G + 1);

@@ -218,3 +218,15 @@ def test_long_rows_aggregate_like_short_ones(jc):
         net.predict([g])
         t.append(min((net.predict([g]), net.predict_stages()[1])[1] for _ in range(9)))
     assert t[0] < 0.95 * t[1]
+
+
+# Of two faulty graphs the first one is reported, whatever its fault
+def test_first_faulty_graph_is_reported(jc):
+    g = jc.gen_path(4)
+    bad_id = jc.Csr(4, g.offsets.copy(), np.where(np.arange(len(g.neighbors)) == 2, 9, g.neighbors).astype(np.uint32))
+    falling = jc.Csr(4, np.array([0, 3, 2, 5, 6], np.uint32), g.neighbors.copy())
+    net = jc.Mpnn(2, 7)
+    for graphs, message in (([g, bad_id, falling], "graph 1: neighbor id 9 out of range"),
+                            ([g, falling, bad_id], "graph 1: offsets must be non-decreasing")):
+        with pytest.raises(jc.JcError, match=message):
+            net.predict(graphs)
