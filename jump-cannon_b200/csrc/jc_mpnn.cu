@@ -1710,6 +1710,10 @@ struct DevSet {
   Buf<uint32_t> go, off, nbr, deg, gid, item_off, hubs, longs;
   Buf<int4> items;
   void upload(HostSet&& hs, cudaStream_t s) {
+    enqueue_upload(std::move(hs), s);
+    JC_CUDA_CHECK(cudaStreamSynchronize(s));
+  }
+  void enqueue_upload(HostSet&& hs, cudaStream_t s) {  // (host vectors stay owned by h)
     h = std::move(hs);
     go.upload(h.go.data(), h.go.size(), s);
     off.upload(h.off.data(), h.off.size(), s);
@@ -1720,7 +1724,6 @@ struct DevSet {
     hubs.upload(h.hubs.data(), h.hubs.size(), s);
     longs.upload(h.longs.data(), h.longs.size(), s);
     items.upload(h.items.data(), h.items.size(), s);
-    JC_CUDA_CHECK(cudaStreamSynchronize(s));  // host vectors stay owned by h
   }
   Batch batch(uint32_t g0, uint32_t g1) const {
     Batch b{};
@@ -2097,7 +2100,10 @@ class Net {
   void predict(uint32_t G, const uint32_t* graph_nodes, const uint32_t* offsets, const uint32_t* neighbors,
                float* out_xyz, float* ms) {
     HostSet hs = assemble(G, graph_nodes, offsets, neighbors, false);  // undirected: predict_device
-    if (hs.n && !out_xyz) fail(JC_ERR_ARG, "out_xyz must be non-null");
+    if (hs.n && !out_xyz) {
+      check_undirected(hs);
+      fail(JC_ERR_ARG, "out_xyz must be non-null");
+    }
     predict_device(std::move(hs), ms);
     if (pred_.h.n) {
       JC_CUDA_CHECK(cudaMemcpyAsync(out_xyz, out_.p, (size_t)pred_.h.n * 12, cudaMemcpyDeviceToHost, st_));
@@ -2107,24 +2113,28 @@ class Net {
 
   // Features, forward and hand-off of a graph set into out_ (3 floats per
   // node, device); returns with the stream drained. Fails on graphs that are
-  // not undirected: the device checks beside the prediction (which reads
-  // nothing out of range whatever the entries are), the verdict is read at the
-  // end.
+  // not undirected before it predicts anything: the device checks behind the
+  // upload, whose one wait brings the verdict.
   void predict_device(HostSet&& hs, float* ms) {
-    pred_.upload(std::move(hs), st_);
+    pred_.enqueue_upload(std::move(hs), st_);
     const uint32_t n = pred_.h.n, G = pred_.h.G;
     const Batch b = pred_.batch(0, G);
-    ensure_work(b, false);
-    red_.ensure(n, (uint32_t)pred_.h.items.size(), G);
-    out_.alloc((size_t)n * 3);
-    gscale_.alloc(G);
     directed_.alloc(1);
     directed_.zero(st_);
     if (n) {
       const uint32_t nh = (uint32_t)pred_.h.hubs.size();
       k_undirected<<<nh + cdiv((uint64_t)n * 8, 256), 256, 0, st_>>>(pred_.view(b), pred_.hubs.p, nh, directed_.p);
+      JC_CUDA_CHECK(cudaGetLastError());
     }
     uint32_t directed = 0;
+    JC_CUDA_CHECK(cudaMemcpyAsync(&directed, directed_.p, 4, cudaMemcpyDeviceToHost, st_));
+    JC_CUDA_CHECK(cudaStreamSynchronize(st_));
+    if (directed & 2u) check_undirected(pred_.h);
+    else if (directed) fail_directed();
+    ensure_work(b, false);
+    red_.ensure(n, (uint32_t)pred_.h.items.size(), G);
+    out_.alloc((size_t)n * 3);
+    gscale_.alloc(G);
     JC_CUDA_CHECK(cudaEventRecord(ev0_, st_));
     compute_features(pred_, seed_, hp_.smooth_steps, hp_.cheb_steps, hp_.cheb_b, PX_, P_, P2_, P3_, red_, red2_,
                      st_);
@@ -2133,10 +2143,7 @@ class Net {
     JC_CUDA_CHECK(cudaEventRecord(evn_, st_));
     if (n) hand_off(pred_, b);
     JC_CUDA_CHECK(cudaEventRecord(ev1_, st_));
-    JC_CUDA_CHECK(cudaMemcpyAsync(&directed, directed_.p, 4, cudaMemcpyDeviceToHost, st_));
     JC_CUDA_CHECK(cudaStreamSynchronize(st_));
-    if (directed & 2u) check_undirected(pred_.h);
-    else if (directed) fail_directed();
     check_err();
     float t = 0.0f;
     JC_CUDA_CHECK(cudaEventElapsedTime(&t, ev0_, ev1_));
@@ -2573,8 +2580,10 @@ inline void warm_start(Net& net, Evaluator& ev, uint32_t G, const uint32_t* grap
                        const uint32_t* neighbors, const float* seed_xyz, float* out_xyz, uint8_t* kept,
                        float* device_ms) {
   HostSet hs = assemble(G, graph_nodes, offsets, neighbors, false);  // undirected: predict_device
-  if (!ev.same_graphs(hs)) fail(JC_ERR_ARG, "the evaluator was built for other graphs");
+  const bool same = ev.same_graphs(hs);
   const uint32_t n = hs.n;
+  if (!same || (n && (!seed_xyz || !out_xyz))) check_undirected(hs);  // (that fault first)
+  if (!same) fail(JC_ERR_ARG, "the evaluator was built for other graphs");
   if (n && (!seed_xyz || !out_xyz)) fail(JC_ERR_ARG, "seed_xyz and out_xyz must be non-null");
   const std::vector<uint32_t> go = hs.go;
   float pred_ms = 0.0f;

@@ -230,3 +230,25 @@ def test_first_faulty_graph_is_reported(jc):
                             ([g, falling, bad_id], "graph 1: offsets must be non-decreasing")):
         with pytest.raises(jc.JcError, match=message):
             net.predict(graphs)
+
+
+# A directed graph is refused before anything is predicted from it, and ahead of an
+# evaluator's mismatch
+def test_directed_graph_is_refused_first(jc):
+    g = jc.gen_path(20000)
+    one_sided = jc.Csr(g.n_nodes, np.minimum(g.offsets, len(g.neighbors) - 1).astype(np.uint32), g.neighbors[:-1].copy())
+    net = jc.Mpnn(2, 7)
+    net.set_params({"smooth_steps": 4000, "cheb_steps": 0})
+    net.predict([g])
+    accepted = _best(lambda: net.predict([g]), 3)
+
+    def refused():
+        with pytest.raises(jc.JcError, match="undirected"):
+            net.predict([one_sided])
+
+    refused()
+    assert _best(refused, 3) < 0.3 * accepted
+    with pytest.raises(jc.JcError, match="undirected"):
+        net.warm_start([one_sided], [jc.seed_uniform(g.n_nodes, 2, 1)], jc.Evaluator([jc.gen_path(5)]))
+    a = net.predict([g])[0][0]
+    assert np.all(np.isfinite(a))
