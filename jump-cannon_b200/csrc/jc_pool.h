@@ -113,4 +113,13 @@ class DevicePool {
   std::vector<Block> free_, used_;
 };
 
+// A block of the pool for one scope.
+struct PoolBlock {
+  uint8_t* const p;
+  explicit PoolBlock(size_t bytes) : p(static_cast<uint8_t*>(DevicePool::instance().alloc(bytes))) {}
+  ~PoolBlock() { DevicePool::instance().free(p); }
+  PoolBlock(const PoolBlock&) = delete;
+  PoolBlock& operator=(const PoolBlock&) = delete;
+};
+
 }  // namespace jc
