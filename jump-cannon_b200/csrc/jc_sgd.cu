@@ -713,7 +713,9 @@ class SgdEngine : public Engine {
     JC_CUDA_CHECK(cudaMemcpyAsync(eta_.p, eta.data(), sizeof(float) * n_eta_, cudaMemcpyHostToDevice, stream_));
     JC_CUDA_CHECK(cudaMemsetAsync(ctr_.p, 0, sizeof(uint32_t), stream_));
     JC_CUDA_CHECK(cudaStreamSynchronize(stream_));
-    if (!wide_) dist32_.free();  // the sweeps read the 16-bit copy
+    // (the sweeps read one of them)
+    if (wide_) dist16_.free();
+    else dist32_.free();
     initialized_ = true;
   }
 
