@@ -3226,11 +3226,15 @@ class Fa2Engine : public Engine {
     forest_.zflat = zflat_.p;
   }
 
-  void alloc_tree(uint32_t n) {
+  void alloc_tree(uint32_t n, uint32_t nodes = 0) {
     // Exact tree: <= n leaves + internal nodes; 3n + 64 covers every layout
     // short of deep coincident clusters, which report JC_ERR_CAPACITY and
-    // grow the buffers before the step is retried.
-    tree_cap_ = std::max<uint32_t>(tree_cap_, 3 * n + 64);
+    // grow the buffers (to `nodes`) before the step is retried. What an earlier
+    // graph of this engine left larger is used, but its child lists (32 bytes a
+    // node) are not made as large as its other arrays.
+    const uint32_t least = std::max<uint32_t>(nodes, 3 * n + 64);
+    const bool lists = n <= KIDS_MAX_N && graph_off_host_.size() <= 2;
+    tree_cap_ = (uint32_t)std::max<size_t>(least, lists ? std::min(nodes_.n, kids_.n / 8) : nodes_.n);
     key_.alloc(n);
     if (graph_off_host_.size() > 2) {  // batches: sorted words, and the CTA-per-graph schedule's low words
       hi_.alloc(n); hi_alt_.alloc(n); lo_.alloc(n);
@@ -3243,7 +3247,7 @@ class Fa2Engine : public Engine {
     if (graph_off_host_.size() > 2) count_.alloc((size_t)n + 1);
     first_.alloc((size_t)n + 2);
     nodes_.alloc(tree_cap_); parent_.alloc(tree_cap_); nchild_.alloc(tree_cap_);
-    if (n <= KIDS_MAX_N && graph_off_host_.size() <= 2) kids_.alloc(8 * (size_t)tree_cap_);
+    if (lists) kids_.alloc(8 * (size_t)tree_cap_);
     top_list_.alloc(TOP_MAX); top_.alloc(2 * TOP_MAX);
     arrive_.alloc(tree_cap_);
     const uint32_t nl = lcp_index_bytes(n), n2p = lcp_m2_bytes(nl);
@@ -3681,9 +3685,9 @@ class Fa2Engine : public Engine {
   void grow_tree() {
     uint32_t need = 0;
     JC_CUDA_CHECK(cudaMemcpy(&need, first_.p + n_, sizeof(uint32_t), cudaMemcpyDeviceToHost));
-    tree_cap_ = std::max<uint32_t>(need + need / 4 + 64, tree_cap_ * 2);
+    const uint32_t nodes = std::max<uint32_t>(need + need / 4 + 64, tree_cap_ * 2);
     nodes_.free(); parent_.free(); nchild_.free(); arrive_.free(); kids_.free();
-    alloc_tree(n_);
+    alloc_tree(n_, nodes);
     warn_accum_ |= hst_->warn;
     uint32_t zero = 0;
     JC_CUDA_CHECK(cudaMemcpy(&state_.p->error, &zero, sizeof(uint32_t), cudaMemcpyHostToDevice));

@@ -290,7 +290,7 @@ print(marks[2] - marks[1])
 # kept: 126 and 36 before; `wide`: distances past 16 bits held in both widths), and what
 # an engine of a million nodes takes when it is re-bound to 400 (child lists for its
 # largest tree: 96 before)
-@pytest.mark.parametrize("kind,most", [("bind", 104), ("wide", 28)])
+@pytest.mark.parametrize("kind,most", [("bind", 104), ("wide", 28), ("rebound", 8)])
 def test_engines_hold_no_more_memory(kind, most):
     r = subprocess.run([sys.executable, "-c", _HELD, kind], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
