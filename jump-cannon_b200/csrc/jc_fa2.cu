@@ -3436,15 +3436,21 @@ class Fa2Engine : public Engine {
   // Child lists (k_com_kids, k_walk_warp): a single graph of few bodies.
   bool kid_lists() const { return forest_.n_graphs == 1 && n_ <= KIDS_MAX_N; }
 
-  // A small single graph's step chains its kernels as programmatic dependents
-  // where nothing but kernels stands between them (no phase events). B200, us a
-  // replayed step without and with: 400 nodes 43.0 -> 41.5, 2,000 69.7 -> 71.5, 4,000
-  // 96.3 -> 95.1, 10,000 141.8 -> 139.4, 20,000 164.6 -> 160.5, but 32,768 175.0 ->
-  // 176.5, 65,537 177 -> 225. (The pass of jc_fa2_bh_forces_noalloc, launched one by
-  // one, is chained at all its sizes: 300 nodes 155 -> 137 us, 20,000 292 -> 273.)
-  static constexpr uint32_t CHAIN_MAX_N = 24576;
+  // The step of a single graph of middle size chains its kernels as programmatic
+  // dependents where nothing but kernels stands between them (no phase events). B200,
+  // us a replayed step without and with, Barabasi-Albert in 3D and random geometric in
+  // 2D: 5,000 nodes 102.6 / 103.4 and 111.4 / 108.1, 8,000 116.7 / 113.3 and 122.7 / 119.1,
+  // 12,000 140.9 / 139.3 and 119.5 / 120.9, 22,000 161.5 / 153.2 and 130.8 / 131.4 (ten sizes
+  // together 1,224 / 1,211 and 1,164 / 1,147); 24,500 159.8 / 159.1 and 131.2 / 135.3, 32,768
+  // 175.0 / 176.5, 65,537 177 / 225. One-launch trees leave three kernels behind them: 600
+  // nodes 45.2 / 47.3 and 48.7 / 49.3, 3,072 86.4 / 88.1 and 92.2 / 93.3 (eight sizes 464 /
+  // 472 and 499 / 499), so those are not chained. (The pass of jc_fa2_bh_forces_noalloc,
+  // launched one by one, is chained at all its sizes: 300 nodes 155 -> 137 us, 20,000 292
+  // -> 273.)
+  static constexpr uint32_t CHAIN_MAX_N = 22528;
   bool chained() const {
-    return n_ <= CHAIN_MAX_N && s_.use_graph && !capture_phases_ && forest_.n_graphs == 1 && !stage_top();
+    return n_ > GB_SINGLE_N && n_ <= CHAIN_MAX_N && bh_ && s_.use_graph && !capture_phases_ && forest_.n_graphs == 1 &&
+           !stage_top();
   }
 
   // The staged-top walk: a single graph, walk group 1.
