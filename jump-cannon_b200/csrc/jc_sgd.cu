@@ -63,6 +63,14 @@ __device__ __forceinline__ uint64_t smix(uint64_t z) {
   return z ^ (z >> 31);
 }
 
+// Threads a block of the sweep and of the search's levels: small enough that the
+// nodes of a small graph spread over the SMs, large enough that an SM's blocks share
+// the schedulers evenly. B200, us a step with 100 pivots at 64 / 128 / 256: 5,000
+// nodes 14.4 / 12.3 / 14.4, 30,000 16.4 / 16.3 / 14.4, 50,000 18.5 / 18.5 / 20.5, 70,000 22.5
+// / 20.5 / 20.5, 90,000 24.6 / 24.6 / 26.6, 140,000 32.8 / 32.8 / 32.7, 200,000 44.2 / 43.0 /
+// 43.6, 250,000 53.3 / 51.7 / 51.2. Binds differ by 2 % at most.
+constexpr uint32_t NODE_THREADS = 128;
+
 // Node i's term with the pivot at q, hop distance d and mu = min(1, eta / d^2):
 // the general operations (any f32 input).
 __device__ __forceinline__ void jacobi_term(float& px, float& py, float& pz, const float4 q, float d, float mu) {
@@ -147,7 +155,7 @@ __device__ __forceinline__ bool jacobi_stage(float4* piv, float2* mu_tab, const 
 // 30,011 with 100 pivots 29 -> 14. Two nodes per thread in packed f32
 // operations gave 95 (grid) but for the moves it needs, and was not kept.
 template <typename D>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(NODE_THREADS)
 k_jacobi(const float4* __restrict__ pin, float4* __restrict__ pout, const uint32_t* __restrict__ pivots,
          const D* __restrict__ dist, uint32_t n, uint32_t k, const float* __restrict__ eta_table, uint32_t n_eta,
          const uint32_t* __restrict__ sweep_ctr, uint32_t mu_len) {
@@ -203,9 +211,6 @@ k_jacobi(const float4* __restrict__ pin, float4* __restrict__ pout, const uint32
   }
   pout[i] = make_float4(px, py, pz, 0.0f);
 }
-
-// Up to here 64-thread blocks, so that the nodes spread over every SM.
-constexpr uint32_t JACOBI_SMALL_N = 148u * 512u;
 
 // A sweep's n samples, drawn in one pass: sample q = sweep * n + t is (node i,
 // pivot j, hop distance as f32 bits; 0 for a skipped pair: the node itself, or
@@ -346,8 +351,8 @@ __global__ void k_pack(const float4* __restrict__ v, uint32_t n, float* __restri
 //
 // A level is a few dependent round trips per node (row bounds, ids, frontier
 // words), so four neighbours' words are in flight, a node that every pivot has
-// reached gathers nothing, a gather ends once it holds every bit still wanted,
-// and blocks are small where nodes are few. Distances go straight into their
+// reached gathers nothing, and a gather ends once it holds every bit still wanted.
+// Distances go straight into their
 // 16-bit rows (u32 from level 65,535 on). Levels are launched MS_CHUNK at a
 // time without waiting; one after the last growing level returns at once.
 // B200, random geometric graphs, us a level: 30,011 nodes with 100 pivots 16 -> 7,
@@ -400,7 +405,7 @@ __device__ __forceinline__ void store_words(word_t* p, const Words<WB>& r) {
 
 // *last: the highest level at which some node grew (0: the seeds).
 template <typename D, int WB>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(NODE_THREADS)
 k_msbfs_level(uint32_t n, uint32_t k, uint32_t stride, const uint32_t* __restrict__ off,
               const uint32_t* __restrict__ nbr, const word_t* __restrict__ front, word_t* __restrict__ next,
               word_t* __restrict__ visited, D* __restrict__ dist, uint32_t level, uint32_t* last) {
@@ -629,16 +634,15 @@ class SgdEngine : public Engine {
     JC_CUDA_CHECK(cudaMemsetAsync(dist16_.p, 0xFF, sizeof(uint16_t) * cells, stream_));
     JC_CUDA_CHECK(cudaMemsetAsync(last, 0, 4, stream_));
     k_msbfs_seed<uint16_t><<<cdiv(k_, 256), 256, 0, stream_>>>(n, k_, W, piv_.p, vis, fa, dist16_.p);
-    const uint32_t threads = n <= JACOBI_SMALL_N ? 64u : 256u;
     auto launch = [&](auto* dist, uint32_t level) {
       using D = std::remove_pointer_t<decltype(dist)>;
-      const uint32_t blocks = cdiv(n, threads);
+      const uint32_t blocks = cdiv(n, NODE_THREADS);
       if (W == 1)
-        k_msbfs_level<D, 1><<<blocks, threads, 0, stream_>>>(n, k_, W, goff, gnbr, fa, fb, vis, dist, level, last);
+        k_msbfs_level<D, 1><<<blocks, NODE_THREADS, 0, stream_>>>(n, k_, W, goff, gnbr, fa, fb, vis, dist, level, last);
       else if (W == 2)
-        k_msbfs_level<D, 2><<<blocks, threads, 0, stream_>>>(n, k_, W, goff, gnbr, fa, fb, vis, dist, level, last);
+        k_msbfs_level<D, 2><<<blocks, NODE_THREADS, 0, stream_>>>(n, k_, W, goff, gnbr, fa, fb, vis, dist, level, last);
       else
-        k_msbfs_level<D, 4><<<blocks, threads, 0, stream_>>>(n, k_, W, goff, gnbr, fa, fb, vis, dist, level, last);
+        k_msbfs_level<D, 4><<<blocks, NODE_THREADS, 0, stream_>>>(n, k_, W, goff, gnbr, fa, fb, vis, dist, level, last);
       std::swap(fa, fb);
     };
     bool wide = false;
@@ -967,10 +971,9 @@ class SgdEngine : public Engine {
                                            200 * 1024 + (int)(sizeof(float) * JACOBI_MU_MAX)));
       float4* in = pos_a_.p;
       float4* out = pos_b_.p;
-      const uint32_t threads = n <= JACOBI_SMALL_N ? 64u : 256u;
       for (uint32_t s = 0; s < sweeps; ++s) {
-        k_jacobi<D><<<cdiv(n, threads), threads, smem, stream_>>>(in, out, piv_.p, dist, n, k, eta_.p, n_eta_, ctr_.p,
-                                                                  mu_len);
+        k_jacobi<D><<<cdiv(n, NODE_THREADS), NODE_THREADS, smem, stream_>>>(in, out, piv_.p, dist, n, k, eta_.p, n_eta_,
+                                                                            ctr_.p, mu_len);
         std::swap(in, out);
         ++L;
       }
