@@ -1194,8 +1194,9 @@ k_walk(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order, cons
   dev::dependent_launch_wait();
   const int lane = threadIdx.x & 31;
   const uint32_t a = blockIdx.x * WALK_THREADS + threadIdx.x;
-  const uint32_t body0 = a < n ? order[a] : 0u;
-  const bool have = a < n && JC_IN_BOUNDS(body0, n, &st->error);
+  const bool failed = st->error != 0u;  // (a sort that gave up leaves no permutation to follow)
+  const uint32_t body0 = a < n && !failed ? order[a] : 0u;
+  const bool have = a < n && !failed && JC_IN_BOUNDS(body0, n, &st->error);
   const uint32_t body = have ? body0 : 0u;
   // In a batch a walk group shares a node stream only among lanes of the
   // same graph (each graph has its own root).
@@ -1361,9 +1362,10 @@ k_walk_ahead(const TNode* nodes, const uint32_t* order, const float4* __restrict
              const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* frep, Forest F) {
   dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t T = st->error ? 0u : st->n_tree;
+  const bool failed = st->error != 0u;  // (no permutation to follow: see k_walk)
+  const uint32_t T = st->n_tree;
   uint32_t n_inter = 0, n_open = 0;
-  if (a < n) {
+  if (a < n && !failed) {
     const uint32_t body = order[a];
     if (!JC_IN_BOUNDS(body, n, &st->error)) return;
     const uint32_t root = T == 0u ? END : F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
@@ -1383,15 +1385,16 @@ k_walk_rope(const TNode* __restrict__ nodes, const uint32_t* __restrict__ order,
             const float* __restrict__ degf, uint32_t n, KParams P, DevState* st, float4* __restrict__ frep, Forest F) {
   dev::dependent_launch_wait();
   const uint32_t a = blockIdx.x * WALK_THREADS + threadIdx.x;
-  const uint32_t T = st->error ? 0u : st->n_tree;
+  const bool failed = st->error != 0u;  // (no permutation to follow: see k_walk)
+  const uint32_t T = st->n_tree;
   uint32_t n_inter = 0, n_open = 0;
-  if (a < n && T > 0u) {
+  if (a < n && T > 0u && !failed) {
     const uint32_t body = order[a];
     if (!JC_IN_BOUNDS(body, n, &st->error)) return;
     const uint32_t root = F.n_graphs > 1 ? F.tree_root[F.node_graph[body]] : 0u;
     walk_one<FAST, false>(nodes, body, pos[body], __fmul_rn(P.scaling_ratio, degf[body]), root, T, P.theta2, st, frep,
                    n_inter, n_open);
-  } else if (a < n) {
+  } else if (a < n && !failed) {
     const uint32_t body = order[a];
     if (JC_IN_BOUNDS(body, n, &st->error)) frep[body] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -1441,7 +1444,8 @@ k_walk_warp(const TNode* nodes, const uint32_t* kids, const uint32_t* order, con
   uint16_t* list = reinterpret_cast<uint16_t*>(base + ((10 * (size_t)words + 15) / 16) * 16);
   uint16_t* queue = list + WW_LIST;                       // two of WW_QUEUE
   float* terms = reinterpret_cast<float*>(queue);         // [3][WW_ROW], after the traversal
-  const uint32_t T = st->error ? 0u : st->n_tree;
+  if (__shfl_sync(0xFFFFFFFFu, st->error, 0)) return;  // (no permutation to follow: see k_walk)
+  const uint32_t T = st->n_tree;
   if (T > 64u * words && n > WW_LANES_N) {  // (the whole grid)
     const uint32_t a = blockIdx.x * (32 * WW_WARPS) + threadIdx.x;
     if (blockIdx.x * (32 * WW_WARPS) >= n) return;
@@ -1650,13 +1654,14 @@ k_walk_top(const TNode* __restrict__ nodes, const uint4* __restrict__ top, const
            float4* __restrict__ frep) {
   dev::dependent_launch_wait();
   __shared__ uint4 tsm[2 * TOP_MAX];
-  const uint32_t T = st->error ? 0u : st->n_tree;
+  const bool failed = st->error != 0u;  // (no permutation to follow: see k_walk)
+  const uint32_t T = st->n_tree;
   const uint32_t nt = min(st->n_top, TOP_MAX);
   for (uint32_t k = threadIdx.x; k < 2 * nt; k += WALK_THREADS) tsm[k] = __ldcg(top + k);
   __syncthreads();
   const uint32_t a = blockIdx.x * WALK_THREADS + threadIdx.x;
   uint32_t n_inter = 0, n_open = 0;
-  if (a < n) {
+  if (a < n && !failed) {
     const uint32_t body = order[a];
     if (!JC_IN_BOUNDS(body, n, &st->error)) return;
     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
@@ -1819,7 +1824,7 @@ __global__ void __launch_bounds__(256)
 k_graph_trees(const uint64_t* __restrict__ hi, const uint32_t* __restrict__ first, const DevState* st, Forest F) {
   const uint32_t a = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t N = st->n_valid;
-  if (a >= N) return;
+  if (a >= N || st->error) return;  // (a sort that gave up leaves no keys to trust)
   const uint32_t g = key_graph(hi[a], F.gbits);
   if (a == 0 || key_graph(hi[a - 1], F.gbits) != g) F.tree_root[g] = first[a];
   if (a + 1 == N || key_graph(hi[a + 1], F.gbits) != g) F.tree_end[g] = first[a + 1];

@@ -109,3 +109,18 @@ def test_chained_kernel_reads(kernel):
             if f == "walk_one" and re.search(r"if \(CHAINED\) load_node_c\(.*?;\s*else load_node\(", body):
                 calls.discard("load_node")
             todo += calls
+
+
+# A sort that gave up waiting leaves a permutation (and a batch's sorted keys) that may
+# hold anything: the kernels behind it read neither once the error word is set.
+@pytest.mark.parametrize("kernel,reads", [("k_walk", "order["), ("k_walk_ahead", "order["), ("k_walk_rope", "order["),
+                                          ("k_walk_top", "order["), ("k_walk_warp", "order["), ("k_fill", "val["),
+                                          ("k_graph_trees", "hi[a]")])
+def test_no_permutation_is_followed_after_an_error(kernel, reads):
+    (_, body), = FUNCTIONS[kernel]
+    checked, previous = False, ""
+    for line in body[: body.rindex(reads) + len(reads)].splitlines():
+        checked |= bool(re.search(r"if \(.*st->error.*\) return;", line))
+        if reads in line:
+            assert checked or "!failed" in line or "!failed" in previous, line
+        previous = line or previous
