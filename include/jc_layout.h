@@ -439,6 +439,16 @@ jc_status jc_selftest_sort_wait(uint32_t* device_status, float* wait_ms);
  * *wait_ms: the kernel's duration). */
 jc_status jc_selftest_gemm_wait(uint32_t* device_status, float* wait_ms);
 
+/* Self-test of the division and the square root that the force and stress kernels
+ * use where operands stay clear of the ends of the exponent range (no reference
+ * counterpart): bit-for-bit comparisons with the IEEE operations on the device.
+ * mismatches[0..5]: roots of every f32 in [2^-40, 2^60); smaller arguments whose
+ * root leaves the 1e-6 clamp; quotients of every numerator significand by the
+ * all-ones divisor and three beside it; of `pairs` random pairs in [2^-60, 2^60);
+ * of `pairs` pairs in the stress sweep's ranges; of numerators at and beside the
+ * halfway points between two quotients. All are 0. */
+jc_status jc_selftest_exact(uint64_t pairs, uint64_t* mismatches);
+
 /* Library build facts: compute capability the kernels were built for. */
 const char* jc_build_info(void);
 

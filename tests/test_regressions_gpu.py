@@ -1,4 +1,5 @@
 """Faults that were found in use, each held by the smallest call that shows it."""
+import ctypes
 import subprocess
 import sys
 import threading
@@ -295,3 +296,11 @@ def test_engines_hold_no_more_memory(kind, most):
     r = subprocess.run([sys.executable, "-c", _HELD, kind], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert float(r.stdout.split()[-1]) < most
+
+
+# The division and the root that stand for the IEEE operations where operands stay
+# clear of the exponent range's ends: the same bits over all that their users pass
+def test_in_range_division_and_root_are_exact(jc):
+    bad = (ctypes.c_uint64 * 6)(*[1] * 6)
+    assert jc.lib().jc_selftest_exact(1 << 28, bad) == jc.JC_OK
+    assert list(bad) == [0] * 6
