@@ -439,6 +439,12 @@ jc_status jc_selftest_sort_wait(uint32_t* device_status, float* wait_ms);
  * *wait_ms: the kernel's duration). */
 jc_status jc_selftest_gemm_wait(uint32_t* device_status, float* wait_ms);
 
+/* The same of the tree's other bounded waits: device_status[0], the radix pass over
+ * 4-byte keys with a tile whose predecessor never publishes; device_status[1], the
+ * full re-sort's grid barrier with a block that never comes (a sixteenth of the
+ * poll limit that the re-sort uses). */
+jc_status jc_selftest_tree_waits(uint32_t* device_status, float* wait_ms);
+
 /* Self-test of the division and the square root that the force and stress kernels
  * use where operands stay clear of the ends of the exponent range (no reference
  * counterpart): bit-for-bit comparisons with the IEEE operations on the device.

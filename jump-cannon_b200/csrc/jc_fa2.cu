@@ -544,7 +544,7 @@ k_seg_fix(K* sorted, uint32_t* val, const ulonglong2* key, uint32_t n, DevState*
 constexpr int TIE_THREADS = 1024;
 constexpr uint32_t TIE_PART = 2048;           // bodies per block, up to one block per SM
 constexpr uint32_t TIE_SPIN_LIMIT = 1u << 22;  // seconds of polling
-__device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target) {
+__device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target, uint32_t limit = TIE_SPIN_LIMIT) {
   __shared__ bool ok;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -554,7 +554,7 @@ __device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target) {
     uint32_t spins = 0, seen;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&st->tie_bar) : "memory");
-      if (seen < target && ++spins > TIE_SPIN_LIMIT) {
+      if (seen < target && ++spins > limit) {
         set_error(st, JC_ERR_DEVICE_TIMEOUT);
         ok = false;
         break;
@@ -563,6 +563,11 @@ __device__ __forceinline__ bool tie_barrier(DevState* st, uint32_t target) {
   }
   __syncthreads();
   return ok;
+}
+
+// One block at a barrier for two: it gives up after `limit` polls (jc_selftest_tree_waits).
+__global__ void __launch_bounds__(TIE_THREADS) k_selftest_barrier(DevState* st, uint32_t limit, uint32_t* passed) {
+  if (tie_barrier(st, 2u, limit) && threadIdx.x == 0) *passed = 1u;
 }
 
 __global__ void __launch_bounds__(TIE_THREADS)
@@ -4029,6 +4034,64 @@ extern "C" jc_status jc_selftest_sort_wait(uint32_t* device_status, float* wait_
   if (e1) cudaEventDestroy(e1);
   for (void* p : {(void*)keys, (void*)keys_out, (void*)vals, (void*)vals_out, (void*)work, (void*)err})
     if (p) cudaFree(p);
+  if (s) cudaStreamDestroy(s);
+  return rc;
+}
+
+// The 4-byte key pass with a tile that waits for one that never publishes, and the
+// re-sort's grid barrier with a block that never comes.
+extern "C" jc_status jc_selftest_tree_waits(uint32_t* device_status, float* wait_ms) {
+  using namespace jc;
+  using namespace jc::fa2;
+  if (!device_status) return JC_ERR_ARG;
+  constexpr uint32_t TILE = dev::RS_THREADS * 2, N = 2 * TILE, WORDS = dev::RS_RADIX + 1 + 2 * dev::RS_RADIX;
+  cudaStream_t s = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  jc_status rc = JC_OK;
+  try {
+    // keys and values in and out, the sort's words; the barrier's state and its flag
+    const PoolBlock block(4 * (4 * (size_t)N + WORDS + 1) + sizeof(DevState) + 64);
+    uint32_t *keys = reinterpret_cast<uint32_t*>(block.p), *vals = keys + N, *keys_out = vals + N, *vals_out = keys_out + N,
+             *work = vals_out + N, *passed = work + WORDS;
+    DevState* st = reinterpret_cast<DevState*>(block.p + ((4 * (4 * (size_t)N + WORDS + 1) + 63) & ~(size_t)63));
+    JC_CUDA_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    JC_CUDA_CHECK(cudaEventCreate(&e0));
+    JC_CUDA_CHECK(cudaEventCreate(&e1));
+    std::vector<uint32_t> h(2 * N);
+    SplitMix64 rng(0x5E1F7E57ull);
+    for (uint32_t i = 0; i < N; ++i) {
+      h[i] = (uint32_t)rng.next_u64();
+      h[N + i] = i;
+    }
+    const uint32_t one = 1u;
+    DevState got{};
+    JC_CUDA_CHECK(cudaMemcpyAsync(keys, h.data(), 8 * (size_t)N, cudaMemcpyHostToDevice, s));
+    JC_CUDA_CHECK(cudaMemsetAsync(work, 0, 4 * (WORDS + 1), s));
+    JC_CUDA_CHECK(cudaMemsetAsync(st, 0, sizeof(DevState), s));
+    JC_CUDA_CHECK(cudaEventRecord(e0, s));
+    dev::os_hist<uint32_t><<<2, dev::RS_THREADS, 0, s>>>(keys, N, 0, 1, work);
+    JC_CUDA_CHECK(cudaMemcpyAsync(work + dev::RS_RADIX, &one, 4, cudaMemcpyHostToDevice, s));  // tile 0 is taken
+    dev::os_pass<uint32_t, 2><<<1, dev::RS_THREADS, 0, s>>>(keys, vals, keys_out, vals_out, N, 0, work,
+                                                             work + dev::RS_RADIX + 1, work + dev::RS_RADIX, &st->error);
+    JC_CUDA_CHECK(cudaGetLastError());
+    JC_CUDA_CHECK(cudaMemcpyAsync(&got, st, sizeof got, cudaMemcpyDeviceToHost, s));
+    JC_CUDA_CHECK(cudaStreamSynchronize(s));
+    device_status[0] = got.error;
+    JC_CUDA_CHECK(cudaMemsetAsync(st, 0, sizeof(DevState), s));
+    k_selftest_barrier<<<1, TIE_THREADS, 0, s>>>(st, TIE_SPIN_LIMIT / 16, passed);
+    JC_CUDA_CHECK(cudaGetLastError());
+    JC_CUDA_CHECK(cudaEventRecord(e1, s));
+    uint32_t through = 1;
+    JC_CUDA_CHECK(cudaMemcpyAsync(&got, st, sizeof got, cudaMemcpyDeviceToHost, s));
+    JC_CUDA_CHECK(cudaMemcpyAsync(&through, passed, 4, cudaMemcpyDeviceToHost, s));
+    JC_CUDA_CHECK(cudaStreamSynchronize(s));
+    device_status[1] = through ? 0u : got.error;
+    if (wait_ms) JC_CUDA_CHECK(cudaEventElapsedTime(wait_ms, e0, e1));
+  } catch (const Error& e) {
+    rc = e.code;
+  }
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
   if (s) cudaStreamDestroy(s);
   return rc;
 }

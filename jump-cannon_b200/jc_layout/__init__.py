@@ -112,6 +112,7 @@ _SIGNATURES = {
     "jc_set_device": (ctypes.c_int32, [ctypes.c_int32]),
     "jc_selftest_sort_wait": (ctypes.c_int32, [_u32p, _f32p]),
     "jc_selftest_gemm_wait": (ctypes.c_int32, [_u32p, _f32p]),
+    "jc_selftest_tree_waits": (ctypes.c_int32, [_u32p, _f32p]),
     "jc_selftest_exact": (ctypes.c_int32, [ctypes.c_uint64, _u64p]),
 }
 

@@ -304,3 +304,20 @@ def test_in_range_division_and_root_are_exact(jc):
     bad = (ctypes.c_uint64 * 6)(*[1] * 6)
     assert jc.lib().jc_selftest_exact(1 << 28, bad) == jc.JC_OK
     assert list(bad) == [0] * 6
+
+
+# The tree's other bounded waits run out too: the radix pass over 4-byte keys and the
+# re-sort's grid barrier report it and leave the context usable
+def test_tree_waits_give_up_and_the_context_survives(jc, orc):
+    status, ms = (ctypes.c_uint32 * 2)(0, 0), ctypes.c_float(0.0)
+    assert jc.lib().jc_selftest_tree_waits(status, ctypes.byref(ms)) == jc.JC_OK
+    assert list(status) == [jc.JC_ERR_DEVICE_TIMEOUT] * 2
+    assert 1.0 < ms.value < 5000.0
+    g, x = jc.gen_scale_free(5000, 3, 9), jc.seed_uniform(5000, 3, 9)
+    e = jc.LayoutEngine("fa2-bh")
+    e.set_params({"theta": 0.8, "hub_threshold": 1 << 30})
+    e.init(g, x)
+    e.step()
+    ref = orc.Fa2(g, x, bh=True, theta=0.8)
+    ref.step()
+    assert np.array_equal(bits(e.forces()[0]), bits(ref.get()["force"]))
