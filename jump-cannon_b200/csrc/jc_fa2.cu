@@ -3958,7 +3958,7 @@ extern "C" jc_status jc_fa2_bh_forces_noalloc(uint32_t n_nodes, const uint32_t* 
                      st, frep, F1);
     launch_chained(true, s, cdiv(n, ATT_THREADS), ATT_THREADS, 0, k_att<true>, order, d_offsets, d_neighbors, pos4, frep, old4,
                    degf, P, st, force4, stats, partials, 1u);
-  } catch (const Error&) {
+  } catch (...) {  // (a failed launch, or no memory for its message)
     return JC_ERR_CUDA;
   }
   k_pack_xyz<<<cdiv(n, 256), 256, 0, s>>>(force4, n, d_forces_xyz);
@@ -4089,6 +4089,8 @@ extern "C" jc_status jc_selftest_tree_waits(uint32_t* device_status, float* wait
     if (wait_ms) JC_CUDA_CHECK(cudaEventElapsedTime(wait_ms, e0, e1));
   } catch (const Error& e) {
     rc = e.code;
+  } catch (...) {
+    rc = JC_ERR_ARG;
   }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);

@@ -84,6 +84,8 @@ extern "C" jc_status jc_selftest_exact(uint64_t pairs, uint64_t* mismatches) {
     JC_CUDA_CHECK(cudaMemcpy(mismatches, bad, 6 * sizeof(*bad), cudaMemcpyDeviceToHost));
   } catch (const Error& e) {
     rc = e.code;
+  } catch (...) {
+    rc = JC_ERR_ARG;
   }
   if (bad) cudaFree(bad);
   return rc;

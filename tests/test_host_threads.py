@@ -26,3 +26,11 @@ def test_join_threads_take_no_memory():
     assert len(loops) == 2
     for loop in loops:
         assert not re.search(r"push_back|emplace|insert\(|resize\(|reserve\(|std::string|std::vector|\bnew\b|\bfail\(", loop)
+
+
+def test_no_exception_leaves_the_no_allocation_pass():
+    """Its launches throw on failure; any exception has to become a status."""
+    text = re.sub(r"//[^\n]*", "", (SOURCE.parent / "jc_fa2.cu").read_text())
+    entry = _block(text, text.index('extern "C" jc_status jc_fa2_bh_forces_noalloc('))
+    assert "launch_chained(" in entry
+    assert "catch (...)" in entry
