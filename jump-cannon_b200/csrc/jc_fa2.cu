@@ -3181,18 +3181,22 @@ class Fa2Engine : public Engine {
     forest_.gbits = 0;
     forest_.lh = 21;
     biggest_ = 0;
-    graph_tally_.alloc(1);
-    JC_CUDA_CHECK(cudaMemsetAsync(graph_tally_.p, 0, sizeof(GraphTally), stream_));
-    if (G <= 1) return;
-    std::vector<uint32_t> order(G);
     auto size = [&](uint32_t g) { return graph_off_host_[g + 1] - graph_off_host_[g]; };
-    for (uint32_t g = 0; g < G; ++g) {
-      order[g] = g;
-      biggest_ = std::max(biggest_, size(g));
+    for (uint32_t g = 0; g < G; ++g) biggest_ = std::max(biggest_, size(g));
+    const bool one_launch = G > 1 ? biggest_ <= GB_MAX_N : n <= GB_SINGLE_N;  // (k_graph_build's state)
+    if (one_launch) {
+      graph_tally_.alloc(1);
+      JC_CUDA_CHECK(cudaMemsetAsync(graph_tally_.p, 0, sizeof(GraphTally), stream_));
     }
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return size(a) > size(b); });
-    graph_order_.alloc(G);
-    JC_CUDA_CHECK(cudaMemcpyAsync(graph_order_.p, order.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, stream_));
+    if (G <= 1) return;
+    std::vector<uint32_t> order;
+    if (one_launch) {
+      order.resize(G);
+      for (uint32_t g = 0; g < G; ++g) order[g] = g;
+      std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return size(a) > size(b); });
+      graph_order_.alloc(G);
+      JC_CUDA_CHECK(cudaMemcpyAsync(graph_order_.p, order.data(), sizeof(uint32_t) * G, cudaMemcpyHostToDevice, stream_));
+    }
     uint32_t gb = 1;
     while ((1u << gb) < G) ++gb;
     forest_.gbits = gb;
