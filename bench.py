@@ -37,9 +37,9 @@ METRIC = "FA2 iters/s on 1M-node RMAT"
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12  # derived: SMs x FP32 lanes x FMA x max clock
 # DRAM bytes (read + write) of one k_walk_rope launch on the default R-MAT
 # workload, from an ncu capture (profiles/fa2_rmat20_kernels.md).
-WALK_TRAFFIC_BYTES = 78.798080e6 + 6.949632e6  # dram read + write of one walk launch (ncu capture)
-WALK_L1_FRAC = 0.885  # L1TEX throughput of the same capture (the walk's binding resource)
-ATT_TRAFFIC_BYTES = 236.895488e6 + 13.988352e6  # the same for the attraction pass
+WALK_TRAFFIC_BYTES = 80.805632e6 + 7.374336e6  # dram read + write of one walk launch (ncu capture)
+WALK_L1_FRAC = 0.887  # L1TEX throughput of the same capture (the walk's binding resource)
+ATT_TRAFFIC_BYTES = 235.787264e6 + 13.697792e6  # the same for the attraction pass
 FLOPS_PER_INTERACTION = 20
 FLOPS_PER_OPEN = 8
 
@@ -838,7 +838,7 @@ def main():
                                   "(profiles/fa2_rmat20_kernels.md)" if default_graph else None,
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in pk else "fallback 6650 GB/s",
                 "algorithmic": f"88 B x {n} nodes + 20 B x {n_att} edge entries per launch",
-                "note": "the gathers are L1-throughput bound (83 % in ncu), not HBM bound"}
+                "note": "the gathers are L1-throughput bound (84 % in ncu), not HBM bound"}
     if ph["walk"] < ph["attraction_speed"]:
         roof = roof_hbm
 

@@ -488,7 +488,7 @@ typedef struct jc_fa2_params {
  * NULL when every row is empty). offsets[n_nodes] must not exceed the
  * length of the caller's neighbour array, which cannot be checked here.
  * All scratch memory (keys, sort workspace, octree, partial sums) lives in
- * one static device array sized for n_nodes <= 32768 (about 9 MB, held by
+ * one static device array sized for n_nodes <= 32768 (about 12 MB, held by
  * every GPU that loads the library until the process exits); larger n is
  * JC_ERR_CAPACITY. The octree has room for 3*32768+64 nodes and does not
  * grow (the engine's does): a layout with deep chains of nearly coincident

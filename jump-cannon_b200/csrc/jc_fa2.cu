@@ -91,7 +91,7 @@ constexpr int BBOX_BLOCKS = 296;  // 2 x 148 SMs, the most; small graphs take a 
 inline uint32_t bbox_blocks(uint32_t n) { return std::min<uint32_t>(BBOX_BLOCKS, std::max(1u, (n + 1023u) / 1024u)); }
 constexpr uint32_t DEFAULT_HUB_THRESHOLD = 2048;
 // Lists at least this long (and below the hub threshold) are gathered by a
-// whole warp, 32 neighbours at a time, and summed in list order by lane 0: a
+// whole warp, 32 neighbours at a time, and summed in list order by every lane: a
 // thread alone would wait on hundreds of dependent gather rounds.
 // Where the graph does not fill the GPU the warps are free and a thread's list
 // only adds latency, so smaller graphs hand over shorter lists. B200, us a pass

@@ -256,8 +256,8 @@ struct Fa2Settings {
   // global subtrees diverge, so every iteration issues both load paths).
   bool walk_stage_top = false;
   // Replay each step from a captured CUDA graph (default). false launches the
-  // same kernels one by one (for profilers that cannot see into graphs with
-  // conditional nodes); results are identical.
+  // same kernels one by one, none chained (for profilers, which see a graph's
+  // kernels only partly); results are identical.
   bool use_graph = true;
   // Tolerance mode of the Barnes-Hut walk (off by default): each repulsion
   // term srd*m/r2 uses the approximate reciprocal and the sums fuse into
