@@ -3538,20 +3538,16 @@ class Fa2Engine : public Engine {
   }
 
   int capture_step(cudaGraphExec_t* out, bool phases) {
-    cudaGraph_t g;
-    JC_CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     int L = 0;
     capture_phases_ = phases;
+    cudaGraph_t g = nullptr;
     try {
-      L = enqueue_step();
+      g = record_graph(stream_, [&] { L = enqueue_step(); });
     } catch (...) {
       capture_phases_ = false;
-      cudaStreamEndCapture(stream_, &g);
-      if (g) cudaGraphDestroy(g);
       throw;
     }
     capture_phases_ = false;
-    JC_CUDA_CHECK(cudaStreamEndCapture(stream_, &g));
     cudaError_t e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) fail(JC_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));

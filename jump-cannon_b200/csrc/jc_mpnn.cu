@@ -60,6 +60,7 @@
 #include <vector>
 
 #include "jc_common.h"
+#include "jc_pool.h"
 #include "jc_engine.h"
 #include "jc_params.h"
 #include "jc_exact.cuh"
@@ -2875,7 +2876,7 @@ extern "C" jc_status jc_tc_gemm_bf16(int32_t M, int32_t N, int32_t K, const uint
       cudaFree(dErr);
       throw;
     }
-    JC_CUDA_CHECK(cudaDeviceSynchronize());
+    JC_CUDA_CHECK(drain_device());
     std::vector<float> parts(nc);
     uint32_t err = 0;
     JC_CUDA_CHECK(cudaMemcpy(parts.data(), dC, nc * 4, cudaMemcpyDeviceToHost));

@@ -25,6 +25,40 @@
 
 namespace jc {
 
+// A stream capture and a wait for the whole device exclude one another: the wait
+// (another thread's engine freeing a block) would fail and break the capture, and the
+// block would go on to the next engine without it. Held for the recording alone (host
+// work, tens of microseconds), not for the instantiation.
+inline std::mutex& capture_mutex() {
+  static std::mutex* m = new std::mutex();
+  return *m;
+}
+
+// Waits for all work on the current device, outside every engine's capture.
+inline cudaError_t drain_device() {
+  std::lock_guard<std::mutex> lock(capture_mutex());
+  return cudaDeviceSynchronize();
+}
+
+// Records what enqueue() launches on the stream, in thread-local mode; the caller owns
+// the graph. A throw of enqueue() ends the capture and passes on.
+template <class F>
+cudaGraph_t record_graph(cudaStream_t stream, F&& enqueue) {
+  cudaGraph_t g = nullptr;
+  std::lock_guard<std::mutex> lock(capture_mutex());
+  JC_CUDA_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+  try {
+    enqueue();
+  } catch (...) {
+    cudaStreamEndCapture(stream, &g);
+    if (g) cudaGraphDestroy(g);
+    (void)cudaGetLastError();
+    throw;
+  }
+  JC_CUDA_CHECK(cudaStreamEndCapture(stream, &g));
+  return g;
+}
+
 class DevicePool {
  public:
   static DevicePool& instance() {
@@ -64,8 +98,10 @@ class DevicePool {
   }
 
   // Back to the cache once the device has finished with it (the
-  // synchronisation cudaFree would have made). No exception leaves this call
-  // (it runs in destructors).
+  // synchronisation cudaFree would have made). Where that wait is refused (a
+  // capture of the caller's own on another thread), the block goes to cudaFree
+  // instead of to the next engine. No exception leaves this call (it runs in
+  // destructors).
   void free(void* p) {
     if (!p) return;
     Block b{};
@@ -80,9 +116,11 @@ class DevicePool {
     int cur = 0;
     const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != b.device;
     if (other) cudaSetDevice(b.device);
-    cudaDeviceSynchronize();
+    const bool idle = drain_device() == cudaSuccess;
+    if (!idle) cudaFree(p);
     if (other) cudaSetDevice(cur);
     (void)cudaGetLastError();
+    if (!idle) return;
     std::lock_guard<std::mutex> lock(mu_);
     free_.push_back(b);
   }

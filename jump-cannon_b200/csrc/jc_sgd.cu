@@ -1006,17 +1006,9 @@ class SgdEngine : public Engine {
 
   void ensure_graph() {
     if (gexec_) return;
-    cudaGraph_t g;
-    JC_CUDA_CHECK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     int L = 0;
-    try {
-      L = wide_ ? enqueue_sweeps<uint32_t>(dist32_.p) : enqueue_sweeps<uint16_t>(dist16_.p);
-    } catch (...) {
-      cudaStreamEndCapture(stream_, &g);
-      if (g) cudaGraphDestroy(g);
-      throw;
-    }
-    JC_CUDA_CHECK(cudaStreamEndCapture(stream_, &g));
+    cudaGraph_t g = record_graph(
+        stream_, [&] { L = wide_ ? enqueue_sweeps<uint32_t>(dist32_.p) : enqueue_sweeps<uint16_t>(dist16_.p); });
     cudaError_t e = cudaGraphInstantiate(&gexec_, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) fail(JC_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));

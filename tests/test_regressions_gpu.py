@@ -321,3 +321,31 @@ def test_tree_waits_give_up_and_the_context_survives(jc, orc):
     ref = orc.Fa2(g, x, bh=True, theta=0.8)
     ref.step()
     assert np.array_equal(bits(e.forces()[0]), bits(ref.get()["force"]))
+
+
+# An engine that gives its blocks back waits for the whole device, which must not fall
+# into the recording of another thread's step: it broke that recording (and the wait).
+@pytest.mark.parametrize("kind", ["fa2-bh", "sgd-stress-gpu", "batch"])
+def test_engines_come_and_go_on_two_threads(jc, kind):
+    graphs = [jc.gen_scale_free(n, 2, n) for n in (20, 300)]
+    xyz = [jc.seed_uniform(g.n_nodes, 2, 1) * np.float32(50) for g in graphs]
+
+    def layout(k):
+        if kind == "batch":
+            e = jc.LayoutEngine("fa2-bh")
+            e.init_batch(graphs[: 1 + k], xyz[: 1 + k])
+        else:
+            e = jc.LayoutEngine(kind)
+            e.init(graphs[k], xyz[k])
+        e.step()
+        out = bits(e.step()).copy()
+        e.close()
+        return out
+
+    expected = [layout(0), layout(1)]
+
+    def work(k):
+        for _ in range(150):
+            assert np.array_equal(layout(k), expected[k])
+
+    assert _concurrently([lambda: work(0), lambda: work(1)]) == []
